@@ -115,6 +115,7 @@ struct Ctx {
     uint32_t last_paths_over = 0, last_pool_used = 0;
     DevBuf segs, seg_leaves, seg_order, seg_ctl, leaves, pool_path, pool_cnt, pool_idx;
     DevBuf tile_fills, tile_state, col_above, col_final, fills, path_fill, path_cls, bin_stage;
+    size_t stage_slots = 0;
     DevBuf row_first, row_paths, scene_row_first;
     DevBuf z, fb_count, list, image, status, scan_temp;
     DevBuf canon_state, canon_clip;  // clipped frames: tile states after the clip rules (read-back only)
@@ -904,6 +905,7 @@ Batch make_batch(Ctx *c) {
     b.fills = c->fills.as<uint2>();
     b.fill_cap = (uint32_t)std::min<size_t>(c->fills.cap / 8, 0xffffffffu);
     b.stage = c->bin_stage.as<uint2>();
+    b.stage_tile = c->bin_stage.as<uint32_t>() + 2 * c->stage_slots;
     b.row_first = c->row_first.as<uint32_t>();
     b.row_paths = c->row_paths.as<uint4>();
     b.row_cap = (uint32_t)std::min<size_t>(c->row_paths.cap / 16, 0xffffffffu);
@@ -995,9 +997,8 @@ int begin_frame(Ctx *c, uint32_t first, uint32_t count) {
     PF_CUDA(c->row_first.ensure((size_t(c->r_rows) + 1) * 4));
     PF_CUDA(c->bin_list.ensure(size_t(N) * 20 + 16));
     PF_CUDA(c->path_fill.ensure(size_t(N) * 4 + 16));
-    size_t stage_bytes = 0;
-    PF_CUDA(bin_stage_bytes(c->tune, &stage_bytes));
-    PF_CUDA(c->bin_stage.ensure(stage_bytes));
+    PF_CUDA(bin_stage_slots(c->tune, &c->stage_slots));
+    PF_CUDA(c->bin_stage.ensure(c->stage_slots * 12));
     PF_CUDA(c->path_cls.ensure(size_t(N) + 16));
     PF_CUDA(c->bin_ctl.ensure(1024));
     PF_CUDA(c->path_leaf_range.ensure(size_t(N) * 8 + 16));

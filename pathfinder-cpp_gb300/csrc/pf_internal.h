@@ -150,7 +150,8 @@ struct Batch {
     int32_t *col_final;                  // [cols]
     uint2 *fills;                        // [fills] packed u16 x4
     uint32_t fill_cap;
-    uint2 *stage;                        // per binning CTA: fills staged during its count walk
+    uint2 *stage;                        // per binning CTA: tile visits staged during its count walk,
+    uint32_t *stage_tile;                // their points and their tiles with the fills kept
 
     // per framebuffer-tile row of each scene: the paths whose tile rect spans the row,
     // in path order
@@ -332,8 +333,8 @@ cudaError_t launch_bin_paths(const Batch &b, const Tuning &t, const BinStreams *
 // The most CTAs of each binning class one SM holds.
 cudaError_t bin_class_max_ctas(int out[3]);
 cudaError_t launch_pool_lists(const Batch &b, bool scatter, cudaStream_t st);
-// Bytes of the binning CTAs' fill stage on the current device for these launch parameters.
-cudaError_t bin_stage_bytes(const Tuning &t, size_t *bytes);
+// Slots of the binning CTAs' stage on the current device for these launch parameters.
+cudaError_t bin_stage_slots(const Tuning &t, size_t *slots);
 cudaError_t launch_mlp_predict(const __nv_bfloat16 *w, const float *feat, uint32_t n, float *out, cudaStream_t st);
 cudaError_t launch_mlp_grad(const __nv_bfloat16 *w, const float *feat, const float *target, const uint32_t *index,
                             uint32_t n, float *grad, float *loss, cudaStream_t st);

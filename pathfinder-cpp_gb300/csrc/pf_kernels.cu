@@ -784,6 +784,187 @@ __device__ void walk_line_warp(const WalkCtx &w, float4 f, OnFill &&on_fill, OnD
     }
 }
 
+// The same walk for 32 lines at once, one per lane, with the lanes in step: the walk the binning
+// kernels spend their time in.  It is bound by instructions, so it does the reference's float
+// operations in the form that takes fewest:
+//
+// * Coordinates are kept in tiles (x / 16), which changes no rounding: scaling by a power of two
+//   is exact, so boundaries, parameters and positions are the same values over 16.  (It is not
+//   exact below 2^-122; a line with such a coordinate takes walk_line.)
+// * add_fill's quantisation of a coordinate v (times 256, rounded half to even, clamped to
+//   [0, 4095]) is a subtract of the tile and one fused multiply-add to 1.5 * 2^23, whose low
+//   mantissa bits are then the rounded integer (the product is exact, so the addition rounds
+//   once, as rint does), and one clamp of both coordinates as packed 16-bit integers.
+// * A crossing point is quantised once, in the tile it leaves; the tile it enters differs by one
+//   in the crossed coordinate, which is 4096 in quantised units.  (Both subtractions of the tile
+//   are exact, or - around the axes, where a coordinate has finer bits than the difference - the
+//   point is so close to the boundary that both forms give 0 and 4095.)
+// * The extra fill of a vertical crossing runs between the crossing point and the tile's corner,
+//   which quantises to (0, 0): it reuses the quantised crossing point.
+// * A tile visit's fills and backdrop delta are added to the tile's counter with one atomic.
+// * One reciprocal per direction gives the boundary spacing: |1 / vx| is |16 / vx| over 16.
+// * A line takes one step per tile boundary between its end points' tiles, so the loop is counted.
+//   A walk that rounding sends past one of those boundaries never comes to the end tile (steps
+//   only go on from it): it reports the walk error after its last step instead of at the step bound.
+// With the tile visits staged as they are walked (12 bytes for up to two fills, their slots from a
+// ballot instead of a counter in shared memory) binning takes, against one walk_line per lane:
+// 10.00 -> 7.86 ms on 256 scenes (162M lines, 485M fills), 1.05 -> 0.81 ms on 20,000 paths.  A round
+// of 32 steps is about 90 instructions, the set-up of 32 lines about 150.
+constexpr float kMagic = 12582912.0f;  // 1.5 * 2^23
+constexpr uint32_t kFillMax = 0x0fff0fffu;
+constexpr int32_t kMaxLaneSpan = 255;  // tiles; longer lines are always walked by the whole warp
+
+// a tile-unit point in tile (tx, ty), rounded to 1/256 px but not clamped: x | y << 16, signed
+__device__ __forceinline__ uint32_t round_point(float x, float y, float tx, float ty) {
+    const float qx = __fmaf_rn(fsub(x, tx), 4096.0f, kMagic), qy = __fmaf_rn(fsub(y, ty), 4096.0f, kMagic);
+    return __byte_perm(__float_as_uint(qx), __float_as_uint(qy), 0x5410);
+}
+
+// One line of a lane.
+struct LaneLine {
+    float x0, y0, vx, vy, tmx, tmy, tdx, tdy, ftx, fty, fex;
+    uint32_t pa;     // the tile's first point, quantised
+    int32_t lx, ly;  // the first tile, in the path's rect
+    int32_t steps;   // tile boundaries to cross; -1: no line
+    bool right, down;
+};
+
+// The steps of up to 32 lines.  visit(live, m, e, pa, pb, down, local, inc) is called by all lanes
+// once per step: live, the lane's line is still being walked; m, the tile's fill (pa, pb) is kept;
+// e, the vertical crossing's extra fill - (0, pa) going down, (pb, 0) going up - is kept; inc, the
+// number of both plus the backdrop delta << 24.  The values are meaningless unless live.
+// kChecked: tiles may lie outside the path's rect, and on_above(column, delta) gets the deltas above it.
+template <bool kChecked, class Visit, class OnAbove>
+__device__ __forceinline__ void lane_steps(const WalkCtx &w, const LaneLine &s, int32_t steps, Visit &&visit,
+                                           OnAbove &&on_above, uint32_t *status) {
+    float tmx = s.tmx, tmy = s.tmy, ftx = s.ftx, fty = s.fty;
+    int32_t lx = s.lx, ly = s.ly;
+    uint32_t local = (uint32_t)(s.ly * w.rw + s.lx);
+    uint32_t pa = s.pa;
+    uint32_t last = 0;  // the boundary the tile was entered through: 0 none, 1 vertical, 2 horizontal
+    const int32_t sx = s.right ? 1 : -1, sy = s.down ? 1 : -1, srow = s.down ? w.rw : -w.rw;
+    const float sxf = s.right ? 1.0f : -1.0f, syf = s.down ? 1.0f : -1.0f;
+    const uint32_t shx = s.right ? 0xf000u : 0x1000u, shy = s.down ? 0xf0000000u : 0x10000000u;
+    const uint32_t dval = s.right ? 0xff000000u : 0x01000000u, top = (uint32_t)(w.rw * w.rh) - 1u;
+    const int32_t rounds = __reduce_max_sync(0xffffffffu, steps);
+    bool lost = false;
+#pragma unroll 1
+    for (int32_t it = 0; it <= rounds; it++) {
+        const bool live = it <= steps, done = it == steps;
+        const bool stepx = tmx < tmy || (s.right && tmx <= tmy);
+        const uint32_t next = done ? 0u : stepx ? 1u : 2u;
+        const float nt = fminf(fminf(tmx, tmy), 1.0f);
+        const uint32_t pu = round_point(fadd(s.x0, fmul(s.vx, nt)), fadd(s.y0, fmul(s.vy, nt)), ftx, fty);
+        const uint32_t pb = __vimin_s16x2_relu(pu, kFillMax);
+        bool m = ((pa ^ pb) & 0xffffu) != 0;
+        bool e = (s.down ? last : next) == 2u && ((s.down ? pa : pb) & 0xffffu) != 0;
+        const bool cross = (s.right ? next : last) == 1u;
+        uint32_t d = cross ? dval : 0u;
+        if (kChecked) {
+            const bool col = (uint32_t)lx < (uint32_t)w.rw, in = col && (uint32_t)ly < (uint32_t)w.rh;
+            if (live && col && ly < 0 && cross) on_above(lx, s.right ? -1 : 1);
+            m = m && in;
+            e = e && in;
+            d = in ? d : 0u;
+            local = (uint32_t)(ly * w.rw + lx);
+        } else {
+            local = min(local, top);  // a lost line's tiles stay inside the counters
+        }
+        visit(live, m, e, pa, pb, s.down, local, (uint32_t)m + (uint32_t)e + d);
+        lost = lost || (done && ftx != s.fex);
+        pa = __viaddmin_s16x2_relu(pu, stepx ? shx : shy, kFillMax);
+        tmx = fadd(tmx, stepx ? s.tdx : 0.0f);
+        tmy = fadd(tmy, stepx ? 0.0f : s.tdy);
+        ftx += stepx ? sxf : 0.0f;
+        fty += stepx ? 0.0f : syf;
+        if (kChecked) {
+            lx += stepx ? sx : 0;
+            ly += stepx ? 0 : sy;
+        } else {
+            local += (uint32_t)(stepx ? sx : srow);
+        }
+        last = next;
+    }
+    if (lost) atomicOr(status, kErrWalk);
+}
+
+// Walks 32 lines (have: this lane has one).  Lines spanning more than long_line tiles are walked by
+// the whole warp, and the few outside the fast form's range (coordinates beyond 2^20, or tiny) by
+// their lane alone, both with on_fill / on_delta after begin_single() and before end_single().
+template <class Visit, class OnAbove, class OnFill, class OnDelta, class Begin, class End>
+__device__ __forceinline__ void walk_lines(const WalkCtx &w, float4 f, bool have, float long_line, Visit &&visit,
+                                           OnAbove &&on_above, OnFill &&on_fill, OnDelta &&on_delta,
+                                           Begin &&begin_single, End &&end_single, uint32_t *status) {
+    const float inv = 1.0f / kTile, low = -1048576.0f;
+    LaneLine s;
+    s.x0 = s.y0 = s.vx = s.vy = s.ftx = s.fty = 0.0f;
+    s.tmx = s.tmy = s.tdx = s.tdy = INFINITY;
+    s.fex = 0.0f;
+    s.pa = 0;
+    s.lx = s.ly = 0;
+    s.steps = -1;
+    s.right = s.down = true;
+    bool alone = false, along = false, safe = true;
+    if (have) {
+        float ax = f.x, ay = f.y, bx = f.z, by = f.w;
+        const bool inside = ax >= w.vb_left && ax <= w.vb_right && ay <= w.vb_bottom && bx >= w.vb_left &&
+                            bx <= w.vb_right && by <= w.vb_bottom;
+        bool keep = true;
+        if (!inside) {
+            keep = isfinite(ax) && isfinite(ay) && isfinite(bx) && isfinite(by);
+            if (keep) keep = clip_line(w, ax, ay, bx, by, status);
+        }
+        if (keep) {
+            alone = !(ay >= low && by >= low);
+            s.x0 = fmul(ax, inv);
+            s.y0 = fmul(ay, inv);
+            const float x1 = fmul(bx, inv), y1 = fmul(by, inv);
+            s.vx = fsub(x1, s.x0);
+            s.vy = fsub(y1, s.y0);
+            s.ftx = floorf(s.x0);
+            s.fty = floorf(s.y0);
+            const int32_t lx = (int32_t)s.ftx - w.rx0, ly = (int32_t)s.fty - w.ry0;
+            s.fex = floorf(x1);
+            const int32_t ex = (int32_t)s.fex - w.rx0, ey = (int32_t)floorf(y1) - w.ry0;
+            s.lx = lx;
+            s.ly = ly;
+            s.right = s.vx >= 0.0f;
+            s.down = s.vy >= 0.0f;
+            s.pa = __vimin_s16x2_relu(round_point(s.x0, s.y0, s.ftx, s.fty), kFillMax);
+            safe = max((uint32_t)lx, (uint32_t)ex) < (uint32_t)w.rw && max((uint32_t)ly, (uint32_t)ey) < (uint32_t)w.rh;
+            const int32_t nx = abs(ex - lx), ny = abs(ey - ly);
+            s.steps = nx + ny;
+            // a line inside one tile goes to its end at once (t = 1)
+            if (s.steps != 0 && !alone) {
+                // 2 |bits| - 1 is below 2^-122's for tiny values only (zero wraps to the largest)
+                const uint32_t tiny = min(min(2u * __float_as_uint(ax) - 1u, 2u * __float_as_uint(ay) - 1u),
+                                          min(2u * __float_as_uint(bx) - 1u, 2u * __float_as_uint(by) - 1u));
+                alone = tiny < 2u * 0x02800000u - 1u;
+                along = !alone && ((float)(s.steps + 1) > long_line || s.steps > kMaxLaneSpan);
+                s.tmx = fdiv(fsub(s.right ? s.ftx + 1.0f : s.ftx, s.x0), s.vx);
+                s.tmy = fdiv(fsub(s.down ? s.fty + 1.0f : s.fty, s.y0), s.vy);
+                s.tdx = fabsf(__frcp_rn(s.vx));
+                s.tdy = fabsf(__frcp_rn(s.vy));
+            }
+            if (alone || along) s.steps = -1;
+        }
+    }
+    lane_steps<false>(w, s, safe ? s.steps : -1, visit, on_above, status);
+    if (!__all_sync(0xffffffffu, safe)) lane_steps<true>(w, s, safe ? -1 : s.steps, visit, on_above, status);
+    unsigned k = __ballot_sync(0xffffffffu, along);
+    if (__any_sync(0xffffffffu, alone || along)) {
+        begin_single();
+        if (alone) walk_line(w, f.x, f.y, f.z, f.w, on_fill, on_delta, status);
+        for (; k; k &= k - 1) {
+            const int l = __ffs(k) - 1;
+            const float4 g = make_float4(__shfl_sync(0xffffffffu, f.x, l), __shfl_sync(0xffffffffu, f.y, l),
+                                         __shfl_sync(0xffffffffu, f.z, l), __shfl_sync(0xffffffffu, f.w, l));
+            walk_line_warp(w, g, on_fill, on_delta, status);
+        }
+        end_single();
+    }
+}
+
 // Flattening shared by the lanes of a warp, for both frames:
 // * learned frame (kExact false): each path's leaf lines go to the path's region, laid out from
 //   the sizer's budget; lines past the budget spill into the shared pool, and an exhausted pool
@@ -1241,9 +1422,9 @@ __host__ __device__ constexpr int class_threads(int c) { return c == 2 ? 384 : c
 // class 0 at 20 (48 registers) and class 1 at 8 (64 registers, no spills) beat 24 and 12 at 40
 // registers with 148-208 B of spills (binning 20.00 -> 19.30 ms per 512-scene frame)
 __host__ __device__ constexpr int class_min_ctas(int c) { return c == 2 ? 3 : c == 1 ? 8 : 20; }
-// Fills a CTA stages during its count walk (8 bytes each, in its own slice of a global buffer
-// that stays in L2): the fills are then placed without walking the lines again.  A path with
-// more fills than this walks its lines twice.
+// Tile visits with fills a CTA stages during its count walk (12 bytes each, in its own slice of a
+// global buffer that stays in L2, an equal part for each of its warps): the fills are then placed
+// without walking the lines again.  A path with more than this walks its lines twice.
 __host__ __device__ constexpr uint32_t class_stage(int c) { return c == 0 ? 3072u : c == 1 ? 6144u : 12288u; }
 // One line gives a tile at most two fills (the walk visits a tile once, with at most one
 // extra fill for a vertical crossing), so with at most 2^22 lines per CTA-binned path the
@@ -1405,37 +1586,27 @@ __global__ void k_bin_scatter(Batch b) {
     b.bin_list[(size_t)(key >> 5) * b.n_paths + base + __popc(g & ((1u << lane) - 1u))] = p;
 }
 
-// Tiles a line's walk visits at most (its end points' tile distance, before clipping, plus one):
-// lines above Batch::long_line (8 unless tuned) are walked by a whole warp.
-__device__ __forceinline__ float line_span(const float4 &f) {
-    return fabsf(floorf(f.z * 0.0625f) - floorf(f.x * 0.0625f)) + fabsf(floorf(f.w * 0.0625f) - floorf(f.y * 0.0625f)) +
-           1.0f;
-}
-
-// A staged fill: the four 12-bit coordinates of the packed u16 fill and the tile (< 2^16).
-__device__ __forceinline__ uint2 stage_pack(uint2 q, uint32_t local) {
-    const uint32_t x0 = q.x & 0xfffu, y0 = q.x >> 16, x1 = q.y & 0xfffu, y1 = q.y >> 16;
-    return make_uint2(x0 | y0 << 12 | (x1 & 0xffu) << 24, x1 >> 8 | y1 << 4 | local << 16);
-}
-__device__ __forceinline__ uint2 stage_fill(uint2 v) {
-    const uint32_t x0 = v.x & 0xfffu, y0 = (v.x >> 12) & 0xfffu, x1 = v.x >> 24 | (v.y & 0xfu) << 8,
-                   y1 = (v.y >> 4) & 0xfffu;
-    return make_uint2(x0 | y0 << 16, x1 | y1 << 16);
-}
+// The fills of one tile visit, as a binning warp stages them: the visit's points and a word with
+// the tile (below 2^16) and which fills are kept - the tile's fill, the vertical crossing's extra
+// one, and whether that runs from the tile's corner (going down) or to it.
+constexpr uint32_t kVisitFill = 1u << 16, kVisitExtra = 1u << 17, kVisitDown = 1u << 18;
 
 template <int kCls>
 __global__ void __launch_bounds__(class_threads(kCls), class_min_ctas(kCls)) k_bin_fused(Batch b) {
     constexpr int kThr = class_threads(kCls), kWarps = kThr / 32;
-    constexpr uint32_t kStage = class_stage(kCls);
+    constexpr uint32_t kStage = class_stage(kCls) / kWarps;  // fills a warp stages
     static_assert(class_words(kCls) <= 65536u, "a staged fill holds its tile in 16 bits");
     extern __shared__ uint32_t sm[];
-    __shared__ uint32_t s_item, s_base, s_write, s_next, s_nstage;
-    uint2 *const stage = b.stage ? b.stage + (size_t)blockIdx.x * kStage : nullptr;
+    __shared__ uint32_t s_item, s_base, s_write, s_next, s_over;
+    __shared__ uint32_t s_slot[kWarps];
     __shared__ int32_t s_seg[kThr];
     __shared__ uint32_t s_warp[kWarps];
     __shared__ unsigned long long s_wsum[kWarps];
     const uint32_t tid = threadIdx.x;
     const int lane = (int)(tid & 31), warp = (int)(tid >> 5);
+    const unsigned below = (1u << lane) - 1u;
+    uint2 *const stage = b.stage + ((size_t)blockIdx.x * kWarps + warp) * kStage;
+    uint32_t *const stage_tile = b.stage_tile + ((size_t)blockIdx.x * kWarps + warp) * kStage;
     const uint32_t *list = b.bin_list + (size_t)kCls * b.n_paths;
     const uint32_t n_items = b.bin_ctl[kCtlCount + kCls];
     uint32_t *const err = &b.status[kStErr];
@@ -1454,7 +1625,7 @@ __global__ void __launch_bounds__(class_threads(kCls), class_min_ctas(kCls)) k_b
         for (uint32_t t = tid; t < T + rw; t += kThr) sm[t] = 0;
         if (tid == 0) {
             s_next = 0;
-            s_nstage = 0;
+            s_over = 0;
         }
         __syncthreads();
 
@@ -1463,14 +1634,40 @@ __global__ void __launch_bounds__(class_threads(kCls), class_min_ctas(kCls)) k_b
         //    A line of many tiles (a contour's closing line spans the canvas) would hold its
         //    warp, and at the barrier its CTA, for tens of steps: such lines are walked by the
         //    whole warp after its short lines.
+        uint32_t nstage = 0;  // visits this warp staged (the same in every lane)
         auto on_fill = [&](int32_t local, uint2 q) {
             atomicAdd(&cnt[local], 1u);
-            const uint32_t slot = atomicAdd(&s_nstage, 1u);
-            if (stage && slot < kStage) stage[slot] = stage_pack(q, (uint32_t)local);
+            const uint32_t slot = atomicAdd(&s_slot[warp], 1u);
+            if (slot < kStage) {
+                stage[slot] = q;
+                stage_tile[slot] = (uint32_t)local | kVisitFill;
+            }
         };
         auto on_delta = [&](int32_t where, int d) {
             if (where >= 0) atomicAdd(&cnt[where], (uint32_t)d << 24);
             else atomicAdd(&above[-1 - where], d);
+        };
+        auto on_above = [&](int32_t x, int d) { atomicAdd(&above[x], d); };
+        auto begin_single = [&]() {
+            if (lane == 0) s_slot[warp] = nstage;
+            __syncwarp();
+        };
+        auto end_single = [&]() {
+            __syncwarp();
+            nstage = s_slot[warp];
+        };
+        // a step of the warp's lines: one atomic per lane for its tile, one stage slot per lane
+        // with a fill
+        auto visit = [&](bool live, bool m, bool e, uint32_t pa, uint32_t pb, bool down, uint32_t local,
+                         uint32_t inc) {
+            const unsigned keep = __ballot_sync(0xffffffffu, live && (m || e));
+            if (live && inc) atomicAdd(&cnt[local], inc);
+            const uint32_t slot = nstage + __popc(keep & below);
+            if ((keep >> lane & 1u) && slot < kStage) {
+                stage[slot] = make_uint2(pa, pb);
+                stage_tile[slot] = local | (m ? kVisitFill : 0u) | (e ? kVisitExtra : 0u) | (down ? kVisitDown : 0u);
+            }
+            nstage += __popc(keep);
         };
         for (;;) {
             uint32_t k0 = 0;
@@ -1478,20 +1675,11 @@ __global__ void __launch_bounds__(class_threads(kCls), class_min_ctas(kCls)) k_b
             k0 = __shfl_sync(0xffffffffu, k0, 0);
             if (k0 >= L.n) break;
             const uint32_t k = k0 + (uint32_t)lane;
-            float4 f = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-            bool along = false;
-            if (k < L.n) {
-                f = b.leaves[L.index(b, k)];
-                along = line_span(f) > b.long_line;
-                if (!along) walk_line(w, f.x, f.y, f.z, f.w, on_fill, on_delta, err);
-            }
-            for (unsigned m = __ballot_sync(0xffffffffu, along); m; m &= m - 1) {
-                const int l = __ffs(m) - 1;
-                const float4 g = make_float4(__shfl_sync(0xffffffffu, f.x, l), __shfl_sync(0xffffffffu, f.y, l),
-                                             __shfl_sync(0xffffffffu, f.z, l), __shfl_sync(0xffffffffu, f.w, l));
-                walk_line_warp(w, g, on_fill, on_delta, err);
-            }
+            const bool have = k < L.n;
+            const float4 f = have ? b.leaves[L.index(b, k)] : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+            walk_lines(w, f, have, b.long_line, visit, on_above, on_fill, on_delta, begin_single, end_single, err);
         }
+        if (lane == 0 && nstage > kStage) s_over = 1;
         __syncthreads();
 
         // 2. the count of each warp's chunk of tiles; thread 0 reserves the path's block of
@@ -1592,19 +1780,28 @@ __global__ void __launch_bounds__(class_threads(kCls), class_min_ctas(kCls)) k_b
         }
         __syncthreads();
 
-        // 5. the fills, grouped by tile: from the stage (four loads in flight per thread), or by
-        //    walking the lines again
-        const uint32_t nstage = s_nstage;
-        if (s_write && stage && nstage <= kStage) {
-            for (uint32_t k = tid; k < nstage; k += 4 * kThr) {
+        // 5. the fills, grouped by tile: each warp's from its stage (four loads in flight per
+        //    lane), or, when a warp's stage was too small, by walking the lines again
+        if (s_write && !s_over) {
+            auto place = [&](uint2 v, uint32_t t) {
+                const uint32_t m = t >> 16 & 1u, e = t >> 17 & 1u;
+                const uint32_t at = atomicAdd(&cnt[t & 0xffffu], m + e);
+                if (m) b.fills[at] = v;
+                if (e) b.fills[at + m] = t & kVisitDown ? make_uint2(0u, v.x) : make_uint2(v.y, 0u);
+            };
+            uint32_t k = lane;
+            for (; k + 96 < nstage; k += 128) {
                 uint2 v[4];
+                uint32_t t[4];
 #pragma unroll
-                for (int j = 0; j < 4; j++)
-                    if (k + j * kThr < nstage) v[j] = stage[k + j * kThr];
+                for (int j = 0; j < 4; j++) {
+                    v[j] = stage[k + j * 32];
+                    t[j] = stage_tile[k + j * 32];
+                }
 #pragma unroll
-                for (int j = 0; j < 4; j++)
-                    if (k + j * kThr < nstage) b.fills[atomicAdd(&cnt[v[j].y >> 16], 1u)] = stage_fill(v[j]);
+                for (int j = 0; j < 4; j++) place(v[j], t[j]);
             }
+            for (; k < nstage; k += 32) place(stage[k], stage_tile[k]);
         } else if (s_write) {
             for (uint32_t k = tid; k < L.n; k += kThr) {
                 const float4 f = b.leaves[L.index(b, k)];
@@ -2580,7 +2777,7 @@ static cudaError_t launch_fused(const Batch &b, uint32_t per_sm, cudaStream_t st
     return cudaGetLastError();
 }
 
-cudaError_t bin_stage_bytes(const Tuning &t, size_t *bytes) {
+cudaError_t bin_stage_slots(const Tuning &t, size_t *slots) {
     unsigned g0 = 0, g1 = 0, g2 = 0;
     cudaError_t e;
     if ((e = fused_grid<0>(&g0, t.bin_ctas_per_sm[0])) != cudaSuccess) return e;
@@ -2588,7 +2785,7 @@ cudaError_t bin_stage_bytes(const Tuning &t, size_t *bytes) {
     if ((e = fused_grid<2>(&g2, t.bin_ctas_per_sm[2])) != cudaSuccess) return e;
     const size_t s0 = size_t(g0) * class_stage(0), s1 = size_t(g1) * class_stage(1), s2 = size_t(g2) * class_stage(2);
     // concurrent classes each keep their own slice of the stage
-    *bytes = 8 * (t.bin_concurrent ? s0 + s1 + s2 : std::max({s0, s1, s2}));
+    *slots = t.bin_concurrent ? s0 + s1 + s2 : std::max({s0, s1, s2});
     return cudaSuccess;
 }
 
@@ -2632,8 +2829,10 @@ cudaError_t launch_bin_paths(const Batch &b, const Tuning &t, const BinStreams *
     for (int k = 0; k < 2; k++)
         if ((e = cudaStreamWaitEvent(bs->side[k], bs->fork, 0)) != cudaSuccess) return e;
     Batch b1 = b, b0 = b;
-    b1.stage = b.stage ? b.stage + size_t(g2) * class_stage(2) : nullptr;
-    b0.stage = b.stage ? b1.stage + size_t(g1) * class_stage(1) : nullptr;
+    b1.stage = b.stage + size_t(g2) * class_stage(2);
+    b0.stage = b1.stage + size_t(g1) * class_stage(1);
+    b1.stage_tile = b.stage_tile + size_t(g2) * class_stage(2);
+    b0.stage_tile = b1.stage_tile + size_t(g1) * class_stage(1);
     if ((e = launch_fused<2>(b, t.bin_ctas_per_sm[2], st)) != cudaSuccess) return e;
     if ((e = launch_fused<1>(b1, t.bin_ctas_per_sm[1], bs->side[0])) != cudaSuccess) return e;
     if ((e = launch_fused<0>(b0, t.bin_ctas_per_sm[0], bs->side[1])) != cudaSuccess) return e;
