@@ -116,7 +116,7 @@ struct Ctx {
     DevBuf segs, seg_leaves, seg_order, seg_ctl, leaves, pool_path, pool_cnt, pool_idx;
     DevBuf tile_fills, tile_state, col_above, col_final, fills, path_fill, path_cls, bin_stage;
     size_t stage_slots = 0;
-    DevBuf row_first, row_paths, scene_row_first;
+    DevBuf row_first, row_mat, row_paths, scene_rblk_first;
     DevBuf z, fb_count, list, image, status, scan_temp;
     DevBuf canon_state, canon_clip;  // clipped frames: tile states after the clip rules (read-back only)
     // host image target (pf_set_host_image): frames composite straight into this host buffer
@@ -137,11 +137,13 @@ struct Ctx {
     // the scene range of the last frame and its totals
     uint32_t r_first = 0, r_count = 0, r_paths = 0, r_contours = 0, r_fb = 0, r_rows = 0;
     uint32_t r_path_base = 0, r_contour_base = 0, r_fb_base = 0, r_row_base = 0;
+    uint32_t r_rblks = 0, r_rblk_base = 0, r_rmat = 0, r_rmat_base = 0;
     uint32_t n_segs = 0, n_tiles = 0, n_cols = 0, n_leaves = 0, n_list = 0, n_row_entries = 0;
     uint64_t n_fills = 0;
     uint64_t fill_hint = 0;  // fills of the largest frame so far: the next frame's starting capacity
     bool lists_dumped = false;
-    std::vector<uint32_t> h_scene_row_first;
+    std::vector<uint32_t> h_scene_row_first, h_scene_rblk_first, h_scene_rmat_first;
+    uint32_t row_chunk = 0;  // paths a block of the row lists takes
     uint32_t syncs = 0;
 
     HostCanon canon;
@@ -683,6 +685,26 @@ int upload(Ctx *c, const pf_scene_view *scenes, uint32_t n) {
     c->n_fb = (uint32_t)fb;
     c->image_bytes = img;
 
+    // the row lists' blocks and count matrices: chunks of 256 paths, or more where canvases of
+    // many rows with very many paths would take a matrix of over 2^26 counts
+    c->h_scene_rblk_first.assign(n + 1, 0);
+    c->h_scene_rmat_first.assign(n + 1, 0);
+    for (uint64_t chunk = 256;; chunk *= 2) {
+        uint64_t blks = 0, mat = 0;
+        for (uint32_t i = 0; i < n; i++) {
+            SceneDev &S = c->h_scenes[i];
+            const uint64_t k = std::max<uint64_t>(1, (scenes[i].n_paths + chunk - 1) / chunk);
+            c->h_scene_rblk_first[i] = S.rblk_first = (uint32_t)blks;
+            c->h_scene_rmat_first[i] = S.rmat_first = (uint32_t)mat;
+            blks += k * ((S.fbh + kRowWindow - 1) / kRowWindow);
+            mat += k * S.fbh;
+        }
+        c->h_scene_rblk_first[n] = (uint32_t)blks;
+        c->h_scene_rmat_first[n] = (uint32_t)mat;
+        c->row_chunk = (uint32_t)chunk;
+        if (mat <= std::max<uint64_t>(1ull << 26, rows)) break;
+    }
+
     bool strokes = false;
     for (uint32_t i = 0; i < n && !strokes; i++)
         for (uint32_t p = 0; scenes[i].path_stroke && p < scenes[i].n_paths; p++)
@@ -705,7 +727,7 @@ int upload(Ctx *c, const pf_scene_view *scenes, uint32_t n) {
     PF_CUDA(c->scene_path_first.ensure((n + 1) * 4));
     PF_CUDA(c->scene_contour_first.ensure((n + 1) * 4));
     PF_CUDA(c->scene_fb_first.ensure((n + 1) * 4));
-    PF_CUDA(c->scene_row_first.ensure((n + 1) * 4));
+    PF_CUDA(c->scene_rblk_first.ensure((n + 1) * 4));
     {
         // a new image buffer starts transparent, so a first frame with PF_LOAD_LOAD loads zeros
         void *const before = c->image.p;
@@ -818,8 +840,8 @@ int upload(Ctx *c, const pf_scene_view *scenes, uint32_t n) {
                             c->stream));
     PF_CUDA(c->fb_scene.ensure(size_t(fb) * 4 + 16));
     PF_CUDA(launch_fb_scene(c->scene_fb_first.as<uint32_t>(), n, c->fb_scene.as<uint32_t>(), c->stream));
-    PF_CUDA(cudaMemcpyAsync(c->scene_row_first.p, c->h_scene_row_first.data(), (n + 1) * 4, cudaMemcpyHostToDevice,
-                            c->stream));
+    PF_CUDA(cudaMemcpyAsync(c->scene_rblk_first.p, c->h_scene_rblk_first.data(), (n + 1) * 4,
+                            cudaMemcpyHostToDevice, c->stream));
     if (strokes) {
         if (int e = stroke_upload(c, scenes, n, scf)) {
             cudaStreamSynchronize(c->stream);
@@ -854,7 +876,7 @@ Batch make_batch(Ctx *c) {
     b.scene_contour_first = c->scene_contour_first.as<uint32_t>();
     b.scene_fb_first = c->scene_fb_first.as<uint32_t>();
     b.fb_scene = c->fb_scene.as<uint32_t>();
-    b.scene_row_first = c->scene_row_first.as<uint32_t>();
+    b.scene_rblk_first = c->scene_rblk_first.as<uint32_t>();
     const bool clips = !c->h_path_clip.empty();
     b.path_clip_cat = clips ? c->path_clip.as<uint32_t>() : nullptr;
     b.path_is_clip_cat = clips ? c->path_is_clip.as<uint8_t>() : nullptr;
@@ -871,6 +893,11 @@ Batch make_batch(Ctx *c) {
     b.n_contours = c->r_contours;
     b.fb_base = c->r_fb_base;
     b.row_base = c->r_row_base;
+    b.row_mat = c->row_mat.as<uint32_t>();
+    b.row_chunk = c->row_chunk;
+    b.rblk_base = c->r_rblk_base;
+    b.n_rblks = c->r_rblks;
+    b.rmat_base = c->r_rmat_base;
     b.contour_point_first = c->contour_point_first.as<uint32_t>();
     b.contour_path = c->contour_path.as<uint32_t>();
     b.paths = c->paths.as<PathDev>();
@@ -970,6 +997,10 @@ void set_range(Ctx *c, uint32_t first, uint32_t count) {
     c->r_fb = c->h_scene_fb_first[first + count] - a.fb_first;
     c->r_row_base = a.row_first;
     c->r_rows = c->h_scene_row_first[first + count] - a.row_first;
+    c->r_rblk_base = a.rblk_first;
+    c->r_rblks = c->h_scene_rblk_first[first + count] - a.rblk_first;
+    c->r_rmat_base = a.rmat_first;
+    c->r_rmat = c->h_scene_rmat_first[first + count] - a.rmat_first;
 }
 
 int begin_frame(Ctx *c, uint32_t first, uint32_t count) {
@@ -995,6 +1026,7 @@ int begin_frame(Ctx *c, uint32_t first, uint32_t count) {
     PF_CUDA(c->path_contours.ensure(size_t(N) * 8 + 8));
     PF_CUDA(c->path_bounds.ensure(size_t(N) * 16 + 16));
     PF_CUDA(c->row_first.ensure((size_t(c->r_rows) + 1) * 4));
+    PF_CUDA(c->row_mat.ensure(size_t(c->r_rmat) * 4));
     PF_CUDA(c->bin_list.ensure(size_t(N) * 20 + 16));
     PF_CUDA(c->path_fill.ensure(size_t(N) * 4 + 16));
     PF_CUDA(bin_stage_slots(c->tune, &c->stage_slots));
@@ -1010,20 +1042,19 @@ int begin_frame(Ctx *c, uint32_t first, uint32_t count) {
 // frame, the sizer's per-path budgets), ending with the frame's first host synchronisation.
 int stage_setup(Ctx *c, bool learned) {
     cudaStream_t st = c->stream;
-    const uint32_t N = c->r_paths, C = c->r_contours, R = c->r_rows;
+    const uint32_t N = c->r_paths, C = c->r_contours;
     Batch b = make_batch(c);
     PF_CUDA(launch_normalize(b, c->path_contours.as<uint2>(), st));
     PF_CUDA(launch_path_setup(b, c->path_contours.as<uint2>(), st));
     PF_CUDA(cudaMemsetAsync(b.contour_segs + C, 0, 4, st));
     PF_CUDA(cudaMemsetAsync(b.path_tiles + N, 0, 4, st));
     PF_CUDA(cudaMemsetAsync(b.path_cols + N, 0, 4, st));
-    PF_CUDA(cudaMemsetAsync(b.row_first + R, 0, 4, st));
     PF_CUDA(launch_contour_segments(b, false, st));
     PF_CUDA(launch_rows(b, false, st));
     if (int e = scan(c, b.contour_segs, C + 1, kStSegs)) return e;
     if (int e = scan(c, b.path_tiles, N + 1, kStTiles)) return e;
     if (int e = scan(c, b.path_cols, N + 1, kStCols)) return e;
-    if (int e = scan(c, b.row_first, R + 1, kStRows)) return e;
+    if (int e = scan(c, b.row_mat, c->r_rmat, kStRows)) return e;
     PF_CUDA(launch_path_offsets(b, st));
     if (learned) {
         PF_CUDA(c->path_feat.ensure(size_t(N) * kSizerIn * 4 + 16));
@@ -1245,7 +1276,7 @@ int render_learned_frame(Ctx *c, uint32_t first, uint32_t count, pf_frame_stats 
 // The buffers a learned frame uses, by address (a reallocated one invalidates the graph).
 std::vector<void *> frame_buffers(const Ctx *c) {
     const DevBuf *bufs[] = {&c->status, &c->contour_point_first, &c->contour_path, &c->paths, &c->path_tiles,
-                            &c->path_cols, &c->path_contours, &c->path_bounds, &c->row_first, &c->bin_list,
+                            &c->path_cols, &c->path_contours, &c->path_bounds, &c->row_first, &c->row_mat, &c->bin_list,
                             &c->bin_ctl, &c->path_leaf_range, &c->path_fill, &c->path_cls, &c->bin_stage,
                             &c->path_feat, &c->contour_feat, &c->path_pred, &c->path_leaf_first, &c->path_leaf_budget,
                             &c->path_leaf_cursor, &c->path_fill_budget, &c->segs, &c->seg_leaves, &c->seg_order,
@@ -1858,8 +1889,8 @@ int pf_ctx_destroy(void *ctx) {
                       &c->contour_path, &c->paths, &c->path_tiles, &c->path_cols, &c->contour_segs,
                       &c->path_contours, &c->segs, &c->seg_leaves, &c->seg_order, &c->seg_ctl, &c->leaves, &c->pool_path, &c->pool_cnt,
                       &c->pool_idx, &c->tile_fills, &c->path_fill, &c->path_cls, &c->tile_state, &c->col_above,
-                      &c->col_final, &c->fills, &c->bin_stage, &c->row_first,
-                      &c->row_paths, &c->scene_row_first, &c->z, &c->fb_count, &c->list, &c->image,
+                      &c->col_final, &c->fills, &c->bin_stage, &c->row_first, &c->row_mat,
+                      &c->row_paths, &c->scene_rblk_first, &c->z, &c->fb_count, &c->list, &c->image,
                       &c->status, &c->scan_temp, &c->path_clip, &c->path_is_clip, &c->path_clip_rel,
                       &c->in_points, &c->in_pflags, &c->in_cstart, &c->in_pstart, &c->st_stroke, &c->st_closed,
                       &c->st_dashes, &c->st_scenes, &c->st_cfirst, &c->dash_pts, &c->dash_cnt, &c->dash_end,

@@ -16,6 +16,7 @@ constexpr int kCovShift = 20;
 constexpr int kMaxDepth = 32;              // flattening recursion bound (depth of the d3d9 bisection)
 constexpr uint32_t kMaxWalk = 1u << 20;    // tile-walk step bound per line
 constexpr uint32_t kNone = 0xffffffffu;       // also the scene format's "no clip path"
+constexpr int kRowWindow = 64;                 // framebuffer-tile rows a block of the row lists takes
 constexpr uint32_t kPathIsClip = 8u;           // PathDev::flags: a clip path (tiled, never drawn)
 
 // Learned sizer: per-path features -> 64 -> 64 -> (log1p leaf lines, log1p fills).
@@ -53,6 +54,7 @@ struct SceneDev {
     uint32_t cstart_base, pstart_base;  // offsets of the scene's offset arrays
     uint32_t row_first;                  // first framebuffer-tile row of this scene in the batch
     uint32_t load;                       // PF_LOAD_LOAD: composite over the image already there
+    uint32_t rblk_first, rmat_first;     // first block and first matrix entry of the scene's row lists
 };
 
 // Per draw path (device), written by the set-up kernel.
@@ -96,7 +98,7 @@ struct Batch {
     const uint32_t *scene_contour_first; // [n_scenes_all + 1]
     const uint32_t *scene_fb_first;      // [n_scenes_all + 1]
     const uint32_t *fb_scene;            // [framebuffer tiles of all scenes] the scene of each
-    const uint32_t *scene_row_first;     // [n_scenes_all + 1]
+    const uint32_t *scene_rblk_first;    // [n_scenes_all + 1]
     uint32_t n_scenes_all;               // scenes uploaded
     // the scenes rendered by this frame: a contiguous range of the uploaded ones.
     // Per-frame arrays are indexed from 0 = the range's first path / contour / framebuffer tile.
@@ -155,7 +157,10 @@ struct Batch {
 
     // per framebuffer-tile row of each scene: the paths whose tile rect spans the row,
     // in path order
-    uint32_t *row_first;                 // [rows + 1] counts -> scanned
+    uint32_t *row_first;                 // [rows + 1] first entry of each row
+    uint32_t *row_mat;                   // [scene][row][chunk of paths] counts -> scanned
+    uint32_t row_chunk;                  // paths of a chunk
+    uint32_t rblk_base, n_rblks, rmat_base;  // blocks of the row kernels, and the first matrix entry
     uint4 *row_paths;                    // {path, rx0 | rx1 << 16, tile of (0, row) in the path's rect
                                          //  numbering, path flags}
     uint32_t row_cap;

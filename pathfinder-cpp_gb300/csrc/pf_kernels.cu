@@ -1985,71 +1985,107 @@ __global__ void k_pool_scatter(Batch b) {
 }
 
 // ---------------------------------------------------------------------------
-// Per framebuffer-tile row of each scene: the scene's paths whose tile rect spans the row,
-// in path order (one block per row; a block scan keeps the order, no sort is needed).
+// Per framebuffer-tile row of each scene: the scene's paths whose tile rect spans the row, in path
+// order.  A block takes kRowWindow rows of a scene and a chunk of its paths (row_chunk of them, 256
+// at a time, one per thread), counts the paths of each row into row_mat[scene][row][chunk], and,
+// once that is scanned, writes them from there: the matrix is in the order of the lists, so the
+// scan gives every chunk its place in every row and path order needs no sort.  A block's cost is its
+// paths plus its rows, wherever the paths lie.  (One block per row, testing every path of the
+// scene, took 0.83 ms of the 2.3 ms frame of 150,000 glyphs on 128 rows, and 0.12 ms of 2.0 ms with
+// 20,000 paths on 256 rows.)
 
-constexpr int kRowThreads = 256;
+constexpr int kRowThreads = 256, kRowWarps = kRowThreads / 32;
 // Row-entry flag of a clipped path; mask sources of a clipped tile.
 constexpr uint32_t kRowClipped = 16u;
 enum : uint32_t { kMaskOwn = 0, kMaskClip = 1, kMaskBoth = 2 };
 
 template <bool kWrite>
 __global__ void __launch_bounds__(kRowThreads) k_rows(Batch b) {
-    __shared__ uint32_t warp_counts[kRowThreads / 32];
-    __shared__ uint32_t chunk_total;
-    const uint32_t r = blockIdx.x;
-    const uint32_t rg = b.row_base + r;
-    const uint32_t s = upper_bound(b.scene_row_first, b.n_scenes_all + 1, rg) - 1;
+    __shared__ int s_cnt[kRowWarps][kRowWindow + 1];  // per warp: the rows' paths (as differences, then summed)
+    __shared__ uint32_t s_out[kRowWindow];            // the rows' next entries (kWrite), or counts so far
+    const uint32_t blk = b.rblk_base + blockIdx.x;
+    const uint32_t s = upper_bound(b.scene_rblk_first + b.scene_base, b.n_scenes + 1, blk) - 1 + b.scene_base;
     const SceneDev &S = b.scenes[s];
-    const int32_t y = (int32_t)(rg - S.row_first);
-    const uint32_t p0 = S.path_first - b.path_base, p1 = S.path_end - b.path_base;
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    uint32_t out = kWrite ? b.row_first[r] : 0u;
-    uint32_t total = 0;
+    const uint32_t paths = S.path_end - S.path_first, chunks = max(1u, (paths + b.row_chunk - 1) / b.row_chunk);
+    const uint32_t local = blk - S.rblk_first, chunk = local % chunks;
+    const int32_t y0 = (int32_t)(local / chunks * kRowWindow), rows = min((int32_t)S.fbh - y0, kRowWindow);
+    uint32_t *const mat = b.row_mat + (S.rmat_first - b.rmat_base) + (size_t)y0 * chunks + chunk;
+    const uint32_t p0 = S.path_first - b.path_base + chunk * b.row_chunk;
+    const uint32_t p1 = min(p0 + b.row_chunk, S.path_end - b.path_base);
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const unsigned below = (1u << lane) - 1u;
+    if (tid < rows) s_out[tid] = kWrite ? mat[(size_t)tid * chunks] : 0u;
+    if (kWrite && chunk == 0 && tid < rows) b.row_first[S.row_first - b.row_base + y0 + tid] = mat[(size_t)tid * chunks];
+    if (kWrite && blockIdx.x == 0 && tid == 0) b.row_first[b.n_rows] = b.status[kStRows];
     for (uint32_t base = p0; base < p1; base += kRowThreads) {
-        const uint32_t p = base + threadIdx.x;
-        bool spans = false;
-        int4 rect = make_int4(0, 0, 0, 0);
-        int32_t cx0 = 0, cx1 = 0;  // the rect's columns inside the framebuffer
+        for (int k = lane; k <= kRowWindow; k += 32) s_cnt[warp][k] = 0;
+        __syncwarp();
+        // the path's rows in this window, its columns inside the framebuffer
+        const uint32_t p = base + tid;
+        PathDev P{};
+        int32_t cx0 = 0, cx1 = 0, a = 0, e = 0;
         if (p < p1) {
-            rect = *reinterpret_cast<const int4 *>(&b.paths[p].rx0);
-            cx0 = max(rect.x, 0);
-            cx1 = min(rect.z, (int32_t)S.fbw);
-            spans = rect.y <= y && y < rect.w && cx0 < cx1 && !(b.paths[p].flags & kPathIsClip);
+            P = b.paths[p];
+            cx0 = max(P.rx0, 0);
+            cx1 = min(P.rx1, (int32_t)S.fbw);
+            if (cx0 < cx1 && !(P.flags & kPathIsClip)) {
+                a = max(P.ry0 - y0, 0);
+                e = min(P.ry1 - y0, rows);
+            }
         }
-        const uint32_t ballot = __ballot_sync(0xffffffffu, spans);
-        if (lane == 0) warp_counts[warp] = __popc(ballot);
+        const bool spans = a < e;
+        if (spans) {
+            atomicAdd(&s_cnt[warp][a], 1);
+            atomicAdd(&s_cnt[warp][e], -1);
+        }
+        __syncwarp();
+        // differences to counts: two rows a lane
+        {
+            const int u = s_cnt[warp][2 * lane], v = s_cnt[warp][2 * lane + 1];
+            int incl = u + v;
+#pragma unroll
+            for (int o = 1; o < 32; o <<= 1) {
+                const int n = __shfl_up_sync(0xffffffffu, incl, o);
+                if (lane >= o) incl += n;
+            }
+            s_cnt[warp][2 * lane] = incl - v;
+            s_cnt[warp][2 * lane + 1] = incl;
+        }
         __syncthreads();
-        if (threadIdx.x == 0) {
-            uint32_t run = 0;
-            for (int k = 0; k < kRowThreads / 32; k++) {
-                const uint32_t c = warp_counts[k];
-                warp_counts[k] = run;
+        // per row: the warps' first entries (kWrite), and the rows' totals
+        if (tid < rows) {
+            uint32_t run = s_out[tid];
+            for (int k = 0; k < kRowWarps; k++) {
+                const uint32_t c = (uint32_t)s_cnt[k][tid];
+                s_cnt[k][tid] = (int)run;
                 run += c;
             }
-            chunk_total = run;
+            s_out[tid] = run;
         }
         __syncthreads();
-        if (kWrite && spans) {
-            const uint32_t rank = warp_counts[warp] + __popc(ballot & ((1u << lane) - 1u));
-            // tile index of column 0 of this row in the path's numbering (may underflow by rx0;
+        if (kWrite) {
+            const int lo = __reduce_min_sync(0xffffffffu, spans ? a : kRowWindow);
+            const int hi = __reduce_max_sync(0xffffffffu, spans ? e : 0);
+            const bool clipped = spans && b.path_clip_cat && b.path_clip_rel[p] != kNone;
+            const uint32_t flags = P.flags | (clipped ? kRowClipped : 0u), rw = (uint32_t)(P.rx1 - P.rx0);
+            // tile index of column 0 of a row in the path's numbering (may underflow by rx0;
             // adding fx >= rx0 brings it back into range)
-            const uint32_t row_tile = b.paths[p].tile_first + (uint32_t)(y - rect.y) * (uint32_t)(rect.z - rect.x) -
-                                      (uint32_t)rect.x;
-            // flags: bit 0 even-odd, bit 1 occludes, bit 2 the rect's first tile (its first
-            // row, first column) is in this row of the framebuffer, bit 4 the path is clipped
-            const bool clipped = b.path_clip_cat && b.path_clip_rel[p] != kNone;
-            const bool first = y == rect.y && rect.x >= 0;
-            if (out + rank < b.row_cap)
-                b.row_paths[out + rank] = make_uint4(p, (uint32_t)cx0 | ((uint32_t)cx1 << 16), row_tile,
-                                                     b.paths[p].flags | (first ? 4u : 0u) |
-                                                         (clipped ? kRowClipped : 0u));
+            uint32_t row_tile = P.tile_first + (uint32_t)(y0 + lo - P.ry0) * rw - (uint32_t)P.rx0;
+            for (int r = lo; r < hi; r++, row_tile += rw) {
+                const bool in = spans && a <= r && r < e;
+                const unsigned m = __ballot_sync(0xffffffffu, in);
+                const uint32_t at = (uint32_t)s_cnt[warp][r] + __popc(m & below);
+                // flags: bit 0 even-odd, bit 1 occludes, bit 2 the rect's first tile (its first
+                // row, first column) is in this row of the framebuffer, bit 4 the path is clipped
+                const bool first = y0 + r == P.ry0 && P.rx0 >= 0;
+                if (in && at < b.row_cap)
+                    b.row_paths[at] = make_uint4(p, (uint32_t)cx0 | ((uint32_t)cx1 << 16), row_tile,
+                                                 flags | (first ? 4u : 0u));
+            }
+            __syncthreads();  // the counts are read before the next paths clear them
         }
-        out += chunk_total;
-        total += chunk_total;
-        __syncthreads();
     }
-    if (!kWrite && threadIdx.x == 0) b.row_first[r] = total;
+    if (!kWrite && tid < rows) mat[(size_t)tid * chunks] = s_out[tid];
 }
 
 // ---------------------------------------------------------------------------
@@ -2883,9 +2919,9 @@ cudaError_t launch_gather_words(uint32_t *dst, const WordSources &s, cudaStream_
 }
 
 cudaError_t launch_rows(const Batch &b, bool write, cudaStream_t st) {
-    if (!b.n_rows) return cudaSuccess;
-    if (write) PF_LAUNCH(k_rows<true><<<b.n_rows, kRowThreads, 0, st>>>(b));
-    else PF_LAUNCH(k_rows<false><<<b.n_rows, kRowThreads, 0, st>>>(b));
+    if (!b.n_rblks) return cudaSuccess;
+    if (write) PF_LAUNCH(k_rows<true><<<b.n_rblks, kRowThreads, 0, st>>>(b));
+    else PF_LAUNCH(k_rows<false><<<b.n_rblks, kRowThreads, 0, st>>>(b));
     return cudaGetLastError();
 }
 
