@@ -113,7 +113,7 @@ struct Ctx {
     bool sz_ready = false;
     float sz_mul = 1.25f, sz_add = 8.0f, sz_pool = 0.10f;
     uint32_t last_paths_over = 0, last_pool_used = 0;
-    DevBuf segs, seg_leaves, seg_order, seg_ctl, leaves, pool_path, pool_cnt, pool_idx;
+    DevBuf segs, path_seg_first, seg_leaves, leaves, pool_path, pool_cnt, pool_idx;
     DevBuf tile_fills, tile_state, col_above, col_final, fills, path_fill, path_cls, bin_stage;
     size_t stage_slots = 0;
     DevBuf row_first, row_mat, row_paths, scene_rblk_first;
@@ -915,9 +915,9 @@ Batch make_batch(Ctx *c) {
     b.path_cols = c->path_cols.as<uint32_t>();
     b.contour_segs = c->contour_segs.as<uint32_t>();
     b.segs = c->segs.as<SegDev>();
+    b.path_seg_first = c->path_seg_first.as<uint32_t>();
     b.seg_cap = (uint32_t)std::min<size_t>(c->segs.cap / sizeof(SegDev), 0xffffffffu);
     b.seg_leaves = c->seg_leaves.as<uint32_t>();
-    b.seg_order = c->seg_order.as<uint32_t>();
     b.leaves = c->leaves.as<float4>();
     b.leaf_cap = (uint32_t)std::min<size_t>(c->leaves.cap / 16, 0xffffffffu);
     b.pool_path = nullptr;  // set by a learned frame
@@ -946,7 +946,6 @@ Batch make_batch(Ctx *c) {
     b.counters = (c->flags & PF_CONFIG_FRAME_COUNTERS) ? 1u : 0u;
     b.long_line = c->tune.long_line;
     b.comp_ticket = c->tune.comp_ticket;
-    if (!c->tune.seg_sorted) b.seg_order = nullptr;
     return b;
 }
 
@@ -1029,6 +1028,7 @@ int begin_frame(Ctx *c, uint32_t first, uint32_t count) {
     PF_CUDA(c->row_mat.ensure(size_t(c->r_rmat) * 4));
     PF_CUDA(c->bin_list.ensure(size_t(N) * 20 + 16));
     PF_CUDA(c->path_fill.ensure(size_t(N) * 4 + 16));
+    PF_CUDA(c->path_seg_first.ensure(size_t(N) * 4 + 16));
     PF_CUDA(bin_stage_slots(c->tune, &c->stage_slots));
     PF_CUDA(c->bin_stage.ensure(c->stage_slots * 12));
     PF_CUDA(c->path_cls.ensure(size_t(N) + 16));
@@ -1085,8 +1085,6 @@ int stage_setup(Ctx *c, bool learned) {
     c->n_row_entries = c->h_status[kStRows];
     PF_CUDA(c->segs.ensure(size_t(c->n_segs) * sizeof(SegDev) + 16));
     PF_CUDA(c->seg_leaves.ensure((size_t(c->n_segs) + 1) * 4));
-    PF_CUDA(c->seg_order.ensure(size_t(c->n_segs) * 4 + 16));
-    PF_CUDA(c->seg_ctl.ensure(seg_ctl_bytes()));
     PF_CUDA(c->row_paths.ensure(size_t(c->n_row_entries) * 16 + 16));
     const size_t T = c->n_tiles, K = c->n_cols;
     PF_CUDA(c->tile_fills.ensure(T * 4 + 16));
@@ -1192,16 +1190,16 @@ int render_exact(Ctx *c, uint32_t first, uint32_t count, pf_frame_stats *stats) 
     Batch b = make_batch(c);
     PF_CUDA(launch_contour_segments(b, true, st));
     PF_CUDA(launch_rows(b, true, st));
-    if (c->tune.seg_sorted) PF_CUDA(launch_seg_order(b, c->n_segs, c->seg_ctl.as<uint32_t>(), st));
     PF_CUDA(cudaMemsetAsync(b.seg_leaves + c->n_segs, 0, 4, st));
-    PF_CUDA(launch_flatten(b, c->n_segs, false, st));
+    const bool shallow = uint64_t(c->h_status[kStSampledDeep]) * 64 < c->h_status[kStSampled];
+    PF_CUDA(launch_flatten(b, c->n_segs, false, shallow, st));
     if (int e = scan(c, b.seg_leaves, c->n_segs + 1, kStLeaves)) return e;
     if (int e = read_status(c)) return e;
     if (int e = check_kernel_status(c)) return e;
     c->n_leaves = c->h_status[kStLeaves];
     PF_CUDA(c->leaves.ensure(size_t(c->n_leaves) * 16 + 16));
     b = make_batch(c);
-    PF_CUDA(launch_flatten(b, c->n_segs, true, st, c->n_leaves));
+    PF_CUDA(launch_flatten(b, c->n_segs, true, shallow, st));
     record(c, 2);
 
     // 3. binning (one CTA per path: counts, backdrops, fill offsets, fills grouped by tile),
@@ -1245,7 +1243,6 @@ int render_learned_frame(Ctx *c, uint32_t first, uint32_t count, pf_frame_stats 
     b.pool_idx = c->pool_idx.as<uint32_t>();
     PF_CUDA(launch_contour_segments(b, true, st));
     PF_CUDA(launch_rows(b, true, st));
-    if (c->tune.seg_sorted) PF_CUDA(launch_seg_order(b, c->n_segs, c->seg_ctl.as<uint32_t>(), st));
     PF_CUDA(launch_flatten_budget(b, c->n_segs, st));
     record(c, 2);
     // the spill pool's lines listed by path, so each path's CTA finds them
@@ -1279,8 +1276,8 @@ std::vector<void *> frame_buffers(const Ctx *c) {
                             &c->path_cols, &c->path_contours, &c->path_bounds, &c->row_first, &c->row_mat, &c->bin_list,
                             &c->bin_ctl, &c->path_leaf_range, &c->path_fill, &c->path_cls, &c->bin_stage,
                             &c->path_feat, &c->contour_feat, &c->path_pred, &c->path_leaf_first, &c->path_leaf_budget,
-                            &c->path_leaf_cursor, &c->path_fill_budget, &c->segs, &c->seg_leaves, &c->seg_order,
-                            &c->seg_ctl, &c->row_paths, &c->tile_fills, &c->tile_state, &c->col_above,
+                            &c->path_leaf_cursor, &c->path_fill_budget, &c->path_seg_first, &c->segs, &c->seg_leaves,
+                            &c->row_paths, &c->tile_fills, &c->tile_state, &c->col_above,
                             &c->col_final, &c->leaves, &c->pool_path, &c->pool_idx, &c->pool_cnt, &c->fills,
                             &c->scan_temp, &c->image, &c->sz_w, &c->path_clip_rel};
     std::vector<void *> v;
@@ -1887,7 +1884,7 @@ int pf_ctx_destroy(void *ctx) {
                       &c->points, &c->pflags, &c->cstart, &c->pstart, &c->fill_rule, &c->color, &c->scenes,
                       &c->scene_path_first, &c->scene_contour_first, &c->scene_fb_first, &c->fb_scene, &c->contour_point_first,
                       &c->contour_path, &c->paths, &c->path_tiles, &c->path_cols, &c->contour_segs,
-                      &c->path_contours, &c->segs, &c->seg_leaves, &c->seg_order, &c->seg_ctl, &c->leaves, &c->pool_path, &c->pool_cnt,
+                      &c->path_contours, &c->path_seg_first, &c->segs, &c->seg_leaves, &c->leaves, &c->pool_path, &c->pool_cnt,
                       &c->pool_idx, &c->tile_fills, &c->path_fill, &c->path_cls, &c->tile_state, &c->col_above,
                       &c->col_final, &c->fills, &c->bin_stage, &c->row_first, &c->row_mat,
                       &c->row_paths, &c->scene_rblk_first, &c->z, &c->fb_count, &c->list, &c->image,
@@ -2486,18 +2483,16 @@ int pf_autotune(void *ctx, uint32_t first, uint32_t count, uint32_t frames, pf_t
         {2, {0, 1, 2, 3}},            // bin_ctas_per_sm[2]
         {3, {4, 6, 8, 12, 16, 32}},   // long_line
         {4, {0, 1}},                  // bin_concurrent
-        {5, {0, 1}},                  // seg_sorted
-        {6, {0, 1, 2, 4, 8, 16}},     // composite_ticket
+        {5, {0, 1, 2, 4, 8, 16}},     // composite_ticket
     };
     auto get = [](const pf_tuning &t, int i) -> float {
         return i < 3 ? (float)t.bin_ctas_per_sm[i] : i == 3 ? t.long_line : i == 4 ? (float)t.bin_concurrent
-               : i == 5 ? (float)t.seg_sorted : (float)t.composite_ticket;
+                                                                                  : (float)t.composite_ticket;
     };
     auto put = [](pf_tuning &t, int i, float v) {
         if (i < 3) t.bin_ctas_per_sm[i] = (uint32_t)v;
         else if (i == 3) t.long_line = v;
         else if (i == 4) t.bin_concurrent = (uint32_t)v;
-        else if (i == 5) t.seg_sorted = (uint32_t)v;
         else t.composite_ticket = (uint32_t)v;
     };
     for (int pass = 0; pass < 3; pass++) {

@@ -128,8 +128,8 @@ struct Batch {
 
     // segments / leaves
     SegDev *segs;
+    uint32_t *path_seg_first;            // [n_paths] first segment of each path
     uint32_t seg_cap;
-    uint32_t *seg_order;                 // [segs] the order the flattening kernels take them in
     uint32_t *seg_leaves;                // [segs + 1] -> scanned
     float4 *leaves;
     uint32_t leaf_cap;
@@ -187,7 +187,7 @@ struct Tuning {
     uint32_t bin_ctas_per_sm[3] = {0, 0, 0};  // 0: as many as fit
     float long_line = 8.0f;
     bool bin_concurrent = false;
-    bool seg_sorted = true;
+    bool seg_sorted = true;  // kept for pf_tuning; changes nothing
     uint32_t comp_ticket = 0;
 };
 
@@ -212,8 +212,11 @@ enum : int {
     kStFill64 = 16,    // two words: fills reserved by the frame's paths (64-bit)
     kStPoolListed = 18,// learned frame: pooled lines listed by path
     kStVisible = 19,   // frame counters: visible tiles of the draw paths (alpha, or a nonzero backdrop)
-    kStFlatTicket = 20,// learned frame: groups of 32 segments taken by the flattening warps
-    kStCount = 21,
+    kStFlatTicket = 20,// groups of segments taken by the flattening warps (exact frame: the count pass)
+    kStFlatTicket2 = 21,// exact frame: the same for the write pass
+    kStSampled = 22,   // segments of the contours sampled for their depth, and the deep ones of them
+    kStSampledDeep = 23,
+    kStCount = 24,
 };
 
 // Kernels launched by this library (host-side counter, all contexts).
@@ -301,7 +304,7 @@ cudaError_t launch_normalize(const Batch &b, uint2 *path_contours, cudaStream_t 
 cudaError_t launch_path_setup(const Batch &b, const uint2 *path_contours, cudaStream_t st);
 cudaError_t launch_path_offsets(const Batch &b, cudaStream_t st);
 cudaError_t launch_contour_segments(const Batch &b, bool write, cudaStream_t st);
-cudaError_t launch_flatten(const Batch &b, uint32_t n_segs, bool write, cudaStream_t st, uint64_t n_lines = 0);
+cudaError_t launch_flatten(const Batch &b, uint32_t n_segs, bool write, bool shallow, cudaStream_t st);
 cudaError_t launch_rows(const Batch &b, bool write, cudaStream_t st);
 cudaError_t launch_composite(const Batch &b, cudaStream_t st);  // b.comp_ticket picks the grid
 // fb_scene[t] = the scene of framebuffer tile t, for every uploaded scene (at upload).
@@ -321,9 +324,6 @@ cudaError_t launch_budgets(const Batch &b, const float *pred, float mul, float a
 cudaError_t launch_path_counts(const Batch &b, const uint2 *path_contours, uint32_t *leaves, uint32_t *fills,
                                cudaStream_t st);
 cudaError_t launch_flatten_budget(const Batch &b, uint32_t n_segs, cudaStream_t st);
-// Orders the segments by estimated subdivision depth (seg_order); ctl holds 32 words.
-cudaError_t launch_seg_order(const Batch &b, uint32_t n_segs, uint32_t *ctl, cudaStream_t st);
-size_t seg_ctl_bytes();  // the per-block bucket counts launch_seg_order keeps in ctl
 // Binning by path: classify (leaf ranges, size classes), then bin every path (counts,
 // backdrops, fill offsets, fills).  A learned frame first lists its pooled lines by path:
 // count, scan pool_cnt, scatter.

@@ -174,10 +174,36 @@ __global__ void k_path_offsets(Batch b) {
 // Segments of a contour, as SegmentsIter::get_next(force_closed = true) yields them
 // (pathfinder/core/data/contour.cpp:110-175): stop at the first malformed point pattern;
 // at the end, an implicit closing line unless first ~= last within 1e-4.
+//
+// One warp per contour, a point per lane.  Every segment ends on the on-curve point the next one
+// starts from, so up to the first malformed pattern the segments are the on-curve points but the
+// last, each with a kind read off the three flags after it, and their order is a ballot's.  (A
+// thread walking its contour point by point: 101 + 16 us for 300,000 glyph contours, 270 + 126 us
+// for the 420,000 of a stroked batch, 22 + 11 us where 240 contours are all there is.)
+
+//
+// The count pass also looks at the segments of every sample-th contour (about 2048 of them): how
+// many would bisect into more than kDeepLines lines, by the flatness value at the root, which a
+// bisection shrinks about 16-fold.  launch_flatten picks its kernel by that.
+constexpr float kDeepFlatness = 4096.0f;  // 8^4: more than 8 lines
+
+__device__ __forceinline__ bool deep_segment(const float2 *p, uint32_t kind) {
+    float m = 0.0f;
+    if (kind == kSegQuad) {
+        const float dx = p[1].x - 0.5f * (p[0].x + p[2].x), dy = p[1].y - 0.5f * (p[0].y + p[2].y);
+        m = 4.0f * (dx * dx + dy * dy);
+    } else if (kind == kSegCubic) {
+        const float ux = 3.0f * p[1].x - 2.0f * p[0].x - p[3].x, uy = 3.0f * p[1].y - 2.0f * p[0].y - p[3].y;
+        const float vx = 3.0f * p[2].x - 2.0f * p[3].x - p[0].x, vy = 3.0f * p[2].y - 2.0f * p[3].y - p[0].y;
+        m = fmaxf(ux * ux, vx * vx) + fmaxf(uy * uy, vy * vy);
+    }
+    return m > kDeepFlatness;
+}
 
 template <bool kWrite>
-__global__ void k_contour_segments(Batch b) {
-    const uint32_t c = global_tid();
+__global__ void __launch_bounds__(kThreads) k_contour_segments(Batch b, uint32_t sample) {
+    const uint32_t c = blockIdx.x * (kThreads / 32) + (threadIdx.x >> 5);
+    const int lane = threadIdx.x & 31;
     if (c >= b.n_contours) return;
     const uint32_t a = b.contour_point_first[c], n = b.contour_point_first[c + 1] - a;
     const uint8_t *fl = b.flags + a;
@@ -185,55 +211,54 @@ __global__ void k_contour_segments(Batch b) {
     if (kWrite) {
         out = b.contour_segs[c];
         path = b.contour_path[c];
+        if (lane == 0 && b.path_contours[path].x == c) b.path_seg_first[path] = out;
         if (out > b.seg_cap) return;
     }
-    uint32_t count = 0, head = 0;
-    auto emit = [&](uint32_t kind, uint32_t first, uint32_t second) {
-        if (kWrite) {
-            const uint32_t k = out + count;
-            if (k < b.seg_cap) b.segs[k] = SegDev{first, second, kind, path};
-            else atomicOr(&b.status[kStErr], kErrOverflowSeg);
-        }
-        count++;
+    auto emit = [&](uint32_t k, const SegDev &s) {
+        if (k < b.seg_cap) b.segs[k] = s;
+        else atomicOr(&b.status[kStErr], kErrOverflowSeg);
     };
-    if (n != 0) {
-        for (;;) {
-            if (head >= n || fl[head] != 0) break;
-            if (head + 1 < n) {
-                const uint8_t f1 = fl[head + 1];
-                if (f1 == 0) {
-                    emit(kSegLine, a + head, 0);
-                    head += 1;
-                } else if (head + 2 < n) {
-                    const uint8_t f2 = fl[head + 2];
-                    if (f1 == 1 && f2 == 0) {
-                        emit(kSegQuad, a + head, 0);
-                        head += 2;
-                    } else if (head + 3 < n) {
-                        if (f1 == 1 && f2 == 2 && fl[head + 3] == 0) {
-                            emit(kSegCubic, a + head, 0);
-                            head += 3;
-                        } else {
-                            break;
-                        }
-                    } else {
-                        break;
-                    }
-                } else {
-                    break;
-                }
-            } else {
-                if (n > 1) {
-                    const float2 f = b.points[a], l = b.points[a + n - 1];
-                    const float dx = fsub(f.x, l.x), dy = fsub(f.y, l.y);
-                    const float len = __fsqrt_rn(fadd(fmul(dx, dx), fmul(dy, dy)));
-                    if (!(len <= 0.0001f)) emit(kSegClose, a + n - 1, a);
-                }
-                break;
-            }
+    uint32_t count = 0, deep = 0;
+    bool ends = n != 0 && fl[0] == 0;  // no malformed pattern so far
+    for (uint32_t base = 0; ends && base < n; base += 32) {
+        const uint32_t i = base + (uint32_t)lane;
+        uint32_t kind = kSegClose;  // none
+        bool bad = false;
+        if (i < n && fl[i] == 0 && i + 1 < n) {
+            const uint8_t f1 = fl[i + 1], f2 = i + 2 < n ? fl[i + 2] : 3, f3 = i + 3 < n ? fl[i + 3] : 3;
+            if (f1 == 0) kind = kSegLine;
+            else if (f1 == 1 && f2 == 0) kind = kSegQuad;
+            else if (f1 == 1 && f2 == 2 && f3 == 0) kind = kSegCubic;
+            else bad = true;
+        }
+        const unsigned bads = __ballot_sync(0xffffffffu, bad);
+        const unsigned before = bads ? (bads & (0u - bads)) - 1u : 0xffffffffu;  // lanes before the first one
+        const unsigned heads = __ballot_sync(0xffffffffu, kind != kSegClose) & before;
+        if (kWrite && (heads >> lane & 1u))
+            emit(out + count + __popc(heads & ((1u << lane) - 1u)), SegDev{a + i, 0, kind, path});
+        if (!kWrite && c % sample == 0) {
+            const bool head = (heads >> lane & 1u) != 0;
+            deep += __popc(__ballot_sync(0xffffffffu, head && deep_segment(b.points + a + i, kind)));
+        }
+        count += __popc(heads);
+        ends = bads == 0;
+    }
+    if (ends && n > 1) {
+        const float2 f = b.points[a], l = b.points[a + n - 1];
+        const float dx = fsub(f.x, l.x), dy = fsub(f.y, l.y);
+        const float len = __fsqrt_rn(fadd(fmul(dx, dx), fmul(dy, dy)));
+        if (!(len <= 0.0001f)) {
+            if (kWrite && lane == 0) emit(out + count, SegDev{a + n - 1, a, kSegClose, path});
+            count++;
         }
     }
-    if (!kWrite) b.contour_segs[c] = count;
+    if (!kWrite && lane == 0) {
+        b.contour_segs[c] = count;
+        if (c % sample == 0) {
+            atomicAdd(&b.status[kStSampled], count);
+            if (deep) atomicAdd(&b.status[kStSampledDeep], deep);
+        }
+    }
 }
 
 // ---------------------------------------------------------------------------
@@ -382,136 +407,14 @@ __device__ void flatten_quad(float b0, float b1, float b2, float b3, float c0, f
     }
 }
 
-// Segment order for the flattening kernels.  A warp's lanes flatten 32 segments in step, so
-// its time is its largest segment's.  Segments are bucketed by sixteenths of the depth a
-// uniform bisection would need, ceil(4 log2 of the root's flatness value) - the value shrinks
-// about 16-fold per level - and the kernels take them bucket by bucket, deepest first, so a
-// warp's segments have like leaf counts, and the learned frame's leaf regions get runs of like
-// lines, which the binning walk takes 32 at a time.  (512-scene frame, flattening + binning:
-// whole levels 6.28 + 20.66 ms, quarters 5.92 + 20.44 ms, eighths 5.90 + 20.18 ms, sixteenths
-// 5.98 + 20.02 ms.)  The order changes no output: every segment writes its own leaf range (exact
-// frame) or reserves slots in its path's region (learned frame).
-constexpr int kSegBuckets = 256;
-
-__device__ __forceinline__ int seg_bucket(const Batch &b, const SegDev &sg) {
-    if (sg.kind == kSegLine || sg.kind == kSegClose) return 0;
-    const float2 p0 = b.points[sg.a], c0 = b.points[sg.a + 1], c1 = b.points[sg.a + 2];
-    float m;
-    if (sg.kind == kSegQuad) {
-        const float dx = c0.x - 0.5f * (p0.x + c1.x), dy = c0.y - 0.5f * (p0.y + c1.y);
-        m = 4.0f * (dx * dx + dy * dy);
-    } else {
-        const float2 p3 = b.points[sg.a + 3];
-        const float ux = 3.0f * c0.x - 2.0f * p0.x - p3.x, uy = 3.0f * c0.y - 2.0f * p0.y - p3.y;
-        const float vx = 3.0f * c1.x - 2.0f * p3.x - p0.x, vy = 3.0f * c1.y - 2.0f * p3.y - p0.y;
-        m = fmaxf(ux * ux, vx * vx) + fmaxf(uy * uy, vy * vy);
-    }
-    if (!(m > 1.0f)) return 0;  // also NaN
-    const int d = (int)ceilf(__log2f(m) * 4.0f);
-    return d < kSegBuckets - 1 ? d : kSegBuckets - 1;
-}
-
-// A fixed grid of kSegBlocks blocks walks the segments grid-stride.  The count pass leaves
-// each block's per-bucket counts in ctl[kSegBuckets * block + bucket]; the totals and starts
-// kernels turn them into each block's first slot per bucket (buckets deepest first); the scatter
-// pass walks the same segments and places them from those slots.  Counters live in shared
-// memory: no global atomics (one hot global counter per bucket serialised millions of them).
-constexpr int kSegBlocks = 1216;  // 8 blocks per SM of 152
-
-template <bool kScatter>
-__global__ void __launch_bounds__(kThreads) k_seg_buckets(Batch b, uint32_t *ctl) {
-    __shared__ uint32_t s_cnt[kSegBuckets];
-    const uint32_t n = b.status[kStSegs];
-    const int lane = threadIdx.x & 31;
-    if (threadIdx.x < kSegBuckets)
-        s_cnt[threadIdx.x] = kScatter ? ctl[kSegBuckets * blockIdx.x + threadIdx.x] : 0u;
-    __syncthreads();
-    const uint32_t stride = gridDim.x * blockDim.x;
-    for (uint32_t base = blockIdx.x * blockDim.x; base < n; base += stride) {
-        const uint32_t i = base + threadIdx.x;
-        const int bk = i < n ? seg_bucket(b, b.segs[i]) : -1;
-        const unsigned group = __match_any_sync(0xffffffffu, bk);
-        const int leader = __ffs(group) - 1;
-        uint32_t slot = 0;
-        if (bk >= 0 && lane == leader) slot = atomicAdd(&s_cnt[bk], (uint32_t)__popc(group));
-        slot = __shfl_sync(0xffffffffu, slot, leader);
-        if (kScatter && bk >= 0) b.seg_order[slot + __popc(group & ((1u << lane) - 1u))] = i;
-    }
-    __syncthreads();
-    if (!kScatter && threadIdx.x < kSegBuckets) ctl[kSegBuckets * blockIdx.x + threadIdx.x] = s_cnt[threadIdx.x];
-}
-
-// Each bucket's total over the blocks (one CTA per bucket), stored after the per-block counts.
-__global__ void __launch_bounds__(kThreads) k_seg_bucket_totals(uint32_t *ctl) {
-    __shared__ uint32_t red[kThreads / 32];
-    const int bk = blockIdx.x, tid = threadIdx.x;
-    uint32_t t = 0;
-    for (int blk = tid; blk < kSegBlocks; blk += kThreads) t += ctl[kSegBuckets * blk + bk];
-    t = __reduce_add_sync(0xffffffffu, t);
-    if ((tid & 31) == 0) red[tid >> 5] = t;
-    __syncthreads();
-    if (tid == 0) {
-        uint32_t sum = 0;
-        for (int w = 0; w < kThreads / 32; w++) sum += red[w];
-        ctl[kSegBuckets * kSegBlocks + bk] = sum;
-    }
-}
-
-// Every block's first slot per bucket, buckets deepest first (one CTA per bucket): the deeper
-// buckets' totals, then an exclusive scan of the bucket's per-block counts.
-__global__ void __launch_bounds__(kThreads) k_seg_bucket_starts(uint32_t *ctl) {
-    constexpr int kPer = (kSegBlocks + kThreads - 1) / kThreads;  // blocks per thread
-    __shared__ uint32_t red[kThreads / 32];
-    __shared__ uint32_t s_base;
-    const int bk = blockIdx.x, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    const uint32_t *total = ctl + kSegBuckets * kSegBlocks;
-    uint32_t deeper = 0;
-    for (int k = bk + 1 + tid; k < kSegBuckets; k += kThreads) deeper += total[k];
-    deeper = __reduce_add_sync(0xffffffffu, deeper);
-    if (lane == 0) red[warp] = deeper;
-    __syncthreads();
-    if (tid == 0) {
-        uint32_t sum = 0;
-        for (int w = 0; w < kThreads / 32; w++) sum += red[w];
-        s_base = sum;
-    }
-    uint32_t v[kPer];
-    uint32_t own = 0;
-#pragma unroll
-    for (int j = 0; j < kPer; j++) {
-        const int blk = tid * kPer + j;
-        v[j] = blk < kSegBlocks ? ctl[kSegBuckets * blk + bk] : 0u;
-        own += v[j];
-    }
-    uint32_t incl = own;
-#pragma unroll
-    for (int o = 1; o < 32; o <<= 1) {
-        const uint32_t n = __shfl_up_sync(0xffffffffu, incl, o);
-        if (lane >= o) incl += n;
-    }
-    __syncthreads();  // red is reused
-    if (lane == 31) red[warp] = incl;
-    __syncthreads();
-    uint32_t before = s_base;
-    for (int w = 0; w < warp; w++) before += red[w];
-    uint32_t run = before + incl - own;
-#pragma unroll
-    for (int j = 0; j < kPer; j++) {
-        const int blk = tid * kPer + j;
-        if (blk < kSegBlocks) ctl[kSegBuckets * blk + bk] = run;
-        run += v[j];
-    }
-}
-
 template <bool kWrite>
 __global__ void __launch_bounds__(kThreads) k_flatten(Batch b, uint32_t n_segs) {
-    const uint32_t t = global_tid();
-    if (t >= n_segs || t >= b.status[kStSegs]) return;
+    const uint32_t i = global_tid();
+    if (i >= n_segs || i >= b.status[kStSegs]) return;
     if (kWrite && b.status[kStLeaves] > b.leaf_cap) {
-        if (t == 0) atomicOr(&b.status[kStErr], kErrOverflowLeaf);
+        if (i == 0) atomicOr(&b.status[kStErr], kErrOverflowLeaf);
         return;
     }
-    const uint32_t i = b.seg_order ? b.seg_order[t] : t;
     const SegDev sg = b.segs[i];
     uint32_t out = kWrite ? b.seg_leaves[i] : 0u;
     uint32_t count = 0;
@@ -966,11 +869,13 @@ __device__ __forceinline__ void walk_lines(const WalkCtx &w, float4 f, bool have
 }
 
 // Flattening shared by the lanes of a warp, for both frames:
-// * learned frame (kExact false): each path's leaf lines go to the path's region, laid out from
+// * learned frame: each path's leaf lines go to the path's region, laid out from
 //   the sizer's budget; lines past the budget spill into the shared pool, and an exhausted pool
 //   sets the overflow bit (the frame is then redone by the exact two-pass method);
-// * exact frame's write pass (kExact true): each segment's lines go to its range of the leaf
+// * exact frame's write pass: each segment's lines go to its range of the leaf
 //   buffer, counted by the count pass.
+//
+// * exact frame's count pass: only the number of each segment's lines is kept.
 //
 // The bisection is shared by the 32 lanes of a warp.  With one segment per lane (as the exact
 // frame's k_flatten does) a warp runs the split branch and the emit branch of every step one after
@@ -980,7 +885,8 @@ __device__ __forceinline__ void walk_lines(const WalkCtx &w, float4 f, bool have
 //
 // * a split round: each lane takes a pending (not flat) piece from the warp's pool in shared
 //   memory, splits it at t = 0.5, and tests both halves: a flat half (or one at the depth bound)
-//   joins the warp's leaf queue, the other goes back on the pool;
+//   joins the warp's leaf queue (count pass: adds to its segment's count), the other goes back on
+//   the pool;
 // * an emit round: each lane takes a queued leaf line and stores it.  Learned frame: the
 //   segment's first leaf (its leftmost piece) at the segment's own slot in its path's region, the
 //   others at slots reserved with one atomic per path among the round's lines (lanes grouped by
@@ -993,26 +899,37 @@ __device__ __forceinline__ void walk_lines(const WalkCtx &w, float4 f, bool have
 // output depends on (fills are counted and placed per tile, coverage sums are integers).  The
 // pool is a stack, so it stays near 32 pieces per level of the warp's deepest segments; a half
 // that finds it full is flattened depth first by its lane alone (about 0.02% of the lines of the
-// 512-scene batch, in a CPU model of this kernel).  Warps take their segments 32 at a time, in the bucketed order, from a
-// frame-wide ticket, up to kPoolSets groups in flight: a group's slot in the segment table is
-// reused once no pending piece or queued line refers to it.
+// 512-scene batch, in a CPU model of this kernel).  Warps take their segments a group at a time from
+// a frame-wide ticket: 32, or fewer (a power of two) when that would leave a resident warp under 8
+// groups, so the last groups end together and small frames use every SM.  A group's slots in the
+// segment table are reused once no pending piece or queued line refers to them.
+//
+// Segments are taken as they lie.  Sorting them by depth first (four kernels, 33 us with 700,000
+// segments) had kept the last groups small and, when a lane flattened its segment alone, a warp's
+// lanes alike; with shared lanes and small groups it no longer pays (flattening and binning, sorted
+// against not: 256 scenes by the learned frame 10.06 / 10.00 ms, 20,000 paths 1.26 / 1.28 ms, 24
+// clipped scenes 0.72 / 0.70 ms, 240 paths 0.20 / 0.18 ms).
 constexpr int kPoolWarps = 2;     // warps per block
 constexpr int kPoolCap = 224;     // pending pieces per warp
 constexpr int kPoolLeafCap = 96;  // queued leaf lines per warp: < 32 before a round, + 2 per lane
-constexpr int kPoolSets = 4;      // groups of 32 segments in flight per warp
+constexpr int kPoolEntries = 128; // segments in flight per warp (at most 32 groups)
+enum : int { kPoolLearned = 0, kPoolCount = 1, kPoolWrite = 2 };
 // piece and line tags: bits 0-6 the segment's table entry (group * 32 + lane), bit 7 the
 // segment's leftmost piece, bit 8 a cubic (else a quadratic), bits 9-13 the depth
 constexpr uint32_t kTagEntry = 127u, kTagLeft = 1u << 7, kTagCubic = 1u << 8;
 constexpr int kTagDepthShift = 9;
 
+template <int kMode>
 struct FlattenPool {
     float4 pend_ends[kPoolCap];   // x0, y0, x1, y1
     float4 pend_ctrl[kPoolCap];   // first control x, y, second control x, y (quadratic: first only)
     uint32_t pend_tag[kPoolCap];
-    float4 leaf[kPoolLeafCap];    // x0, y0, x1, y1
-    uint32_t leaf_tag[kPoolLeafCap];
-    uint4 seg[kPoolSets * 32];    // learned frame: path, region, budget, own slot; exact frame:
-                                  // the segment's first leaf slot and its lines stored so far
+    float4 leaf[kMode == kPoolCount ? 1 : kPoolLeafCap];  // x0, y0, x1, y1
+    uint32_t leaf_tag[kMode == kPoolCount ? 1 : kPoolLeafCap];
+    // learned frame: path, region, budget, own slot; write pass: the segment's first leaf slot and
+    // its lines stored so far; count pass: the segment (kNone: none) and its lines so far
+    uint4 seg[kMode == kPoolLearned ? kPoolEntries : 1];
+    uint2 seg2[kMode == kPoolLearned ? 1 : kPoolEntries];
 };
 
 // Where a lane stores leaf lines by itself.
@@ -1075,28 +992,50 @@ __device__ __noinline__ void flatten_piece_alone_exact(float4 *leaves, uint32_t 
         flatten_quad(ends.x, ends.y, ends.z, ends.w, ctrl.x, ctrl.y, emit, &status[kStErr], depth);
 }
 
+// And for the count pass: the number of the piece's lines.
+__device__ __noinline__ uint32_t count_piece_alone(uint32_t *status, float4 ends, float4 ctrl, uint32_t tag) {
+    uint32_t n = 0;
+    auto emit = [&](float, float, float, float) { n++; };
+    const int depth = (int)(tag >> kTagDepthShift) & 31;
+    if (tag & kTagCubic)
+        flatten_cubic(ends.x, ends.y, ends.z, ends.w, ctrl.x, ctrl.y, ctrl.z, ctrl.w, emit, &status[kStErr], depth);
+    else
+        flatten_quad(ends.x, ends.y, ends.z, ends.w, ctrl.x, ctrl.y, emit, &status[kStErr], depth);
+    return n;
+}
+
 __device__ __forceinline__ bool piece_flat(bool cubic, float4 e, float4 c) {
     const float bb[4] = {e.x, e.y, e.z, e.w}, cc[4] = {c.x, c.y, c.z, c.w};
     return cubic ? flat_cubic(bb, cc) : flat_quad(bb, cc);
 }
 
-template <bool kExact>
-__global__ void __launch_bounds__(kPoolWarps * 32) k_flatten_pool(Batch b, uint32_t n_segs) {
-    __shared__ FlattenPool pools[kPoolWarps];
-    FlattenPool &W = pools[threadIdx.x >> 5];
+template <int kMode>
+__global__ void __launch_bounds__(kPoolWarps * 32) k_flatten_pool(Batch b, uint32_t n_segs, int group_shift) {
+    __shared__ FlattenPool<kMode> pools[kPoolWarps];
+    FlattenPool<kMode> &W = pools[threadIdx.x >> 5];
     const int lane = threadIdx.x & 31;
     const unsigned below = (1u << lane) - 1u;
     uint32_t *const err = &b.status[kStErr];
-    if (kExact && b.status[kStLeaves] > b.leaf_cap) {
+    if (kMode == kPoolWrite && b.status[kStLeaves] > b.leaf_cap) {
         if (blockIdx.x == 0 && threadIdx.x == 0) atomicOr(err, kErrOverflowLeaf);
         return;
     }
     n_segs = min(n_segs, b.status[kStSegs]);
-    const uint32_t n_groups = (n_segs + 31u) / 32u;
-    // a group of 32 segments: lane 0 takes the ticket, and the lanes read it when they need it,
-    // so the atomic's round trip overlaps the work in between
-    uint32_t ticket = lane == 0 ? atomicAdd(&b.status[kStFlatTicket], 1u) : 0u;
+    constexpr int kTicket = kMode == kPoolWrite ? kStFlatTicket2 : kStFlatTicket;
+    const uint32_t group = 1u << group_shift, n_groups = (n_segs + group - 1u) >> group_shift;
+    const uint32_t n_sets = min(32u, (uint32_t)kPoolEntries >> group_shift);
+    const uint32_t all_sets = n_sets == 32u ? ~0u : (1u << n_sets) - 1u;
+    // a group of segments: lane 0 takes the ticket, and the lanes read it when they need it, so the
+    // atomic's round trip overlaps the work in between
+    uint32_t ticket = lane == 0 ? atomicAdd(&b.status[kTicket], 1u) : 0u;
     auto current_group = [&]() { return __shfl_sync(~0u, ticket, 0); };
+    uint32_t open = 0;  // count pass: the table's groups whose counts are not stored yet
+    auto store_counts = [&](uint32_t set) {
+        if ((uint32_t)lane < group) {
+            const uint2 c = W.seg2[(set << group_shift) + lane];
+            if (c.x != kNone) b.seg_leaves[c.x] = c.y;
+        }
+    };
     int top = 0, nleaf = 0;  // pool and queue sizes (the same in every lane)
     uint32_t produced = 0;
 
@@ -1141,7 +1080,7 @@ __global__ void __launch_bounds__(kPoolWarps * 32) k_flatten_pool(Batch b, uint3
     // n (1..32) queued lines from the top of the queue, one per lane: a segment's leftmost line
     // goes to the segment's own slot, the others reserve slots (one atomic per path)
     auto emit_round = [&](int n) {
-        if constexpr (kExact) {
+        if constexpr (kMode == kPoolWrite) {
             // exact frame: each segment's lines fill its counted range, slots taken from the
             // segment's counter by one lane per segment among the round's lines
             const bool act = lane < n;
@@ -1159,11 +1098,11 @@ __global__ void __launch_bounds__(kPoolWarps * 32) k_flatten_pool(Batch b, uint3
                 const int leader = __ffs(same) - 1;
                 uint32_t stored = 0;
                 if (lane == leader) {
-                    stored = W.seg[entry].y;
-                    W.seg[entry].y = stored + __popc(same);
+                    stored = W.seg2[entry].y;
+                    W.seg2[entry].y = stored + __popc(same);
                 }
                 stored = __shfl_sync(act_mask, stored, leader);
-                const uint32_t idx = W.seg[entry].x + stored + __popc(same & below);
+                const uint32_t idx = W.seg2[entry].x + stored + __popc(same & below);
                 if (idx < b.leaf_cap) b.leaves[idx] = v;
                 else atomicOr(err, kErrOverflowLeaf);
             }
@@ -1209,45 +1148,47 @@ __global__ void __launch_bounds__(kPoolWarps * 32) k_flatten_pool(Batch b, uint3
         if (top < 32 && current_group() < n_groups) {
             // a table group that no pending piece or queued line refers to
             uint32_t used = 0;
-            for (int k = lane; k < top; k += 32) used |= 1u << ((W.pend_tag[k] & kTagEntry) >> 5);
-            for (int k = lane; k < nleaf; k += 32) used |= 1u << ((W.leaf_tag[k] & kTagEntry) >> 5);
+            for (int k = lane; k < top; k += 32) used |= 1u << ((W.pend_tag[k] & kTagEntry) >> group_shift);
+            for (int k = lane; k < nleaf; k += 32) used |= 1u << ((W.leaf_tag[k] & kTagEntry) >> group_shift);
             used = __reduce_or_sync(~0u, used);
-            if (used != (1u << kPoolSets) - 1u) {
+            if (used != all_sets) {
                 const uint32_t set = __ffs(~used) - 1;
-                const uint32_t t = current_group() * 32u + (uint32_t)lane;
-                const bool valid = t < n_segs;
+                const uint32_t i = (current_group() << group_shift) + (uint32_t)lane;
+                const bool slot = (uint32_t)lane < group, valid = slot && i < n_segs;
+                const uint32_t entry = (set << group_shift) + (uint32_t)lane;
+                if (kMode == kPoolCount) {
+                    if (open >> set & 1u) store_counts(set);
+                    open |= 1u << set;
+                }
                 bool is_leaf = false, is_piece = false;
                 float4 ends = make_float4(0.0f, 0.0f, 0.0f, 0.0f), ctrl = ends;
-                uint32_t tag = set * 32u + (uint32_t)lane | kTagLeft;
+                uint32_t tag = (entry & kTagEntry) | kTagLeft;
                 if (valid) {
-                    const uint32_t i = b.seg_order ? b.seg_order[t] : t;
                     const SegDev sg = b.segs[i];
-                    if constexpr (kExact) {
-                        W.seg[set * 32u + lane] = make_uint4(b.seg_leaves[i], 0u, 0u, 0u);
-                    } else {
+                    if constexpr (kMode == kPoolLearned) {
                         const uint32_t region = b.path_leaf_first[sg.path];
-                        const uint32_t own = region + (i - b.contour_segs[b.path_contours[sg.path].x]);
-                        W.seg[set * 32u + lane] = make_uint4(sg.path, region, b.path_leaf_budget[sg.path], own);
+                        W.seg[entry] = make_uint4(sg.path, region, b.path_leaf_budget[sg.path],
+                                                  region + (i - b.path_seg_first[sg.path]));
                     }
-                    const float2 p0 = b.points[sg.a];
-                    if (sg.kind == kSegLine || sg.kind == kSegClose) {
-                        const float2 p1 = b.points[sg.kind == kSegLine ? sg.a + 1 : sg.b];
-                        ends = make_float4(p0.x, p0.y, p1.x, p1.y);
-                        is_leaf = true;
-                    } else if (sg.kind == kSegQuad) {
-                        const float2 c = b.points[sg.a + 1], p2 = b.points[sg.a + 2];
+                    if constexpr (kMode == kPoolWrite) W.seg2[entry] = make_uint2(b.seg_leaves[i], 0u);
+                    const float2 p0 = b.points[sg.a], p1 = b.points[sg.kind == kSegClose ? sg.b : sg.a + 1];
+                    ends = make_float4(p0.x, p0.y, p1.x, p1.y);
+                    if (sg.kind == kSegQuad) {
+                        const float2 p2 = b.points[sg.a + 2];
                         ends = make_float4(p0.x, p0.y, p2.x, p2.y);
-                        ctrl = make_float4(c.x, c.y, 0.0f, 0.0f);
-                    } else {
-                        const float2 c0 = b.points[sg.a + 1], c1 = b.points[sg.a + 2], p3 = b.points[sg.a + 3];
+                        ctrl = make_float4(p1.x, p1.y, 0.0f, 0.0f);
+                    } else if (sg.kind == kSegCubic) {
+                        const float2 p2 = b.points[sg.a + 2], p3 = b.points[sg.a + 3];
                         ends = make_float4(p0.x, p0.y, p3.x, p3.y);
-                        ctrl = make_float4(c0.x, c0.y, c1.x, c1.y);
+                        ctrl = make_float4(p1.x, p1.y, p2.x, p2.y);
                         tag |= kTagCubic;
                     }
-                    if (!is_leaf) {
-                        is_leaf = piece_flat(tag & kTagCubic, ends, ctrl);
-                        is_piece = !is_leaf;
-                    }
+                    is_leaf = sg.kind == kSegLine || sg.kind == kSegClose || piece_flat(tag & kTagCubic, ends, ctrl);
+                    is_piece = !is_leaf;
+                }
+                if constexpr (kMode == kPoolCount) {
+                    if (slot) W.seg2[entry] = make_uint2(valid ? i : kNone, is_leaf ? 1u : 0u);
+                    is_leaf = false;
                 }
                 const unsigned leaf_mask = __ballot_sync(~0u, is_leaf), piece_mask = __ballot_sync(~0u, is_piece);
                 // nleaf < 32 and top < 32 here: the group fits (checked all the same)
@@ -1273,7 +1214,7 @@ __global__ void __launch_bounds__(kPoolWarps * 32) k_flatten_pool(Batch b, uint3
                 nleaf = min(nleaf + __popc(leaf_mask), kPoolLeafCap);
                 top = min(top + __popc(piece_mask), kPoolCap);
                 __syncwarp();
-                if (lane == 0) ticket = atomicAdd(&b.status[kStFlatTicket], 1u);
+                if (lane == 0) ticket = atomicAdd(&b.status[kTicket], 1u);
                 drain();
             }
         }
@@ -1328,6 +1269,10 @@ __global__ void __launch_bounds__(kPoolWarps * 32) k_flatten_pool(Batch b, uint3
         const bool leaf0 = act && (deep || piece_flat(cubic, e0, c0));
         const bool leaf1 = act && (deep || piece_flat(cubic, e1, c1));
         const unsigned l0 = __ballot_sync(~0u, leaf0), l1 = __ballot_sync(~0u, leaf1);
+        if constexpr (kMode == kPoolCount) {
+            const uint32_t lines = (leaf0 ? 1u : 0u) + (leaf1 ? 1u : 0u);
+            if (lines) atomicAdd(&W.seg2[tag & kTagEntry].y, lines);
+        } else {
         // nleaf < 32 before the round, so at most 31 + 64 lines are queued after it (the
         // bounds checks below never fail; a failure would send the frame to the exact redo)
         if (leaf0) {
@@ -1349,6 +1294,7 @@ __global__ void __launch_bounds__(kPoolWarps * 32) k_flatten_pool(Batch b, uint3
             }
         }
         nleaf = min(nleaf + __popc(l0) + __popc(l1), kPoolLeafCap);
+        }
         // halves that are not flat go back on the pool, the second below the first
         const bool keep0 = act && !leaf0, keep1 = act && !leaf1;
         const unsigned m0 = __ballot_sync(~0u, keep0), m1 = __ballot_sync(~0u, keep1);
@@ -1369,13 +1315,18 @@ __global__ void __launch_bounds__(kPoolWarps * 32) k_flatten_pool(Batch b, uint3
         }
         top = min(top + __popc(m0) + __popc(m1), kPoolCap);
         if ((keep1 && k1 >= kPoolCap) || (keep0 && k0 >= kPoolCap)) {
-            if constexpr (kExact) {
+            if constexpr (kMode == kPoolCount) {
+                if (keep1 && k1 >= kPoolCap)
+                    atomicAdd(&W.seg2[tag1 & kTagEntry].y, count_piece_alone(b.status, e1, c1, tag1));
+                if (keep0 && k0 >= kPoolCap)
+                    atomicAdd(&W.seg2[tag0 & kTagEntry].y, count_piece_alone(b.status, e0, c0, tag0));
+            } else if constexpr (kMode == kPoolWrite) {
                 if (keep1 && k1 >= kPoolCap) {
-                    uint4 &sg = W.seg[tag1 & kTagEntry];
+                    uint2 &sg = W.seg2[tag1 & kTagEntry];
                     flatten_piece_alone_exact(b.leaves, b.leaf_cap, b.status, &sg.y, sg.x, e1, c1, tag1);
                 }
                 if (keep0 && k0 >= kPoolCap) {
-                    uint4 &sg = W.seg[tag0 & kTagEntry];
+                    uint2 &sg = W.seg2[tag0 & kTagEntry];
                     flatten_piece_alone_exact(b.leaves, b.leaf_cap, b.status, &sg.y, sg.x, e0, c0, tag0);
                 }
             } else {
@@ -1389,7 +1340,11 @@ __global__ void __launch_bounds__(kPoolWarps * 32) k_flatten_pool(Batch b, uint3
         }
         __syncwarp();
     }
-    if constexpr (!kExact) {
+    if constexpr (kMode == kPoolCount) {
+        for (uint32_t set = 0; set < n_sets; set++)
+            if (open >> set & 1u) store_counts(set);
+    }
+    if constexpr (kMode == kPoolLearned) {
         store_held();
         const uint32_t total = __reduce_add_sync(~0u, produced);
         if (lane == 0) atomicAdd(&b.status[kStLeafCount], total);
@@ -2704,70 +2659,52 @@ cudaError_t launch_path_offsets(const Batch &b, cudaStream_t st) {
 
 cudaError_t launch_contour_segments(const Batch &b, bool write, cudaStream_t st) {
     if (!b.n_contours) return cudaSuccess;
-    if (write) PF_LAUNCH(k_contour_segments<true><<<grid_for(b.n_contours), kThreads, 0, st>>>(b));
-    else PF_LAUNCH(k_contour_segments<false><<<grid_for(b.n_contours), kThreads, 0, st>>>(b));
+    const unsigned grid = grid_for(b.n_contours, kThreads / 32);
+    const uint32_t sample = b.n_contours / 2048 + 1;
+    if (write) PF_LAUNCH(k_contour_segments<true><<<grid, kThreads, 0, st>>>(b, sample));
+    else PF_LAUNCH(k_contour_segments<false><<<grid, kThreads, 0, st>>>(b, sample));
     return cudaGetLastError();
 }
 
 // The warp-shared flattening runs as many blocks as fit on every SM (they take segments by
-// ticket), fewer when the frame has fewer groups of 32 segments than resident warps.
-template <bool kExact>
-static cudaError_t flatten_pool_blocks(uint64_t *resident) {
+// ticket).  Groups of 32 segments, or of the power of two below that leaves 8 groups to every
+// resident warp (20,000 paths, 700,000 segments: 0.48 ms of flattening with 16 groups a warp, 0.46
+// with 8, 0.49 with 4; 240 paths, 4,000 segments, one to a group: 0.13 ms with one lane per
+// segment -> 0.066).
+template <int kMode>
+static cudaError_t launch_flatten_pool(const Batch &b, uint32_t n_segs, cudaStream_t st) {
     int dev = 0, sms = 152, per_sm = 0;
     cudaGetDevice(&dev);
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-    const cudaError_t e =
-        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_flatten_pool<kExact>, kPoolWarps * 32, 0);
-    *resident = uint64_t(std::max(1, per_sm)) * uint64_t(sms);
-    return e;
-}
-
-template <bool kExact>
-static cudaError_t launch_flatten_pool(const Batch &b, uint32_t n_segs, cudaStream_t st) {
-    uint64_t resident = 0;
-    if (const cudaError_t e = flatten_pool_blocks<kExact>(&resident)) return e;
-    const uint64_t groups = (uint64_t(n_segs) + 31) / 32;
+    if (const cudaError_t e =
+            cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_flatten_pool<kMode>, kPoolWarps * 32, 0))
+        return e;
+    const uint64_t resident = uint64_t(std::max(1, per_sm)) * uint64_t(sms);
+    int shift = 0;
+    while (shift < 5 && (uint64_t(16) << shift) * resident * kPoolWarps <= n_segs) shift++;
+    const uint64_t groups = ((uint64_t(n_segs) - 1) >> shift) + 1;
     const uint64_t blocks = std::min<uint64_t>(resident, (groups + kPoolWarps - 1) / kPoolWarps);
-    PF_LAUNCH(k_flatten_pool<kExact><<<(unsigned)blocks, kPoolWarps * 32, 0, st>>>(b, n_segs));
+    PF_LAUNCH(k_flatten_pool<kMode><<<(unsigned)blocks, kPoolWarps * 32, 0, st>>>(b, n_segs, shift));
     return cudaGetLastError();
 }
 
-// Exact frame: the count pass one segment per thread (it stores nothing, so its stack stays in
-// L1).  The write pass is shared by the lanes of a warp when the segments bisect deeply enough
-// and are many enough to give every resident warp a group of 32; otherwise one segment per
-// thread keeps more of them in flight (GB300, exact frames: 512-scene batch, 51 lines per
-// segment, 38.28 -> 34.48 ms with the shared pass; 20,000 paths, 25 per segment, 2.28 -> 2.10 ms;
-// 150,000 glyphs, 2.3 per segment, 2.29 -> 2.37 ms; 240 paths, 4,062 segments, 0.445 -> 0.453 ms).
-constexpr uint64_t kPoolMinLinesPerSeg = 8;
-
-cudaError_t launch_flatten(const Batch &b, uint32_t n_segs, bool write, cudaStream_t st, uint64_t n_lines) {
+// Exact frame.  Segments that bisect deeply are shared by the lanes of a warp; where nearly all are
+// shallow (under 1 in 64 of the sampled ones takes more than 8 lines), one segment per thread keeps
+// more of them in flight (count and write pass with their segments, GB300: 150,000 glyphs, none
+// deep, 0.24 ms against 0.36 shared; stroked batch, 1.8 lines per segment but some deep, 0.72
+// against 0.60; 20,000 paths, 25 per segment, 0.80 against 0.46).
+cudaError_t launch_flatten(const Batch &b, uint32_t n_segs, bool write, bool shallow, cudaStream_t st) {
     if (!n_segs) return cudaSuccess;
-    if (write) {
-        uint64_t resident = 0;
-        if (const cudaError_t e = flatten_pool_blocks<true>(&resident)) return e;
-        if (n_lines >= kPoolMinLinesPerSeg * n_segs && n_segs >= resident * kPoolWarps * 32)
-            return launch_flatten_pool<true>(b, n_segs, st);
-        PF_LAUNCH(k_flatten<true><<<grid_for(n_segs), kThreads, 0, st>>>(b, n_segs));
-        return cudaGetLastError();
-    }
-    PF_LAUNCH(k_flatten<false><<<grid_for(n_segs), kThreads, 0, st>>>(b, n_segs));
-    return cudaGetLastError();
-}
-
-size_t seg_ctl_bytes() { return (size_t(kSegBlocks) + 1) * kSegBuckets * 4; }
-
-cudaError_t launch_seg_order(const Batch &b, uint32_t n_segs, uint32_t *ctl, cudaStream_t st) {
-    if (!n_segs) return cudaSuccess;
-    PF_LAUNCH(k_seg_buckets<false><<<kSegBlocks, kThreads, 0, st>>>(b, ctl));
-    PF_LAUNCH(k_seg_bucket_totals<<<kSegBuckets, kThreads, 0, st>>>(ctl));
-    PF_LAUNCH(k_seg_bucket_starts<<<kSegBuckets, kThreads, 0, st>>>(ctl));
-    PF_LAUNCH(k_seg_buckets<true><<<kSegBlocks, kThreads, 0, st>>>(b, ctl));
+    if (!shallow)
+        return write ? launch_flatten_pool<kPoolWrite>(b, n_segs, st) : launch_flatten_pool<kPoolCount>(b, n_segs, st);
+    if (write) PF_LAUNCH(k_flatten<true><<<grid_for(n_segs), kThreads, 0, st>>>(b, n_segs));
+    else PF_LAUNCH(k_flatten<false><<<grid_for(n_segs), kThreads, 0, st>>>(b, n_segs));
     return cudaGetLastError();
 }
 
 cudaError_t launch_flatten_budget(const Batch &b, uint32_t n_segs, cudaStream_t st) {
     if (!n_segs) return cudaSuccess;
-    return launch_flatten_pool<false>(b, n_segs, st);
+    return launch_flatten_pool<kPoolLearned>(b, n_segs, st);
 }
 
 cudaError_t launch_bin_classify(const Batch &b, bool learned, cudaStream_t st) {
