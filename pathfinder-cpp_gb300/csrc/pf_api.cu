@@ -88,6 +88,8 @@ struct Ctx {
     std::vector<uint8_t> h_path_is_clip;
     // stroked paths: the uploaded outline and what the upload's stroke pass works in
     DevBuf in_points, in_pflags, in_cstart, in_pstart, st_stroke, st_closed, st_dashes, st_scenes, st_cfirst;
+    DevBuf dash_chunks;
+    uint64_t dash_points_hint = 0;  // points of the chunks the largest dashed upload took
     DevBuf dash_pts, dash_cnt, dash_end, dash_points, dash_flags, job_first, jobs, job_pts, st_bounds;
     DevBuf job_units, job_nfwd, job_flags, job_cap1, job_end, units, unit_leaves, st_leaves, leaf_pts;
     DevBuf st_order_ctl, unit_order, dash_order;
@@ -454,13 +456,26 @@ int stroke_upload(Ctx *c, const pf_scene_view *scenes, uint32_t n, const std::ve
         PF_CUDA(launch_stroke_order(in, 1, c->st_order_ctl.as<uint32_t>(), c->dash_order.as<uint32_t>(), st));
         in.dash_order = c->dash_order.as<uint32_t>();
         in.n_dashed = c->ustats.dashed_paths;
+        // the chunk pool: two chunks to begin each path, and 16 points for each input point or what
+        // the largest upload so far took; at most 2^26 points (0.6 GB)
+        const uint64_t chunk_points = std::max<uint64_t>(c->dash_points_hint, uint64_t(c->n_points) * 16);
+        const uint64_t chunk_cap = std::min<uint64_t>(2 * uint64_t(in.n_dashed) + chunk_points / kDashChunk,
+                                                      (1ull << 26) / kDashChunk);
+        PF_CUDA(c->dash_chunks.ensure(chunk_cap * (16 + 9 * kDashChunk) + 16));
+        char *pool = c->dash_chunks.as<char>();
+        in.dash_chunk_head = reinterpret_cast<uint4 *>(pool);
+        in.dash_chunk_points = reinterpret_cast<float2 *>(pool + chunk_cap * 16);
+        in.dash_chunk_flags = reinterpret_cast<uint8_t *>(pool + chunk_cap * (16 + 8 * kDashChunk));
+        in.dash_chunk_count = status + kStDashChunks;
+        in.dash_chunk_cap = (uint32_t)chunk_cap;
+        PF_CUDA(cudaMemsetAsync(pool, 0xff, chunk_cap * 16, st));  // no path
         PF_CUDA(launch_dash(in, false, status, st));
         PF_CUDA(scan_exclusive_u32(in.dash_pts, in.dash_pts, N, in.dash_pts + N, c->scan_temp.p, st, status));
         PF_CUDA(scan_exclusive_u32(in.dash_cnt, in.dash_cnt, N, in.dash_cnt + N, c->scan_temp.p, st, status));
-        uint32_t tot[3], w[5];
+        uint32_t tot[3], w[6];
         PF_CUDA(mark(1));
         if (int e = read_words(c, {in.dash_pts + N, in.dash_cnt + N, status + kStFill64, status + kStFill64 + 1,
-                                   status + kStErr}, w))
+                                   status + kStErr, status + kStDashChunks}, w))
             return e;
         tot[0] = w[0], tot[1] = w[1], tot[2] = w[4];
         const uint64_t wide = uint64_t(w[2]) | uint64_t(w[3]) << 32;  // the dash points' 64-bit total
@@ -476,7 +491,10 @@ int stroke_upload(Ctx *c, const pf_scene_view *scenes, uint32_t n, const std::ve
         in.dash_flags = c->dash_flags.as<uint8_t>();
         in.dash_end = c->dash_end.as<uint32_t>();
         PF_CUDA(mark(2));
-        PF_CUDA(launch_dash(in, true, status, st));
+        in.n_dash_chunks = w[5];
+        c->dash_points_hint = std::max(c->dash_points_hint, uint64_t(w[5]) * kDashChunk);
+        if (w[5] <= in.dash_chunk_cap) PF_CUDA(launch_dash_gather(in, st));
+        else PF_CUDA(launch_dash(in, true, status, st));
         PF_CUDA(mark(3));
     }
     // one job per output contour
@@ -1890,7 +1908,7 @@ int pf_ctx_destroy(void *ctx) {
                       &c->row_paths, &c->scene_rblk_first, &c->z, &c->fb_count, &c->list, &c->image,
                       &c->status, &c->scan_temp, &c->path_clip, &c->path_is_clip, &c->path_clip_rel,
                       &c->in_points, &c->in_pflags, &c->in_cstart, &c->in_pstart, &c->st_stroke, &c->st_closed,
-                      &c->st_dashes, &c->st_scenes, &c->st_cfirst, &c->dash_pts, &c->dash_cnt, &c->dash_end,
+                      &c->st_dashes, &c->st_scenes, &c->st_cfirst, &c->dash_chunks, &c->dash_pts, &c->dash_cnt, &c->dash_end,
                       &c->dash_points, &c->dash_flags, &c->job_first, &c->jobs, &c->job_pts, &c->st_bounds,
                       &c->job_units, &c->job_nfwd, &c->job_flags, &c->job_cap1, &c->job_end, &c->units,
                       &c->unit_leaves, &c->st_leaves, &c->leaf_pts, &c->path_grad, &c->grad_paint, &c->image_snap,

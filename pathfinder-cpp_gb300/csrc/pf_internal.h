@@ -216,7 +216,8 @@ enum : int {
     kStFlatTicket2 = 21,// exact frame: the same for the write pass
     kStSampled = 22,   // segments of the contours sampled for their depth, and the deep ones of them
     kStSampledDeep = 23,
-    kStCount = 24,
+    kStDashChunks = 24,// upload: chunks of dashed points taken
+    kStCount = 25,
 };
 
 // Kernels launched by this library (host-side counter, all contexts).
@@ -246,6 +247,13 @@ struct StrokeIn {
     uint32_t *dash_end;                 // [dash contours] one past each contour's last point
     float2 *dash_points;
     uint8_t *dash_flags;
+    // chunks the count pass stores the dashed points in: (path, its first point in the path, the
+    // path's contours begun before it, -), points, flags with bit 7 on a contour's first point
+    uint4 *dash_chunk_head;
+    float2 *dash_chunk_points;
+    uint8_t *dash_chunk_flags;
+    uint32_t *dash_chunk_count;         // chunks taken (may run past dash_chunk_cap)
+    uint32_t dash_chunk_cap, n_dash_chunks;
     uint32_t *job_first;                // [n_paths + 1] counts -> scanned
     uint4 *jobs;                        // [n_jobs]
     uint32_t *job_pts;                  // [n_jobs + 1] counts -> scanned
@@ -268,7 +276,9 @@ struct StrokeIn {
 };
 size_t stroke_order_ctl_bytes();
 cudaError_t launch_stroke_order(const StrokeIn &in, int what, uint32_t *ctl, uint32_t *order, cudaStream_t st);
+constexpr uint32_t kDashChunk = 64;  // points
 cudaError_t launch_dash(const StrokeIn &in, bool write, uint32_t *status, cudaStream_t st);
+cudaError_t launch_dash_gather(const StrokeIn &in, cudaStream_t st);
 cudaError_t launch_copy_words(uint32_t *dst, const uint32_t *src, uint32_t n, cudaStream_t st);
 // up to 8 single words gathered into dst[0, n)
 struct WordSources {
