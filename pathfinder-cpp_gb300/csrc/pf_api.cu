@@ -71,6 +71,7 @@ struct HostCanon {
 
 struct Ctx {
     int device = 0;
+    uint32_t n_sms = 152;
     cudaStream_t stream = nullptr;
     bool own_stream = false;
     uint32_t flags = 0;
@@ -956,6 +957,7 @@ Batch make_batch(Ctx *c) {
     b.row_cap = (uint32_t)std::min<size_t>(c->row_paths.cap / 16, 0xffffffffu);
     b.n_rows = c->r_rows;
     b.n_fb = c->r_fb;
+    b.n_sms = c->n_sms;
     b.z = c->z.as<int32_t>();
     b.fb_count = c->fb_count.as<uint32_t>();
     b.list = c->list.as<uint32_t>();
@@ -1115,8 +1117,9 @@ int stage_setup(Ctx *c, bool learned) {
 // Binning and composite of a frame whose leaf lines are in place.  The fills buffer starts
 // at the largest frame's size (or about three fills per line); a frame that overruns it is
 // counted to the exact total, the buffer grows, and binning and composite run again.  Ends
-// with the status words read back.
-int bin_and_composite(Ctx *c, Batch b, bool learned) {
+// with the status words read back.  max_leaves: the most leaf lines a path can have.
+int bin_and_composite(Ctx *c, Batch b, bool learned, uint64_t max_leaves) {
+    const bool large = c->h_status[kStLargeRects] != 0 || max_leaves > kCtaMaxLeaves;
     cudaStream_t st = c->stream;
     for (int attempt = 0;; attempt++) {
         PF_CUDA(cudaMemsetAsync(b.bin_ctl, 0, 1024, st));
@@ -1128,7 +1131,7 @@ int bin_and_composite(Ctx *c, Batch b, bool learned) {
             for (auto &e : c->bs.join) PF_CUDA(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
             c->bs_ready = true;
         }
-        PF_CUDA(launch_bin_paths(b, c->tune, c->bs_ready ? &c->bs : nullptr, st));
+        PF_CUDA(launch_bin_paths(b, c->tune, large, c->bs_ready ? &c->bs : nullptr, st));
         record(c, 3);
         record(c, 4);
         record(c, 5);
@@ -1224,7 +1227,7 @@ int render_exact(Ctx *c, uint32_t first, uint32_t count, pf_frame_stats *stats) 
     //    then coverage and the front-to-back composite with the z-cull walk
     PF_CUDA(c->fills.ensure(std::max<uint64_t>(c->fill_hint, uint64_t(c->n_leaves) * 3) * 8 + 16));
     b = make_batch(c);
-    if (int e = bin_and_composite(c, b, false)) return e;
+    if (int e = bin_and_composite(c, b, false, c->n_leaves)) return e;
     return finish_frame(c, first, count, launches0, stats);
 }
 
@@ -1269,7 +1272,7 @@ int render_learned_frame(Ctx *c, uint32_t first, uint32_t count, pf_frame_stats 
     PF_CUDA(launch_pool_lists(b, false, st));
     if (int e = scan(c, b.pool_cnt, N + 1, kStPoolListed)) return e;
     PF_CUDA(launch_pool_lists(b, true, st));
-    if (int e = bin_and_composite(c, b, true)) return e;
+    if (int e = bin_and_composite(c, b, true, leaf_slots)) return e;
     if (c->h_status[kStErr] & kErrOverflowLeaf) {
         // a path overran its leaf region and the pool: redo the frame exactly
         const int e = render_exact(c, first, count, stats);
@@ -1863,6 +1866,9 @@ int pf_ctx_create(const pf_config *config, void **out) {
         c->flags = config->flags;
     }
     cudaError_t e = cudaSetDevice(c->device);
+    int sms = 0;
+    if (e == cudaSuccess) e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, c->device);
+    c->n_sms = (uint32_t)std::max(sms, 1);
     if (e == cudaSuccess && !c->stream) {
         e = cudaStreamCreateWithFlags(&c->stream, cudaStreamNonBlocking);
         c->own_stream = e == cudaSuccess;

@@ -16,6 +16,7 @@ constexpr int kCovShift = 20;
 constexpr int kMaxDepth = 32;              // flattening recursion bound (depth of the d3d9 bisection)
 constexpr uint32_t kMaxWalk = 1u << 20;    // tile-walk step bound per line
 constexpr uint32_t kNone = 0xffffffffu;       // also the scene format's "no clip path"
+constexpr uint32_t kCtaMaxLeaves = 1u << 22;   // most leaf lines of a path that a CTA bins
 constexpr int kRowWindow = 64;                 // framebuffer-tile rows a block of the row lists takes
 constexpr uint32_t kPathIsClip = 8u;           // PathDev::flags: a clip path (tiled, never drawn)
 
@@ -166,6 +167,7 @@ struct Batch {
     uint32_t row_cap;
     uint32_t n_rows;
     uint32_t n_fb;
+    uint32_t n_sms;                      // of the device
 
     // composite-list dump (canonical output only)
     int32_t *z;                          // [fb tiles]
@@ -217,7 +219,8 @@ enum : int {
     kStSampled = 22,   // segments of the contours sampled for their depth, and the deep ones of them
     kStSampledDeep = 23,
     kStDashChunks = 24,// upload: chunks of dashed points taken
-    kStCount = 25,
+    kStLargeRects = 25,// nonzero: a path's rect takes the binning's global passes
+    kStCount = 26,
 };
 
 // Kernels launched by this library (host-side counter, all contexts).
@@ -344,7 +347,8 @@ struct BinStreams {
     cudaStream_t side[2];
     cudaEvent_t fork, join[2];
 };
-cudaError_t launch_bin_paths(const Batch &b, const Tuning &t, const BinStreams *bs, cudaStream_t st);
+// large: a path may be of the class of the global passes.
+cudaError_t launch_bin_paths(const Batch &b, const Tuning &t, bool large, const BinStreams *bs, cudaStream_t st);
 // The most CTAs of each binning class one SM holds.
 cudaError_t bin_class_max_ctas(int out[3]);
 cudaError_t launch_pool_lists(const Batch &b, bool scatter, cudaStream_t st);

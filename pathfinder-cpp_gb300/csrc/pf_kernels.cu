@@ -32,6 +32,8 @@ namespace pfc {
 namespace {
 
 constexpr int kThreads = 256;
+// Shared words of the binning's CTA classes (see "Binning by path").
+__host__ __device__ constexpr uint32_t class_words(int c) { return c == 0 ? 1088u : c == 1 ? 4352u : 16896u; }
 
 __device__ __forceinline__ float fadd(float a, float b) { return __fadd_rn(a, b); }
 __device__ __forceinline__ float fsub(float a, float b) { return __fsub_rn(a, b); }
@@ -161,6 +163,8 @@ __global__ void k_path_setup(Batch b, const uint2 *path_contours) {
     b.paths[p] = P;
     b.path_tiles[p] = (uint32_t)(w * h);
     b.path_cols[p] = (uint32_t)w;
+    // a rect for the binning's global passes: the host leaves them out of frames without one
+    if ((uint64_t)w * (uint32_t)(h + 1) > class_words(2)) b.status[kStLargeRects] = 1;
 }
 
 __global__ void k_path_offsets(Batch b) {
@@ -1366,7 +1370,6 @@ __global__ void __launch_bounds__(kPoolWarps * 32) k_flatten_pool(Batch b, uint3
 // backdrop deltas in bits 24-31, later the tile's write cursor) and one per column (deltas
 // landing above the rect, summed as int32).
 constexpr int kCtaClasses = 3;
-__host__ __device__ constexpr uint32_t class_words(int c) { return c == 0 ? 1088u : c == 1 ? 4352u : 16896u; }
 // Small CTAs for the small classes: a path's barriers then hold few warps, and more paths are in
 // flight per SM (A/B on the 512-scene batch, binning: 21.56 ms with 256-thread CTAs, 6 per SM, for
 // classes 0 and 1; 20.80 ms with 128-thread CTAs, 12 per SM; 20.72 ms with class 0 at 64 threads,
@@ -1383,8 +1386,7 @@ __host__ __device__ constexpr int class_min_ctas(int c) { return c == 2 ? 3 : c 
 __host__ __device__ constexpr uint32_t class_stage(int c) { return c == 0 ? 3072u : c == 1 ? 6144u : 12288u; }
 // One line gives a tile at most two fills (the walk visits a tile once, with at most one
 // extra fill for a vertical crossing), so with at most 2^22 lines per CTA-binned path the
-// 24-bit counters cannot carry into the delta byte.
-constexpr uint32_t kCtaMaxLeaves = 1u << 22;
+// 24-bit counters cannot carry into the delta byte (kCtaMaxLeaves).
 // bin_ctl slots: paths per CTA class, work tickets per CTA class, tickets of the class-3
 // zeroing and set-up passes, and at slot 12 a 64-bit word: class-3 paths << 40 | their lines.
 enum : int { kCtlCount = 0, kCtlTicket = 4, kCtlTicketZero = 8, kCtlTicketPrep = 9, kCtl3 = 12 };
@@ -1402,13 +1404,27 @@ __device__ __forceinline__ unsigned long long *fill_total(const Batch &b) {
     return reinterpret_cast<unsigned long long *>(b.status + kStFill64);
 }
 
-// -1: no columns (nothing can land); 0-2: CTA classes; 3: global passes
-__device__ __forceinline__ int path_class(const PathDev &P, uint32_t leaves) {
+// -1: no columns (nothing can land); 0-2: CTA classes; 3: global passes.  A CTA class holds the path's
+// words; a larger one is taken where the smaller one's warps would have to walk more than
+// warp_lines lines each (bin_warp_lines).
+__device__ __forceinline__ int path_class(const PathDev &P, uint32_t leaves, uint32_t warp_lines) {
     const int32_t rw = max(P.rx1 - P.rx0, 0), rh = max(P.ry1 - P.ry0, 0);
     if (rw == 0) return -1;
     if (leaves > kCtaMaxLeaves) return 3;
     const uint32_t words = (uint32_t)rw * (uint32_t)rh + (uint32_t)rw;
-    return words <= class_words(0) ? 0 : words <= class_words(1) ? 1 : words <= class_words(2) ? 2 : 3;
+    if (words > class_words(2)) return 3;
+    int c = words <= class_words(0) ? 0 : words <= class_words(1) ? 1 : 2;
+    if (c == 0 && leaves > class_threads(0) / 32 * warp_lines) c = 1;
+    if (c == 1 && leaves > class_threads(1) / 32 * warp_lines) c = 2;
+    return c;
+}
+
+// The lines a warp would get if the frame's were spread evenly over the binning warps the GPU holds
+// (36 per SM), at least 64 (two rounds).  A path of far more lines for its size than that - a
+// dashed outline, or any path of a frame too small to fill the GPU - is the frame's critical path,
+// so it gets a CTA of more warps.
+__device__ __forceinline__ uint32_t bin_warp_lines(const Batch &b, bool learned) {
+    return max(64u, b.status[learned ? kStLeafCount : kStLeaves] / (36u * b.n_sms));
 }
 
 // The leaf lines of one path: its region of the leaf buffer, then (learned frame) its lines
@@ -1491,7 +1507,7 @@ __global__ void k_bin_classify(Batch b, bool learned) {
         b.path_leaf_range[p] = range;
         uint32_t n = range.y - range.x;
         if (b.pool_cnt) n += b.pool_cnt[p] - b.pool_cnt[(int64_t)p - 1];
-        cls = path_class(P, n);
+        cls = path_class(P, n, bin_warp_lines(b, learned));
         b.path_cls[p] = (uint8_t)cls;
         if (cls < 0) b.path_fill[p] = 0;
         if (cls == 3) {
@@ -2822,17 +2838,19 @@ cudaError_t bin_class_max_ctas(int out[3]) {
     return cudaSuccess;
 }
 
-// Class 3 (zero, count, backdrops and offsets, write; each returns at once when the class is
-// empty), then the CTA classes, largest rects first.
-cudaError_t launch_bin_paths(const Batch &b, const Tuning &t, const BinStreams *bs, cudaStream_t st) {
+// Class 3 when it can have paths (zero, count, backdrops and offsets, write), then the CTA classes,
+// largest rects first.
+cudaError_t launch_bin_paths(const Batch &b, const Tuning &t, bool large, const BinStreams *bs, cudaStream_t st) {
     if (!b.n_paths) return cudaSuccess;
     int dev = 0, sms = 152;
     cudaGetDevice(&dev);
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-    PF_LAUNCH(k_bin_zero_large<<<sms * 2, 256, 0, st>>>(b));
-    PF_LAUNCH(k_bin_large<false><<<sms * 8, kThreads, 0, st>>>(b));
-    PF_LAUNCH(k_bin_large_prep<<<sms * 2, kPrepThreads, 0, st>>>(b));
-    PF_LAUNCH(k_bin_large<true><<<sms * 8, kThreads, 0, st>>>(b));
+    if (large) {
+        PF_LAUNCH(k_bin_zero_large<<<sms * 2, 256, 0, st>>>(b));
+        PF_LAUNCH(k_bin_large<false><<<sms * 8, kThreads, 0, st>>>(b));
+        PF_LAUNCH(k_bin_large_prep<<<sms * 2, kPrepThreads, 0, st>>>(b));
+        PF_LAUNCH(k_bin_large<true><<<sms * 8, kThreads, 0, st>>>(b));
+    }
     cudaError_t e;
     if (!t.bin_concurrent || !bs) {
         if ((e = launch_fused<2>(b, t.bin_ctas_per_sm[2], st)) != cudaSuccess) return e;

@@ -193,19 +193,6 @@ __device__ __forceinline__ bool svalid(const Seg &s) {  // :189-200
     if (s.kind == kQuad || s.kind == kCubic) return lfinite(s.b) && lfinite(s.c);
     return false;
 }
-__device__ float sarc_length(const Seg &s) {  // :141-187 (quadratics through to_cubic)
-    if (s.kind == kLine) return vlen(lvec(s.b));
-    if (s.kind != kQuad && s.kind != kCubic) return 0.0f;
-    LSeg c = s.c;
-    if (s.kind == kQuad) {
-        const V2 p1_2 = vadd(s.c.f, s.c.f);
-        const V2 c0 = vadd(s.b.f, p1_2), c1 = vadd(p1_2, s.b.t);
-        c = ls(mk(fd(c0.x, 3.0f), fd(c0.y, 3.0f)), mk(fd(c1.x, 3.0f), fd(c1.y, 3.0f)));
-    }
-    const float chord = vlen(lvec(s.b));
-    const float net = fa(fa(vlen(vsub(s.b.f, c.f)), vlen(lvec(c))), vlen(vsub(s.b.t, c.t)));
-    return fm(fa(net, chord), 0.5f);
-}
 __device__ __forceinline__ Seg quarter_arc() {  // :202-211
     const float r2 = fsqrt(2.0f);
     const V2 p0 = mk(fm(r2, 0.5f), fm(r2, 0.5f));
@@ -561,7 +548,7 @@ __device__ __forceinline__ uint2 path_contours(const StrokeIn &in, uint32_t p) {
 // path per lane, 2.30 ms with a warp per path walked by one lane, 1.83 by all.)
 
 // Segment::arc_length (core/data/segment.cpp:141-187) of a segment all lanes hold; lane l % 4 takes
-// leg l of the control polygon, with sarc_length's operations.
+// leg l of the control polygon (quadratics through to_cubic).
 __device__ __forceinline__ float warp_arc_length(const Seg &s) {
     if (s.kind == kLine) return vlen(lvec(s.b));
     const int l = threadIdx.x & 3;
