@@ -335,7 +335,8 @@ typedef struct pf_tuning {
                                     whose rect plus a row of column sums takes <= 1088, 4352,
                                     16896 words); 0: as many as fit */
     float long_line;             /* lines spanning more tiles than this are walked by a whole warp */
-    uint32_t bin_concurrent;     /* 1: the three binning classes run at once on side streams */
+    uint32_t bin_concurrent;     /* 1: the binning classes always run at once, on side streams; 0: they do
+                                    where several classes have paths and the frame is not too long */
     uint32_t seg_sorted;         /* 0 or 1; changes nothing (segments are no longer ordered by depth) */
     uint32_t composite_ticket;   /* 0: the composite runs a warp per framebuffer tile; n > 0: its warps
                                     stay resident and take n consecutive tiles per ticket from a

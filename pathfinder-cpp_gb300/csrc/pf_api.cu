@@ -1049,7 +1049,7 @@ int begin_frame(Ctx *c, uint32_t first, uint32_t count) {
     PF_CUDA(c->bin_list.ensure(size_t(N) * 20 + 16));
     PF_CUDA(c->path_fill.ensure(size_t(N) * 4 + 16));
     PF_CUDA(c->path_seg_first.ensure(size_t(N) * 4 + 16));
-    PF_CUDA(bin_stage_slots(c->tune, &c->stage_slots));
+    PF_CUDA(bin_stage_slots(c->tune, c->n_sms, c->r_paths, &c->stage_slots));
     PF_CUDA(c->bin_stage.ensure(c->stage_slots * 12));
     PF_CUDA(c->path_cls.ensure(size_t(N) + 16));
     PF_CUDA(c->bin_ctl.ensure(1024));
@@ -1119,19 +1119,26 @@ int stage_setup(Ctx *c, bool learned) {
 // counted to the exact total, the buffer grows, and binning and composite run again.  Ends
 // with the status words read back.  max_leaves: the most leaf lines a path can have.
 int bin_and_composite(Ctx *c, Batch b, bool learned, uint64_t max_leaves) {
-    const bool large = c->h_status[kStLargeRects] != 0 || max_leaves > kCtaMaxLeaves;
+    const uint32_t *rects = c->h_status + kStRectClass;
+    const bool large = rects[3] != 0 || max_leaves > kCtaMaxLeaves;
+    // the binning classes at once where several have paths (20,000 paths 1607 -> 1497 us, mixed 8,192
+    // paths 1456 -> 1247 us, stroked batch 3.10 -> 2.63 ms), but not in frames so long that their
+    // tails no longer count (256 scenes, 178,734 paths, 13.43 -> 13.45 ms); the forks and joins cost
+    // 10 to 15 us (150,000 glyphs, all of one class, 1219 -> 1233 us)
+    const bool several = (rects[0] != 0) + (rects[1] != 0) + (rects[2] != 0) + large > 1;
+    const bool at_once = c->tune.bin_concurrent || (several && c->r_paths <= 1u << 16);
     cudaStream_t st = c->stream;
     for (int attempt = 0;; attempt++) {
         PF_CUDA(cudaMemsetAsync(b.bin_ctl, 0, 1024, st));
         PF_CUDA(cudaMemsetAsync(b.status + kStFill64, 0, 8, st));
         PF_CUDA(launch_bin_classify(b, learned, st));
-        if (c->tune.bin_concurrent && !c->bs_ready) {
+        if (at_once && !c->bs_ready) {
             for (auto &s : c->bs.side) PF_CUDA(cudaStreamCreateWithFlags(&s, cudaStreamNonBlocking));
             PF_CUDA(cudaEventCreateWithFlags(&c->bs.fork, cudaEventDisableTiming));
             for (auto &e : c->bs.join) PF_CUDA(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
             c->bs_ready = true;
         }
-        PF_CUDA(launch_bin_paths(b, c->tune, large, c->bs_ready ? &c->bs : nullptr, st));
+        PF_CUDA(launch_bin_paths(b, c->tune, large, at_once ? &c->bs : nullptr, st));
         record(c, 3);
         record(c, 4);
         record(c, 5);

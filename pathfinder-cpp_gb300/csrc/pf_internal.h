@@ -188,7 +188,7 @@ struct Batch {
 struct Tuning {
     uint32_t bin_ctas_per_sm[3] = {0, 0, 0};  // 0: as many as fit
     float long_line = 8.0f;
-    bool bin_concurrent = false;
+    bool bin_concurrent = false;  // true: the binning classes always run at once
     bool seg_sorted = true;  // kept for pf_tuning; changes nothing
     uint32_t comp_ticket = 0;
 };
@@ -219,8 +219,8 @@ enum : int {
     kStSampled = 22,   // segments of the contours sampled for their depth, and the deep ones of them
     kStSampledDeep = 23,
     kStDashChunks = 24,// upload: chunks of dashed points taken
-    kStLargeRects = 25,// nonzero: a path's rect takes the binning's global passes
-    kStCount = 26,
+    kStRectClass = 25, // four words: nonzero if a path's rect asks for that binning class
+    kStCount = 29,
 };
 
 // Kernels launched by this library (host-side counter, all contexts).
@@ -341,8 +341,7 @@ cudaError_t launch_flatten_budget(const Batch &b, uint32_t n_segs, cudaStream_t 
 // backdrops, fill offsets, fills).  A learned frame first lists its pooled lines by path:
 // count, scan pool_cnt, scatter.
 cudaError_t launch_bin_classify(const Batch &b, bool learned, cudaStream_t st);
-// side[0..1], fork, join[0..1]: streams and events for running the CTA classes concurrently
-// (tuning.bin_concurrent), or null.
+// side[0..1], fork, join[0..1]: streams and events for running the classes at once, or null.
 struct BinStreams {
     cudaStream_t side[2];
     cudaEvent_t fork, join[2];
@@ -353,7 +352,7 @@ cudaError_t launch_bin_paths(const Batch &b, const Tuning &t, bool large, const 
 cudaError_t bin_class_max_ctas(int out[3]);
 cudaError_t launch_pool_lists(const Batch &b, bool scatter, cudaStream_t st);
 // Slots of the binning CTAs' stage on the current device for these launch parameters.
-cudaError_t bin_stage_slots(const Tuning &t, size_t *slots);
+cudaError_t bin_stage_slots(const Tuning &t, uint32_t n_sms, uint32_t n_paths, size_t *slots);
 cudaError_t launch_mlp_predict(const __nv_bfloat16 *w, const float *feat, uint32_t n, float *out, cudaStream_t st);
 cudaError_t launch_mlp_grad(const __nv_bfloat16 *w, const float *feat, const float *target, const uint32_t *index,
                             uint32_t n, float *grad, float *loss, cudaStream_t st);

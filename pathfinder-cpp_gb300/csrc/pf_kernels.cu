@@ -34,6 +34,10 @@ namespace {
 constexpr int kThreads = 256;
 // Shared words of the binning's CTA classes (see "Binning by path").
 __host__ __device__ constexpr uint32_t class_words(int c) { return c == 0 ? 1088u : c == 1 ? 4352u : 16896u; }
+// The class that holds a rect of that many words; 3: none (global passes).
+__device__ __forceinline__ int rect_class(uint64_t words) {
+    return words <= class_words(0) ? 0 : words <= class_words(1) ? 1 : words <= class_words(2) ? 2 : 3;
+}
 
 __device__ __forceinline__ float fadd(float a, float b) { return __fadd_rn(a, b); }
 __device__ __forceinline__ float fsub(float a, float b) { return __fsub_rn(a, b); }
@@ -106,10 +110,9 @@ __global__ void k_normalize_paths(Batch b, uint2 *path_contours) {
 // round_rect_out_to_tile_bounds (pathfinder/core/data/data.h:131-133), Tiler::Tiler
 // (pathfinder/core/d3d9/tiler.cpp:317-335).
 
-__global__ void k_path_setup(Batch b, const uint2 *path_contours) {
-    const uint32_t p = global_tid() >> 5;
-    const int lane = threadIdx.x & 31;
-    if (p >= b.n_paths) return;
+// One warp: the path's bounds and tile rect; in lane 0 the binning class its rect asks for (-1: no
+// columns).
+__device__ __forceinline__ int path_rect(const Batch &b, const uint2 *path_contours, uint32_t p, int lane) {
     const uint2 cr = path_contours[p];
     const uint32_t a = b.contour_point_first[cr.x], e = b.contour_point_first[cr.y];
     float l = INFINITY, t = INFINITY, r = -INFINITY, bt = -INFINITY;
@@ -130,7 +133,7 @@ __global__ void k_path_setup(Batch b, const uint2 *path_contours) {
         bt = fmaxf(bt, __shfl_xor_sync(0xffffffffu, bt, d));
     }
     bad = __any_sync(0xffffffffu, bad);
-    if (lane != 0) return;
+    if (lane != 0) return -1;
     if (bad) atomicOr(&b.status[kStErr], kErrNonFinite);
     PathDev P = b.paths[p];
     const SceneDev &S = b.scenes[P.scene];
@@ -163,8 +166,21 @@ __global__ void k_path_setup(Batch b, const uint2 *path_contours) {
     b.paths[p] = P;
     b.path_tiles[p] = (uint32_t)(w * h);
     b.path_cols[p] = (uint32_t)w;
-    // a rect for the binning's global passes: the host leaves them out of frames without one
-    if ((uint64_t)w * (uint32_t)(h + 1) > class_words(2)) b.status[kStLargeRects] = 1;
+    return w ? rect_class((uint32_t)w * (uint64_t)(uint32_t)(h + 1)) : -1;
+}
+
+__global__ void k_path_setup(Batch b, const uint2 *path_contours) {
+    __shared__ uint32_t s_classes;  // a bit per binning class by rect (0-3) among the block's paths
+    const uint32_t p = blockIdx.x * (kThreads / 32) + (threadIdx.x >> 5);
+    const int lane = threadIdx.x & 31;
+    if (threadIdx.x == 0) s_classes = 0;
+    __syncthreads();
+    if (p < b.n_paths) {
+        const int c = path_rect(b, path_contours, p, lane);
+        if (lane == 0 && c >= 0) atomicOr(&s_classes, 1u << c);
+    }
+    __syncthreads();
+    if (threadIdx.x < 4 && (s_classes >> threadIdx.x & 1u)) b.status[kStRectClass + threadIdx.x] = 1;
 }
 
 __global__ void k_path_offsets(Batch b) {
@@ -1411,9 +1427,7 @@ __device__ __forceinline__ int path_class(const PathDev &P, uint32_t leaves, uin
     const int32_t rw = max(P.rx1 - P.rx0, 0), rh = max(P.ry1 - P.ry0, 0);
     if (rw == 0) return -1;
     if (leaves > kCtaMaxLeaves) return 3;
-    const uint32_t words = (uint32_t)rw * (uint32_t)rh + (uint32_t)rw;
-    if (words > class_words(2)) return 3;
-    int c = words <= class_words(0) ? 0 : words <= class_words(1) ? 1 : 2;
+    int c = rect_class((uint64_t)rw * (uint32_t)(rh + 1));
     if (c == 0 && leaves > class_threads(0) / 32 * warp_lines) c = 1;
     if (c == 1 && leaves > class_threads(1) / 32 * warp_lines) c = 2;
     return c;
@@ -2711,7 +2725,7 @@ cudaError_t launch_normalize(const Batch &b, uint2 *path_contours, cudaStream_t 
 }
 
 cudaError_t launch_path_setup(const Batch &b, const uint2 *path_contours, cudaStream_t st) {
-    if (b.n_paths) PF_LAUNCH(k_path_setup<<<grid_for(uint64_t(b.n_paths) * 32), kThreads, 0, st>>>(b, path_contours));
+    if (b.n_paths) PF_LAUNCH(k_path_setup<<<grid_for(b.n_paths, kThreads / 32), kThreads, 0, st>>>(b, path_contours));
     return cudaGetLastError();
 }
 
@@ -2779,102 +2793,98 @@ cudaError_t launch_bin_classify(const Batch &b, bool learned, cudaStream_t st) {
     return cudaGetLastError();
 }
 
-// Grid of a CTA class: as many CTAs as fit on every SM (they take paths by ticket), or
-// per_sm_wanted per SM when that is nonzero and fits.
+// CTAs of a class that one SM holds.
 template <int kCls>
-static cudaError_t fused_grid(unsigned *grid, uint32_t per_sm_wanted = 0) {
+static cudaError_t fused_per_sm(int *per_sm) {
     const size_t smem = size_t(class_words(kCls)) * 4;
-    static int configured_device = -1;
-    int dev = 0, sms = 152;
-    cudaGetDevice(&dev);
-    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-    if (configured_device != dev) {
-        const cudaError_t e =
-            cudaFuncSetAttribute(k_bin_fused<kCls>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-        if (e != cudaSuccess) return e;
-        configured_device = dev;
-    }
-    int per_sm = 0;
-    const cudaError_t e =
-        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_bin_fused<kCls>, class_threads(kCls), smem);
+    static std::atomic<uint64_t> configured{0};  // devices the kernel's shared memory is set up on, and
+    static std::atomic<int> known[64];           // what fits there
+    int dev = 0;
+    cudaError_t e = cudaGetDevice(&dev);
     if (e != cudaSuccess) return e;
-    per_sm = std::max(1, per_sm);
+    if (dev < 64 && (configured.load() >> dev & 1u)) {
+        *per_sm = known[dev].load();
+        return cudaSuccess;
+    }
+    e = cudaFuncSetAttribute(k_bin_fused<kCls>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    if (e != cudaSuccess) return e;
+    e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(per_sm, k_bin_fused<kCls>, class_threads(kCls), smem);
+    if (e != cudaSuccess) return e;
+    *per_sm = std::max(1, *per_sm);
+    if (dev < 64) {
+        known[dev].store(*per_sm);
+        configured.fetch_or(uint64_t(1) << dev);
+    }
+    return cudaSuccess;
+}
+
+// Grid of a CTA class: as many CTAs as fit on every SM (they take paths by ticket), or
+// per_sm_wanted per SM when that is nonzero and fits; no more than there are paths.
+template <int kCls>
+static cudaError_t fused_grid(unsigned *grid, uint32_t n_sms, uint32_t n_paths, uint32_t per_sm_wanted) {
+    int per_sm = 0;
+    const cudaError_t e = fused_per_sm<kCls>(&per_sm);
+    if (e != cudaSuccess) return e;
     if (per_sm_wanted) per_sm = std::min(per_sm, (int)per_sm_wanted);
-    *grid = (unsigned)per_sm * (unsigned)sms;
+    *grid = std::min((unsigned)per_sm * n_sms, std::max(n_paths, 1u));
     return cudaSuccess;
 }
 
 template <int kCls>
-static cudaError_t launch_fused(const Batch &b, uint32_t per_sm, cudaStream_t st) {
-    unsigned grid = 0;
-    const cudaError_t e = fused_grid<kCls>(&grid, per_sm);
-    if (e != cudaSuccess) return e;
-    PF_LAUNCH(k_bin_fused<kCls><<<grid, class_threads(kCls), size_t(class_words(kCls)) * 4, st>>>(b));
+static cudaError_t launch_fused(const Batch &b, unsigned grid, size_t stage_first, cudaStream_t st) {
+    Batch c = b;
+    c.stage += stage_first;
+    c.stage_tile += stage_first;
+    PF_LAUNCH(k_bin_fused<kCls><<<grid, class_threads(kCls), size_t(class_words(kCls)) * 4, st>>>(c));
     return cudaGetLastError();
 }
 
-cudaError_t bin_stage_slots(const Tuning &t, size_t *slots) {
-    unsigned g0 = 0, g1 = 0, g2 = 0;
-    cudaError_t e;
-    if ((e = fused_grid<0>(&g0, t.bin_ctas_per_sm[0])) != cudaSuccess) return e;
-    if ((e = fused_grid<1>(&g1, t.bin_ctas_per_sm[1])) != cudaSuccess) return e;
-    if ((e = fused_grid<2>(&g2, t.bin_ctas_per_sm[2])) != cudaSuccess) return e;
-    const size_t s0 = size_t(g0) * class_stage(0), s1 = size_t(g1) * class_stage(1), s2 = size_t(g2) * class_stage(2);
-    // concurrent classes each keep their own slice of the stage
-    *slots = t.bin_concurrent ? s0 + s1 + s2 : std::max({s0, s1, s2});
+static cudaError_t fused_grids(const Tuning &t, uint32_t n_sms, uint32_t n_paths, unsigned g[3]) {
+    cudaError_t e = fused_grid<0>(&g[0], n_sms, n_paths, t.bin_ctas_per_sm[0]);
+    if (e == cudaSuccess) e = fused_grid<1>(&g[1], n_sms, n_paths, t.bin_ctas_per_sm[1]);
+    if (e == cudaSuccess) e = fused_grid<2>(&g[2], n_sms, n_paths, t.bin_ctas_per_sm[2]);
+    return e;
+}
+
+// The classes' slices of the stage follow each other, largest class first: they may run at once.
+cudaError_t bin_stage_slots(const Tuning &t, uint32_t n_sms, uint32_t n_paths, size_t *slots) {
+    unsigned g[3];
+    if (const cudaError_t e = fused_grids(t, n_sms, n_paths, g)) return e;
+    *slots = size_t(g[0]) * class_stage(0) + size_t(g[1]) * class_stage(1) + size_t(g[2]) * class_stage(2);
     return cudaSuccess;
 }
 
 cudaError_t bin_class_max_ctas(int out[3]) {
-    unsigned g[3];
-    cudaError_t e;
-    if ((e = fused_grid<0>(&g[0])) != cudaSuccess) return e;
-    if ((e = fused_grid<1>(&g[1])) != cudaSuccess) return e;
-    if ((e = fused_grid<2>(&g[2])) != cudaSuccess) return e;
-    int dev = 0, sms = 152;
-    cudaGetDevice(&dev);
-    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-    for (int c = 0; c < 3; c++) out[c] = (int)(g[c] / (unsigned)sms);
-    return cudaSuccess;
+    cudaError_t e = fused_per_sm<0>(&out[0]);
+    if (e == cudaSuccess) e = fused_per_sm<1>(&out[1]);
+    if (e == cudaSuccess) e = fused_per_sm<2>(&out[2]);
+    return e;
 }
 
-// Class 3 when it can have paths (zero, count, backdrops and offsets, write), then the CTA classes,
-// largest rects first.
+// Class 3 when it can have paths (zero, count, backdrops and offsets, write), and the CTA classes,
+// largest rects first; at once (bs not null) on streams of their own, joined before the composite,
+// so that the block scheduler fills the SMs that one class's last paths leave idle with the others'.
 cudaError_t launch_bin_paths(const Batch &b, const Tuning &t, bool large, const BinStreams *bs, cudaStream_t st) {
     if (!b.n_paths) return cudaSuccess;
-    int dev = 0, sms = 152;
-    cudaGetDevice(&dev);
-    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+    unsigned g[3];
+    cudaError_t e = fused_grids(t, b.n_sms, b.n_paths, g);
+    if (e != cudaSuccess) return e;
+    if (bs) {
+        if ((e = cudaEventRecord(bs->fork, st)) != cudaSuccess) return e;
+        for (int k = 0; k < 2; k++)
+            if ((e = cudaStreamWaitEvent(bs->side[k], bs->fork, 0)) != cudaSuccess) return e;
+    }
     if (large) {
-        PF_LAUNCH(k_bin_zero_large<<<sms * 2, 256, 0, st>>>(b));
-        PF_LAUNCH(k_bin_large<false><<<sms * 8, kThreads, 0, st>>>(b));
-        PF_LAUNCH(k_bin_large_prep<<<sms * 2, kPrepThreads, 0, st>>>(b));
-        PF_LAUNCH(k_bin_large<true><<<sms * 8, kThreads, 0, st>>>(b));
+        PF_LAUNCH(k_bin_zero_large<<<b.n_sms * 2, 256, 0, st>>>(b));
+        PF_LAUNCH(k_bin_large<false><<<b.n_sms * 8, kThreads, 0, st>>>(b));
+        PF_LAUNCH(k_bin_large_prep<<<b.n_sms * 2, kPrepThreads, 0, st>>>(b));
+        PF_LAUNCH(k_bin_large<true><<<b.n_sms * 8, kThreads, 0, st>>>(b));
     }
-    cudaError_t e;
-    if (!t.bin_concurrent || !bs) {
-        if ((e = launch_fused<2>(b, t.bin_ctas_per_sm[2], st)) != cudaSuccess) return e;
-        if ((e = launch_fused<1>(b, t.bin_ctas_per_sm[1], st)) != cudaSuccess) return e;
-        return launch_fused<0>(b, t.bin_ctas_per_sm[0], st);
-    }
-    // the three classes at once: classes 1 and 0 on side streams, each with its own slice of
-    // the fill stage (the classes' grids follow each other in it), joined back before the
-    // composite; the block scheduler fills the SMs a class's tail leaves idle with the others
-    unsigned g2 = 0, g1 = 0;
-    if ((e = fused_grid<2>(&g2, t.bin_ctas_per_sm[2])) != cudaSuccess) return e;
-    if ((e = fused_grid<1>(&g1, t.bin_ctas_per_sm[1])) != cudaSuccess) return e;
-    if ((e = cudaEventRecord(bs->fork, st)) != cudaSuccess) return e;
-    for (int k = 0; k < 2; k++)
-        if ((e = cudaStreamWaitEvent(bs->side[k], bs->fork, 0)) != cudaSuccess) return e;
-    Batch b1 = b, b0 = b;
-    b1.stage = b.stage + size_t(g2) * class_stage(2);
-    b0.stage = b1.stage + size_t(g1) * class_stage(1);
-    b1.stage_tile = b.stage_tile + size_t(g2) * class_stage(2);
-    b0.stage_tile = b1.stage_tile + size_t(g1) * class_stage(1);
-    if ((e = launch_fused<2>(b, t.bin_ctas_per_sm[2], st)) != cudaSuccess) return e;
-    if ((e = launch_fused<1>(b1, t.bin_ctas_per_sm[1], bs->side[0])) != cudaSuccess) return e;
-    if ((e = launch_fused<0>(b0, t.bin_ctas_per_sm[0], bs->side[1])) != cudaSuccess) return e;
-    for (int k = 0; k < 2; k++) {
+    const size_t s1 = size_t(g[2]) * class_stage(2), s0 = s1 + size_t(g[1]) * class_stage(1);
+    if ((e = launch_fused<2>(b, g[2], 0, bs ? bs->side[0] : st)) != cudaSuccess) return e;
+    if ((e = launch_fused<1>(b, g[1], s1, st)) != cudaSuccess) return e;
+    if ((e = launch_fused<0>(b, g[0], s0, bs ? bs->side[1] : st)) != cudaSuccess) return e;
+    for (int k = 0; bs && k < 2; k++) {
         if ((e = cudaEventRecord(bs->join[k], bs->side[k])) != cudaSuccess) return e;
         if ((e = cudaStreamWaitEvent(st, bs->join[k], 0)) != cudaSuccess) return e;
     }
