@@ -34,9 +34,12 @@ namespace {
 constexpr int kThreads = 256;
 // Shared words of the binning's CTA classes (see "Binning by path").
 __host__ __device__ constexpr uint32_t class_words(int c) { return c == 0 ? 1088u : c == 1 ? 4352u : 16896u; }
+constexpr uint32_t kSmallWords = 128;  // of the class binned by a warp
+constexpr int kSmallClass = kRectSmall;
 // The class that holds a rect of that many words; 3: none (global passes).
 __device__ __forceinline__ int rect_class(uint64_t words) {
-    return words <= class_words(0) ? 0 : words <= class_words(1) ? 1 : words <= class_words(2) ? 2 : 3;
+    return words <= kSmallWords ? kSmallClass
+           : words <= class_words(0) ? 0 : words <= class_words(1) ? 1 : words <= class_words(2) ? 2 : 3;
 }
 
 __device__ __forceinline__ float fadd(float a, float b) { return __fadd_rn(a, b); }
@@ -170,7 +173,7 @@ __device__ __forceinline__ int path_rect(const Batch &b, const uint2 *path_conto
 }
 
 __global__ void k_path_setup(Batch b, const uint2 *path_contours) {
-    __shared__ uint32_t s_classes;  // a bit per binning class by rect (0-3) among the block's paths
+    __shared__ uint32_t s_classes;  // a bit per binning class by rect among the block's paths
     const uint32_t p = blockIdx.x * (kThreads / 32) + (threadIdx.x >> 5);
     const int lane = threadIdx.x & 31;
     if (threadIdx.x == 0) s_classes = 0;
@@ -180,7 +183,7 @@ __global__ void k_path_setup(Batch b, const uint2 *path_contours) {
         if (lane == 0 && c >= 0) atomicOr(&s_classes, 1u << c);
     }
     __syncthreads();
-    if (threadIdx.x < 4 && (s_classes >> threadIdx.x & 1u)) b.status[kStRectClass + threadIdx.x] = 1;
+    if (threadIdx.x <= kSmallClass && (s_classes >> threadIdx.x & 1u)) b.status[kStRectClass + threadIdx.x] = 1;
 }
 
 __global__ void k_path_offsets(Batch b) {
@@ -1406,12 +1409,27 @@ __host__ __device__ constexpr uint32_t class_stage(int c) { return c == 0 ? 3072
 // bin_ctl slots: paths per CTA class, work tickets per CTA class, tickets of the class-3
 // zeroing and set-up passes, and at slot 12 a 64-bit word: class-3 paths << 40 | their lines.
 enum : int { kCtlCount = 0, kCtlTicket = 4, kCtlTicketZero = 8, kCtlTicketPrep = 9, kCtl3 = 12 };
-// and from slot 16 the CTA classes' paths counted by log2 of their leaf lines (3 x 32), then
-// the write cursors of those buckets (3 x 32): each class's list runs from its largest paths to
-// its smallest, so the last CTAs to start take the shortest paths
-enum : int { kCtlBucket = 16, kCtlCursor = 16 + 3 * 32, kCtlWords = 16 + 6 * 32, kCtlCompTicket = kCtlWords };
-static_assert((kCtlCompTicket + 1) * 4 <= 1024, "bin_ctl holds 1024 bytes");
+// and from slot 16 the listed classes' paths (the CTA classes, then the small one) counted by log2 of
+// their leaf lines (4 x 32), then the write cursors of those buckets (4 x 32): each class's list runs
+// from its largest paths to its smallest, so the last to start take the shortest paths
+constexpr int kLists = kCtaClasses + 1;
+enum : int {
+    kCtlBucket = 16,
+    kCtlCursor = 16 + kLists * 32,
+    kCtlWords = 16 + 2 * kLists * 32,
+    kCtlCompTicket = kCtlWords
+};
+static_assert((kCtlCompTicket + 1) * 4 <= kBinCtlBytes, "bin_ctl is too small");
+// The list of a class (-1: none, class 3 has its own); list 3 lies behind class 3's two rows.
+__device__ __forceinline__ int class_list(int cls) {
+    return cls == kSmallClass ? kCtaClasses : cls < kCtaClasses ? cls : -1;
+}
+__device__ __forceinline__ uint32_t *list_row(const Batch &b, int list) {
+    return b.bin_list + (size_t)(list < kCtaClasses ? list : 5) * b.n_paths;
+}
 constexpr uint64_t kLow40 = (1ull << 40) - 1;
+
+constexpr uint32_t kSmallLines = 384;  // most lines of a path that a warp bins
 
 __device__ __forceinline__ unsigned long long *ctl3_word(const Batch &b) {
     return reinterpret_cast<unsigned long long *>(b.bin_ctl + kCtl3);
@@ -1420,14 +1438,15 @@ __device__ __forceinline__ unsigned long long *fill_total(const Batch &b) {
     return reinterpret_cast<unsigned long long *>(b.status + kStFill64);
 }
 
-// -1: no columns (nothing can land); 0-2: CTA classes; 3: global passes.  A CTA class holds the path's
-// words; a larger one is taken where the smaller one's warps would have to walk more than
-// warp_lines lines each (bin_warp_lines).
+// -1: no columns (nothing can land); kSmallClass: a warp; 0-2: CTA classes; 3: global passes.  A
+// class holds the path's words; a larger one is taken where the smaller one's warps would have to
+// walk more than warp_lines lines each (bin_warp_lines), and a warp takes no more than it can stage.
 __device__ __forceinline__ int path_class(const PathDev &P, uint32_t leaves, uint32_t warp_lines) {
     const int32_t rw = max(P.rx1 - P.rx0, 0), rh = max(P.ry1 - P.ry0, 0);
     if (rw == 0) return -1;
     if (leaves > kCtaMaxLeaves) return 3;
     int c = rect_class((uint64_t)rw * (uint32_t)(rh + 1));
+    if (c == kSmallClass && leaves > min(warp_lines, kSmallLines)) c = 0;
     if (c == 0 && leaves > class_threads(0) / 32 * warp_lines) c = 1;
     if (c == 1 && leaves > class_threads(1) / 32 * warp_lines) c = 2;
     return c;
@@ -1531,21 +1550,22 @@ __global__ void k_bin_classify(Batch b, bool learned) {
             b.bin_list[(size_t)4 * b.n_paths + item] = (uint32_t)(old & kLow40);
         }
     }
+    const int list = class_list(cls);
 #pragma unroll
-    for (int c = 0; c < kCtaClasses; c++) {
-        const uint32_t m = __ballot_sync(0xffffffffu, cls == c);
+    for (int c = 0; c < kLists; c++) {
+        const uint32_t m = __ballot_sync(0xffffffffu, list == c);
         if (m && lane == __ffs(m) - 1) atomicAdd(&b.bin_ctl[kCtlCount + c], (uint32_t)__popc(m));
     }
-    // the bucket of a CTA-class path: log2 of its leaf lines
-    const int key = cls >= 0 && cls < kCtaClasses ? cls * 32 + bin_bucket(b, p) : -1;
+    // the bucket of a listed path: log2 of its leaf lines
+    const int key = list >= 0 ? list * 32 + bin_bucket(b, p) : -1;
     const unsigned g = __match_any_sync(0xffffffffu, key);
     if (key >= 0 && lane == __ffs(g) - 1) atomicAdd(&b.bin_ctl[kCtlBucket + key], (uint32_t)__popc(g));
 }
 
-// The buckets' cursors, largest lines first within each class.
+// The buckets' cursors, largest lines first within each list.
 __global__ void k_bin_bucket_starts(Batch b) {
     const int c = threadIdx.x;
-    if (c >= kCtaClasses) return;
+    if (c >= kLists) return;
     uint32_t off = 0;
     for (int k = 31; k >= 0; k--) {
         b.bin_ctl[kCtlCursor + c * 32 + k] = off;
@@ -1553,14 +1573,14 @@ __global__ void k_bin_bucket_starts(Batch b) {
     }
 }
 
-// Each CTA-class path into its class list at its bucket's cursor.
+// Each listed path into its list at its bucket's cursor.
 __global__ void k_bin_scatter(Batch b) {
     const uint32_t p = global_tid();
     const int lane = threadIdx.x & 31;
     int key = -1;
     if (p < b.n_paths) {
-        const int cls = (int)(int8_t)b.path_cls[p];
-        if (cls >= 0 && cls < kCtaClasses) key = cls * 32 + bin_bucket(b, p);
+        const int list = class_list((int)(int8_t)b.path_cls[p]);
+        if (list >= 0) key = list * 32 + bin_bucket(b, p);
     }
     const unsigned g = __match_any_sync(0xffffffffu, key);
     if (key < 0) return;
@@ -1568,7 +1588,7 @@ __global__ void k_bin_scatter(Batch b) {
     uint32_t base = 0;
     if (lane == leader) base = atomicAdd(&b.bin_ctl[kCtlCursor + key], (uint32_t)__popc(g));
     base = __shfl_sync(g, base, leader);
-    b.bin_list[(size_t)(key >> 5) * b.n_paths + base + __popc(g & ((1u << lane) - 1u))] = p;
+    list_row(b, key >> 5)[base + __popc(g & ((1u << lane) - 1u))] = p;
 }
 
 // The fills of one tile visit, as a binning warp stages them: the visit's points and a word with
@@ -1797,6 +1817,159 @@ __global__ void __launch_bounds__(class_threads(kCls), class_min_ctas(kCls)) k_b
             }
         }
         __syncthreads();
+    }
+}
+
+// The small class: one warp bins a path, as k_bin_fused does with a CTA.  A glyph's path has some 60
+// lines and 10 tiles; a CTA spends most of its time on it in barriers and in waiting for the path's
+// record, while warps on paths of their own have no barriers and wait side by side.  Visits are
+// staged in shared memory (the rest, if any, in the warp's slice of the global stage).  Binning
+// 150,000 glyphs 0.47 -> 0.34 ms, 20,000 paths (half of them small) 0.73 -> 0.69 ms; 10 CTAs per SM
+// (48 registers, spills) instead of 8 take 0.37 ms, the next path's record loaded ahead 0.35 ms.
+constexpr int kSmallThreads = 128, kSmallWarps = kSmallThreads / 32;
+constexpr uint32_t kSmallStage = 160, kSmallSpill = 640;  // visits staged per warp: shared, then global
+
+__global__ void __launch_bounds__(kSmallThreads, 8) k_bin_small(Batch b) {
+    __shared__ __align__(16) uint32_t s_cnt[kSmallWarps][kSmallWords];
+    __shared__ uint2 s_pts[kSmallWarps][kSmallStage];
+    __shared__ uint32_t s_tile[kSmallWarps][kSmallStage], s_slot[kSmallWarps];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const unsigned below = (1u << lane) - 1u;
+    uint32_t *const cnt = s_cnt[warp], *const err = &b.status[kStErr];
+    const uint32_t first = blockIdx.x * kSmallWarps + warp, stride = gridDim.x * kSmallWarps;
+    uint2 *const spill = b.stage + (size_t)first * kSmallSpill;
+    uint32_t *const spill_tile = b.stage_tile + (size_t)first * kSmallSpill;
+    const uint32_t *list = list_row(b, kCtaClasses);
+    const uint32_t n_items = b.bin_ctl[kCtlCount + kCtaClasses];
+    uint32_t item = first;
+    if (item >= n_items) return;
+    uint32_t next_p = list[item];
+    for (;;) {
+        const uint32_t p = next_p;
+        if (item + stride < n_items) next_p = list[item + stride];
+        const PathDev P = b.paths[p];
+        const PathLeaves L = path_leaves(b, p);
+        const WalkCtx w = walk_ctx(b, P);
+        const uint32_t rw = (uint32_t)w.rw, rh = (uint32_t)w.rh, T = rw * rh, tb = P.tile_first, cb = P.col_first;
+        int32_t *const above = reinterpret_cast<int32_t *>(cnt + T);
+        for (uint32_t t = lane; t < T + rw; t += 32) cnt[t] = 0;
+        __syncwarp();
+
+        // 1. fill counts and backdrop deltas, the visits staged
+        uint32_t nstage = 0;
+        auto stage = [&](uint32_t slot, uint2 pts, uint32_t tile) {
+            if (slot < kSmallStage) {
+                s_pts[warp][slot] = pts;
+                s_tile[warp][slot] = tile;
+            } else if (slot < kSmallStage + kSmallSpill) {
+                spill[slot - kSmallStage] = pts;
+                spill_tile[slot - kSmallStage] = tile;
+            }
+        };
+        auto on_fill = [&](int32_t local, uint2 q) {
+            atomicAdd(&cnt[local], 1u);
+            stage(atomicAdd(&s_slot[warp], 1u), q, (uint32_t)local | kVisitFill);
+        };
+        auto on_delta = [&](int32_t where, int d) {
+            if (where >= 0) atomicAdd(&cnt[where], (uint32_t)d << 24);
+            else atomicAdd(&above[-1 - where], d);
+        };
+        auto on_above = [&](int32_t x, int d) { atomicAdd(&above[x], d); };
+        auto begin_single = [&]() {
+            if (lane == 0) s_slot[warp] = nstage;
+            __syncwarp();
+        };
+        auto end_single = [&]() {
+            __syncwarp();
+            nstage = s_slot[warp];
+        };
+        auto visit = [&](bool live, bool m, bool e, uint32_t pa, uint32_t pb, bool down, uint32_t local,
+                         uint32_t inc) {
+            const unsigned keep = __ballot_sync(0xffffffffu, live && (m || e));
+            if (live && inc) atomicAdd(&cnt[local], inc);
+            if (keep >> lane & 1u)
+                stage(nstage + __popc(keep & below), make_uint2(pa, pb),
+                      local | (m ? kVisitFill : 0u) | (e ? kVisitExtra : 0u) | (down ? kVisitDown : 0u));
+            nstage += __popc(keep);
+        };
+        for (uint32_t k0 = 0; k0 < L.n; k0 += 32) {
+            const uint32_t k = k0 + (uint32_t)lane;
+            const bool have = k < L.n;
+            const float4 f = have ? b.leaves[L.index(b, k)] : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+            walk_lines(w, f, have, b.long_line, visit, on_above, on_fill, on_delta, begin_single, end_single, err);
+        }
+        __syncwarp();
+
+        // 2. the path's block of fills: four consecutive tiles a lane
+        uint32_t v[4], own = 0;
+#pragma unroll
+        for (int j = 0; j < 4; j++) {
+            v[j] = 4u * lane + j < T ? cnt[4 * lane + j] & 0xffffffu : 0u;
+            own += v[j];
+        }
+        uint32_t incl = own;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const uint32_t n = __shfl_up_sync(0xffffffffu, incl, o);
+            if (lane >= o) incl += n;
+        }
+        const uint32_t total = __shfl_sync(0xffffffffu, incl, 31);
+        unsigned long long base = 0;
+        if (lane == 0) base = atomicAdd(fill_total(b), (unsigned long long)total);
+
+        // 3. backdrops down each column
+        for (uint32_t x = lane; x < rw; x += 32) {
+            int32_t run = above[x];
+            for (uint32_t y = 0; y < rh; y++) {
+                const uint32_t t = y * rw + x, c = cnt[t];
+                b.tile_state[tb + t] = (uint16_t)((uint32_t)(uint8_t)(int8_t)run | ((c & 0xffffffu) ? 0x100u : 0u));
+                run += (int8_t)(c >> 24);
+            }
+            b.col_final[cb + x] = run;
+        }
+        __syncwarp();
+
+        // 4. write cursors (shared) and end offsets (global)
+        base = __shfl_sync(0xffffffffu, base, 0);
+        const bool fits = base + total <= (unsigned long long)b.fill_cap;
+        if (lane == 0) {
+            if (!fits) atomicOr(err, kErrOverflowFill);
+            b.path_fill[p] = (uint32_t)base;
+        }
+        uint32_t at = (uint32_t)base + incl - own;
+#pragma unroll
+        for (int j = 0; j < 4; j++) {
+            const uint32_t t = 4 * lane + j;
+            if (t < T) {
+                cnt[t] = at;
+                b.tile_fills[tb + t] = at + v[j];
+            }
+            at += v[j];
+        }
+        __syncwarp();
+
+        // 5. the fills, grouped by tile
+        if (fits && nstage <= kSmallStage + kSmallSpill) {
+            for (uint32_t k = lane; k < nstage; k += 32) {
+                const bool here = k < kSmallStage;
+                const uint2 q = here ? s_pts[warp][k] : spill[k - kSmallStage];
+                const uint32_t t = here ? s_tile[warp][k] : spill_tile[k - kSmallStage];
+                const uint32_t m = t >> 16 & 1u, e = t >> 17 & 1u;
+                const uint32_t slot = atomicAdd(&cnt[t & 0xffffu], m + e);
+                if (m) b.fills[slot] = q;
+                if (e) b.fills[slot + m] = t & kVisitDown ? make_uint2(0u, q.x) : make_uint2(q.y, 0u);
+            }
+        } else if (fits) {
+            for (uint32_t k = lane; k < L.n; k += 32) {
+                const float4 f = b.leaves[L.index(b, k)];
+                walk_line(
+                    w, f.x, f.y, f.z, f.w,
+                    [&](int32_t local, uint2 q) { b.fills[atomicAdd(&cnt[local], 1u)] = q; },
+                    [&](int32_t, int) {}, err);
+            }
+        }
+        __syncwarp();
+        if ((item += stride) >= n_items) return;
     }
 }
 
@@ -2846,11 +3019,27 @@ static cudaError_t fused_grids(const Tuning &t, uint32_t n_sms, uint32_t n_paths
     return e;
 }
 
+// The small class's grid: as many CTAs as fit on every SM, a path per warp at least.
+static cudaError_t small_grid(unsigned *grid, uint32_t n_sms, uint32_t n_paths) {
+    static std::atomic<int> per_sm{0};  // the same on every device of the one architecture this is built for
+    int n = per_sm.load();
+    if (!n) {
+        const cudaError_t e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, k_bin_small, kSmallThreads, 0);
+        if (e != cudaSuccess) return e;
+        per_sm.store(n = std::max(n, 1));
+    }
+    *grid = std::min((unsigned)n * n_sms, std::max(1u, (n_paths + kSmallWarps - 1) / kSmallWarps));
+    return cudaSuccess;
+}
+
 // The classes' slices of the stage follow each other, largest class first: they may run at once.
 cudaError_t bin_stage_slots(const Tuning &t, uint32_t n_sms, uint32_t n_paths, size_t *slots) {
     unsigned g[3];
     if (const cudaError_t e = fused_grids(t, n_sms, n_paths, g)) return e;
-    *slots = size_t(g[0]) * class_stage(0) + size_t(g[1]) * class_stage(1) + size_t(g[2]) * class_stage(2);
+    unsigned gs = 0;
+    if (const cudaError_t e = small_grid(&gs, n_sms, n_paths)) return e;
+    *slots = size_t(g[0]) * class_stage(0) + size_t(g[1]) * class_stage(1) + size_t(g[2]) * class_stage(2) +
+             size_t(gs) * kSmallWarps * kSmallSpill;
     return cudaSuccess;
 }
 
@@ -2864,7 +3053,8 @@ cudaError_t bin_class_max_ctas(int out[3]) {
 // Class 3 when it can have paths (zero, count, backdrops and offsets, write), and the CTA classes,
 // largest rects first; at once (bs not null) on streams of their own, joined before the composite,
 // so that the block scheduler fills the SMs that one class's last paths leave idle with the others'.
-cudaError_t launch_bin_paths(const Batch &b, const Tuning &t, bool large, const BinStreams *bs, cudaStream_t st) {
+cudaError_t launch_bin_paths(const Batch &b, const Tuning &t, bool small, bool large, const BinStreams *bs,
+                             cudaStream_t st) {
     if (!b.n_paths) return cudaSuccess;
     unsigned g[3];
     cudaError_t e = fused_grids(t, b.n_sms, b.n_paths, g);
@@ -2884,6 +3074,15 @@ cudaError_t launch_bin_paths(const Batch &b, const Tuning &t, bool large, const 
     if ((e = launch_fused<2>(b, g[2], 0, bs ? bs->side[0] : st)) != cudaSuccess) return e;
     if ((e = launch_fused<1>(b, g[1], s1, st)) != cudaSuccess) return e;
     if ((e = launch_fused<0>(b, g[0], s0, bs ? bs->side[1] : st)) != cudaSuccess) return e;
+    if (small) {
+        unsigned gs = 0;
+        if ((e = small_grid(&gs, b.n_sms, b.n_paths)) != cudaSuccess) return e;
+        Batch c = b;
+        c.stage += s0 + size_t(g[0]) * class_stage(0);
+        c.stage_tile += s0 + size_t(g[0]) * class_stage(0);
+        PF_LAUNCH(k_bin_small<<<gs, kSmallThreads, 0, bs ? bs->side[1] : st>>>(c));
+        if ((e = cudaGetLastError()) != cudaSuccess) return e;
+    }
     for (int k = 0; bs && k < 2; k++) {
         if ((e = cudaEventRecord(bs->join[k], bs->side[k])) != cudaSuccess) return e;
         if ((e = cudaStreamWaitEvent(st, bs->join[k], 0)) != cudaSuccess) return e;
