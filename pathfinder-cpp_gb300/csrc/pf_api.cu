@@ -1046,7 +1046,7 @@ int begin_frame(Ctx *c, uint32_t first, uint32_t count) {
     PF_CUDA(c->path_bounds.ensure(size_t(N) * 16 + 16));
     PF_CUDA(c->row_first.ensure((size_t(c->r_rows) + 1) * 4));
     PF_CUDA(c->row_mat.ensure(size_t(c->r_rmat) * 4));
-    PF_CUDA(c->bin_list.ensure(size_t(N) * 24 + 16));
+    PF_CUDA(c->bin_list.ensure(size_t(N) * 28 + 16));
     PF_CUDA(c->path_fill.ensure(size_t(N) * 4 + 16));
     PF_CUDA(c->path_seg_first.ensure(size_t(N) * 4 + 16));
     PF_CUDA(bin_stage_slots(c->tune, c->n_sms, c->r_paths, &c->stage_slots));
@@ -1125,8 +1125,8 @@ int bin_and_composite(Ctx *c, Batch b, bool learned, uint64_t max_leaves) {
     // paths 1456 -> 1247 us, stroked batch 3.10 -> 2.63 ms), but not in frames so long that their
     // tails no longer count (256 scenes, 178,734 paths, 13.43 -> 13.45 ms); the forks and joins cost
     // 10 to 15 us (150,000 glyphs, all of one class, 1219 -> 1233 us)
-    const bool small = rects[kRectSmall] != 0;
-    const bool several = small + (rects[0] != 0) + (rects[1] != 0) + (rects[2] != 0) + large > 1;
+    const BinClasses has{rects[kRectSmall] != 0, rects[kRectCluster] != 0, large};
+    const bool several = has.small + has.cluster + (rects[0] != 0) + (rects[1] != 0) + (rects[2] != 0) + large > 1;
     const bool at_once = c->tune.bin_concurrent || (several && c->r_paths <= 1u << 16);
     cudaStream_t st = c->stream;
     for (int attempt = 0;; attempt++) {
@@ -1139,7 +1139,7 @@ int bin_and_composite(Ctx *c, Batch b, bool learned, uint64_t max_leaves) {
             for (auto &e : c->bs.join) PF_CUDA(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
             c->bs_ready = true;
         }
-        PF_CUDA(launch_bin_paths(b, c->tune, small, large, at_once ? &c->bs : nullptr, st));
+        PF_CUDA(launch_bin_paths(b, c->tune, has, at_once ? &c->bs : nullptr, st));
         record(c, 3);
         record(c, 4);
         record(c, 5);

@@ -18,7 +18,7 @@ constexpr uint32_t kMaxWalk = 1u << 20;    // tile-walk step bound per line
 constexpr uint32_t kNone = 0xffffffffu;       // also the scene format's "no clip path"
 constexpr uint32_t kCtaMaxLeaves = 1u << 22;   // most leaf lines of a path that a CTA bins
 constexpr size_t kBinCtlBytes = 2048;
-constexpr int kRectSmall = 4;                  // the binning class of paths small enough for a warp
+constexpr int kRectSmall = 4, kRectCluster = 5;  // the binning classes of a warp and of a cluster of CTAs
 constexpr int kRowWindow = 64;                 // framebuffer-tile rows a block of the row lists takes
 constexpr uint32_t kPathIsClip = 8u;           // PathDev::flags: a clip path (tiled, never drawn)
 
@@ -123,7 +123,7 @@ struct Batch {
     // per-path binning: leaf range of every path, paths bucketed by tile count
     uint2 *path_leaf_range;              // [n_paths] [first, end) in the leaf buffer
     const uint2 *path_contours;          // [n_paths] [first, end) contours of each path
-    uint32_t *bin_list;                  // [6][n_paths] paths of each size class
+    uint32_t *bin_list;                  // [7][n_paths] paths of each size class
     uint32_t *bin_ctl;                   // class counts, work tickets (kBinCtlBytes)
     uint32_t *path_tiles;                // [n_paths + 1] -> scanned to first tile
     uint32_t *path_cols;                 // [n_paths + 1] -> scanned to first column
@@ -221,8 +221,8 @@ enum : int {
     kStSampled = 22,   // segments of the contours sampled for their depth, and the deep ones of them
     kStSampledDeep = 23,
     kStDashChunks = 24,// upload: chunks of dashed points taken
-    kStRectClass = 25, // five words: nonzero if a path's rect asks for that binning class
-    kStCount = 30,
+    kStRectClass = 25, // six words: nonzero if a path's rect asks for that binning class
+    kStCount = 31,
 };
 
 // Kernels launched by this library (host-side counter, all contexts).
@@ -348,9 +348,12 @@ struct BinStreams {
     cudaStream_t side[2];
     cudaEvent_t fork, join[2];
 };
-// small, large: a path may be of the class that a warp bins, or of that of the global passes.
-cudaError_t launch_bin_paths(const Batch &b, const Tuning &t, bool small, bool large, const BinStreams *bs,
-                             cudaStream_t st);
+// The classes beside the CTA ones that a path of the frame may be of: a warp's, a cluster's, that of
+// the global passes.
+struct BinClasses {
+    bool small, cluster, large;
+};
+cudaError_t launch_bin_paths(const Batch &b, const Tuning &t, BinClasses has, const BinStreams *bs, cudaStream_t st);
 // The most CTAs of each binning class one SM holds.
 cudaError_t bin_class_max_ctas(int out[3]);
 cudaError_t launch_pool_lists(const Batch &b, bool scatter, cudaStream_t st);

@@ -35,11 +35,20 @@ constexpr int kThreads = 256;
 // Shared words of the binning's CTA classes (see "Binning by path").
 __host__ __device__ constexpr uint32_t class_words(int c) { return c == 0 ? 1088u : c == 1 ? 4352u : 16896u; }
 constexpr uint32_t kSmallWords = 128;  // of the class binned by a warp
-constexpr int kSmallClass = kRectSmall;
-// The class that holds a rect of that many words; 3: none (global passes).
-__device__ __forceinline__ int rect_class(uint64_t words) {
+constexpr int kSmallClass = kRectSmall, kClusterClass = kRectCluster;
+// The class binned by a cluster of CTAs, each with the tiles of a band of rows and a word per column
+// for two purposes.
+constexpr uint32_t kClusterCtas = 4, kClusterTiles = 16384, kClusterCols = 512;
+__device__ __forceinline__ uint32_t cluster_rows(uint32_t rh) { return (rh + kClusterCtas - 1) / kClusterCtas; }
+__device__ __forceinline__ bool fits_cluster(uint32_t rw, uint32_t rh) {
+    return rw <= kClusterCols && (uint64_t)cluster_rows(rh) * rw <= kClusterTiles;
+}
+// The class that holds a rect; 3: none (global passes).
+__device__ __forceinline__ int rect_class(uint32_t rw, uint32_t rh) {
+    const uint64_t words = (uint64_t)rw * ((uint64_t)rh + 1);
     return words <= kSmallWords ? kSmallClass
-           : words <= class_words(0) ? 0 : words <= class_words(1) ? 1 : words <= class_words(2) ? 2 : 3;
+           : words <= class_words(0) ? 0 : words <= class_words(1) ? 1 : words <= class_words(2) ? 2
+           : fits_cluster(rw, rh) ? kClusterClass : 3;
 }
 
 __device__ __forceinline__ float fadd(float a, float b) { return __fadd_rn(a, b); }
@@ -169,7 +178,7 @@ __device__ __forceinline__ int path_rect(const Batch &b, const uint2 *path_conto
     b.paths[p] = P;
     b.path_tiles[p] = (uint32_t)(w * h);
     b.path_cols[p] = (uint32_t)w;
-    return w ? rect_class((uint32_t)w * (uint64_t)(uint32_t)(h + 1)) : -1;
+    return w ? rect_class((uint32_t)w, (uint32_t)h) : -1;
 }
 
 __global__ void k_path_setup(Batch b, const uint2 *path_contours) {
@@ -183,7 +192,7 @@ __global__ void k_path_setup(Batch b, const uint2 *path_contours) {
         if (lane == 0 && c >= 0) atomicOr(&s_classes, 1u << c);
     }
     __syncthreads();
-    if (threadIdx.x <= kSmallClass && (s_classes >> threadIdx.x & 1u)) b.status[kStRectClass + threadIdx.x] = 1;
+    if (threadIdx.x <= kClusterClass && (s_classes >> threadIdx.x & 1u)) b.status[kStRectClass + threadIdx.x] = 1;
 }
 
 __global__ void k_path_offsets(Batch b) {
@@ -1406,13 +1415,14 @@ __host__ __device__ constexpr uint32_t class_stage(int c) { return c == 0 ? 3072
 // One line gives a tile at most two fills (the walk visits a tile once, with at most one
 // extra fill for a vertical crossing), so with at most 2^22 lines per CTA-binned path the
 // 24-bit counters cannot carry into the delta byte (kCtaMaxLeaves).
-// bin_ctl slots: paths per CTA class, work tickets per CTA class, tickets of the class-3
-// zeroing and set-up passes, and at slot 12 a 64-bit word: class-3 paths << 40 | their lines.
-enum : int { kCtlCount = 0, kCtlTicket = 4, kCtlTicketZero = 8, kCtlTicketPrep = 9, kCtl3 = 12 };
-// and from slot 16 the listed classes' paths (the CTA classes, then the small one) counted by log2 of
-// their leaf lines (4 x 32), then the write cursors of those buckets (4 x 32): each class's list runs
-// from its largest paths to its smallest, so the last to start take the shortest paths
-constexpr int kLists = kCtaClasses + 1;
+// bin_ctl slots: paths per list (the CTA classes, the small one, the cluster one), work tickets of the
+// CTA classes and of the cluster one, tickets of the class-3 zeroing and set-up passes, and at slot
+// 12 a 64-bit word: class-3 paths << 40 | their lines.
+enum : int { kCtlCount = 0, kCtlTicket = 5, kCtlTicketCluster = 8, kCtlTicketZero = 9, kCtlTicketPrep = 10, kCtl3 = 12 };
+// and from slot 16 the lists' paths counted by log2 of their leaf lines (5 x 32), then the write
+// cursors of those buckets (5 x 32): each list runs from its largest paths to its smallest, so the
+// last to start take the shortest paths
+constexpr int kListSmall = kCtaClasses, kListCluster = kCtaClasses + 1, kLists = kCtaClasses + 2;
 enum : int {
     kCtlBucket = 16,
     kCtlCursor = 16 + kLists * 32,
@@ -1420,12 +1430,12 @@ enum : int {
     kCtlCompTicket = kCtlWords
 };
 static_assert((kCtlCompTicket + 1) * 4 <= kBinCtlBytes, "bin_ctl is too small");
-// The list of a class (-1: none, class 3 has its own); list 3 lies behind class 3's two rows.
+// The list of a class (-1: none, class 3 has its own); lists 3 and 4 lie behind class 3's two rows.
 __device__ __forceinline__ int class_list(int cls) {
-    return cls == kSmallClass ? kCtaClasses : cls < kCtaClasses ? cls : -1;
+    return cls == kSmallClass ? kListSmall : cls == kClusterClass ? kListCluster : cls < kCtaClasses ? cls : -1;
 }
 __device__ __forceinline__ uint32_t *list_row(const Batch &b, int list) {
-    return b.bin_list + (size_t)(list < kCtaClasses ? list : 5) * b.n_paths;
+    return b.bin_list + (size_t)(list < kCtaClasses ? list : list + 2) * b.n_paths;
 }
 constexpr uint64_t kLow40 = (1ull << 40) - 1;
 
@@ -1438,14 +1448,15 @@ __device__ __forceinline__ unsigned long long *fill_total(const Batch &b) {
     return reinterpret_cast<unsigned long long *>(b.status + kStFill64);
 }
 
-// -1: no columns (nothing can land); kSmallClass: a warp; 0-2: CTA classes; 3: global passes.  A
+// -1: no columns (nothing can land); kSmallClass: a warp; 0-2: CTA classes; kClusterClass: a cluster
+// of CTAs; 3: global passes.  A
 // class holds the path's words; a larger one is taken where the smaller one's warps would have to
 // walk more than warp_lines lines each (bin_warp_lines), and a warp takes no more than it can stage.
 __device__ __forceinline__ int path_class(const PathDev &P, uint32_t leaves, uint32_t warp_lines) {
     const int32_t rw = max(P.rx1 - P.rx0, 0), rh = max(P.ry1 - P.ry0, 0);
     if (rw == 0) return -1;
     if (leaves > kCtaMaxLeaves) return 3;
-    int c = rect_class((uint64_t)rw * (uint32_t)(rh + 1));
+    int c = rect_class((uint32_t)rw, (uint32_t)rh);
     if (c == kSmallClass && leaves > min(warp_lines, kSmallLines)) c = 0;
     if (c == 0 && leaves > class_threads(0) / 32 * warp_lines) c = 1;
     if (c == 1 && leaves > class_threads(1) / 32 * warp_lines) c = 2;
@@ -1839,8 +1850,8 @@ __global__ void __launch_bounds__(kSmallThreads, 8) k_bin_small(Batch b) {
     const uint32_t first = blockIdx.x * kSmallWarps + warp, stride = gridDim.x * kSmallWarps;
     uint2 *const spill = b.stage + (size_t)first * kSmallSpill;
     uint32_t *const spill_tile = b.stage_tile + (size_t)first * kSmallSpill;
-    const uint32_t *list = list_row(b, kCtaClasses);
-    const uint32_t n_items = b.bin_ctl[kCtlCount + kCtaClasses];
+    const uint32_t *list = list_row(b, kListSmall);
+    const uint32_t n_items = b.bin_ctl[kCtlCount + kListSmall];
     uint32_t item = first;
     if (item >= n_items) return;
     uint32_t next_p = list[item];
@@ -1970,6 +1981,234 @@ __global__ void __launch_bounds__(kSmallThreads, 8) k_bin_small(Batch b) {
         }
         __syncwarp();
         if ((item += stride) >= n_items) return;
+    }
+}
+
+// The cluster class: rects too large for one CTA's shared memory (beyond 2048 x 2048 px or so) are
+// binned by four CTAs of a cluster, each holding the counters of a band of rows.  All four walk the
+// path's lines, a quarter each, and add to each other's counters through distributed shared memory;
+// the bands' column sums and totals are exchanged the same way.  The global passes that these
+// rects took before walk every line twice with global atomics on two arrays (mixed 8,192 paths on
+// 4095 x 4095, some 150 of such rects: binning 0.83 ms, of which 0.61 in those passes; now 0.38).
+__device__ __forceinline__ void cluster_sync() {
+    asm volatile("barrier.cluster.arrive.aligned;\n\tbarrier.cluster.wait.aligned;" ::: "memory");
+}
+// The address of a shared variable of the cluster's CTA `rank`, in the cluster's shared window.
+__device__ __forceinline__ uint32_t cluster_addr(const void *p, uint32_t rank) {
+    uint32_t a;
+    asm("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(a) : "r"((uint32_t)__cvta_generic_to_shared(p)), "r"(rank));
+    return a;
+}
+__device__ __forceinline__ void cluster_add(uint32_t addr, uint32_t v) {
+    asm volatile("red.relaxed.cluster.shared::cluster.add.u32 [%0], %1;" ::"r"(addr), "r"(v) : "memory");
+}
+__device__ __forceinline__ uint32_t cluster_fetch_add(uint32_t addr, uint32_t v) {
+    uint32_t old;
+    asm volatile("atom.relaxed.cluster.shared::cluster.add.u32 %0, [%1], %2;" : "=r"(old) : "r"(addr), "r"(v) : "memory");
+    return old;
+}
+__device__ __forceinline__ uint32_t cluster_load(uint32_t addr) {
+    uint32_t v;
+    asm volatile("ld.shared::cluster.u32 %0, [%1];" : "=r"(v) : "r"(addr) : "memory");
+    return v;
+}
+__device__ __forceinline__ void cluster_store(uint32_t addr, uint32_t v) {
+    asm volatile("st.shared::cluster.u32 [%0], %1;" ::"r"(addr), "r"(v) : "memory");
+}
+
+constexpr int kClusterThreads = 384, kClusterWarps = kClusterThreads / 32;
+constexpr uint32_t kClusterStage = 1024;  // visits staged per warp
+constexpr size_t kClusterSmem = (kClusterTiles + 2 * kClusterCols) * 4;
+
+__global__ void __cluster_dims__(kClusterCtas, 1, 1) __launch_bounds__(kClusterThreads, 3) k_bin_cluster(Batch b) {
+    extern __shared__ uint32_t sm[];
+    uint32_t *const cnt = sm;                                              // this band's tiles
+    int32_t *const above = reinterpret_cast<int32_t *>(sm + kClusterTiles);  // CTA 0: deltas above the rect
+    int32_t *const colsum = above + kClusterCols;                          // this band's delta sums
+    __shared__ uint32_t s_item, s_base, s_write, s_next, s_over;
+    __shared__ uint32_t s_total[2 * kClusterCtas];  // every CTA's fills (64 bits each)
+    __shared__ uint32_t s_slot[kClusterWarps], s_warp[kClusterWarps];
+    __shared__ unsigned long long s_wsum[kClusterWarps];
+    const uint32_t tid = threadIdx.x;
+    const int lane = (int)(tid & 31), warp = (int)(tid >> 5);
+    const unsigned below = (1u << lane) - 1u;
+    const uint32_t rank = blockIdx.x % kClusterCtas;
+    uint2 *const stage = b.stage + ((size_t)blockIdx.x * kClusterWarps + warp) * kClusterStage;
+    uint32_t *const stage_tile = b.stage_tile + ((size_t)blockIdx.x * kClusterWarps + warp) * kClusterStage;
+    const uint32_t *list = list_row(b, kListCluster);
+    const uint32_t n_items = b.bin_ctl[kCtlCount + kListCluster];
+    uint32_t *const err = &b.status[kStErr];
+    for (;;) {
+        if (rank == 0 && tid == 0) {
+            const uint32_t t = atomicAdd(&b.bin_ctl[kCtlTicketCluster], 1u);
+            for (uint32_t r = 0; r < kClusterCtas; r++) cluster_store(cluster_addr(&s_item, r), t);
+        }
+        cluster_sync();  // the ticket; and every CTA is done with the path before
+        const uint32_t item = s_item;
+        if (item >= n_items) return;
+        const uint32_t p = list[item];
+        const PathDev P = b.paths[p];
+        const WalkCtx w = walk_ctx(b, P);
+        const PathLeaves L = path_leaves(b, p);
+        const uint32_t rw = (uint32_t)w.rw, rh = (uint32_t)w.rh;
+        const uint32_t rows = cluster_rows(rh), band = rows * rw;  // tiles of a whole band
+        const uint32_t y0 = min(rh, rank * rows), y1 = min(rh, y0 + rows), T = (y1 - y0) * rw;
+        const uint32_t tb = P.tile_first + y0 * rw, cb = P.col_first;
+        for (uint32_t t = tid; t < T; t += kClusterThreads) cnt[t] = 0;
+        for (uint32_t x = tid; x < rw; x += kClusterThreads) above[x] = 0;
+        if (tid == 0) {
+            s_next = 0;
+            s_over = 0;
+        }
+        cluster_sync();
+
+        // 1. fill counts and backdrop deltas into the bands' counters, the visits staged.  CTA r
+        //    takes every fourth group of 32 lines from group r.
+        auto tile_addr = [&](uint32_t local) {
+            const uint32_t r = (uint32_t)(local >= band) + (uint32_t)(local >= 2 * band) + (uint32_t)(local >= 3 * band);
+            return cluster_addr(cnt + (local - r * band), r);
+        };
+        uint32_t nstage = 0;
+        auto on_fill = [&](int32_t local, uint2 q) {
+            cluster_add(tile_addr((uint32_t)local), 1u);
+            const uint32_t slot = atomicAdd(&s_slot[warp], 1u);
+            if (slot < kClusterStage) {
+                stage[slot] = q;
+                stage_tile[slot] = (uint32_t)local | kVisitFill;
+            }
+        };
+        auto on_above = [&](int32_t x, int d) { cluster_add(cluster_addr(above + x, 0), (uint32_t)d); };
+        auto on_delta = [&](int32_t where, int d) {
+            if (where >= 0) cluster_add(tile_addr((uint32_t)where), (uint32_t)d << 24);
+            else on_above(-1 - where, d);
+        };
+        auto begin_single = [&]() {
+            if (lane == 0) s_slot[warp] = nstage;
+            __syncwarp();
+        };
+        auto end_single = [&]() {
+            __syncwarp();
+            nstage = s_slot[warp];
+        };
+        auto visit = [&](bool live, bool m, bool e, uint32_t pa, uint32_t pb, bool down, uint32_t local,
+                         uint32_t inc) {
+            const unsigned keep = __ballot_sync(0xffffffffu, live && (m || e));
+            if (live && inc) cluster_add(tile_addr(local), inc);
+            const uint32_t slot = nstage + __popc(keep & below);
+            if ((keep >> lane & 1u) && slot < kClusterStage) {
+                stage[slot] = make_uint2(pa, pb);
+                stage_tile[slot] = local | (m ? kVisitFill : 0u) | (e ? kVisitExtra : 0u) | (down ? kVisitDown : 0u);
+            }
+            nstage += __popc(keep);
+        };
+        for (;;) {
+            uint32_t g = 0;
+            if (lane == 0) g = atomicAdd(&s_next, 1u);
+            const uint32_t k0 = (__shfl_sync(0xffffffffu, g, 0) * kClusterCtas + rank) * 32u;
+            if (k0 >= L.n) break;
+            const uint32_t k = k0 + (uint32_t)lane;
+            const bool have = k < L.n;
+            const float4 f = have ? b.leaves[L.index(b, k)] : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+            walk_lines(w, f, have, b.long_line, visit, on_above, on_fill, on_delta, begin_single, end_single, err);
+        }
+        if (lane == 0 && nstage > kClusterStage) s_over = 1;
+        cluster_sync();
+
+        // 2. the band's fills (each warp's chunk of tiles) and column sums, told to every CTA
+        const uint32_t chunk = ((T + kClusterWarps - 1) / kClusterWarps + 127u) & ~127u;
+        const uint32_t c0 = min(T, (uint32_t)warp * chunk), c1 = min(T, c0 + chunk);
+        unsigned long long wsum = 0;
+        for (uint32_t t = c0 + lane; t < c1; t += 32) wsum += cnt[t] & 0xffffffu;
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) wsum += __shfl_down_sync(0xffffffffu, wsum, o);
+        if (lane == 0) s_wsum[warp] = wsum;
+        for (uint32_t x = tid; x < rw; x += kClusterThreads) {
+            int32_t sum = 0;
+            for (uint32_t t = x; t < T; t += rw) sum += (int8_t)(cnt[t] >> 24);
+            colsum[x] = sum;
+        }
+        __syncthreads();
+        if (tid == 0) {
+            unsigned long long total = 0;
+            for (int k = 0; k < kClusterWarps; k++) {
+                const unsigned long long v = s_wsum[k];
+                s_warp[k] = (uint32_t)total;
+                total += v;
+            }
+            for (uint32_t r = 0; r < kClusterCtas; r++) {
+                cluster_store(cluster_addr(&s_total[2 * rank], r), (uint32_t)total);
+                cluster_store(cluster_addr(&s_total[2 * rank + 1], r), (uint32_t)(total >> 32));
+            }
+        }
+        cluster_sync();
+        unsigned long long before = 0, total = 0;  // fills of the bands above, of the path
+        for (uint32_t r = 0; r < kClusterCtas; r++) {
+            const unsigned long long v = s_total[2 * r] | (unsigned long long)s_total[2 * r + 1] << 32;
+            if (r < rank) before += v;
+            total += v;
+        }
+        if (rank == 0 && tid == 0) {
+            const unsigned long long base = atomicAdd(fill_total(b), total);
+            const bool fits = base + total <= (unsigned long long)b.fill_cap;
+            if (!fits) atomicOr(err, kErrOverflowFill);
+            b.path_fill[p] = (uint32_t)base;
+            for (uint32_t r = 0; r < kClusterCtas; r++) {
+                cluster_store(cluster_addr(&s_base, r), (uint32_t)base);
+                cluster_store(cluster_addr(&s_write, r), fits && total > 0 ? 1u : 0u);
+            }
+        }
+
+        // 3. backdrops down the band's columns, from the sums of the bands above
+        for (uint32_t x = tid; x < rw; x += kClusterThreads) {
+            int32_t run = (int32_t)cluster_load(cluster_addr(above + x, 0));
+            for (uint32_t r = 0; r < rank; r++) run += (int32_t)cluster_load(cluster_addr(colsum + x, r));
+            for (uint32_t t = x; t < T; t += rw) {
+                const uint32_t c = cnt[t];
+                b.tile_state[tb + t] = (uint16_t)((uint32_t)(uint8_t)(int8_t)run | ((c & 0xffffffu) ? 0x100u : 0u));
+                run += (int8_t)(c >> 24);
+            }
+            if (rank == kClusterCtas - 1) b.col_final[cb + x] = run;
+        }
+        cluster_sync();  // the base; and the counters are read before they become cursors
+
+        // 4. write cursors and end offsets: a warp scan of each warp's chunk
+        uint32_t carry = s_base + (uint32_t)before + s_warp[warp];
+        for (uint32_t t0 = c0; t0 < c1; t0 += 32) {
+            const uint32_t t = t0 + (uint32_t)lane, own = t < c1 ? cnt[t] & 0xffffffu : 0u;
+            uint32_t incl = own;
+#pragma unroll
+            for (int o = 1; o < 32; o <<= 1) {
+                const uint32_t n = __shfl_up_sync(0xffffffffu, incl, o);
+                if (lane >= o) incl += n;
+            }
+            if (t < c1) {
+                cnt[t] = carry + incl - own;
+                b.tile_fills[tb + t] = carry + incl;
+            }
+            carry += __shfl_sync(0xffffffffu, incl, 31);
+        }
+        cluster_sync();
+
+        // 5. the fills, grouped by tile, from this CTA's stages or by walking its lines again
+        if (s_write && !s_over) {
+            for (uint32_t k = lane; k < nstage; k += 32) {
+                const uint2 q = stage[k];
+                const uint32_t t = stage_tile[k], m = t >> 16 & 1u, e = t >> 17 & 1u;
+                const uint32_t at = cluster_fetch_add(tile_addr(t & 0xffffu), m + e);
+                if (m) b.fills[at] = q;
+                if (e) b.fills[at + m] = t & kVisitDown ? make_uint2(0u, q.x) : make_uint2(q.y, 0u);
+            }
+        } else if (s_write) {
+            for (uint32_t k0 = ((uint32_t)warp * kClusterCtas + rank) * 32u; k0 < L.n;
+                 k0 += kClusterWarps * kClusterCtas * 32u) {
+                if (k0 + (uint32_t)lane >= L.n) continue;
+                const float4 f = b.leaves[L.index(b, k0 + (uint32_t)lane)];
+                walk_line(
+                    w, f.x, f.y, f.z, f.w,
+                    [&](int32_t local, uint2 q) { b.fills[cluster_fetch_add(tile_addr((uint32_t)local), 1u)] = q; },
+                    [&](int32_t, int) {}, err);
+            }
+        }
     }
 }
 
@@ -3032,14 +3271,48 @@ static cudaError_t small_grid(unsigned *grid, uint32_t n_sms, uint32_t n_paths) 
     return cudaSuccess;
 }
 
+// The cluster class's grid: as many clusters as the GPU holds, a path each at least.
+static cudaError_t cluster_grid(unsigned *grid, uint32_t n_paths) {
+    static std::atomic<uint64_t> configured{0};  // devices the kernel's shared memory is set up on, and
+    static std::atomic<int> known[64];           // the clusters that fit there
+    int dev = 0, clusters = 0;
+    cudaError_t e = cudaGetDevice(&dev);
+    if (e != cudaSuccess) return e;
+    if (dev < 64 && (configured.load() >> dev & 1u)) {
+        clusters = known[dev].load();
+    } else {
+        e = cudaFuncSetAttribute(k_bin_cluster, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kClusterSmem);
+        if (e != cudaSuccess) return e;
+        cudaLaunchConfig_t cfg{};
+        cfg.gridDim = dim3(kClusterCtas);
+        cfg.blockDim = dim3(kClusterThreads);
+        cfg.dynamicSmemBytes = kClusterSmem;
+        cudaLaunchAttribute attr{};
+        attr.id = cudaLaunchAttributeClusterDimension;
+        attr.val.clusterDim.x = kClusterCtas;
+        attr.val.clusterDim.y = attr.val.clusterDim.z = 1;
+        cfg.attrs = &attr;
+        cfg.numAttrs = 1;
+        if ((e = cudaOccupancyMaxActiveClusters(&clusters, k_bin_cluster, &cfg)) != cudaSuccess) return e;
+        clusters = std::max(clusters, 1);
+        if (dev < 64) {
+            known[dev].store(clusters);
+            configured.fetch_or(uint64_t(1) << dev);
+        }
+    }
+    *grid = std::min((unsigned)clusters, std::max(n_paths, 1u)) * kClusterCtas;
+    return cudaSuccess;
+}
+
 // The classes' slices of the stage follow each other, largest class first: they may run at once.
 cudaError_t bin_stage_slots(const Tuning &t, uint32_t n_sms, uint32_t n_paths, size_t *slots) {
     unsigned g[3];
     if (const cudaError_t e = fused_grids(t, n_sms, n_paths, g)) return e;
-    unsigned gs = 0;
+    unsigned gs = 0, gc = 0;
     if (const cudaError_t e = small_grid(&gs, n_sms, n_paths)) return e;
+    if (const cudaError_t e = cluster_grid(&gc, n_paths)) return e;
     *slots = size_t(g[0]) * class_stage(0) + size_t(g[1]) * class_stage(1) + size_t(g[2]) * class_stage(2) +
-             size_t(gs) * kSmallWarps * kSmallSpill;
+             size_t(gs) * kSmallWarps * kSmallSpill + size_t(gc) * kClusterWarps * kClusterStage;
     return cudaSuccess;
 }
 
@@ -3050,11 +3323,10 @@ cudaError_t bin_class_max_ctas(int out[3]) {
     return e;
 }
 
-// Class 3 when it can have paths (zero, count, backdrops and offsets, write), and the CTA classes,
-// largest rects first; at once (bs not null) on streams of their own, joined before the composite,
+// Class 3 and the cluster class when they can have paths, and the CTA classes, largest rects first, and
+// the small class; at once (bs not null) on streams of their own, joined before the composite,
 // so that the block scheduler fills the SMs that one class's last paths leave idle with the others'.
-cudaError_t launch_bin_paths(const Batch &b, const Tuning &t, bool small, bool large, const BinStreams *bs,
-                             cudaStream_t st) {
+cudaError_t launch_bin_paths(const Batch &b, const Tuning &t, BinClasses has, const BinStreams *bs, cudaStream_t st) {
     if (!b.n_paths) return cudaSuccess;
     unsigned g[3];
     cudaError_t e = fused_grids(t, b.n_sms, b.n_paths, g);
@@ -3064,17 +3336,29 @@ cudaError_t launch_bin_paths(const Batch &b, const Tuning &t, bool small, bool l
         for (int k = 0; k < 2; k++)
             if ((e = cudaStreamWaitEvent(bs->side[k], bs->fork, 0)) != cudaSuccess) return e;
     }
-    if (large) {
+    if (has.large) {
         PF_LAUNCH(k_bin_zero_large<<<b.n_sms * 2, 256, 0, st>>>(b));
         PF_LAUNCH(k_bin_large<false><<<b.n_sms * 8, kThreads, 0, st>>>(b));
         PF_LAUNCH(k_bin_large_prep<<<b.n_sms * 2, kPrepThreads, 0, st>>>(b));
         PF_LAUNCH(k_bin_large<true><<<b.n_sms * 8, kThreads, 0, st>>>(b));
     }
+    if (has.cluster) {
+        unsigned gs = 0, gc = 0;
+        if ((e = small_grid(&gs, b.n_sms, b.n_paths)) != cudaSuccess) return e;
+        if ((e = cluster_grid(&gc, b.n_paths)) != cudaSuccess) return e;
+        const size_t first = size_t(g[0]) * class_stage(0) + size_t(g[1]) * class_stage(1) +
+                             size_t(g[2]) * class_stage(2) + size_t(gs) * kSmallWarps * kSmallSpill;
+        Batch c = b;
+        c.stage += first;
+        c.stage_tile += first;
+        PF_LAUNCH(k_bin_cluster<<<gc, kClusterThreads, kClusterSmem, st>>>(c));
+        if ((e = cudaGetLastError()) != cudaSuccess) return e;
+    }
     const size_t s1 = size_t(g[2]) * class_stage(2), s0 = s1 + size_t(g[1]) * class_stage(1);
     if ((e = launch_fused<2>(b, g[2], 0, bs ? bs->side[0] : st)) != cudaSuccess) return e;
     if ((e = launch_fused<1>(b, g[1], s1, st)) != cudaSuccess) return e;
     if ((e = launch_fused<0>(b, g[0], s0, bs ? bs->side[1] : st)) != cudaSuccess) return e;
-    if (small) {
+    if (has.small) {
         unsigned gs = 0;
         if ((e = small_grid(&gs, b.n_sms, b.n_paths)) != cudaSuccess) return e;
         Batch c = b;
