@@ -9,6 +9,9 @@
 // the fallback when a prediction overflows.
 #include <math.h>
 
+#include <algorithm>
+#include <atomic>
+
 #include "pf_internal.h"
 
 namespace pfc {
@@ -34,11 +37,10 @@ __device__ __forceinline__ float turn(float2 a, float2 b, float2 c) {
 
 // Per contour: its point-flag counts, control-polygon length and summed turning angle
 // (closed around the contour).  Paths sum them over their contours, so a path of thousands of
-// contours (a dashed stroke's outline) costs its warp one strided pass over those sums.  A
-// thread takes its contour alone up to kBigContour points; longer contours are taken by the
-// whole warp afterwards, one at a time, so no thread walks thousands of points.
-constexpr uint32_t kBigContour = 64;
-
+// contours (a dashed stroke's outline) costs its warp one strided pass over those sums.  A warp per
+// contour, its points over the lanes: a point's turn is an arc tangent and its neighbours' loads (a
+// thread per contour of up to 64 points took 74 us on the 12,383 contours of mixed 8,192 paths, now
+// 11 us).
 __device__ __forceinline__ void point_terms(const Batch &b, uint32_t a, uint32_t n, uint32_t i, float &n_on,
                                             float &n_c0, float &n_c1, float &length, float &turning) {
     const uint8_t f = b.flags[a + i];
@@ -53,41 +55,24 @@ __device__ __forceinline__ void point_terms(const Batch &b, uint32_t a, uint32_t
     }
 }
 
-__global__ void k_contour_features(Batch b, float4 *cf) {
-    const uint32_t c = global_tid();
+__global__ void __launch_bounds__(kThreads) k_contour_features(Batch b, float4 *cf) {
+    const uint32_t c = blockIdx.x * (kThreads / 32) + (threadIdx.x >> 5);
     const int lane = threadIdx.x & 31;
-    const bool in = c < b.n_contours;
-    uint32_t a = 0, n = 0;
-    if (in) {
-        a = b.contour_point_first[c];
-        n = b.contour_point_first[c + 1] - a;
+    if (c >= b.n_contours) return;
+    const uint32_t a = b.contour_point_first[c], n = b.contour_point_first[c + 1] - a;
+    float n_on = 0, n_c0 = 0, n_c1 = 0, length = 0, turning = 0;
+    for (uint32_t i = lane; i < n; i += 32) point_terms(b, a, n, i, n_on, n_c0, n_c1, length, turning);
+#pragma unroll
+    for (int d = 16; d > 0; d >>= 1) {
+        n_on += __shfl_xor_sync(0xffffffffu, n_on, d);
+        n_c0 += __shfl_xor_sync(0xffffffffu, n_c0, d);
+        n_c1 += __shfl_xor_sync(0xffffffffu, n_c1, d);
+        length += __shfl_xor_sync(0xffffffffu, length, d);
+        turning += __shfl_xor_sync(0xffffffffu, turning, d);
     }
-    const bool big = in && n > kBigContour;
-    if (in && !big) {
-        float n_on = 0, n_c0 = 0, n_c1 = 0, length = 0, turning = 0;
-        for (uint32_t i = 0; i < n; i++) point_terms(b, a, n, i, n_on, n_c0, n_c1, length, turning);
+    if (lane == 0) {
         cf[2 * (size_t)c] = make_float4(n_on, n_c0, n_c1, length);
         cf[2 * (size_t)c + 1] = make_float4(turning, 0.0f, 0.0f, 0.0f);
-    }
-    unsigned pending = __ballot_sync(0xffffffffu, big);
-    while (pending) {
-        const int src = __ffs(pending) - 1;
-        pending &= pending - 1;
-        const uint32_t ba = __shfl_sync(0xffffffffu, a, src), bn = __shfl_sync(0xffffffffu, n, src);
-        float n_on = 0, n_c0 = 0, n_c1 = 0, length = 0, turning = 0;
-        for (uint32_t i = lane; i < bn; i += 32) point_terms(b, ba, bn, i, n_on, n_c0, n_c1, length, turning);
-#pragma unroll
-        for (int d = 16; d > 0; d >>= 1) {
-            n_on += __shfl_xor_sync(0xffffffffu, n_on, d);
-            n_c0 += __shfl_xor_sync(0xffffffffu, n_c0, d);
-            n_c1 += __shfl_xor_sync(0xffffffffu, n_c1, d);
-            length += __shfl_xor_sync(0xffffffffu, length, d);
-            turning += __shfl_xor_sync(0xffffffffu, turning, d);
-        }
-        if (lane == src) {
-            cf[2 * (size_t)c] = make_float4(n_on, n_c0, n_c1, length);
-            cf[2 * (size_t)c + 1] = make_float4(turning, 0.0f, 0.0f, 0.0f);
-        }
     }
 }
 
@@ -178,139 +163,228 @@ constexpr int kOffW1 = 0, kOffB1 = kOffW1 + kH * kI, kOffW2 = kOffB1 + kH, kOffB
               kOffW3 = kOffB2 + kH, kOffB3 = kOffW3 + kO * kH, kParams = kOffB3 + kO;
 static_assert(kParams == kSizerParams, "parameter count");
 
-// Weights are stored and used in bf16; accumulation is fp32.
-__device__ __forceinline__ void load_params_smem(const __nv_bfloat16 *w, float *s) {
-    for (int i = threadIdx.x; i < kParams; i += blockDim.x) s[i] = __bfloat162float(w[i]);
-    __syncthreads();
-}
+// Weights are stored and used in bf16; activations and accumulation are fp32, so the contractions run
+// on the fp32 pipes: 14,000 multiply-adds a sample in training, 5,000 in prediction.  What bounds
+// them is how many operands each needs from shared memory, so a block works on kTile samples at a
+// time with a tile of 8 x 4 results per thread (12 16-byte reads per 128 multiply-adds), all
+// activations in shared memory, sample by sample.  Blocks stay on their SM (three fit) and take tiles
+// in turn, so the weight gradients stay in registers until the end: one atomic per block and
+// parameter.  (A sample per thread, weights read one by one, and the gradients of 64 samples added
+// with 5,122 atomics each: 65,536 samples trained in 298 us, predicted in 108 us; now 88 and
+// 35 us.)
+constexpr int kMlpThreads = 128, kMlpTile = 64, kMlpBlocks = 3;  // blocks per SM
+static_assert(kMlpThreads == kO * kH && kOffW2 % 8 == 0, "the weights' loads");
+constexpr int kPad = kH + 4;  // row of a sample's activations: 16-byte aligned, rows in other banks
 
-__device__ __forceinline__ void mlp_forward(const float *s, const float x[kI], float h1[kH], float h2[kH],
-                                            float y[kO]) {
+struct MlpShared {
+    float w1t[kI][kH];   // [k][i]
+    float w2t[kH][kH];   // [k][i]
+    float w2[kH][kH];    // [i][k]
+    float w3[kO][kH];
+    float b1[kH], b2[kH], b3[4];
+    float x[kMlpTile][kI];
+    float h1[kMlpTile][kPad];  // then dL/d(pre-activation 1)
+    float h2[kMlpTile][kPad];  // then dL/d(pre-activation 2)
+    float dy[kMlpTile][kO];
+};
+
+// acc[j][i] += sum over k of w[k][o + i] * act[s + j][k], for this thread's 8 outputs and 4 samples
+template <int kK, int kStride>
+__device__ __forceinline__ void mlp_gemm(const float (*w)[kH], const float *act, int o, int s, float acc[4][8]) {
 #pragma unroll 4
-    for (int i = 0; i < kH; i++) {
-        float a = s[kOffB1 + i];
+    for (int k = 0; k < kK; k += 4) {
+        float4 v[4];
 #pragma unroll
-        for (int k = 0; k < kI; k++) a += s[kOffW1 + i * kI + k] * x[k];
-        h1[i] = fmaxf(a, 0.0f);
-    }
-#pragma unroll 2
-    for (int i = 0; i < kH; i++) {
-        float a = s[kOffB2 + i];
-#pragma unroll 8
-        for (int k = 0; k < kH; k++) a += s[kOffW2 + i * kH + k] * h1[k];
-        h2[i] = fmaxf(a, 0.0f);
-    }
+        for (int j = 0; j < 4; j++) v[j] = *reinterpret_cast<const float4 *>(act + (s + j) * kStride + k);
 #pragma unroll
-    for (int o = 0; o < kO; o++) {
-        float a = s[kOffB3 + o];
-#pragma unroll 8
-        for (int k = 0; k < kH; k++) a += s[kOffW3 + o * kH + k] * h2[k];
-        y[o] = a;
+        for (int q = 0; q < 4; q++) {
+            const float4 u0 = *reinterpret_cast<const float4 *>(&w[k + q][o]);
+            const float4 u1 = *reinterpret_cast<const float4 *>(&w[k + q][o + 4]);
+            const float u[8] = {u0.x, u0.y, u0.z, u0.w, u1.x, u1.y, u1.z, u1.w};
+#pragma unroll
+            for (int j = 0; j < 4; j++) {
+                const float a = q == 0 ? v[j].x : q == 1 ? v[j].y : q == 2 ? v[j].z : v[j].w;
+#pragma unroll
+                for (int i = 0; i < 8; i++) acc[j][i] = fmaf(u[i], a, acc[j][i]);
+            }
+        }
     }
 }
 
-__global__ void __launch_bounds__(128) k_mlp_predict(const __nv_bfloat16 *w, const float *feat, uint32_t n,
-                                                     float *out) {
-    __shared__ float s[kParams];
-    load_params_smem(w, s);
-    const uint32_t i = global_tid();
-    if (i >= n) return;
-    float x[kI], h1[kH], h2[kH], y[kO];
+__device__ __forceinline__ void mlp_store(float (*dst)[kPad], int o, int s, const float v[4][8]) {
 #pragma unroll
-    for (int k = 0; k < kI; k++) x[k] = feat[(size_t)i * kI + k];
-    mlp_forward(s, x, h1, h2, y);
-#pragma unroll
-    for (int o = 0; o < kO; o++) out[(size_t)i * kO + o] = y[o];
+    for (int j = 0; j < 4; j++) {
+        *reinterpret_cast<float4 *>(&dst[s + j][o]) = make_float4(v[j][0], v[j][1], v[j][2], v[j][3]);
+        *reinterpret_cast<float4 *>(&dst[s + j][o + 4]) = make_float4(v[j][4], v[j][5], v[j][6], v[j][7]);
+    }
 }
 
-// Training step, part 1: forward + backward of a mini-batch, weight gradients summed over
-// the block's samples (a reduction over the batch dimension, no per-sample atomics) and
-// added to the global gradient.  Loss: mean over samples and outputs of (y - t)^2.
-constexpr int kTrainSamples = 64;  // samples per block
-
-__global__ void __launch_bounds__(kTrainSamples) k_mlp_grad(const __nv_bfloat16 *w, const float *feat,
-                                                            const float *target, const uint32_t *index,
-                                                            uint32_t n, float inv_count, float *grad,
-                                                            float *loss) {
-    __shared__ float s[kParams];
-    __shared__ float sx[kTrainSamples][kI];
-    __shared__ float sh1[kTrainSamples][kH + 1];
-    __shared__ float sh2[kTrainSamples][kH + 1];
-    __shared__ float sd2[kTrainSamples][kH + 1];  // dL/d(pre-activation 2)
-    __shared__ float sd1[kTrainSamples][kH + 1];  // dL/d(pre-activation 1)
-    __shared__ float sdy[kTrainSamples][kO];
-    load_params_smem(w, s);
+// kTrain false: predictions into out.  kTrain true: forward and backward of the mini-batch, weight
+// gradients added to grad and squared errors to loss (mean over samples and outputs of (y - t)^2
+// once the caller divides).  Samples past n have zero features and no error.
+template <bool kTrain>
+__global__ void __launch_bounds__(kMlpThreads, kMlpBlocks) k_mlp(const __nv_bfloat16 *w, const float *feat,
+                                                        const float *target, const uint32_t *index, uint32_t n,
+                                                        float inv_count, float *out, float *grad, float *loss) {
+    extern __shared__ float4 smem[];
+    MlpShared &S = *reinterpret_cast<MlpShared *>(smem);
     const int t = threadIdx.x;
-    const uint32_t j = blockIdx.x * kTrainSamples + t;
-    const bool valid = j < n;
-    float x[kI], h1[kH], h2[kH], y[kO];
-    float l = 0.0f;
-    if (valid) {
-        const uint32_t src = index ? index[j] : j;
+    // the weights, read eight (W2) or two (W1) at a time along k and stored along i
+    const uint32_t *const pairs = reinterpret_cast<const uint32_t *>(w);
+    auto low = [](uint32_t v) { return __uint_as_float(v << 16); };  // bf16 to fp32
+    auto high = [](uint32_t v) { return __uint_as_float(v & 0xffff0000u); };
 #pragma unroll
-        for (int k = 0; k < kI; k++) x[k] = feat[(size_t)src * kI + k];
-        mlp_forward(s, x, h1, h2, y);
+    for (int q = t; q < kH * kI / 2; q += kMlpThreads) {
+        const int i = q % kH, k = q / kH * 2;
+        const uint32_t v = pairs[(kOffW1 + i * kI + k) / 2];
+        S.w1t[k][i] = low(v);
+        S.w1t[k + 1][i] = high(v);
+    }
 #pragma unroll
-        for (int o = 0; o < kO; o++) {
-            const float e = y[o] - target[(size_t)src * kO + o];
-            l += e * e;
-            sdy[t][o] = 2.0f * e * inv_count;
+    for (int q = t; q < kH * kH / 8; q += kMlpThreads) {
+        const int i = q % kH, k = q / kH * 8;
+        const uint4 v = *reinterpret_cast<const uint4 *>(pairs + (kOffW2 + i * kH + k) / 2);
+        const float f[8] = {low(v.x), high(v.x), low(v.y), high(v.y), low(v.z), high(v.z), low(v.w), high(v.w)};
+#pragma unroll
+        for (int j = 0; j < 8; j++) S.w2t[k + j][i] = f[j];
+        if (kTrain) {
+            *reinterpret_cast<float4 *>(&S.w2[i][k]) = make_float4(f[0], f[1], f[2], f[3]);
+            *reinterpret_cast<float4 *>(&S.w2[i][k + 4]) = make_float4(f[4], f[5], f[6], f[7]);
         }
-    } else {
-#pragma unroll
-        for (int k = 0; k < kI; k++) x[k] = 0.0f;
-#pragma unroll
-        for (int k = 0; k < kH; k++) h1[k] = h2[k] = 0.0f;
-#pragma unroll
-        for (int o = 0; o < kO; o++) sdy[t][o] = 0.0f;
     }
-#pragma unroll
-    for (int k = 0; k < kI; k++) sx[t][k] = x[k];
-    for (int k = 0; k < kH; k++) {
-        sh1[t][k] = h1[k];
-        sh2[t][k] = h2[k];
+    S.w3[t / kH][t % kH] = __bfloat162float(w[kOffW3 + t]);
+    if (t < kH) {
+        S.b1[t] = __bfloat162float(w[kOffB1 + t]);
+        S.b2[t] = __bfloat162float(w[kOffB2 + t]);
     }
-    // backprop through layer 3 and the ReLU of layer 2
-    for (int k = 0; k < kH; k++) {
-        float d = 0.0f;
-#pragma unroll
-        for (int o = 0; o < kO; o++) d += s[kOffW3 + o * kH + k] * sdy[t][o];
-        sd2[t][k] = h2[k] > 0.0f ? d : 0.0f;
-    }
-    // backprop through layer 2 and the ReLU of layer 1
-    for (int k = 0; k < kH; k++) {
-        float d = 0.0f;
-        for (int i = 0; i < kH; i++) d += s[kOffW2 + i * kH + k] * sd2[t][i];
-        sd1[t][k] = h1[k] > 0.0f ? d : 0.0f;
-    }
-    __syncthreads();
-    // weight gradients: every thread owns a strided set of parameters and sums over samples
-    for (int q = t; q < kParams; q += kTrainSamples) {
-        float g = 0.0f;
-        if (q < kOffB1) {
-            const int i = q / kI, k = q % kI;
-            for (int m = 0; m < kTrainSamples; m++) g += sd1[m][i] * sx[m][k];
-        } else if (q < kOffW2) {
-            const int i = q - kOffB1;
-            for (int m = 0; m < kTrainSamples; m++) g += sd1[m][i];
-        } else if (q < kOffB2) {
-            const int i = (q - kOffW2) / kH, k = (q - kOffW2) % kH;
-            for (int m = 0; m < kTrainSamples; m++) g += sd2[m][i] * sh1[m][k];
-        } else if (q < kOffW3) {
-            const int i = q - kOffB2;
-            for (int m = 0; m < kTrainSamples; m++) g += sd2[m][i];
-        } else if (q < kOffB3) {
-            const int o = (q - kOffW3) / kH, k = (q - kOffW3) % kH;
-            for (int m = 0; m < kTrainSamples; m++) g += sdy[m][o] * sh2[m][k];
-        } else {
-            const int o = q - kOffB3;
-            for (int m = 0; m < kTrainSamples; m++) g += sdy[m][o];
+    if (t < kO) S.b3[t] = __bfloat162float(w[kOffB3 + t]);
+    const int o = (t & 7) * 8, s = (t >> 3) * 4;            // this thread's outputs and samples of a layer
+    const int gi = (t >> 4) * 8, gk = (t & 15) * 4;         // its part of W2's gradient
+    const int xi = t >> 1, xk = (t & 1) * 6;                // of W1's
+    float g2[8][4] = {}, g1[6] = {}, g3 = 0.0f, gb = 0.0f, gb3 = 0.0f, err = 0.0f;
+    const uint32_t tiles = (n + kMlpTile - 1) / kMlpTile;
+    for (uint32_t tile = blockIdx.x; tile < tiles; tile += gridDim.x) {
+        __syncthreads();
+        for (int q = t; q < kMlpTile * kI; q += kMlpThreads) {
+            const uint32_t j = tile * kMlpTile + q / kI;
+            float v = 0.0f;
+            if (j < n) v = feat[(size_t)(kTrain && index ? index[j] : j) * kI + q % kI];
+            S.x[q / kI][q % kI] = v;
         }
-        atomicAdd(&grad[q], g);
+        __syncthreads();
+        float acc[4][8];
+        auto layer = [&](const float *bias) {
+#pragma unroll
+            for (int i = 0; i < 8; i++) {
+                const float v = bias ? bias[o + i] : 0.0f;
+#pragma unroll
+                for (int j = 0; j < 4; j++) acc[j][i] = v;
+            }
+        };
+        auto relu = [&]() {
+#pragma unroll
+            for (int j = 0; j < 4; j++)
+#pragma unroll
+                for (int i = 0; i < 8; i++) acc[j][i] = fmaxf(acc[j][i], 0.0f);
+        };
+        layer(S.b1);
+        mlp_gemm<kI, kI>(S.w1t, &S.x[0][0], o, s, acc);
+        relu();
+        mlp_store(S.h1, o, s, acc);
+        __syncthreads();
+        layer(S.b2);
+        mlp_gemm<kH, kPad>(S.w2t, &S.h1[0][0], o, s, acc);
+        relu();
+        mlp_store(S.h2, o, s, acc);
+        __syncthreads();
+        {
+            // the outputs: a sample and output per thread
+            const int m = t >> 1, c = t & 1;
+            float y = S.b3[c];
+#pragma unroll
+            for (int k = 0; k < kH; k += 4) {
+                const float4 h = *reinterpret_cast<const float4 *>(&S.h2[m][k]);
+                const float4 u = *reinterpret_cast<const float4 *>(&S.w3[c][k]);
+                y = fmaf(u.x, h.x, fmaf(u.y, h.y, fmaf(u.z, h.z, fmaf(u.w, h.w, y))));
+            }
+            const uint32_t j = tile * kMlpTile + m;
+            if (!kTrain) {
+                if (j < n) out[(size_t)j * kO + c] = y;
+            } else {
+                const float e = j < n ? y - target[(size_t)(index ? index[j] : j) * kO + c] : 0.0f;
+                err = fmaf(e, e, err);
+                S.dy[m][c] = 2.0f * e * inv_count;
+            }
+        }
+        if constexpr (kTrain) {
+            __syncthreads();
+            // layer 3's gradient: a weight per thread (and the biases by the threads of weight 0)
+            {
+                const int c = t >> 6, k = t & 63;
+#pragma unroll 8
+                for (int m = 0; m < kMlpTile; m++) {
+                    g3 = fmaf(S.dy[m][c], S.h2[m][k], g3);
+                    gb3 += S.dy[m][c];
+                }
+            }
+            __syncthreads();
+            // back through layer 3 and the ReLU of layer 2, in place of its activations
+#pragma unroll
+            for (int j = 0; j < 4; j++)
+#pragma unroll
+                for (int i = 0; i < 8; i++)
+                    acc[j][i] = acc[j][i] > 0.0f ? fmaf(S.w3[0][o + i], S.dy[s + j][0], S.w3[1][o + i] * S.dy[s + j][1]) : 0.0f;
+            mlp_store(S.h2, o, s, acc);
+            __syncthreads();
+            // layer 2's gradient
+#pragma unroll 4
+            for (int m = 0; m < kMlpTile; m++) {
+                const float4 d0 = *reinterpret_cast<const float4 *>(&S.h2[m][gi]);
+                const float4 d1 = *reinterpret_cast<const float4 *>(&S.h2[m][gi + 4]);
+                const float4 h = *reinterpret_cast<const float4 *>(&S.h1[m][gk]);
+                const float d[8] = {d0.x, d0.y, d0.z, d0.w, d1.x, d1.y, d1.z, d1.w};
+#pragma unroll
+                for (int i = 0; i < 8; i++) {
+                    g2[i][0] = fmaf(d[i], h.x, g2[i][0]);
+                    g2[i][1] = fmaf(d[i], h.y, g2[i][1]);
+                    g2[i][2] = fmaf(d[i], h.z, g2[i][2]);
+                    g2[i][3] = fmaf(d[i], h.w, g2[i][3]);
+                }
+            }
+            // back through layer 2 and the ReLU of layer 1
+            layer(nullptr);
+            mlp_gemm<kH, kPad>(S.w2, &S.h2[0][0], o, s, acc);
+#pragma unroll
+            for (int j = 0; j < 4; j++)
+#pragma unroll
+                for (int i = 0; i < 8; i++) acc[j][i] = S.h1[s + j][o + i] > 0.0f ? acc[j][i] : 0.0f;
+            __syncthreads();  // every thread has read layer 1's activations
+            mlp_store(S.h1, o, s, acc);
+            __syncthreads();
+            // layer 1's gradient, and the biases of layers 2 (threads 0-63) and 1
+            const float (*const bias_rows)[kPad] = t < kH ? S.h2 : S.h1;
+#pragma unroll 4
+            for (int m = 0; m < kMlpTile; m++) {
+                const float d = S.h1[m][xi];
+#pragma unroll
+                for (int k = 0; k < 6; k++) g1[k] = fmaf(d, S.x[m][xk + k], g1[k]);
+                gb += bias_rows[m][t & 63];
+            }
+        }
     }
-    // loss (sum of squared errors; the caller divides)
-    for (int d = 16; d > 0; d >>= 1) l += __shfl_xor_sync(0xffffffffu, l, d);
-    if ((t & 31) == 0) atomicAdd(loss, l);
+    if constexpr (kTrain) {
+#pragma unroll
+        for (int i = 0; i < 8; i++)
+#pragma unroll
+            for (int k = 0; k < 4; k++) atomicAdd(&grad[kOffW2 + (gi + i) * kH + gk + k], g2[i][k]);
+#pragma unroll
+        for (int k = 0; k < 6; k++) atomicAdd(&grad[kOffW1 + xi * kI + xk + k], g1[k]);
+        atomicAdd(&grad[kOffW3 + t], g3);
+        atomicAdd(&grad[(t < kH ? kOffB2 : kOffB1) + (t & 63)], gb);
+        if ((t & 63) == 0) atomicAdd(&grad[kOffB3 + (t >> 6)], gb3);
+        for (int d = 16; d > 0; d >>= 1) err += __shfl_xor_sync(0xffffffffu, err, d);
+        if ((t & 31) == 0) atomicAdd(loss, err);
+    }
 }
 
 // Training step, part 2: Adam on fp32 master weights, bf16 copy for the next forward.
@@ -336,7 +410,7 @@ cudaError_t launch_features(const Batch &b, const uint2 *path_contours, float4 *
                             cudaStream_t st) {
     if (b.n_paths) {
         if (b.n_contours) {
-            k_contour_features<<<(b.n_contours + kThreads - 1) / kThreads, kThreads, 0, st>>>(b, contour_scratch);
+            k_contour_features<<<(b.n_contours + kThreads / 32 - 1) / (kThreads / 32), kThreads, 0, st>>>(b, contour_scratch);
             count_launches(1);
         }
         k_features<<<(unsigned)((uint64_t(b.n_paths) * 32 + kThreads - 1) / kThreads), kThreads, 0, st>>>(
@@ -365,22 +439,34 @@ cudaError_t launch_path_counts(const Batch &b, const uint2 *path_contours, uint3
     return cudaGetLastError();
 }
 
-cudaError_t launch_mlp_predict(const __nv_bfloat16 *w, const float *feat, uint32_t n, float *out, cudaStream_t st) {
-    if (n) {
-        k_mlp_predict<<<(n + 127) / 128, 128, 0, st>>>(w, feat, n, out);
-        count_launches(1);
+// As many blocks as the SMs hold, no more than there are tiles of samples.
+template <bool kTrain>
+static cudaError_t launch_mlp(const __nv_bfloat16 *w, const float *feat, const float *target, const uint32_t *index,
+                              uint32_t n, float *out, float *grad, float *loss, cudaStream_t st) {
+    if (!n) return cudaSuccess;
+    static std::atomic<uint64_t> configured{0};  // devices the kernel's shared memory is set up on
+    int dev = 0, sms = 152;
+    cudaError_t e = cudaGetDevice(&dev);
+    if (e == cudaSuccess) e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+    if (e == cudaSuccess && !(dev < 64 && (configured.load() >> dev & 1u))) {
+        e = cudaFuncSetAttribute(k_mlp<kTrain>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(MlpShared));
+        if (e == cudaSuccess && dev < 64) configured.fetch_or(uint64_t(1) << dev);
     }
+    if (e != cudaSuccess) return e;
+    const unsigned tiles = (unsigned)((uint64_t(n) + kMlpTile - 1) / kMlpTile);
+    k_mlp<kTrain><<<std::min(tiles, (unsigned)kMlpBlocks * (unsigned)sms), kMlpThreads, sizeof(MlpShared), st>>>(
+        w, feat, target, index, n, 1.0f / ((float)n * kO), out, grad, loss);
+    count_launches(1);
     return cudaGetLastError();
+}
+
+cudaError_t launch_mlp_predict(const __nv_bfloat16 *w, const float *feat, uint32_t n, float *out, cudaStream_t st) {
+    return launch_mlp<false>(w, feat, nullptr, nullptr, n, out, nullptr, nullptr, st);
 }
 
 cudaError_t launch_mlp_grad(const __nv_bfloat16 *w, const float *feat, const float *target, const uint32_t *index,
                             uint32_t n, float *grad, float *loss, cudaStream_t st) {
-    if (n) {
-        k_mlp_grad<<<(n + kTrainSamples - 1) / kTrainSamples, kTrainSamples, 0, st>>>(
-            w, feat, target, index, n, 1.0f / (float)(n * kO), grad, loss);
-        count_launches(1);
-    }
-    return cudaGetLastError();
+    return launch_mlp<true>(w, feat, target, index, n, nullptr, grad, loss, st);
 }
 
 cudaError_t launch_adam(float *master, __nv_bfloat16 *w, float *grad, float *m, float *v, float lr, int step,
