@@ -140,6 +140,7 @@ struct Ctx {
     // the scene range of the last frame and its totals
     uint32_t r_first = 0, r_count = 0, r_paths = 0, r_contours = 0, r_fb = 0, r_rows = 0;
     uint32_t r_path_base = 0, r_contour_base = 0, r_fb_base = 0, r_row_base = 0;
+    uint32_t r_points = 0;
     uint32_t r_rblks = 0, r_rblk_base = 0, r_rmat = 0, r_rmat_base = 0;
     uint32_t n_segs = 0, n_tiles = 0, n_cols = 0, n_leaves = 0, n_list = 0, n_row_entries = 0;
     uint64_t n_fills = 0;
@@ -1012,6 +1013,7 @@ void set_range(Ctx *c, uint32_t first, uint32_t count) {
     c->r_paths = e.path_end - a.path_first;
     c->r_contour_base = a.contour_first;
     c->r_contours = e.contour_end - a.contour_first;
+    c->r_points = e.point_end - a.point_first;
     c->r_fb_base = a.fb_first;
     c->r_fb = c->h_scene_fb_first[first + count] - a.fb_first;
     c->r_row_base = a.row_first;
@@ -1069,7 +1071,7 @@ int stage_setup(Ctx *c, bool learned) {
     PF_CUDA(cudaMemsetAsync(b.contour_segs + C, 0, 4, st));
     PF_CUDA(cudaMemsetAsync(b.path_tiles + N, 0, 4, st));
     PF_CUDA(cudaMemsetAsync(b.path_cols + N, 0, 4, st));
-    PF_CUDA(launch_contour_segments(b, false, st));
+    PF_CUDA(launch_contour_segments(b, c->r_points, false, st));
     PF_CUDA(launch_rows(b, false, st));
     if (int e = scan(c, b.contour_segs, C + 1, kStSegs)) return e;
     if (int e = scan(c, b.path_tiles, N + 1, kStTiles)) return e;
@@ -1217,7 +1219,7 @@ int render_exact(Ctx *c, uint32_t first, uint32_t count, pf_frame_stats *stats) 
 
     // 2. segments, row lists, leaf counts, leaves
     Batch b = make_batch(c);
-    PF_CUDA(launch_contour_segments(b, true, st));
+    PF_CUDA(launch_contour_segments(b, c->r_points, true, st));
     PF_CUDA(launch_rows(b, true, st));
     PF_CUDA(cudaMemsetAsync(b.seg_leaves + c->n_segs, 0, 4, st));
     const bool shallow = uint64_t(c->h_status[kStSampledDeep]) * 64 < c->h_status[kStSampled];
@@ -1270,7 +1272,7 @@ int render_learned_frame(Ctx *c, uint32_t first, uint32_t count, pf_frame_stats 
     b.leaf_pool_cap = (uint32_t)leaf_pool;
     b.pool_path = c->pool_path.as<uint32_t>();
     b.pool_idx = c->pool_idx.as<uint32_t>();
-    PF_CUDA(launch_contour_segments(b, true, st));
+    PF_CUDA(launch_contour_segments(b, c->r_points, true, st));
     PF_CUDA(launch_rows(b, true, st));
     PF_CUDA(launch_flatten_budget(b, c->n_segs, st));
     record(c, 2);

@@ -318,7 +318,7 @@ cudaError_t launch_gradients(const pf_paint *paints, const uint32_t *grad_path, 
 cudaError_t launch_normalize(const Batch &b, uint2 *path_contours, cudaStream_t st);
 cudaError_t launch_path_setup(const Batch &b, const uint2 *path_contours, cudaStream_t st);
 cudaError_t launch_path_offsets(const Batch &b, cudaStream_t st);
-cudaError_t launch_contour_segments(const Batch &b, bool write, cudaStream_t st);
+cudaError_t launch_contour_segments(const Batch &b, uint64_t n_points, bool write, cudaStream_t st);
 cudaError_t launch_flatten(const Batch &b, uint32_t n_segs, bool write, bool shallow, cudaStream_t st);
 cudaError_t launch_rows(const Batch &b, bool write, cudaStream_t st);
 cudaError_t launch_composite(const Batch &b, cudaStream_t st);  // b.comp_ticket picks the grid

@@ -122,9 +122,10 @@ __global__ void k_normalize_paths(Batch b, uint2 *path_contours) {
 // round_rect_out_to_tile_bounds (pathfinder/core/data/data.h:131-133), Tiler::Tiler
 // (pathfinder/core/d3d9/tiler.cpp:317-335).
 
-// One warp: the path's bounds and tile rect; in lane 0 the binning class its rect asks for (-1: no
-// columns).
-__device__ __forceinline__ int path_rect(const Batch &b, const uint2 *path_contours, uint32_t p, int lane) {
+__global__ void k_path_setup(Batch b, const uint2 *path_contours) {
+    const uint32_t p = blockIdx.x * (kThreads / 32) + (threadIdx.x >> 5);
+    const int lane = threadIdx.x & 31;
+    if (p >= b.n_paths) return;
     const uint2 cr = path_contours[p];
     const uint32_t a = b.contour_point_first[cr.x], e = b.contour_point_first[cr.y];
     float l = INFINITY, t = INFINITY, r = -INFINITY, bt = -INFINITY;
@@ -145,7 +146,7 @@ __device__ __forceinline__ int path_rect(const Batch &b, const uint2 *path_conto
         bt = fmaxf(bt, __shfl_xor_sync(0xffffffffu, bt, d));
     }
     bad = __any_sync(0xffffffffu, bad);
-    if (lane != 0) return -1;
+    if (lane != 0) return;
     if (bad) atomicOr(&b.status[kStErr], kErrNonFinite);
     PathDev P = b.paths[p];
     const SceneDev &S = b.scenes[P.scene];
@@ -178,28 +179,26 @@ __device__ __forceinline__ int path_rect(const Batch &b, const uint2 *path_conto
     b.paths[p] = P;
     b.path_tiles[p] = (uint32_t)(w * h);
     b.path_cols[p] = (uint32_t)w;
-    return w ? rect_class((uint32_t)w, (uint32_t)h) : -1;
 }
 
-__global__ void k_path_setup(Batch b, const uint2 *path_contours) {
-    __shared__ uint32_t s_classes;  // a bit per binning class by rect among the block's paths
-    const uint32_t p = blockIdx.x * (kThreads / 32) + (threadIdx.x >> 5);
-    const int lane = threadIdx.x & 31;
+// The paths' first tiles and columns, and which binning classes their rects ask for.
+__global__ void __launch_bounds__(kThreads) k_path_offsets(Batch b) {
+    __shared__ uint32_t s_classes;
     if (threadIdx.x == 0) s_classes = 0;
     __syncthreads();
+    const uint32_t p = global_tid();
+    int c = -1;
     if (p < b.n_paths) {
-        const int c = path_rect(b, path_contours, p, lane);
-        if (lane == 0 && c >= 0) atomicOr(&s_classes, 1u << c);
+        const int4 rect = *reinterpret_cast<const int4 *>(&b.paths[p].rx0);
+        const int32_t w = max(rect.z - rect.x, 0), h = max(rect.w - rect.y, 0);
+        b.paths[p].tile_first = b.path_tiles[p];
+        b.paths[p].col_first = b.path_cols[p];
+        if (w) c = rect_class((uint32_t)w, (uint32_t)h);
     }
+    const uint32_t classes = __reduce_or_sync(0xffffffffu, c >= 0 ? 1u << c : 0u);
+    if ((threadIdx.x & 31) == 0 && classes) atomicOr(&s_classes, classes);
     __syncthreads();
     if (threadIdx.x <= kClusterClass && (s_classes >> threadIdx.x & 1u)) b.status[kStRectClass + threadIdx.x] = 1;
-}
-
-__global__ void k_path_offsets(Batch b) {
-    const uint32_t p = global_tid();
-    if (p >= b.n_paths) return;
-    b.paths[p].tile_first = b.path_tiles[p];
-    b.paths[p].col_first = b.path_cols[p];
 }
 
 // ---------------------------------------------------------------------------
@@ -207,7 +206,9 @@ __global__ void k_path_offsets(Batch b) {
 // (pathfinder/core/data/contour.cpp:110-175): stop at the first malformed point pattern;
 // at the end, an implicit closing line unless first ~= last within 1e-4.
 //
-// One warp per contour, a point per lane.  Every segment ends on the on-curve point the next one
+// One warp per contour, a point per lane; or eight lanes, where contours are short on average (up to
+// 40 points: a round over the contour's points waits for memory anyway, and four contours' rounds
+// wait together).  Every segment ends on the on-curve point the next one
 // starts from, so up to the first malformed pattern the segments are the on-curve points but the
 // last, each with a kind read off the three flags after it, and their order is a ballot's.  (A
 // thread walking its contour point by point: 101 + 16 us for 300,000 glyph contours, 270 + 126 us
@@ -232,59 +233,62 @@ __device__ __forceinline__ bool deep_segment(const float2 *p, uint32_t kind) {
     return m > kDeepFlatness;
 }
 
-template <bool kWrite>
+template <bool kWrite, int kGroup>
 __global__ void __launch_bounds__(kThreads) k_contour_segments(Batch b, uint32_t sample) {
-    const uint32_t c = blockIdx.x * (kThreads / 32) + (threadIdx.x >> 5);
-    const int lane = threadIdx.x & 31;
-    if (c >= b.n_contours) return;
-    const uint32_t a = b.contour_point_first[c], n = b.contour_point_first[c + 1] - a;
-    const uint8_t *fl = b.flags + a;
-    uint32_t out = 0, path = 0;
-    if (kWrite) {
-        out = b.contour_segs[c];
-        path = b.contour_path[c];
-        if (lane == 0 && b.path_contours[path].x == c) b.path_seg_first[path] = out;
-        if (out > b.seg_cap) return;
+    const int lane = threadIdx.x & 31, shift = lane & ~(kGroup - 1), l = lane & (kGroup - 1);
+    const unsigned group = kGroup == 32 ? 0xffffffffu : (1u << (kGroup & 31)) - 1u;
+    const uint32_t c = blockIdx.x * (kThreads / kGroup) + threadIdx.x / kGroup;
+    uint32_t a = 0, n = 0, out = 0, path = 0;
+    if (c < b.n_contours) {
+        a = b.contour_point_first[c];
+        n = b.contour_point_first[c + 1] - a;
+        if (kWrite) {
+            out = b.contour_segs[c];
+            path = b.contour_path[c];
+            if (l == 0 && b.path_contours[path].x == c) b.path_seg_first[path] = out;
+            if (out > b.seg_cap) n = 0;
+        }
     }
+    const uint8_t *fl = b.flags + a;
     auto emit = [&](uint32_t k, const SegDev &s) {
         if (k < b.seg_cap) b.segs[k] = s;
         else atomicOr(&b.status[kStErr], kErrOverflowSeg);
     };
     uint32_t count = 0, deep = 0;
     bool ends = n != 0 && fl[0] == 0;  // no malformed pattern so far
-    for (uint32_t base = 0; ends && base < n; base += 32) {
-        const uint32_t i = base + (uint32_t)lane;
+    for (uint32_t base = 0; __any_sync(0xffffffffu, ends && base < n); base += kGroup) {
+        const uint32_t i = base + (uint32_t)l;
         uint32_t kind = kSegClose;  // none
         bool bad = false;
-        if (i < n && fl[i] == 0 && i + 1 < n) {
+        if (ends && i < n && fl[i] == 0 && i + 1 < n) {
             const uint8_t f1 = fl[i + 1], f2 = i + 2 < n ? fl[i + 2] : 3, f3 = i + 3 < n ? fl[i + 3] : 3;
             if (f1 == 0) kind = kSegLine;
             else if (f1 == 1 && f2 == 0) kind = kSegQuad;
             else if (f1 == 1 && f2 == 2 && f3 == 0) kind = kSegCubic;
             else bad = true;
         }
-        const unsigned bads = __ballot_sync(0xffffffffu, bad);
-        const unsigned before = bads ? (bads & (0u - bads)) - 1u : 0xffffffffu;  // lanes before the first one
-        const unsigned heads = __ballot_sync(0xffffffffu, kind != kSegClose) & before;
-        if (kWrite && (heads >> lane & 1u))
-            emit(out + count + __popc(heads & ((1u << lane) - 1u)), SegDev{a + i, 0, kind, path});
-        if (!kWrite && c % sample == 0) {
-            const bool head = (heads >> lane & 1u) != 0;
-            deep += __popc(__ballot_sync(0xffffffffu, head && deep_segment(b.points + a + i, kind)));
+        const unsigned bads = __ballot_sync(0xffffffffu, bad) >> shift & group;
+        const unsigned before = bads ? (bads & (0u - bads)) - 1u : group;  // lanes before the first one
+        const unsigned heads = __ballot_sync(0xffffffffu, kind != kSegClose) >> shift & before;
+        const bool head = (heads >> l & 1u) != 0;
+        if (kWrite && head) emit(out + count + __popc(heads & ((1u << l) - 1u)), SegDev{a + i, 0, kind, path});
+        if (!kWrite) {
+            const bool d = head && c % sample == 0 && deep_segment(b.points + a + i, kind);
+            deep += __popc(__ballot_sync(0xffffffffu, d) >> shift & group);
         }
         count += __popc(heads);
-        ends = bads == 0;
+        ends = ends && bads == 0;
     }
     if (ends && n > 1) {
-        const float2 f = b.points[a], l = b.points[a + n - 1];
-        const float dx = fsub(f.x, l.x), dy = fsub(f.y, l.y);
+        const float2 f = b.points[a], z = b.points[a + n - 1];
+        const float dx = fsub(f.x, z.x), dy = fsub(f.y, z.y);
         const float len = __fsqrt_rn(fadd(fmul(dx, dx), fmul(dy, dy)));
         if (!(len <= 0.0001f)) {
-            if (kWrite && lane == 0) emit(out + count, SegDev{a + n - 1, a, kSegClose, path});
+            if (kWrite && l == 0) emit(out + count, SegDev{a + n - 1, a, kSegClose, path});
             count++;
         }
     }
-    if (!kWrite && lane == 0) {
+    if (!kWrite && l == 0 && c < b.n_contours) {
         b.contour_segs[c] = count;
         if (c % sample == 0) {
             atomicAdd(&b.status[kStSampled], count);
@@ -3146,12 +3150,18 @@ cudaError_t launch_path_offsets(const Batch &b, cudaStream_t st) {
     return cudaGetLastError();
 }
 
-cudaError_t launch_contour_segments(const Batch &b, bool write, cudaStream_t st) {
+cudaError_t launch_contour_segments(const Batch &b, uint64_t n_points, bool write, cudaStream_t st) {
     if (!b.n_contours) return cudaSuccess;
-    const unsigned grid = grid_for(b.n_contours, kThreads / 32);
     const uint32_t sample = b.n_contours / 2048 + 1;
-    if (write) PF_LAUNCH(k_contour_segments<true><<<grid, kThreads, 0, st>>>(b, sample));
-    else PF_LAUNCH(k_contour_segments<false><<<grid, kThreads, 0, st>>>(b, sample));
+    if (n_points <= uint64_t(b.n_contours) * 40) {
+        const unsigned grid = grid_for(b.n_contours, kThreads / 8);
+        if (write) PF_LAUNCH(k_contour_segments<true, 8><<<grid, kThreads, 0, st>>>(b, sample));
+        else PF_LAUNCH(k_contour_segments<false, 8><<<grid, kThreads, 0, st>>>(b, sample));
+    } else {
+        const unsigned grid = grid_for(b.n_contours, kThreads / 32);
+        if (write) PF_LAUNCH(k_contour_segments<true, 32><<<grid, kThreads, 0, st>>>(b, sample));
+        else PF_LAUNCH(k_contour_segments<false, 32><<<grid, kThreads, 0, st>>>(b, sample));
+    }
     return cudaGetLastError();
 }
 
