@@ -23,6 +23,8 @@ using namespace pfc;
 
 namespace {
 
+// the status words and the binning's control words, which share a buffer with the scans' state
+constexpr size_t kZeroBytes = kStBinCtl * 4 + kBinCtlBytes;
 constexpr size_t kStageBytes = 64 << 10;  // mapped host staging for small device reads
 
 struct DevBuf {
@@ -111,7 +113,7 @@ struct Ctx {
     // learned sizer: weights (bf16 used by the kernels, fp32 master + Adam moments for training)
     DevBuf sz_w, sz_master, sz_m, sz_v, sz_grad, sz_loss, sz_feat, sz_target, sz_index, sz_pred;
     DevBuf path_feat, contour_feat, path_pred, path_leaf_first, path_leaf_budget, path_leaf_cursor, path_fill_budget;
-    DevBuf bin_list, bin_ctl, path_leaf_range;
+    DevBuf bin_list, path_leaf_range;
     int sz_step = 0;
     bool sz_ready = false;
     float sz_mul = 1.25f, sz_add = 8.0f, sz_pool = 0.10f;
@@ -143,6 +145,8 @@ struct Ctx {
     uint32_t r_points = 0;
     uint32_t r_rblks = 0, r_rblk_base = 0, r_rmat = 0, r_rmat_base = 0;
     uint32_t n_segs = 0, n_tiles = 0, n_cols = 0, n_leaves = 0, n_list = 0, n_row_entries = 0;
+    // the buffer of the status words: bytes cleared for the frame, and taken so far by scan states
+    size_t zero_bytes = 0, zero_used = 0;
     uint64_t n_fills = 0;
     uint64_t fill_hint = 0;  // fills of the largest frame so far: the next frame's starting capacity
     bool lists_dumped = false;
@@ -930,7 +934,7 @@ Batch make_batch(Ctx *c) {
     b.path_leaf_range = c->path_leaf_range.as<uint2>();
     b.path_contours = c->path_contours.as<uint2>();
     b.bin_list = c->bin_list.as<uint32_t>();
-    b.bin_ctl = c->bin_ctl.as<uint32_t>();
+    b.bin_ctl = c->status.as<uint32_t>() + kStBinCtl;
     b.path_tiles = c->path_tiles.as<uint32_t>();
     b.path_cols = c->path_cols.as<uint32_t>();
     b.contour_segs = c->contour_segs.as<uint32_t>();
@@ -970,9 +974,10 @@ Batch make_batch(Ctx *c) {
     return b;
 }
 
-int read_status(Ctx *c) {
+// Waits for the status words.  copied: a kernel before has written them to the host already.
+int read_status(Ctx *c, bool copied = false) {
     if (c->capturing) return PF_OK;  // the captured frame's totals are already in h_status
-    PF_CUDA(launch_copy_words(c->h_status_dev, c->status.as<uint32_t>(), kStCount, c->stream));
+    if (!copied) PF_CUDA(launch_copy_words(c->h_status_dev, c->status.as<uint32_t>(), kStHostWords, c->stream));
     PF_CUDA(cudaStreamSynchronize(c->stream));
     c->syncs++;
     return PF_OK;
@@ -995,6 +1000,39 @@ int scan(Ctx *c, uint32_t *arr, uint32_t n, int slot) {
     PF_CUDA(c->scan_temp.ensure(scan_temp_bytes(n)));
     PF_CUDA(scan_exclusive_u32(arr, arr, n, c->status.as<uint32_t>() + slot, c->scan_temp.p, c->stream,
                                c->status.as<uint32_t>() + kStErr));
+    return PF_OK;
+}
+
+// A frame's scans, several in one launch, in place; the total goes to a status word and, with_end,
+// behind the array.  copy: the status words go to the host with them (read_status then only waits).
+// Their state lies in the buffer of the status words, which begin_frame clears.
+struct FrameScan {
+    uint32_t *arr;
+    uint32_t n;
+    int slot;
+    bool with_end;
+};
+
+int scan_frame(Ctx *c, std::initializer_list<FrameScan> scans, bool copy) {
+    uint32_t *const status = c->status.as<uint32_t>();
+    ScanJobs j{};
+    size_t at = c->zero_used;
+    for (const FrameScan &f : scans) {
+        j.job[j.n++] = ScanJob{f.arr, f.arr, f.n, status + f.slot, f.with_end ? f.arr + f.n : nullptr,
+                               reinterpret_cast<unsigned long long *>(c->status.as<char>() + at), 0, 0};
+        at += scan_state_words(f.n) * 8;
+    }
+    j.err = status + kStErr;
+    j.status = status;
+    j.n_status = kStHostWords;
+    if (copy && !c->capturing) {
+        j.host = c->h_status_dev;
+        j.done = reinterpret_cast<uint32_t *>(c->status.as<char>() + at);
+    }
+    at += 8;
+    if (at > c->zero_bytes) return fail(c, PF_ERR_CUDA, "the frame's scan state is too small");
+    c->zero_used = at;
+    PF_CUDA(scan_jobs(j, c->stream));
     return PF_OK;
 }
 
@@ -1036,8 +1074,14 @@ int begin_frame(Ctx *c, uint32_t first, uint32_t count) {
     c->syncs = 0;
     cudaStream_t st = c->stream;
     const uint32_t N = c->r_paths, C = c->r_contours;
-    PF_CUDA(c->status.ensure(kStCount * 4));
-    PF_CUDA(cudaMemsetAsync(c->status.p, 0, kStCount * 4, st));
+    // everything a frame counts in from zero, cleared at once: the status words, the binning's control
+    // words and the scans' states (set-up's four, one over the segments, which the points bound, and
+    // a learned frame's three over the paths)
+    c->zero_used = kZeroBytes;
+    c->zero_bytes = kZeroBytes + 8 * (scan_state_words(C) + 5 * scan_state_words(N) + scan_state_words(c->r_rmat) +
+                                      scan_state_words(c->r_points) + 16);
+    PF_CUDA(c->status.ensure(c->zero_bytes));
+    PF_CUDA(cudaMemsetAsync(c->status.p, 0, c->zero_bytes, st));
     PF_CUDA(c->contour_point_first.ensure((size_t(C) + 1) * 4));
     PF_CUDA(c->contour_path.ensure(size_t(C) * 4 + 4));
     PF_CUDA(c->contour_segs.ensure((size_t(C) + 1) * 4));
@@ -1054,7 +1098,6 @@ int begin_frame(Ctx *c, uint32_t first, uint32_t count) {
     PF_CUDA(bin_stage_slots(c->tune, c->n_sms, c->r_paths, &c->stage_slots));
     PF_CUDA(c->bin_stage.ensure(c->stage_slots * 12));
     PF_CUDA(c->path_cls.ensure(size_t(N) + 16));
-    PF_CUDA(c->bin_ctl.ensure(kBinCtlBytes));
     PF_CUDA(c->path_leaf_range.ensure(size_t(N) * 8 + 16));
     if (!c->h_path_clip.empty()) PF_CUDA(c->path_clip_rel.ensure(size_t(N) * 4 + 16));
     return PF_OK;
@@ -1068,16 +1111,15 @@ int stage_setup(Ctx *c, bool learned) {
     Batch b = make_batch(c);
     PF_CUDA(launch_normalize(b, c->path_contours.as<uint2>(), st));
     PF_CUDA(launch_path_setup(b, c->path_contours.as<uint2>(), st));
-    PF_CUDA(cudaMemsetAsync(b.contour_segs + C, 0, 4, st));
-    PF_CUDA(cudaMemsetAsync(b.path_tiles + N, 0, 4, st));
-    PF_CUDA(cudaMemsetAsync(b.path_cols + N, 0, 4, st));
     PF_CUDA(launch_contour_segments(b, c->r_points, false, st));
     PF_CUDA(launch_rows(b, false, st));
-    if (int e = scan(c, b.contour_segs, C + 1, kStSegs)) return e;
-    if (int e = scan(c, b.path_tiles, N + 1, kStTiles)) return e;
-    if (int e = scan(c, b.path_cols, N + 1, kStCols)) return e;
-    if (int e = scan(c, b.row_mat, c->r_rmat, kStRows)) return e;
-    PF_CUDA(launch_path_offsets(b, st));
+    if (int e = scan_frame(c,
+                           {{b.contour_segs, C, kStSegs, true},
+                            {b.path_tiles, N, kStTiles, true},
+                            {b.path_cols, N, kStCols, true},
+                            {b.row_mat, c->r_rmat, kStRows, false}},
+                           !learned))
+        return e;
     if (learned) {
         PF_CUDA(c->path_feat.ensure(size_t(N) * kSizerIn * 4 + 16));
         PF_CUDA(c->contour_feat.ensure(size_t(C) * 32 + 32));
@@ -1094,12 +1136,13 @@ int stage_setup(Ctx *c, bool learned) {
         PF_CUDA(launch_budgets(b, c->path_pred.as<float>(), c->sz_mul, c->sz_add, b.path_leaf_first,
                                c->path_fill_budget.as<uint32_t>(), b.path_leaf_cursor, st));
         PF_CUDA(cudaMemcpyAsync(b.path_leaf_budget, b.path_leaf_first, size_t(N) * 4, cudaMemcpyDeviceToDevice, st));
-        PF_CUDA(cudaMemsetAsync(b.path_leaf_first + N, 0, 4, st));
-        PF_CUDA(cudaMemsetAsync(c->path_fill_budget.as<uint32_t>() + N, 0, 4, st));
-        if (int e = scan(c, b.path_leaf_first, N + 1, kStLeafBudget)) return e;
-        if (int e = scan(c, c->path_fill_budget.as<uint32_t>(), N + 1, kStFillBudget)) return e;
+        if (int e = scan_frame(c,
+                               {{b.path_leaf_first, N, kStLeafBudget, true},
+                                {c->path_fill_budget.as<uint32_t>(), N, kStFillBudget, true}},
+                               true))
+            return e;
     }
-    if (int e = read_status(c)) return e;
+    if (int e = read_status(c, true)) return e;
     if (int e = check_kernel_status(c)) return e;
     c->n_segs = c->h_status[kStSegs];
     c->n_tiles = c->h_status[kStTiles];
@@ -1132,8 +1175,10 @@ int bin_and_composite(Ctx *c, Batch b, bool learned, uint64_t max_leaves) {
     const bool at_once = c->tune.bin_concurrent || (several && c->r_paths <= 1u << 16);
     cudaStream_t st = c->stream;
     for (int attempt = 0;; attempt++) {
-        PF_CUDA(cudaMemsetAsync(b.bin_ctl, 0, kBinCtlBytes, st));
-        PF_CUDA(cudaMemsetAsync(b.status + kStFill64, 0, 8, st));
+        if (attempt > 0) {  // else begin_frame cleared them
+            PF_CUDA(cudaMemsetAsync(b.bin_ctl, 0, kBinCtlBytes, st));
+            PF_CUDA(cudaMemsetAsync(b.status + kStFill64, 0, 8, st));
+        }
         PF_CUDA(launch_bin_classify(b, learned, st));
         if (at_once && !c->bs_ready) {
             for (auto &s : c->bs.side) PF_CUDA(cudaStreamCreateWithFlags(&s, cudaStreamNonBlocking));
@@ -1221,11 +1266,11 @@ int render_exact(Ctx *c, uint32_t first, uint32_t count, pf_frame_stats *stats) 
     Batch b = make_batch(c);
     PF_CUDA(launch_contour_segments(b, c->r_points, true, st));
     PF_CUDA(launch_rows(b, true, st));
-    PF_CUDA(cudaMemsetAsync(b.seg_leaves + c->n_segs, 0, 4, st));
     const bool shallow = uint64_t(c->h_status[kStSampledDeep]) * 64 < c->h_status[kStSampled];
     PF_CUDA(launch_flatten(b, c->n_segs, false, shallow, st));
-    if (int e = scan(c, b.seg_leaves, c->n_segs + 1, kStLeaves)) return e;
-    if (int e = read_status(c)) return e;
+    if (c->n_segs > c->r_points) return fail(c, PF_ERR_CUDA, "more segments than points");
+    if (int e = scan_frame(c, {{b.seg_leaves, c->n_segs, kStLeaves, true}}, true)) return e;
+    if (int e = read_status(c, true)) return e;
     if (int e = check_kernel_status(c)) return e;
     c->n_leaves = c->h_status[kStLeaves];
     PF_CUDA(c->leaves.ensure(size_t(c->n_leaves) * 16 + 16));
@@ -1280,7 +1325,7 @@ int render_learned_frame(Ctx *c, uint32_t first, uint32_t count, pf_frame_stats 
     PF_CUDA(cudaMemsetAsync(c->pool_cnt.p, 0, (size_t(N) + 2) * 4, st));
     b.pool_cnt = c->pool_cnt.as<uint32_t>() + 1;
     PF_CUDA(launch_pool_lists(b, false, st));
-    if (int e = scan(c, b.pool_cnt, N + 1, kStPoolListed)) return e;
+    if (int e = scan_frame(c, {{b.pool_cnt, N, kStPoolListed, true}}, false)) return e;
     PF_CUDA(launch_pool_lists(b, true, st));
     if (int e = bin_and_composite(c, b, true, leaf_slots)) return e;
     if (c->h_status[kStErr] & kErrOverflowLeaf) {
@@ -1305,7 +1350,7 @@ int render_learned_frame(Ctx *c, uint32_t first, uint32_t count, pf_frame_stats 
 std::vector<void *> frame_buffers(const Ctx *c) {
     const DevBuf *bufs[] = {&c->status, &c->contour_point_first, &c->contour_path, &c->paths, &c->path_tiles,
                             &c->path_cols, &c->path_contours, &c->path_bounds, &c->row_first, &c->row_mat, &c->bin_list,
-                            &c->bin_ctl, &c->path_leaf_range, &c->path_fill, &c->path_cls, &c->bin_stage,
+                            &c->path_leaf_range, &c->path_fill, &c->path_cls, &c->bin_stage,
                             &c->path_feat, &c->contour_feat, &c->path_pred, &c->path_leaf_first, &c->path_leaf_budget,
                             &c->path_leaf_cursor, &c->path_fill_budget, &c->path_seg_first, &c->segs, &c->seg_leaves,
                             &c->row_paths, &c->tile_fills, &c->tile_state, &c->col_above,
@@ -1883,12 +1928,12 @@ int pf_ctx_create(const pf_config *config, void **out) {
         e = cudaStreamCreateWithFlags(&c->stream, cudaStreamNonBlocking);
         c->own_stream = e == cudaSuccess;
     }
-    if (e == cudaSuccess) e = cudaHostAlloc(&c->h_status, kStCount * 4, cudaHostAllocMapped);
+    if (e == cudaSuccess) e = cudaHostAlloc(&c->h_status, kStHostWords * 4, cudaHostAllocMapped);
     if (e == cudaSuccess) e = cudaHostGetDevicePointer(reinterpret_cast<void **>(&c->h_status_dev), c->h_status, 0);
     if (e == cudaSuccess) e = cudaHostAlloc(&c->h_stage, kStageBytes, cudaHostAllocMapped);
     if (e == cudaSuccess) e = cudaHostGetDevicePointer(reinterpret_cast<void **>(&c->h_stage_dev), c->h_stage, 0);
     for (int i = 0; i < 8 && e == cudaSuccess; i++) e = cudaEventCreate(&c->ev[i]);
-    if (e == cudaSuccess) e = c->status.ensure(kStCount * 4);
+    if (e == cudaSuccess) e = c->status.ensure(kZeroBytes);
     if (e != cudaSuccess) {
         int st = cuda_fail(nullptr, e, "pf_ctx_create");
         pf_ctx_destroy(c);
@@ -1914,7 +1959,7 @@ int pf_ctx_destroy(void *ctx) {
     DevBuf *bufs[] = {&c->sz_w, &c->sz_master, &c->sz_m, &c->sz_v, &c->sz_grad, &c->sz_loss, &c->sz_feat,
                       &c->sz_target, &c->sz_index, &c->sz_pred, &c->path_feat, &c->contour_feat, &c->path_pred, &c->path_leaf_first,
                       &c->path_leaf_budget, &c->path_leaf_cursor, &c->path_fill_budget, &c->path_bounds,
-                      &c->bin_list, &c->bin_ctl, &c->path_leaf_range,
+                      &c->bin_list, &c->path_leaf_range,
                       &c->points, &c->pflags, &c->cstart, &c->pstart, &c->fill_rule, &c->color, &c->scenes,
                       &c->scene_path_first, &c->scene_contour_first, &c->scene_fb_first, &c->fb_scene, &c->contour_point_first,
                       &c->contour_path, &c->paths, &c->path_tiles, &c->path_cols, &c->contour_segs,

@@ -223,6 +223,9 @@ enum : int {
     kStDashChunks = 24,// upload: chunks of dashed points taken
     kStRectClass = 25, // six words: nonzero if a path's rect asks for that binning class
     kStCount = 31,
+    // the binning's control words follow in the same buffer; the host reads the first of them too
+    kStBinCtl = 64,
+    kStHostWords = kStBinCtl + 16,
 };
 
 // Kernels launched by this library (host-side counter, all contexts).
@@ -231,6 +234,28 @@ void count_launches(uint32_t n);
 
 // Scans (exclusive, in place allowed); the total lands in *total (device).
 size_t scan_temp_bytes(uint32_t n);
+// Several scans in one launch: in and out (may be equal), the total to *total and behind the output to
+// *end (either may be null), state: scan_state_words(n) zeroed words.  With host set, the last block
+// copies n_status status words there (done: a zeroed counter).
+struct ScanJob {
+    const uint32_t *in;
+    uint32_t *out;
+    uint32_t n;
+    uint32_t *total, *end;
+    unsigned long long *state;
+    uint32_t first_block, blocks;  // set by scan_jobs
+};
+constexpr uint32_t kMaxScanJobs = 6;
+struct ScanJobs {
+    ScanJob job[kMaxScanJobs];
+    uint32_t n;
+    uint32_t *err;
+    const uint32_t *status;
+    uint32_t n_status;
+    uint32_t *host, *done;
+};
+size_t scan_state_words(uint32_t n);
+cudaError_t scan_jobs(ScanJobs &jobs, cudaStream_t st);
 cudaError_t scan_exclusive_u32(const uint32_t *in, uint32_t *out, uint32_t n, uint32_t *total, void *temp,
                                cudaStream_t st, uint32_t *err);
 
@@ -317,7 +342,6 @@ cudaError_t launch_gradients(const pf_paint *paints, const uint32_t *grad_path, 
 // Stage launchers (all asynchronous on the given stream).
 cudaError_t launch_normalize(const Batch &b, uint2 *path_contours, cudaStream_t st);
 cudaError_t launch_path_setup(const Batch &b, const uint2 *path_contours, cudaStream_t st);
-cudaError_t launch_path_offsets(const Batch &b, cudaStream_t st);
 cudaError_t launch_contour_segments(const Batch &b, uint64_t n_points, bool write, cudaStream_t st);
 cudaError_t launch_flatten(const Batch &b, uint32_t n_segs, bool write, bool shallow, cudaStream_t st);
 cudaError_t launch_rows(const Batch &b, bool write, cudaStream_t st);

@@ -181,26 +181,6 @@ __global__ void k_path_setup(Batch b, const uint2 *path_contours) {
     b.path_cols[p] = (uint32_t)w;
 }
 
-// The paths' first tiles and columns, and which binning classes their rects ask for.
-__global__ void __launch_bounds__(kThreads) k_path_offsets(Batch b) {
-    __shared__ uint32_t s_classes;
-    if (threadIdx.x == 0) s_classes = 0;
-    __syncthreads();
-    const uint32_t p = global_tid();
-    int c = -1;
-    if (p < b.n_paths) {
-        const int4 rect = *reinterpret_cast<const int4 *>(&b.paths[p].rx0);
-        const int32_t w = max(rect.z - rect.x, 0), h = max(rect.w - rect.y, 0);
-        b.paths[p].tile_first = b.path_tiles[p];
-        b.paths[p].col_first = b.path_cols[p];
-        if (w) c = rect_class((uint32_t)w, (uint32_t)h);
-    }
-    const uint32_t classes = __reduce_or_sync(0xffffffffu, c >= 0 ? 1u << c : 0u);
-    if ((threadIdx.x & 31) == 0 && classes) atomicOr(&s_classes, classes);
-    __syncthreads();
-    if (threadIdx.x <= kClusterClass && (s_classes >> threadIdx.x & 1u)) b.status[kStRectClass + threadIdx.x] = 1;
-}
-
 // ---------------------------------------------------------------------------
 // Segments of a contour, as SegmentsIter::get_next(force_closed = true) yields them
 // (pathfinder/core/data/contour.cpp:110-175): stop at the first malformed point pattern;
@@ -2418,6 +2398,7 @@ __global__ void __launch_bounds__(kRowThreads) k_rows(Batch b) {
     if (tid < rows) s_out[tid] = kWrite ? mat[(size_t)tid * chunks] : 0u;
     if (kWrite && chunk == 0 && tid < rows) b.row_first[S.row_first - b.row_base + y0 + tid] = mat[(size_t)tid * chunks];
     if (kWrite && blockIdx.x == 0 && tid == 0) b.row_first[b.n_rows] = b.status[kStRows];
+    uint32_t seen = 0;  // lane 0: a bit per binning class
     for (uint32_t base = p0; base < p1; base += kRowThreads) {
         for (int k = lane; k <= kRowWindow; k += 32) s_cnt[warp][k] = 0;
         __syncwarp();
@@ -2427,12 +2408,25 @@ __global__ void __launch_bounds__(kRowThreads) k_rows(Batch b) {
         int32_t cx0 = 0, cx1 = 0, a = 0, e = 0;
         if (p < p1) {
             P = b.paths[p];
+            if (kWrite) {
+                P.tile_first = b.path_tiles[p];
+                if (y0 == 0) {  // one block of the chunk leaves them to the kernels that follow
+                    b.paths[p].tile_first = P.tile_first;
+                    b.paths[p].col_first = b.path_cols[p];
+                }
+            }
             cx0 = max(P.rx0, 0);
             cx1 = min(P.rx1, (int32_t)S.fbw);
             if (cx0 < cx1 && !(P.flags & kPathIsClip)) {
                 a = max(P.ry0 - y0, 0);
                 e = min(P.ry1 - y0, rows);
             }
+        }
+        if (!kWrite && y0 == 0) {
+            // which binning classes the rects ask for
+            const uint32_t w = (uint32_t)max(P.rx1 - P.rx0, 0), h = (uint32_t)max(P.ry1 - P.ry0, 0);
+            const uint32_t classes = __reduce_or_sync(0xffffffffu, w ? 1u << rect_class(w, h) : 0u);
+            if (lane == 0) seen |= classes;
         }
         const bool spans = a < e;
         if (spans) {
@@ -2486,7 +2480,10 @@ __global__ void __launch_bounds__(kRowThreads) k_rows(Batch b) {
             __syncthreads();  // the counts are read before the next paths clear them
         }
     }
-    if (!kWrite && tid < rows) mat[(size_t)tid * chunks] = s_out[tid];
+    if (kWrite) return;
+    if (tid < rows) mat[(size_t)tid * chunks] = s_out[tid];
+    for (int c = 0; c <= kClusterClass; c++)
+        if (seen >> c & 1u) b.status[kStRectClass + c] = 1;
 }
 
 // ---------------------------------------------------------------------------
@@ -3142,11 +3139,6 @@ cudaError_t launch_normalize(const Batch &b, uint2 *path_contours, cudaStream_t 
 
 cudaError_t launch_path_setup(const Batch &b, const uint2 *path_contours, cudaStream_t st) {
     if (b.n_paths) PF_LAUNCH(k_path_setup<<<grid_for(b.n_paths, kThreads / 32), kThreads, 0, st>>>(b, path_contours));
-    return cudaGetLastError();
-}
-
-cudaError_t launch_path_offsets(const Batch &b, cudaStream_t st) {
-    if (b.n_paths) PF_LAUNCH(k_path_offsets<<<grid_for(b.n_paths), kThreads, 0, st>>>(b));
     return cudaGetLastError();
 }
 

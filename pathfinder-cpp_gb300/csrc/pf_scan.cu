@@ -11,6 +11,11 @@
 // are taken in launch order from an atomic ticket so a block only ever waits on tiles that
 // started before it.  Every wait is bounded: after kSpinLimit polls the block records an
 // error bit and stops.
+//
+// One launch scans several arrays (their tiles one after the other in the grid): a frame's set-up
+// has four of a few thousand elements, whose launches and clears were most of their time.  The last
+// block to finish can also copy the frame's status words to mapped host memory, which saves the
+// host's read-back a launch of its own.
 #include "pf_internal.h"
 
 namespace pfc {
@@ -33,13 +38,20 @@ __device__ __forceinline__ uint32_t warp_inclusive(uint32_t v) {
     return v;
 }
 
-// state[0] = ticket counter, state[1 + t] = status of tile t
-__global__ void __launch_bounds__(kScanThreads) k_scan(const uint32_t *in, uint32_t *out, uint32_t n,
-                                                       unsigned long long *state, uint32_t *total,
-                                                       uint32_t *err) {
+// state[0] = ticket counter, state[1 + t] = status of tile t (all zero at the start)
+__global__ void __launch_bounds__(kScanThreads) k_scan(ScanJobs jobs) {
     __shared__ uint32_t warp_sums[kScanThreads / 32];
     __shared__ uint32_t s_tile;
     __shared__ uint32_t s_prefix;
+    __shared__ bool s_last;
+    uint32_t k = 0;
+    while (k + 1 < jobs.n && jobs.job[k + 1].first_block <= blockIdx.x) k++;
+    const ScanJob &job = jobs.job[k];
+    const uint32_t *const in = job.in;
+    uint32_t *const out = job.out;
+    const uint32_t n = job.n, tiles = job.blocks;
+    unsigned long long *const state = job.state;
+    uint32_t *const err = jobs.err;
     if (threadIdx.x == 0) s_tile = (uint32_t)atomicAdd(&state[0], 1ull);
     __syncthreads();
     const uint32_t tile = s_tile;
@@ -112,8 +124,9 @@ __global__ void __launch_bounds__(kScanThreads) k_scan(const uint32_t *in, uint3
     }
     __syncthreads();
     uint32_t run = s_prefix + warp_sums[warp] + inc - sum;
-    if (tile == gridDim.x - 1 && threadIdx.x == kScanThreads - 1 && total) {
-        total[0] = run + sum;
+    if (tile == tiles - 1 && threadIdx.x == kScanThreads - 1) {
+        if (job.total) *job.total = run + sum;
+        if (job.end) *job.end = run + sum;
     }
     if (base + kScanItems <= n && ((reinterpret_cast<uintptr_t>(out + base) & 15) == 0)) {
         uint32_t o[kScanItems];
@@ -132,24 +145,50 @@ __global__ void __launch_bounds__(kScanThreads) k_scan(const uint32_t *in, uint3
             run += v[k];
         }
     }
+    if (!jobs.host) return;
+    // the last block of the grid copies the status words out
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        __threadfence();
+        s_last = atomicAdd(jobs.done, 1u) == gridDim.x - 1;
+    }
+    __syncthreads();
+    if (s_last) {
+        __threadfence();
+        for (uint32_t i = threadIdx.x; i < jobs.n_status; i += kScanThreads)
+            jobs.host[i] = *(const volatile uint32_t *)(jobs.status + i);
+    }
 }
 
 }  // namespace
 
-size_t scan_temp_bytes(uint32_t n) {
-    const size_t tiles = (size_t(n) + kScanTile - 1) / kScanTile;
-    return (tiles + 1) * sizeof(unsigned long long) + 64;
+static uint32_t scan_blocks(uint32_t n) { return n ? (n + kScanTile - 1) / kScanTile : 1u; }
+
+size_t scan_state_words(uint32_t n) { return size_t(scan_blocks(n)) + 1; }
+
+size_t scan_temp_bytes(uint32_t n) { return scan_state_words(n) * sizeof(unsigned long long) + 64; }
+
+cudaError_t scan_jobs(ScanJobs &jobs, cudaStream_t st) {
+    uint32_t blocks = 0;
+    for (uint32_t k = 0; k < jobs.n; k++) {
+        jobs.job[k].first_block = blocks;
+        blocks += jobs.job[k].blocks = scan_blocks(jobs.job[k].n);
+    }
+    k_scan<<<blocks, kScanThreads, 0, st>>>(jobs);
+    count_launches(1);
+    return cudaGetLastError();
 }
 
 cudaError_t scan_exclusive_u32(const uint32_t *in, uint32_t *out, uint32_t n, uint32_t *total, void *temp,
                                cudaStream_t st, uint32_t *err) {
     if (n == 0) return cudaMemsetAsync(total, 0, sizeof(uint32_t), st);
-    const uint32_t tiles = (n + kScanTile - 1) / kScanTile;
-    cudaError_t e = cudaMemsetAsync(temp, 0, (size_t(tiles) + 1) * sizeof(unsigned long long), st);
+    const cudaError_t e = cudaMemsetAsync(temp, 0, scan_state_words(n) * sizeof(unsigned long long), st);
     if (e != cudaSuccess) return e;
-    k_scan<<<tiles, kScanThreads, 0, st>>>(in, out, n, static_cast<unsigned long long *>(temp), total, err);
-    count_launches(1);
-    return cudaGetLastError();
+    ScanJobs jobs{};
+    jobs.n = 1;
+    jobs.err = err;
+    jobs.job[0] = ScanJob{in, out, n, total, nullptr, static_cast<unsigned long long *>(temp), 0, 0};
+    return scan_jobs(jobs, st);
 }
 
 }  // namespace pfc
