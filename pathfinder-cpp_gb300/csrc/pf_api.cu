@@ -80,7 +80,7 @@ struct Ctx {
     std::string err;
 
     // inputs
-    DevBuf points, pflags, cstart, pstart, fill_rule, color, scenes, scene_path_first, scene_contour_first,
+    DevBuf points, pflags, cstart, pstart, fill_rule, color, scenes, scene_path_first,
         scene_fb_first, fb_scene;
     std::vector<SceneDev> h_scenes;
     std::vector<uint32_t> h_scene_fb_first;
@@ -611,7 +611,6 @@ int stroke_upload(Ctx *c, const pf_scene_view *scenes, uint32_t n, const std::ve
     PF_CUDA(launch_scene_bounds(in, c->st_bounds.as<uint32_t>(), st));
     std::vector<uint32_t> bounds(2 * (size_t(n) + 1));
     if (int e = d2h_wait(c, bounds.data(), c->st_bounds.p, bounds.size())) return e;
-    std::vector<uint32_t> ocf(n + 1);
     for (uint32_t i = 0; i < n; i++) {
         SceneDev &S = c->h_scenes[i];
         S.contour_first = bounds[2 * i];
@@ -619,14 +618,11 @@ int stroke_upload(Ctx *c, const pf_scene_view *scenes, uint32_t n, const std::ve
         S.point_first = bounds[2 * i + 1];
         S.point_end = bounds[2 * i + 3];
         S.cstart_base = S.contour_first + i;
-        ocf[i] = S.contour_first;
     }
-    ocf[n] = J;
     c->n_points = P;
     c->n_contours = J;
     PF_CUDA(c->cstart.ensure((size_t(J) + n) * 4 + 16));
     PF_CUDA(cudaMemcpyAsync(c->scenes.p, c->h_scenes.data(), size_t(n) * sizeof(SceneDev), cudaMemcpyHostToDevice, st));
-    PF_CUDA(cudaMemcpyAsync(c->scene_contour_first.p, ocf.data(), (size_t(n) + 1) * 4, cudaMemcpyHostToDevice, st));
     PF_CUDA(launch_outline_starts(in, c->scenes.as<SceneDev>(), c->cstart.as<uint32_t>(), c->pstart.as<uint32_t>(),
                                   st));
     c->ustats.stroke_contours = J;
@@ -749,7 +745,6 @@ int upload(Ctx *c, const pf_scene_view *scenes, uint32_t n) {
     PF_CUDA(c->color.ensure(N * 4 + 16));
     PF_CUDA(c->scenes.ensure(n * sizeof(SceneDev)));
     PF_CUDA(c->scene_path_first.ensure((n + 1) * 4));
-    PF_CUDA(c->scene_contour_first.ensure((n + 1) * 4));
     PF_CUDA(c->scene_fb_first.ensure((n + 1) * 4));
     PF_CUDA(c->scene_rblk_first.ensure((n + 1) * 4));
     {
@@ -876,8 +871,6 @@ int upload(Ctx *c, const pf_scene_view *scenes, uint32_t n) {
         c->ustats = pf_upload_stats{};
         PF_CUDA(cudaMemcpyAsync(c->scenes.p, c->h_scenes.data(), n * sizeof(SceneDev), cudaMemcpyHostToDevice,
                                 c->stream));
-        PF_CUDA(cudaMemcpyAsync(c->scene_contour_first.p, scf.data(), (n + 1) * 4, cudaMemcpyHostToDevice,
-                                c->stream));
     }
     // the host arrays are borrowed only for this call
     PF_CUDA(cudaStreamSynchronize(c->stream));
@@ -897,7 +890,6 @@ Batch make_batch(Ctx *c) {
     b.color = c->color.as<uint32_t>();
     b.scenes = c->scenes.as<SceneDev>();
     b.scene_path_first = c->scene_path_first.as<uint32_t>();
-    b.scene_contour_first = c->scene_contour_first.as<uint32_t>();
     b.scene_fb_first = c->scene_fb_first.as<uint32_t>();
     b.fb_scene = c->fb_scene.as<uint32_t>();
     b.scene_rblk_first = c->scene_rblk_first.as<uint32_t>();
@@ -1109,8 +1101,7 @@ int stage_setup(Ctx *c, bool learned) {
     cudaStream_t st = c->stream;
     const uint32_t N = c->r_paths, C = c->r_contours;
     Batch b = make_batch(c);
-    PF_CUDA(launch_normalize(b, c->path_contours.as<uint2>(), st));
-    PF_CUDA(launch_path_setup(b, c->path_contours.as<uint2>(), st));
+    PF_CUDA(launch_paths(b, c->path_contours.as<uint2>(), st));
     PF_CUDA(launch_contour_segments(b, c->r_points, false, st));
     PF_CUDA(launch_rows(b, false, st));
     if (int e = scan_frame(c,
@@ -1164,22 +1155,36 @@ int stage_setup(Ctx *c, bool learned) {
 // counted to the exact total, the buffer grows, and binning and composite run again.  Ends
 // with the status words read back.  max_leaves: the most leaf lines a path can have.
 int bin_and_composite(Ctx *c, Batch b, bool learned, uint64_t max_leaves) {
-    const uint32_t *rects = c->h_status + kStRectClass;
-    const bool large = rects[3] != 0 || max_leaves > kCtaMaxLeaves;
+    cudaStream_t st = c->stream;
+    // the classes that have paths: an exact frame's lists are made and counted by now, a learned
+    // frame knows what the rects ask for, and paths of many lines may be moved to larger CTA classes
+    BinClasses has{};
+    const uint32_t *rects = c->h_status + kStRectClass, *counts = c->h_status + kStBinCtl, N = c->r_paths;
+    if (learned) {
+        const bool any = rects[kRectSmall] || rects[0] || rects[1] || rects[2];
+        for (uint32_t &n : has.cta) n = any ? N : 0u;
+        has.small = rects[kRectSmall] ? N : 0u;
+        has.cluster = rects[kRectCluster] ? N : 0u;
+        has.large = rects[3] || max_leaves > kCtaMaxLeaves ? N : 0u;
+    } else {
+        for (int k = 0; k < 3; k++) has.cta[k] = counts[k];
+        has.small = counts[3];
+        has.cluster = counts[4];
+        has.large = counts[13] >> 8;  // the paths, above 40 bits of their lines
+    }
     // the binning classes at once where several have paths (20,000 paths 1607 -> 1497 us, mixed 8,192
     // paths 1456 -> 1247 us, stroked batch 3.10 -> 2.63 ms), but not in frames so long that their
     // tails no longer count (256 scenes, 178,734 paths, 13.43 -> 13.45 ms); the forks and joins cost
     // 10 to 15 us (150,000 glyphs, all of one class, 1219 -> 1233 us)
-    const BinClasses has{rects[kRectSmall] != 0, rects[kRectCluster] != 0, large};
-    const bool several = has.small + has.cluster + (rects[0] != 0) + (rects[1] != 0) + (rects[2] != 0) + large > 1;
-    const bool at_once = c->tune.bin_concurrent || (several && c->r_paths <= 1u << 16);
-    cudaStream_t st = c->stream;
+    int classes = (has.small != 0) + (has.cluster != 0) + (has.large != 0);
+    for (int k = 0; k < 3; k++) classes += (learned ? rects[k] : has.cta[k]) != 0;
+    const bool at_once = c->tune.bin_concurrent || (classes > 1 && N <= 1u << 16);
     for (int attempt = 0;; attempt++) {
         if (attempt > 0) {  // else begin_frame cleared them
             PF_CUDA(cudaMemsetAsync(b.bin_ctl, 0, kBinCtlBytes, st));
             PF_CUDA(cudaMemsetAsync(b.status + kStFill64, 0, 8, st));
         }
-        PF_CUDA(launch_bin_classify(b, learned, st));
+        if (learned || attempt > 0) PF_CUDA(launch_bin_lists(b, learned, StatusCopy{}, st));
         if (at_once && !c->bs_ready) {
             for (auto &s : c->bs.side) PF_CUDA(cudaStreamCreateWithFlags(&s, cudaStreamNonBlocking));
             PF_CUDA(cudaEventCreateWithFlags(&c->bs.fork, cudaEventDisableTiming));
@@ -1269,7 +1274,11 @@ int render_exact(Ctx *c, uint32_t first, uint32_t count, pf_frame_stats *stats) 
     const bool shallow = uint64_t(c->h_status[kStSampledDeep]) * 64 < c->h_status[kStSampled];
     PF_CUDA(launch_flatten(b, c->n_segs, false, shallow, st));
     if (c->n_segs > c->r_points) return fail(c, PF_ERR_CUDA, "more segments than points");
-    if (int e = scan_frame(c, {{b.seg_leaves, c->n_segs, kStLeaves, true}}, true)) return e;
+    if (int e = scan_frame(c, {{b.seg_leaves, c->n_segs, kStLeaves, true}}, false)) return e;
+    const StatusCopy copy{c->h_status_dev, reinterpret_cast<uint32_t *>(c->status.as<char>() + c->zero_used)};
+    if (c->zero_used + 8 > c->zero_bytes) return fail(c, PF_ERR_CUDA, "the frame's scan state is too small");
+    c->zero_used += 8;
+    PF_CUDA(launch_bin_lists(b, false, copy, st));
     if (int e = read_status(c, true)) return e;
     if (int e = check_kernel_status(c)) return e;
     c->n_leaves = c->h_status[kStLeaves];
@@ -1961,7 +1970,7 @@ int pf_ctx_destroy(void *ctx) {
                       &c->path_leaf_budget, &c->path_leaf_cursor, &c->path_fill_budget, &c->path_bounds,
                       &c->bin_list, &c->path_leaf_range,
                       &c->points, &c->pflags, &c->cstart, &c->pstart, &c->fill_rule, &c->color, &c->scenes,
-                      &c->scene_path_first, &c->scene_contour_first, &c->scene_fb_first, &c->fb_scene, &c->contour_point_first,
+                      &c->scene_path_first, &c->scene_fb_first, &c->fb_scene, &c->contour_point_first,
                       &c->contour_path, &c->paths, &c->path_tiles, &c->path_cols, &c->contour_segs,
                       &c->path_contours, &c->path_seg_first, &c->segs, &c->seg_leaves, &c->leaves, &c->pool_path, &c->pool_cnt,
                       &c->pool_idx, &c->tile_fills, &c->path_fill, &c->path_cls, &c->tile_state, &c->col_above,

@@ -98,7 +98,6 @@ struct Batch {
     const uint32_t *grad_ramp;           // [gradients][256] RGBA8 ramps
     const SceneDev *scenes;
     const uint32_t *scene_path_first;    // [n_scenes_all + 1]
-    const uint32_t *scene_contour_first; // [n_scenes_all + 1]
     const uint32_t *scene_fb_first;      // [n_scenes_all + 1]
     const uint32_t *fb_scene;            // [framebuffer tiles of all scenes] the scene of each
     const uint32_t *scene_rblk_first;    // [n_scenes_all + 1]
@@ -340,8 +339,7 @@ cudaError_t launch_gradients(const pf_paint *paints, const uint32_t *grad_path, 
                              float4 *meta, uint32_t *ramps, cudaStream_t st);
 
 // Stage launchers (all asynchronous on the given stream).
-cudaError_t launch_normalize(const Batch &b, uint2 *path_contours, cudaStream_t st);
-cudaError_t launch_path_setup(const Batch &b, const uint2 *path_contours, cudaStream_t st);
+cudaError_t launch_paths(const Batch &b, uint2 *path_contours, cudaStream_t st);
 cudaError_t launch_contour_segments(const Batch &b, uint64_t n_points, bool write, cudaStream_t st);
 cudaError_t launch_flatten(const Batch &b, uint32_t n_segs, bool write, bool shallow, cudaStream_t st);
 cudaError_t launch_rows(const Batch &b, bool write, cudaStream_t st);
@@ -363,21 +361,27 @@ cudaError_t launch_budgets(const Batch &b, const float *pred, float mul, float a
 cudaError_t launch_path_counts(const Batch &b, const uint2 *path_contours, uint32_t *leaves, uint32_t *fills,
                                cudaStream_t st);
 cudaError_t launch_flatten_budget(const Batch &b, uint32_t n_segs, cudaStream_t st);
-// Binning by path: classify (leaf ranges, size classes), then bin every path (counts,
-// backdrops, fill offsets, fills).  A learned frame first lists its pooled lines by path:
+// Where a kernel copies the status words (kStHostWords of them) as its last act: mapped host memory, or
+// null; done: a zeroed counter.
+struct StatusCopy {
+    uint32_t *host, *done;
+};
+// Binning by path: the lists of paths by size class (leaf ranges, classes), then every path binned
+// (counts, backdrops, fill offsets, fills).  A learned frame first lists its pooled lines by path:
 // count, scan pool_cnt, scatter.
-cudaError_t launch_bin_classify(const Batch &b, bool learned, cudaStream_t st);
+cudaError_t launch_bin_lists(const Batch &b, bool learned, const StatusCopy &copy, cudaStream_t st);
 // side[0..1], fork, join[0..1]: streams and events for running the classes at once, or null.
 struct BinStreams {
     cudaStream_t side[2];
     cudaEvent_t fork, join[2];
 };
-// The classes beside the CTA ones that a path of the frame may be of: a warp's, a cluster's, that of
-// the global passes.
+// The paths each class can have at most (0: none): the CTA classes, a warp's, a cluster's, that of the
+// global passes.
 struct BinClasses {
-    bool small, cluster, large;
+    uint32_t cta[3], small, cluster, large;
 };
-cudaError_t launch_bin_paths(const Batch &b, const Tuning &t, BinClasses has, const BinStreams *bs, cudaStream_t st);
+cudaError_t launch_bin_paths(const Batch &b, const Tuning &t, const BinClasses &has, const BinStreams *bs,
+                             cudaStream_t st);
 // The most CTAs of each binning class one SM holds.
 cudaError_t bin_class_max_ctas(int out[3]);
 cudaError_t launch_pool_lists(const Batch &b, bool scatter, cudaStream_t st);

@@ -2,7 +2,7 @@
 //
 // Stage map (reference -> here):
 //   SegmentsD3D11::add_path / SegmentsIter   -> k_contour_segments (count + emit)
-//   BuiltPath / round_rect_out_to_tile_bounds -> k_path_setup
+//   BuiltPath / round_rect_out_to_tile_bounds -> k_paths
 //   dice.comp (here: the d3d9 recursive bisection, tiler.cpp:284-315)  -> k_flatten<count|write>
 //   bin.comp (here: the d3d9 tile walk + add_fill, tiler.cpp:131-279,
 //             object_builder.cpp:19-114),
@@ -74,60 +74,25 @@ inline unsigned grid_for(uint64_t n, int threads = kThreads) {
 }
 
 // ---------------------------------------------------------------------------
-// Normalisation: scene-local offsets -> global offsets.
-
-__global__ void k_normalize_contours(Batch b) {
-    const uint32_t c = global_tid();
-    if (c >= b.n_contours) return;
-    const uint32_t cg = b.contour_base + c;
-    const uint32_t s = upper_bound(b.scene_contour_first, b.n_scenes_all + 1, cg) - 1;
-    const SceneDev &S = b.scenes[s];
-    const uint32_t local = cg - S.contour_first;
-    b.contour_point_first[c] = S.point_first + b.contour_start_cat[S.cstart_base + local];
-    if (c == b.n_contours - 1)
-        b.contour_point_first[b.n_contours] = S.point_first + b.contour_start_cat[S.cstart_base + local + 1];
-}
-
-__global__ void k_normalize_paths(Batch b, uint2 *path_contours) {
-    const uint32_t p = global_tid();
-    if (p >= b.n_paths) return;
-    const uint32_t pg = b.path_base + p;
-    const uint32_t s = upper_bound(b.scene_path_first, b.n_scenes_all + 1, pg) - 1;
-    const SceneDev &S = b.scenes[s];
-    const uint32_t local = pg - S.path_first;
-    const uint32_t c0 = S.contour_first + b.path_start_cat[S.pstart_base + local] - b.contour_base;
-    const uint32_t c1 = S.contour_first + b.path_start_cat[S.pstart_base + local + 1] - b.contour_base;
-    path_contours[p] = make_uint2(c0, c1);
-    for (uint32_t c = c0; c < c1; c++) b.contour_path[c] = p;
-    PathDev P{};
-    P.scene = s;
-    // occludes: an opaque paint (PaintMetadata::is_opaque): an opaque colour, or a gradient
-    // whose stops are all opaque
-    bool opaque = (b.color[pg] >> 24) == 0xffu;
-    if (b.path_grad && b.path_grad[pg] != kNone) opaque = __float_as_uint(b.grad_meta[4 * b.path_grad[pg] + 3].z) != 0;
-    P.flags = (b.fill_rule[pg] ? 1u : 0u) | (opaque ? 2u : 0u);
-    if (b.path_clip_cat) {
-        // clip paths are tiled like the others but never drawn; a clipped path's clip is in its
-        // scene, addressed here within the frame
-        if (b.path_is_clip_cat[pg]) P.flags |= kPathIsClip;
-        const uint32_t lc = b.path_clip_cat[pg];
-        b.path_clip_rel[p] = lc == kNone ? kNone : S.path_first - b.path_base + lc;
-    }
-    b.paths[p] = P;
-}
-
-// ---------------------------------------------------------------------------
-// Per-path bounds and tile rect (one warp per path).
+// Per path, one warp: its contours and points in frame-wide numbering (the scenes' offsets are their
+// own), its flags, and its bounds and tile rect.
 // Outline::bounds (pathfinder/core/data/path.cpp), RectF::intersection and
 // round_rect_out_to_tile_bounds (pathfinder/core/data/data.h:131-133), Tiler::Tiler
 // (pathfinder/core/d3d9/tiler.cpp:317-335).
 
-__global__ void k_path_setup(Batch b, const uint2 *path_contours) {
+__global__ void __launch_bounds__(kThreads) k_paths(Batch b, uint2 *path_contours) {
     const uint32_t p = blockIdx.x * (kThreads / 32) + (threadIdx.x >> 5);
     const int lane = threadIdx.x & 31;
     if (p >= b.n_paths) return;
-    const uint2 cr = path_contours[p];
-    const uint32_t a = b.contour_point_first[cr.x], e = b.contour_point_first[cr.y];
+    const uint32_t pg = b.path_base + p;
+    const uint32_t s = upper_bound(b.scene_path_first + b.scene_base, b.n_scenes + 1, pg) - 1 + b.scene_base;
+    const SceneDev &S = b.scenes[s];
+    const uint32_t local = pg - S.path_first;
+    const uint32_t k0 = b.path_start_cat[S.pstart_base + local], k1 = b.path_start_cat[S.pstart_base + local + 1];
+    const uint32_t c0 = S.contour_first + k0 - b.contour_base, c1 = S.contour_first + k1 - b.contour_base;
+    for (uint32_t c = c0 + lane; c < c1; c += 32) b.contour_path[c] = p;
+    const uint32_t a = S.point_first + b.contour_start_cat[S.cstart_base + k0];
+    const uint32_t e = S.point_first + b.contour_start_cat[S.cstart_base + k1];
     float l = INFINITY, t = INFINITY, r = -INFINITY, bt = -INFINITY;
     bool bad = false;
     for (uint32_t i = a + lane; i < e; i += 32) {
@@ -148,8 +113,21 @@ __global__ void k_path_setup(Batch b, const uint2 *path_contours) {
     bad = __any_sync(0xffffffffu, bad);
     if (lane != 0) return;
     if (bad) atomicOr(&b.status[kStErr], kErrNonFinite);
-    PathDev P = b.paths[p];
-    const SceneDev &S = b.scenes[P.scene];
+    path_contours[p] = make_uint2(c0, c1);
+    PathDev P{};
+    P.scene = s;
+    // occludes: an opaque paint (PaintMetadata::is_opaque): an opaque colour, or a gradient
+    // whose stops are all opaque
+    bool opaque = (b.color[pg] >> 24) == 0xffu;
+    if (b.path_grad && b.path_grad[pg] != kNone) opaque = __float_as_uint(b.grad_meta[4 * b.path_grad[pg] + 3].z) != 0;
+    P.flags = (b.fill_rule[pg] ? 1u : 0u) | (opaque ? 2u : 0u);
+    if (b.path_clip_cat) {
+        // clip paths are tiled like the others but never drawn; a clipped path's clip is in its
+        // scene, addressed here within the frame
+        if (b.path_is_clip_cat[pg]) P.flags |= kPathIsClip;
+        const uint32_t lc = b.path_clip_cat[pg];
+        b.path_clip_rel[p] = lc == kNone ? kNone : S.path_first - b.path_base + lc;
+    }
     float il, it, ir, ib;
     if (e == a) {  // no points: the default (invalid) RectF {1, 1, 0, 0}
         l = 1.0f;
@@ -220,11 +198,19 @@ __global__ void __launch_bounds__(kThreads) k_contour_segments(Batch b, uint32_t
     const uint32_t c = blockIdx.x * (kThreads / kGroup) + threadIdx.x / kGroup;
     uint32_t a = 0, n = 0, out = 0, path = 0;
     if (c < b.n_contours) {
-        a = b.contour_point_first[c];
-        n = b.contour_point_first[c + 1] - a;
-        if (kWrite) {
+        path = b.contour_path[c];
+        if (!kWrite) {
+            // the contour's points in frame-wide numbering, kept for the kernels that follow
+            const SceneDev &S = b.scenes[b.paths[path].scene];
+            const uint32_t *start = b.contour_start_cat + S.cstart_base + (b.contour_base + c - S.contour_first);
+            a = S.point_first + start[0];
+            n = start[1] - start[0];
+            if (l == 0) b.contour_point_first[c] = a;
+            if (l == 0 && c == b.n_contours - 1) b.contour_point_first[b.n_contours] = a + n;
+        } else {
+            a = b.contour_point_first[c];
+            n = b.contour_point_first[c + 1] - a;
             out = b.contour_segs[c];
-            path = b.contour_path[c];
             if (l == 0 && b.path_contours[path].x == c) b.path_seg_first[path] = out;
             if (out > b.seg_cap) n = 0;
         }
@@ -1506,84 +1492,138 @@ __device__ __forceinline__ void add_delta_u16(uint16_t *a, int d, uint32_t *stat
     atomicOr(status, kErrWalk);
 }
 
-// Leaf ranges of every path and the size classes.  Classes 0-2 are listed with one atomic per
-// warp and class; class-3 paths take a 64-bit atomic that also hands out their offsets in the
-// class-3 line numbering the global passes stride over.
-// log2 of a path's leaf lines (its range and its spill-pool lines), after k_bin_classify
-// stored the range
-__device__ __forceinline__ int bin_bucket(const Batch &b, uint32_t p) {
-    const uint2 range = b.path_leaf_range[p];
+// The paths' leaf ranges, size classes and lists.  A listed path's key is its list and the log2 of
+// its leaf lines; the lists are filled bucket by bucket, largest first, from the buckets' counts.
+// Class-3 paths take a 64-bit atomic that also hands out their offsets in the class-3 line
+// numbering the global passes stride over.
+__device__ __forceinline__ uint32_t path_lines(const Batch &b, uint32_t p, uint2 range) {
     uint32_t n = range.y - range.x;
     if (b.pool_cnt) n += b.pool_cnt[p] - b.pool_cnt[(int64_t)p - 1];
-    return 31 - __clz(max(n, 1u));
+    return n;
 }
 
-__global__ void k_bin_classify(Batch b, bool learned) {
-    const uint32_t p = global_tid();
-    const int lane = threadIdx.x & 31;
-    int cls = -1;
-    if (p < b.n_paths) {
-        const PathDev P = b.paths[p];
-        uint2 range;
-        if (learned) {
-            const uint32_t f = b.path_leaf_first[p];
-            range = make_uint2(f, f + min(b.path_leaf_cursor[p], b.path_leaf_budget[p]));
-        } else {
-            const uint2 pc = b.path_contours[p];
-            range = make_uint2(b.seg_leaves[b.contour_segs[pc.x]], b.seg_leaves[b.contour_segs[pc.y]]);
-        }
-        b.path_leaf_range[p] = range;
-        uint32_t n = range.y - range.x;
-        if (b.pool_cnt) n += b.pool_cnt[p] - b.pool_cnt[(int64_t)p - 1];
-        cls = path_class(P, n, bin_warp_lines(b, learned));
-        b.path_cls[p] = (uint8_t)cls;
-        if (cls < 0) b.path_fill[p] = 0;
-        if (cls == 3) {
-            const unsigned long long old = atomicAdd(ctl3_word(b), (1ull << 40) | (unsigned long long)n);
-            const uint32_t item = (uint32_t)(old >> 40);
-            b.bin_list[(size_t)3 * b.n_paths + item] = p;
-            b.bin_list[(size_t)4 * b.n_paths + item] = (uint32_t)(old & kLow40);
-        }
+// Classifies path p; its key, or -1 when it is on no list.
+__device__ __forceinline__ int bin_classify(const Batch &b, uint32_t p, bool learned, uint32_t warp_lines) {
+    const PathDev P = b.paths[p];
+    uint2 range;
+    if (learned) {
+        const uint32_t f = b.path_leaf_first[p];
+        range = make_uint2(f, f + min(b.path_leaf_cursor[p], b.path_leaf_budget[p]));
+    } else {
+        const uint2 pc = b.path_contours[p];
+        range = make_uint2(b.seg_leaves[b.contour_segs[pc.x]], b.seg_leaves[b.contour_segs[pc.y]]);
     }
-    const int list = class_list(cls);
+    b.path_leaf_range[p] = range;
+    const uint32_t n = path_lines(b, p, range);
+    const int cls = path_class(P, n, warp_lines), list = class_list(cls);
+    b.path_cls[p] = (uint8_t)cls;
+    if (cls < 0) b.path_fill[p] = 0;
+    if (cls == 3) {
+        const unsigned long long old = atomicAdd(ctl3_word(b), (1ull << 40) | (unsigned long long)n);
+        const uint32_t item = (uint32_t)(old >> 40);
+        b.bin_list[(size_t)3 * b.n_paths + item] = p;
+        b.bin_list[(size_t)4 * b.n_paths + item] = (uint32_t)(old & kLow40);
+    }
+    return list >= 0 ? list * 32 + (31 - __clz(max(n, 1u))) : -1;
+}
+
+// One warp per list: the buckets' first slots, largest lines first, into start[]; lane 31 returns
+// the list's length.
+__device__ __forceinline__ uint32_t bucket_starts(const uint32_t *count, uint32_t *start, int list, int lane) {
+    const uint32_t v = count[list * 32 + 31 - lane];
+    uint32_t incl = v;
 #pragma unroll
-    for (int c = 0; c < kLists; c++) {
-        const uint32_t m = __ballot_sync(0xffffffffu, list == c);
-        if (m && lane == __ffs(m) - 1) atomicAdd(&b.bin_ctl[kCtlCount + c], (uint32_t)__popc(m));
+    for (int o = 1; o < 32; o <<= 1) {
+        const uint32_t n = __shfl_up_sync(0xffffffffu, incl, o);
+        if (lane >= o) incl += n;
     }
-    // the bucket of a listed path: log2 of its leaf lines
-    const int key = list >= 0 ? list * 32 + bin_bucket(b, p) : -1;
-    const unsigned g = __match_any_sync(0xffffffffu, key);
-    if (key >= 0 && lane == __ffs(g) - 1) atomicAdd(&b.bin_ctl[kCtlBucket + key], (uint32_t)__popc(g));
+    start[list * 32 + 31 - lane] = incl - v;
+    return incl;
 }
 
-// The buckets' cursors, largest lines first within each list.
-__global__ void k_bin_bucket_starts(Batch b) {
-    const int c = threadIdx.x;
-    if (c >= kLists) return;
-    uint32_t off = 0;
-    for (int k = 31; k >= 0; k--) {
-        b.bin_ctl[kCtlCursor + c * 32 + k] = off;
-        off += b.bin_ctl[kCtlBucket + c * 32 + k];
-    }
+__device__ __forceinline__ void copy_status(const Batch &b, const StatusCopy &copy) {
+    for (uint32_t i = threadIdx.x; i < kStHostWords; i += blockDim.x)
+        copy.host[i] = *(const volatile uint32_t *)(b.status + i);
 }
 
-// Each listed path into its list at its bucket's cursor.
-__global__ void k_bin_scatter(Batch b) {
+// A frame of many paths: a pass that classifies and counts, and one that places.
+__global__ void __launch_bounds__(kThreads) k_bin_classify(Batch b, bool learned) {
+    __shared__ uint32_t s_bucket[kLists * 32];
+    if (threadIdx.x < kLists * 32) s_bucket[threadIdx.x] = 0;
+    __syncthreads();
     const uint32_t p = global_tid();
-    const int lane = threadIdx.x & 31;
+    const int key = p < b.n_paths ? bin_classify(b, p, learned, bin_warp_lines(b, learned)) : -1;
+    if (key >= 0) atomicAdd(&s_bucket[key], 1u);
+    __syncthreads();
+    if (threadIdx.x < kLists * 32 && s_bucket[threadIdx.x])
+        atomicAdd(&b.bin_ctl[kCtlBucket + threadIdx.x], s_bucket[threadIdx.x]);
+}
+
+__global__ void __launch_bounds__(kThreads) k_bin_scatter(Batch b, StatusCopy copy) {
+    __shared__ uint32_t s_start[kLists * 32];
+    __shared__ bool s_last;
+    const uint32_t p = global_tid();
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    if (warp < kLists) {
+        const uint32_t n = bucket_starts(b.bin_ctl + kCtlBucket, s_start, warp, lane);
+        if (blockIdx.x == 0 && lane == 31) b.bin_ctl[kCtlCount + warp] = n;
+    }
     int key = -1;
     if (p < b.n_paths) {
         const int list = class_list((int)(int8_t)b.path_cls[p]);
-        if (list >= 0) key = list * 32 + bin_bucket(b, p);
+        if (list >= 0) key = list * 32 + (31 - __clz(max(path_lines(b, p, b.path_leaf_range[p]), 1u)));
     }
     const unsigned g = __match_any_sync(0xffffffffu, key);
-    if (key < 0) return;
     const int leader = __ffs(g) - 1;
     uint32_t base = 0;
-    if (lane == leader) base = atomicAdd(&b.bin_ctl[kCtlCursor + key], (uint32_t)__popc(g));
-    base = __shfl_sync(g, base, leader);
-    list_row(b, key >> 5)[base + __popc(g & ((1u << lane) - 1u))] = p;
+    if (key >= 0 && lane == leader) base = atomicAdd(&b.bin_ctl[kCtlCursor + key], (uint32_t)__popc(g));
+    base = __shfl_sync(0xffffffffu, base, leader);
+    __syncthreads();
+    if (key >= 0) list_row(b, key >> 5)[s_start[key] + base + __popc(g & ((1u << lane) - 1u))] = p;
+    if (!copy.host) return;
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        __threadfence();
+        s_last = atomicAdd(copy.done, 1u) == gridDim.x - 1;
+    }
+    __syncthreads();
+    if (s_last) {
+        __threadfence();
+        copy_status(b, copy);
+    }
+}
+
+// A frame of few paths: both in one block (of up to kOneBlockPaths; 3,000 paths took 12 us in three
+// launches).
+constexpr uint32_t kOneBlockPaths = 4096;
+constexpr int kOneBlockThreads = 1024;
+
+__global__ void __launch_bounds__(kOneBlockThreads) k_bin_lists(Batch b, bool learned, StatusCopy copy) {
+    __shared__ uint32_t s_bucket[kLists * 32], s_start[kLists * 32];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    if (threadIdx.x < kLists * 32) s_bucket[threadIdx.x] = 0;
+    __syncthreads();
+    const uint32_t warp_lines = bin_warp_lines(b, learned);
+    int key[kOneBlockPaths / kOneBlockThreads];
+#pragma unroll
+    for (int k = 0; k < (int)(kOneBlockPaths / kOneBlockThreads); k++) {
+        const uint32_t p = k * kOneBlockThreads + threadIdx.x;
+        key[k] = p < b.n_paths ? bin_classify(b, p, learned, warp_lines) : -1;
+        if (key[k] >= 0) atomicAdd(&s_bucket[key[k]], 1u);
+    }
+    __syncthreads();
+    if (warp < kLists) {
+        const uint32_t n = bucket_starts(s_bucket, s_start, warp, lane);
+        if (lane == 31) b.bin_ctl[kCtlCount + warp] = n;
+    }
+    __syncthreads();
+#pragma unroll
+    for (int k = 0; k < (int)(kOneBlockPaths / kOneBlockThreads); k++)
+        if (key[k] >= 0) list_row(b, key[k] >> 5)[atomicAdd(&s_start[key[k]], 1u)] = k * kOneBlockThreads + threadIdx.x;
+    if (!copy.host) return;
+    __threadfence_block();
+    __syncthreads();
+    copy_status(b, copy);
 }
 
 // The fills of one tile visit, as a binning warp stages them: the visit's points and a word with
@@ -3131,14 +3171,8 @@ void count_launches(uint32_t n) { g_launches += n; }
         count_launches(1);       \
     } while (0)
 
-cudaError_t launch_normalize(const Batch &b, uint2 *path_contours, cudaStream_t st) {
-    if (b.n_contours) PF_LAUNCH(k_normalize_contours<<<grid_for(b.n_contours), kThreads, 0, st>>>(b));
-    if (b.n_paths) PF_LAUNCH(k_normalize_paths<<<grid_for(b.n_paths), kThreads, 0, st>>>(b, path_contours));
-    return cudaGetLastError();
-}
-
-cudaError_t launch_path_setup(const Batch &b, const uint2 *path_contours, cudaStream_t st) {
-    if (b.n_paths) PF_LAUNCH(k_path_setup<<<grid_for(b.n_paths, kThreads / 32), kThreads, 0, st>>>(b, path_contours));
+cudaError_t launch_paths(const Batch &b, uint2 *path_contours, cudaStream_t st) {
+    if (b.n_paths) PF_LAUNCH(k_paths<<<grid_for(b.n_paths, kThreads / 32), kThreads, 0, st>>>(b, path_contours));
     return cudaGetLastError();
 }
 
@@ -3198,11 +3232,12 @@ cudaError_t launch_flatten_budget(const Batch &b, uint32_t n_segs, cudaStream_t 
     return launch_flatten_pool<kPoolLearned>(b, n_segs, st);
 }
 
-cudaError_t launch_bin_classify(const Batch &b, bool learned, cudaStream_t st) {
-    if (b.n_paths) {
+cudaError_t launch_bin_lists(const Batch &b, bool learned, const StatusCopy &copy, cudaStream_t st) {
+    if (b.n_paths <= kOneBlockPaths) {
+        PF_LAUNCH(k_bin_lists<<<1, kOneBlockThreads, 0, st>>>(b, learned, copy));
+    } else {
         PF_LAUNCH(k_bin_classify<<<grid_for(b.n_paths), kThreads, 0, st>>>(b, learned));
-        PF_LAUNCH(k_bin_bucket_starts<<<1, 32, 0, st>>>(b));
-        PF_LAUNCH(k_bin_scatter<<<grid_for(b.n_paths), kThreads, 0, st>>>(b));
+        PF_LAUNCH(k_bin_scatter<<<grid_for(b.n_paths), kThreads, 0, st>>>(b, copy));
     }
     return cudaGetLastError();
 }
@@ -3245,11 +3280,8 @@ static cudaError_t fused_grid(unsigned *grid, uint32_t n_sms, uint32_t n_paths, 
 }
 
 template <int kCls>
-static cudaError_t launch_fused(const Batch &b, unsigned grid, size_t stage_first, cudaStream_t st) {
-    Batch c = b;
-    c.stage += stage_first;
-    c.stage_tile += stage_first;
-    PF_LAUNCH(k_bin_fused<kCls><<<grid, class_threads(kCls), size_t(class_words(kCls)) * 4, st>>>(c));
+static cudaError_t launch_fused(const Batch &b, unsigned grid, cudaStream_t st) {
+    PF_LAUNCH(k_bin_fused<kCls><<<grid, class_threads(kCls), size_t(class_words(kCls)) * 4, st>>>(b));
     return cudaGetLastError();
 }
 
@@ -3325,13 +3357,16 @@ cudaError_t bin_class_max_ctas(int out[3]) {
     return e;
 }
 
-// Class 3 and the cluster class when they can have paths, and the CTA classes, largest rects first, and
-// the small class; at once (bs not null) on streams of their own, joined before the composite,
-// so that the block scheduler fills the SMs that one class's last paths leave idle with the others'.
-cudaError_t launch_bin_paths(const Batch &b, const Tuning &t, BinClasses has, const BinStreams *bs, cudaStream_t st) {
+// Class 3, the cluster class, the CTA classes, largest rects first, and the small class, those that can
+// have paths; at once (bs not null) on streams of their own, joined before the composite, so that the
+// block scheduler fills the SMs that one class's last paths leave idle with the others'.
+cudaError_t launch_bin_paths(const Batch &b, const Tuning &t, const BinClasses &has, const BinStreams *bs,
+                             cudaStream_t st) {
     if (!b.n_paths) return cudaSuccess;
-    unsigned g[3];
+    unsigned g[3], gs = 0, gc = 0;
     cudaError_t e = fused_grids(t, b.n_sms, b.n_paths, g);
+    if (e == cudaSuccess) e = small_grid(&gs, b.n_sms, b.n_paths);
+    if (e == cudaSuccess) e = cluster_grid(&gc, b.n_paths);
     if (e != cudaSuccess) return e;
     if (bs) {
         if ((e = cudaEventRecord(bs->fork, st)) != cudaSuccess) return e;
@@ -3344,29 +3379,25 @@ cudaError_t launch_bin_paths(const Batch &b, const Tuning &t, BinClasses has, co
         PF_LAUNCH(k_bin_large_prep<<<b.n_sms * 2, kPrepThreads, 0, st>>>(b));
         PF_LAUNCH(k_bin_large<true><<<b.n_sms * 8, kThreads, 0, st>>>(b));
     }
-    if (has.cluster) {
-        unsigned gs = 0, gc = 0;
-        if ((e = small_grid(&gs, b.n_sms, b.n_paths)) != cudaSuccess) return e;
-        if ((e = cluster_grid(&gc, b.n_paths)) != cudaSuccess) return e;
-        const size_t first = size_t(g[0]) * class_stage(0) + size_t(g[1]) * class_stage(1) +
-                             size_t(g[2]) * class_stage(2) + size_t(gs) * kSmallWarps * kSmallSpill;
+    // the classes' slices of the stage, as bin_stage_slots sizes them
+    const size_t s1 = size_t(g[2]) * class_stage(2), s0 = s1 + size_t(g[1]) * class_stage(1);
+    const size_t ss = s0 + size_t(g[0]) * class_stage(0), sc = ss + size_t(gs) * kSmallWarps * kSmallSpill;
+    auto slice = [&](size_t first) {
         Batch c = b;
         c.stage += first;
         c.stage_tile += first;
-        PF_LAUNCH(k_bin_cluster<<<gc, kClusterThreads, kClusterSmem, st>>>(c));
+        return c;
+    };
+    if (has.cluster) {
+        PF_LAUNCH(k_bin_cluster<<<std::min(gc, has.cluster * kClusterCtas), kClusterThreads, kClusterSmem, st>>>(slice(sc)));
         if ((e = cudaGetLastError()) != cudaSuccess) return e;
     }
-    const size_t s1 = size_t(g[2]) * class_stage(2), s0 = s1 + size_t(g[1]) * class_stage(1);
-    if ((e = launch_fused<2>(b, g[2], 0, bs ? bs->side[0] : st)) != cudaSuccess) return e;
-    if ((e = launch_fused<1>(b, g[1], s1, st)) != cudaSuccess) return e;
-    if ((e = launch_fused<0>(b, g[0], s0, bs ? bs->side[1] : st)) != cudaSuccess) return e;
+    cudaStream_t const st2 = bs ? bs->side[0] : st, st0 = bs ? bs->side[1] : st;
+    if (has.cta[2] && (e = launch_fused<2>(slice(0), std::min(g[2], has.cta[2]), st2)) != cudaSuccess) return e;
+    if (has.cta[1] && (e = launch_fused<1>(slice(s1), std::min(g[1], has.cta[1]), st)) != cudaSuccess) return e;
+    if (has.cta[0] && (e = launch_fused<0>(slice(s0), std::min(g[0], has.cta[0]), st0)) != cudaSuccess) return e;
     if (has.small) {
-        unsigned gs = 0;
-        if ((e = small_grid(&gs, b.n_sms, b.n_paths)) != cudaSuccess) return e;
-        Batch c = b;
-        c.stage += s0 + size_t(g[0]) * class_stage(0);
-        c.stage_tile += s0 + size_t(g[0]) * class_stage(0);
-        PF_LAUNCH(k_bin_small<<<gs, kSmallThreads, 0, bs ? bs->side[1] : st>>>(c));
+        PF_LAUNCH(k_bin_small<<<std::min(gs, (has.small + kSmallWarps - 1u) / kSmallWarps), kSmallThreads, 0, st0>>>(slice(ss)));
         if ((e = cudaGetLastError()) != cudaSuccess) return e;
     }
     for (int k = 0; bs && k < 2; k++) {

@@ -77,7 +77,7 @@ __global__ void __launch_bounds__(kThreads) k_contour_features(Batch b, float4 *
 }
 
 // One warp per path: features from its contours' sums and its bounds / tile rect (after
-// k_path_setup); they need no segment records, so they are ready before the first host
+// k_paths); they need no segment records, so they are ready before the first host
 // synchronisation of a frame:
 //   0 segments   1 lines   2 quadratics   3 cubics   4 contours   5 box width   6 box height
 //   7 box area   8 control-polygon length   9 summed turning angle   10 tiles in the rect

@@ -45,3 +45,22 @@ def test_classes_match_oracle(renderer, oracle_mod, sizes, n, lines, side):
     got = renderer.canon()
     for key in TILE_KEYS:
         assert np.array_equal(got[key], want[key]), key
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("learned", [False, True])
+@pytest.mark.parametrize("n", [1, 1023, 1024, 1025, 4095, 4096, 4097, 8200])
+def test_lists_by_path_count(pf, oracle_mod, n, learned):
+    """Around one block's threads (1024) and the paths one block lists (4096); every class present."""
+    sizes = [SMALL[i % 12] for i in range(n)]
+    for k, s in enumerate([(33, 33), (66, 66), (130, 130), (513, 34), (256, 2)]):
+        sizes[(k * 997 + 5) % n] = s
+    sc = paths(n, sizes, [3 + i % 9 for i in range(n)], 8400)
+    want = oracle_mod.tile_scene(sc, oracle_mod.Z_D3D11, threads=8)
+    with pf.Renderer() as r:
+        r.sizer_load(pf.DEFAULT_WEIGHTS)
+        r.upload(sc)
+        r.render_learned() if learned else r.render()
+        got = r.canon()
+    for key in TILE_KEYS:
+        assert np.array_equal(got[key], want[key]), key
