@@ -1373,6 +1373,8 @@ constexpr int kCtaClasses = 3;
 // classes 0 and 1; 20.80 ms with 128-thread CTAs, 12 per SM; 20.72 ms with class 0 at 64 threads,
 // 24 per SM).  Class 2 keeps 384 threads: its shared words allow 3 CTAs per SM (256 or 512 threads
 // ran slower).
+// a class's words, and up to 3 before the tiles and 3 after them
+__host__ __device__ constexpr size_t class_smem(int c) { return (size_t(class_words(c)) + 8) * 4; }
 __host__ __device__ constexpr int class_threads(int c) { return c == 2 ? 384 : c == 1 ? 128 : 64; }
 // CTAs per SM the register budget is set for (shared memory allows 3 of class 2, 12 of class 1):
 // class 0 at 20 (48 registers) and class 1 at 8 (64 registers, no spills) beat 24 and 12 at 40
@@ -1636,7 +1638,7 @@ __global__ void __launch_bounds__(class_threads(kCls), class_min_ctas(kCls)) k_b
     constexpr int kThr = class_threads(kCls), kWarps = kThr / 32;
     constexpr uint32_t kStage = class_stage(kCls) / kWarps;  // fills a warp stages
     static_assert(class_words(kCls) <= 65536u, "a staged fill holds its tile in 16 bits");
-    extern __shared__ uint32_t sm[];
+    extern __shared__ __align__(16) uint32_t sm[];
     __shared__ uint32_t s_item, s_base, s_write, s_next, s_over;
     __shared__ uint32_t s_slot[kWarps];
     __shared__ int32_t s_seg[kThr];
@@ -1659,10 +1661,15 @@ __global__ void __launch_bounds__(class_threads(kCls), class_min_ctas(kCls)) k_b
         const PathDev P = b.paths[p];
         const WalkCtx w = walk_ctx(b, P);
         const uint32_t rw = (uint32_t)w.rw, rh = (uint32_t)w.rh, T = rw * rh, tb = P.tile_first, cb = P.col_first;
-        uint32_t *cnt = sm;                                   // per tile: count | delta << 24, then cursor
-        int32_t *above = reinterpret_cast<int32_t *>(sm + T);  // per column
+        // the tiles start as many words into the array as their records in global memory lie past a
+        // multiple of four, so that the passes over them take 16 bytes at a time on both sides; the
+        // words before and after them stay zero
+        const uint32_t pad = tb & 3u, end4 = (pad + T + 3u) & ~3u;
+        uint32_t *cnt = sm + pad;                                 // per tile: count | delta << 24, then cursor
+        int32_t *above = reinterpret_cast<int32_t *>(sm + end4);  // per column
         const PathLeaves L = path_leaves(b, p);
-        for (uint32_t t = tid; t < T + rw; t += kThr) sm[t] = 0;
+        for (uint32_t t = 4 * tid; t < end4 + rw; t += 4 * kThr)
+            *reinterpret_cast<uint4 *>(&sm[t]) = make_uint4(0u, 0u, 0u, 0u);
         if (tid == 0) {
             s_next = 0;
             s_over = 0;
@@ -1724,10 +1731,14 @@ __global__ void __launch_bounds__(class_threads(kCls), class_min_ctas(kCls)) k_b
 
         // 2. the count of each warp's chunk of tiles; thread 0 reserves the path's block of
         //    fills with one atomic whose result it reads only after the column pass
-        const uint32_t chunk = ((T + kWarps - 1) / kWarps + 127u) & ~127u;
-        const uint32_t c0 = min(T, (uint32_t)warp * chunk), c1 = min(T, c0 + chunk);
-        unsigned long long wsum = 0;  // 64-bit: a path's fills need not fit 32 bits (it then overflows)
-        for (uint32_t t = c0 + lane; t < c1; t += 32) wsum += cnt[t] & 0xffffffu;
+        const uint32_t chunk = ((end4 + kWarps - 1) / kWarps + 127u) & ~127u;
+        const uint32_t c0 = min(end4, (uint32_t)warp * chunk), c1 = min(end4, c0 + chunk);
+        uint32_t lsum = 0;  // under 2^8 tiles a lane
+        for (uint32_t t = c0 + 4 * lane; t < c1; t += 128) {
+            const uint4 q = *reinterpret_cast<const uint4 *>(&sm[t]);
+            lsum += (q.x & 0xffffffu) + (q.y & 0xffffffu) + (q.z & 0xffffffu) + (q.w & 0xffffffu);
+        }
+        unsigned long long wsum = lsum;  // 64-bit: a path's fills need not fit 32 bits (it then overflows)
 #pragma unroll
         for (int o = 16; o > 0; o >>= 1) wsum += __shfl_down_sync(0xffffffffu, wsum, o);
         if (lane == 0) s_wsum[warp] = wsum;
@@ -1779,22 +1790,16 @@ __global__ void __launch_bounds__(class_threads(kCls), class_min_ctas(kCls)) k_b
         __syncthreads();
 
         // 4. each warp scans its chunk into write cursors (shared) and end offsets (global): a
-        //    lane takes four consecutive tiles (one 16-byte shared load; chunks start on
-        //    multiples of 128 tiles), and one warp scan covers 128 tiles
+        //    lane takes four consecutive tiles (16 bytes of both), and one warp scan covers 128.
+        //    With the passes over the tiles (zeros, counts, offsets) 16 bytes wide on both sides
+        //    binning takes 7.64 ms instead of 7.93 on 256 scenes, whose large rects have more
+        //    tiles than fills
         uint32_t carry = s_base + s_warp[warp];
         for (uint32_t t0 = c0; t0 < c1; t0 += 128) {
             const uint32_t t = t0 + 4 * (uint32_t)lane;
-            uint32_t v[4];
-            if (t + 4 <= c1) {
-                const uint4 q = *reinterpret_cast<const uint4 *>(&cnt[t]);
-                v[0] = q.x & 0xffffffu;
-                v[1] = q.y & 0xffffffu;
-                v[2] = q.z & 0xffffffu;
-                v[3] = q.w & 0xffffffu;
-            } else {
-#pragma unroll
-                for (int j = 0; j < 4; j++) v[j] = t + j < c1 ? (cnt[t + j] & 0xffffffu) : 0u;
-            }
+            const bool in = t < c1;
+            const uint4 q = in ? *reinterpret_cast<const uint4 *>(&sm[t]) : make_uint4(0u, 0u, 0u, 0u);
+            const uint32_t v[4] = {q.x & 0xffffffu, q.y & 0xffffffu, q.z & 0xffffffu, q.w & 0xffffffu};
             const uint32_t own = v[0] + v[1] + v[2] + v[3];
             uint32_t incl = own;
 #pragma unroll
@@ -1806,16 +1811,17 @@ __global__ void __launch_bounds__(class_threads(kCls), class_min_ctas(kCls)) k_b
             e[0] = carry + incl - own;
 #pragma unroll
             for (int j = 0; j < 4; j++) e[j + 1] = e[j] + v[j];
-            if (t + 4 <= c1) {
-                *reinterpret_cast<uint4 *>(&cnt[t]) = make_uint4(e[0], e[1], e[2], e[3]);
-            } else {
+            if (in) {
+                *reinterpret_cast<uint4 *>(&sm[t]) = make_uint4(e[0], e[1], e[2], e[3]);
+                uint32_t *const fills = b.tile_fills + (tb - pad) + t;
+                if (t >= pad && t + 4 <= pad + T) {
+                    *reinterpret_cast<uint4 *>(fills) = make_uint4(e[1], e[2], e[3], e[4]);
+                } else {
 #pragma unroll
-                for (int j = 0; j < 4; j++)
-                    if (t + j < c1) cnt[t + j] = e[j];
+                    for (int j = 0; j < 4; j++)
+                        if (t + j >= pad && t + j < pad + T) fills[j] = e[j + 1];
+                }
             }
-#pragma unroll
-            for (int j = 0; j < 4; j++)
-                if (t + j < c1) b.tile_fills[tb + t + j] = e[j + 1];
             carry += __shfl_sync(0xffffffffu, incl, 31);
         }
         __syncthreads();
@@ -3245,7 +3251,7 @@ cudaError_t launch_bin_lists(const Batch &b, bool learned, const StatusCopy &cop
 // CTAs of a class that one SM holds.
 template <int kCls>
 static cudaError_t fused_per_sm(int *per_sm) {
-    const size_t smem = size_t(class_words(kCls)) * 4;
+    const size_t smem = class_smem(kCls);
     static std::atomic<uint64_t> configured{0};  // devices the kernel's shared memory is set up on, and
     static std::atomic<int> known[64];           // what fits there
     int dev = 0;
@@ -3281,7 +3287,7 @@ static cudaError_t fused_grid(unsigned *grid, uint32_t n_sms, uint32_t n_paths, 
 
 template <int kCls>
 static cudaError_t launch_fused(const Batch &b, unsigned grid, cudaStream_t st) {
-    PF_LAUNCH(k_bin_fused<kCls><<<grid, class_threads(kCls), size_t(class_words(kCls)) * 4, st>>>(b));
+    PF_LAUNCH(k_bin_fused<kCls><<<grid, class_threads(kCls), class_smem(kCls), st>>>(b));
     return cudaGetLastError();
 }
 
