@@ -1271,7 +1271,7 @@ int render_exact(Ctx *c, uint32_t first, uint32_t count, pf_frame_stats *stats) 
     Batch b = make_batch(c);
     PF_CUDA(launch_contour_segments(b, c->r_points, true, st));
     PF_CUDA(launch_rows(b, true, st));
-    const bool shallow = uint64_t(c->h_status[kStSampledDeep]) * 64 < c->h_status[kStSampled];
+    const bool shallow = uint64_t(c->h_status[kStSampledDeep]) * 1024 < c->h_status[kStSampled];
     PF_CUDA(launch_flatten(b, c->n_segs, false, shallow, st));
     if (c->n_segs > c->r_points) return fail(c, PF_ERR_CUDA, "more segments than points");
     if (int e = scan_frame(c, {{b.seg_leaves, c->n_segs, kStLeaves, true}}, false)) return e;

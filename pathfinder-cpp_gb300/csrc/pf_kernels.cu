@@ -80,37 +80,78 @@ inline unsigned grid_for(uint64_t n, int threads = kThreads) {
 // round_rect_out_to_tile_bounds (pathfinder/core/data/data.h:131-133), Tiler::Tiler
 // (pathfinder/core/d3d9/tiler.cpp:317-335).
 
-__global__ void __launch_bounds__(kThreads) k_paths(Batch b, uint2 *path_contours) {
-    const uint32_t p = blockIdx.x * (kThreads / 32) + (threadIdx.x >> 5);
-    const int lane = threadIdx.x & 31;
-    if (p >= b.n_paths) return;
-    const uint32_t pg = b.path_base + p;
-    const uint32_t s = upper_bound(b.scene_path_first + b.scene_base, b.n_scenes + 1, pg) - 1 + b.scene_base;
-    const SceneDev &S = b.scenes[s];
-    const uint32_t local = pg - S.path_first;
-    const uint32_t k0 = b.path_start_cat[S.pstart_base + local], k1 = b.path_start_cat[S.pstart_base + local + 1];
-    const uint32_t c0 = S.contour_first + k0 - b.contour_base, c1 = S.contour_first + k1 - b.contour_base;
-    for (uint32_t c = c0 + lane; c < c1; c += 32) b.contour_path[c] = p;
-    const uint32_t a = S.point_first + b.contour_start_cat[S.cstart_base + k0];
-    const uint32_t e = S.point_first + b.contour_start_cat[S.cstart_base + k1];
-    float l = INFINITY, t = INFINITY, r = -INFINITY, bt = -INFINITY;
-    bool bad = false;
-    for (uint32_t i = a + lane; i < e; i += 32) {
-        const float2 q = b.points[i];
-        bad |= !(isfinite(q.x) && isfinite(q.y));
-        l = fminf(l, q.x);
-        t = fminf(t, q.y);
-        r = fmaxf(r, q.x);
-        bt = fmaxf(bt, q.y);
+// A path of many points is read by its block: a dashed path can have 100,000, and one warp on it
+// outlasted the other 19,000 paths (set-up of a stroked batch 0.42 -> 0.19 ms).
+constexpr uint32_t kWarpPoints = 4096;
+constexpr int kPathThreads = 128;
+
+struct PointBox {
+    float l = INFINITY, t = INFINITY, r = -INFINITY, b = -INFINITY;
+    uint32_t bad = 0;
+    __device__ __forceinline__ void add(const float2 *points, uint32_t i, uint32_t e, uint32_t step) {
+#pragma unroll 4
+        for (; i < e; i += step) {
+            const float2 q = points[i];
+            bad |= !(isfinite(q.x) && isfinite(q.y));
+            l = fminf(l, q.x);
+            t = fminf(t, q.y);
+            r = fmaxf(r, q.x);
+            b = fmaxf(b, q.y);
+        }
     }
+    __device__ __forceinline__ void reduce() {
 #pragma unroll
-    for (int d = 16; d > 0; d >>= 1) {
-        l = fminf(l, __shfl_xor_sync(0xffffffffu, l, d));
-        t = fminf(t, __shfl_xor_sync(0xffffffffu, t, d));
-        r = fmaxf(r, __shfl_xor_sync(0xffffffffu, r, d));
-        bt = fmaxf(bt, __shfl_xor_sync(0xffffffffu, bt, d));
+        for (int d = 16; d > 0; d >>= 1) {
+            l = fminf(l, __shfl_xor_sync(0xffffffffu, l, d));
+            t = fminf(t, __shfl_xor_sync(0xffffffffu, t, d));
+            r = fmaxf(r, __shfl_xor_sync(0xffffffffu, r, d));
+            b = fmaxf(b, __shfl_xor_sync(0xffffffffu, b, d));
+        }
+        bad = __any_sync(0xffffffffu, bad);
     }
-    bad = __any_sync(0xffffffffu, bad);
+};
+
+__global__ void __launch_bounds__(kPathThreads) k_paths(Batch b, uint2 *path_contours) {
+    __shared__ uint2 s_long[kPathThreads / 32];
+    __shared__ PointBox s_box[kPathThreads / 32];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const uint32_t p = blockIdx.x * (kPathThreads / 32) + warp;
+    const uint32_t pg = b.path_base + p;
+    uint32_t s = 0, c0 = 0, c1 = 0, a = 0, e = 0;
+    if (p < b.n_paths) {
+        s = upper_bound(b.scene_path_first + b.scene_base, b.n_scenes + 1, pg) - 1 + b.scene_base;
+        const SceneDev &S = b.scenes[s];
+        const uint32_t local = pg - S.path_first;
+        const uint32_t k0 = b.path_start_cat[S.pstart_base + local], k1 = b.path_start_cat[S.pstart_base + local + 1];
+        c0 = S.contour_first + k0 - b.contour_base;
+        c1 = S.contour_first + k1 - b.contour_base;
+        for (uint32_t c = c0 + lane; c < c1; c += 32) b.contour_path[c] = p;
+        a = S.point_first + b.contour_start_cat[S.cstart_base + k0];
+        e = S.point_first + b.contour_start_cat[S.cstart_base + k1];
+    }
+    PointBox box;
+    const bool many = e > a && e - a > kWarpPoints;
+    if (!many) box.add(b.points, a + lane, e, 32);
+    if (__syncthreads_or(many)) {
+        if (lane == 0) s_long[warp] = many ? make_uint2(a, e) : make_uint2(0u, 0u);
+        __syncthreads();
+        for (int k = 0; k < kPathThreads / 32; k++) {
+            const uint2 range = s_long[k];
+            if (range.x == range.y) continue;
+            PointBox part;
+            part.add(b.points, range.x + threadIdx.x, range.y, kPathThreads);
+            part.reduce();
+            if (lane == 0) s_box[warp] = part;
+            __syncthreads();
+            if (k == warp && lane < kPathThreads / 32) box = s_box[lane];
+            __syncthreads();
+        }
+    }
+    box.reduce();
+    if (p >= b.n_paths) return;
+    const SceneDev &S = b.scenes[s];
+    float l = box.l, t = box.t, r = box.r, bt = box.b;
+    const bool bad = box.bad;
     if (lane != 0) return;
     if (bad) atomicOr(&b.status[kStErr], kErrNonFinite);
     path_contours[p] = make_uint2(c0, c1);
@@ -3178,7 +3219,7 @@ void count_launches(uint32_t n) { g_launches += n; }
     } while (0)
 
 cudaError_t launch_paths(const Batch &b, uint2 *path_contours, cudaStream_t st) {
-    if (b.n_paths) PF_LAUNCH(k_paths<<<grid_for(b.n_paths, kThreads / 32), kThreads, 0, st>>>(b, path_contours));
+    if (b.n_paths) PF_LAUNCH(k_paths<<<grid_for(b.n_paths, kPathThreads / 32), kPathThreads, 0, st>>>(b, path_contours));
     return cudaGetLastError();
 }
 
@@ -3220,10 +3261,10 @@ static cudaError_t launch_flatten_pool(const Batch &b, uint32_t n_segs, cudaStre
 }
 
 // Exact frame.  Segments that bisect deeply are shared by the lanes of a warp; where nearly all are
-// shallow (under 1 in 64 of the sampled ones takes more than 8 lines), one segment per thread keeps
+// shallow (under 1 in 1,024 of the sampled ones takes more than 8 lines), one segment per thread keeps
 // more of them in flight (count and write pass with their segments, GB300: 150,000 glyphs, none
-// deep, 0.24 ms against 0.36 shared; stroked batch, 1.8 lines per segment but some deep, 0.72
-// against 0.60; 20,000 paths, 25 per segment, 0.80 against 0.46).
+// deep, 0.22 ms against 0.36 shared; stroked batch, 1.8 lines per segment but between 1 in 64 and 1 in
+// 256 deep, 0.69 against 0.57; 20,000 paths, 25 per segment, 0.80 against 0.44).
 cudaError_t launch_flatten(const Batch &b, uint32_t n_segs, bool write, bool shallow, cudaStream_t st) {
     if (!n_segs) return cudaSuccess;
     if (!shallow)
