@@ -258,6 +258,18 @@ cudaError_t scan_jobs(ScanJobs &jobs, cudaStream_t st);
 cudaError_t scan_exclusive_u32(const uint32_t *in, uint32_t *out, uint32_t n, uint32_t *total, void *temp,
                                cudaStream_t st, uint32_t *err);
 
+// Ranges of a staging buffer and where they go: bytes [first, end) to dst.  first and dst are equal
+// modulo 16, and no two ranges share 16 aligned bytes of the buffer.
+constexpr uint32_t kCopySegs = 32;
+struct CopySegs {
+    uint32_t n;
+    struct {
+        uint8_t *dst;
+        uint32_t first, end;
+    } s[kCopySegs];
+};
+cudaError_t launch_unstage(const uint8_t *src, const CopySegs &c, cudaStream_t st);
+
 // Stroke-to-fill and dashing at upload (pf_stroke.cu).  Inputs: the uploaded outline in the
 // upload's per-scene layout; outputs: the dashed contours, one job per output contour, and the
 // new outline.

@@ -3483,6 +3483,30 @@ __global__ void k_gather_words(uint32_t *dst, WordSources s) {
     if (threadIdx.x < s.n) dst[threadIdx.x] = *s.p[threadIdx.x];
 }
 
+// Spreads a mapped host buffer over device buffers.  Bound by the link's latency and rate; 16 bytes a
+// thread, so that even a small upload has all its reads in flight.
+__global__ void __launch_bounds__(256) k_unstage(const uint8_t *src, CopySegs c) {
+    const uint32_t step = gridDim.x * blockDim.x * 16u, end = c.s[c.n - 1].end;
+    uint32_t k = 0;
+    for (uint32_t at = (c.s[0].first & ~15u) + (blockIdx.x * blockDim.x + threadIdx.x) * 16u; at < end; at += step) {
+        while (c.s[k].end <= at) k++;  // ends: the last range's end is above at
+        const uint32_t lo = max(at, c.s[k].first), hi = min(at + 16u, c.s[k].end);
+        uint8_t *const dst = c.s[k].dst + ((int64_t)at - (int64_t)c.s[k].first);
+        if (hi - lo == 16u && lo < hi) {
+            *reinterpret_cast<uint4 *>(dst) = *reinterpret_cast<const uint4 *>(src + at);
+        } else {
+            for (uint32_t i = lo; i < hi; i++) dst[i - at] = src[i];
+        }
+    }
+}
+
+cudaError_t launch_unstage(const uint8_t *src, const CopySegs &c, cudaStream_t st) {
+    if (!c.n) return cudaSuccess;
+    const uint32_t units = (c.s[c.n - 1].end - (c.s[0].first & ~15u) + 15) / 16;
+    PF_LAUNCH(k_unstage<<<std::min<uint32_t>((units + 255) / 256, 1216), 256, 0, st>>>(src, c));
+    return cudaGetLastError();
+}
+
 cudaError_t launch_copy_bytes(uint8_t *dst, const uint8_t *src, uint32_t n, cudaStream_t st) {
     if (n) PF_LAUNCH(k_copy_bytes<<<std::min<uint32_t>((n + 255) / 256, 64), 256, 0, st>>>(dst, src, n));
     return cudaGetLastError();
