@@ -21,6 +21,8 @@
 // bit: Segment::offset and its helpers (core/stroke.cpp:370-540), LineSegmentF
 // (core/data/line_segment.cpp), Segment (core/data/segment.cpp), Mat2 / Transform2 /
 // UnitVector (common/math).
+#include <type_traits>
+
 #include "pf_internal.h"
 
 namespace pfc {
@@ -179,6 +181,19 @@ __device__ void ssplit(const Seg &s, float t, Seg &a, Seg &b) {
         a = Seg{ls(p0, p0123), ls(p01, p012), kCubic};
         b = Seg{ls(p0123, p3), ls(p123, p23), kCubic};
     }
+}
+// the same for t < 1
+__device__ __forceinline__ void split_below(const Seg &s, float t, Seg &a, Seg &b) {
+    if (s.kind != kCubic || t <= 0.0f) {
+        ssplit(s, t, a, b);
+        return;
+    }
+    const V2 p0 = s.b.f, p3 = s.b.t, p1 = s.c.f, p2 = s.c.t;
+    const V2 p01 = lerp_t(p0, p1, t), p12 = lerp_t(p1, p2, t), p23 = lerp_t(p2, p3, t);
+    const V2 p012 = lerp_t(p01, p12, t), p123 = lerp_t(p12, p23, t);
+    const V2 p0123 = lerp_t(p012, p123, t);
+    a = Seg{ls(p0, p0123), ls(p01, p012), kCubic};
+    b = Seg{ls(p0123, p3), ls(p123, p23), kCubic};
 }
 __device__ __forceinline__ V2 ssample(const Seg &s, float t) {  // :160-165
     Seg a, b;
@@ -539,13 +554,16 @@ __device__ __forceinline__ uint2 path_contours(const StrokeIn &in, uint32_t p) {
 //   would take turns, as they meet segments of different kinds, while warps run side by side, and
 //   the lanes share what a step has of the same kind: the square roots of a curve's four legs
 //   (serial ones took a third of a step), a quadratic's divisions, the points to store;
-// * no state beside the segment in hand: points go straight out, not through a contour's ring;
+// * no state beside the segment in hand: pieces stay in the lanes, a point each, until the next would
+//   not fit, and all then go out together; the loop over a segment knows its kind and selects rather
+//   than branches, since a lone warp waits out each branch (a step is some 130 instructions);
 // * the path is walked once.  Its points go to chunks of kDashChunk points, taken from a pool as
 //   they are needed (the next one a chunk ahead), and k_dash_gather copies them to the path's place
 //   once the counts are scanned.  A pool that runs out costs a second walk, straight to that place.
 //
 // (5,689 dashed paths, 1.3M points, the longest of 4,000 steps: 5.65 ms for the two passes of one
-// path per lane, 2.30 ms with a warp per path walked by one lane, 1.83 by all.)
+// path per lane, 2.30 ms with a warp per path walked by one lane, 1.85 by all with each piece put out
+// by itself, 1.42 so; all with the ordering by size before and the gather after.)
 
 // Segment::arc_length (core/data/segment.cpp:141-187) of a segment all lanes hold; lane l % 4 takes
 // leg l of the control polygon (quadratics through to_cubic).
@@ -595,92 +613,136 @@ __global__ void __launch_bounds__(64) k_dash(StrokeIn in, uint32_t *status) {
         return;
     }
     float left = offset;
-    float ahead = dashes[idx + 1 == count ? 0 : idx + 1];  // the next entry of the pattern
-    uint32_t pts = 0, cnt = 0;      // points and contours of the path so far
-    uint32_t contour = 0;           // points of the contour in hand
+    uint32_t next = idx + 1 == count ? 0u : idx + 1;  // the next entry of the pattern
+    float ahead = dashes[next];
     const uint32_t pt0 = kWrite ? in.dash_pts[p] : 0u, c0 = kWrite ? in.dash_cnt[p] : 0u;
+    uint32_t pts = 0, begun = 0;  // points of the path so far, and the contours they begin
+    bool open = false;            // the last of those contours has not ended
     // count pass: the chunk in hand, and the next one (lane 0)
     uint32_t chunk = 0, next_chunk = 0;
     if (!kWrite && lane == 0) next_chunk = atomicAdd(in.dash_chunk_count, 1u);
-    auto put_seg = [&](const Seg &s) {  // core/data/contour.cpp:11-41: a point per lane
-        const uint32_t n = s.kind == kLine ? 2u : s.kind == kQuad ? 3u : 4u;
-        const bool mine = lane < n;
-        const V2 q = lane == 0 ? s.b.f : lane + 1 == n ? s.b.t : lane == 1 ? s.c.f : s.c.t;
-        const uint8_t f = lane == 0 || lane + 1 == n ? kOn : lane == 1 ? kC0 : kC1;
-        if (__any_sync(0xffffffffu, mine && !(isfinite(q.x) && isfinite(q.y)))) return;  // svalid
+    // the pieces since the last drain: a point per lane, the lanes where pieces begin, and those
+    // whose points end a contour
+    float2 point = make_float2(0.0f, 0.0f);
+    uint32_t flag = 0, held = 0;
+    unsigned firsts = 0, ends = 0;
+    auto drain = [&]() {
+        const bool mine = lane < held;
+        unsigned live = held == 32 ? 0xffffffffu : (1u << held) - 1u;
+        unsigned bad = __ballot_sync(0xffffffffu, mine && !(isfinite(point.x) && isfinite(point.y)));
+        while (bad) {  // svalid: the pieces with such points are not pushed
+            const int f = 31 - __clz(firsts & (0xffffffffu >> __clz(bad)));
+            const unsigned above = firsts & ~(0xffffffffu >> (31 - f));
+            const unsigned piece = (above ? (above & -above) - 1u : 0xffffffffu) & ~((1u << f) - 1u);
+            live &= ~piece;
+            bad &= ~piece;
+        }
+        const unsigned below = (1u << lane) - 1u;
+        const unsigned cut = ends & below;  // contour ends before this lane's point
+        const unsigned since = cut ? below & ~(0xffffffffu >> __clz(cut)) : below;
+        const bool out = live >> lane & 1u, first = out && (cut || !open) && !(live & since);
+        const unsigned starts = __ballot_sync(0xffffffffu, first);
+        const uint32_t n = __popc(live), at = pts + __popc(live & below);
         if (kWrite) {
-            if (mine) {
-                in.dash_points[pt0 + pts + lane] = make_float2(q.x, q.y);
-                in.dash_flags[pt0 + pts + lane] = f;
+            if (out) {
+                in.dash_points[pt0 + at] = point;
+                in.dash_flags[pt0 + at] = (uint8_t)flag;
+                // a contour ends where the next begins
+                const uint32_t k = begun + __popc(starts & below);
+                if (first && k > 0) in.dash_end[c0 + k - 1] = pt0 + at;
             }
         } else {
-            const uint32_t at = pts + lane, border = (pts + kDashChunk - 1) / kDashChunk * kDashChunk;
+            const uint32_t border = (pts + kDashChunk - 1) / kDashChunk * kDashChunk;
             uint32_t mychunk = chunk;
             if (pts + n > border) {  // the next chunk begins among these points
                 chunk = __shfl_sync(0xffffffffu, next_chunk, 0);
                 if (at >= border) mychunk = chunk;
+                const unsigned before = __ballot_sync(0xffffffffu, first && at < border);
                 if (lane == 0) {
                     if (chunk < in.dash_chunk_cap)
-                        in.dash_chunk_head[chunk] =
-                            make_uint4(p, border, cnt + (contour + (border - pts) != 0 ? 1u : 0u), 0u);
+                        in.dash_chunk_head[chunk] = make_uint4(p, border, begun + __popc(before), 0u);
                     next_chunk = atomicAdd(in.dash_chunk_count, 1u);
                 }
             }
-            if (mine && mychunk < in.dash_chunk_cap) {
+            if (out && mychunk < in.dash_chunk_cap) {
                 const uint32_t slot = mychunk * kDashChunk + at % kDashChunk;
-                in.dash_chunk_points[slot] = make_float2(q.x, q.y);
-                // bit 7: the first point of a contour
-                in.dash_chunk_flags[slot] = f | (contour == 0 && lane == 0 ? 0x80u : 0u);
+                in.dash_chunk_points[slot] = point;
+                in.dash_chunk_flags[slot] = (uint8_t)(flag | (first ? 0x80u : 0u));  // bit 7: of a contour
             }
         }
+        begun += __popc(starts);
+        const unsigned tail = ends ? ~(0xffffffffu >> __clz(ends)) : 0xffffffffu;
+        open = (live & tail) || (!ends && open);
         pts += n;
-        contour += n;
+        held = 0;
+        firsts = ends = 0;
     };
     uint32_t steps = 0;
-    auto flush = [&]() {  // Outline::push_contour: empty contours are dropped
-        if (contour == 0) return;
-        if (kWrite && lane == 0) in.dash_end[c0 + cnt] = pt0 + pts;
-        cnt++;
-        contour = 0;
+    bool failed = false;
+    auto end_contour = [&]() {  // Outline::push_contour: empty contours are dropped
+        if (held) ends |= 1u << (held - 1);
+        else open = false;
+    };
+    // one segment, of a kind the compiler knows
+    auto walk = [&](Seg rest, auto kind) {
+        constexpr int kKind = decltype(kind)::value;
+        constexpr uint32_t kN = kKind == kLine ? 2u : kKind == kQuad ? 3u : 4u;
+        rest.kind = kKind;
+        bool more;
+        do {
+            const float length = warp_arc_length(rest);
+            float distance = left;
+            const float t = fd(left, length);
+            Seg piece = rest;
+            more = t < 1.0f;
+            if (more) split_below(Seg(rest), t, piece, rest);
+            else distance = length;
+            // core/data/contour.cpp:11-41: a point per lane.  Selects, not branches: a lone warp
+            // waits out each branch
+            const bool on = (idx & 1u) == 0;
+            if (on && held + kN > 32) drain();
+            const uint32_t k = on ? lane - held : kN;
+            const V2 q = k == 0 ? piece.b.f : k + 1 == kN ? piece.b.t : k == 1 ? piece.c.f : piece.c.t;
+            point.x = k < kN ? q.x : point.x;
+            point.y = k < kN ? q.y : point.y;
+            flag = k < kN ? (k == 0 || k + 1 == kN ? kOn : k == 1 ? kC0 : kC1) : flag;
+            firsts |= on ? 1u << held : 0u;
+            held += on ? kN : 0u;
+            left = fs(left, distance);
+            const bool over = left < kFloatEps;  // the dash (or gap) ends: flush() of an even one
+            ends |= on && over && held ? 1u << ((held - 1) & 31u) : 0u;
+            open = open && !(on && over && !held);
+            idx = over ? next : idx;
+            next = over ? (next + 1 == count ? 0u : next + 1) : next;
+            left = over ? ahead : left;
+            if (over) ahead = dashes[next];
+        } while (++steps < kDashStepLimit && more);
+        failed = more;
     };
     const uint2 kr = path_contours(in, p);
     for (uint32_t k = kr.x; k < kr.y; k++) {
         const Contour c = raw_contour(in, k);
         // ContourDash::dash, dash.cpp:68-124
         SegIter it{&c, 0, true};
-        while (it.has_next) {
-            Seg rest = it.next();
-            if (rest.kind == kNone) break;
-            for (bool more = true; more;) {
-                if (++steps > kDashStepLimit) {
-                    if (lane == 0) atomicOr(&status[kStErr], kErrStroke);
-                    return;
-                }
-                const float length = warp_arc_length(rest);
-                float distance = left;
-                const float t = fd(left, length);
-                Seg piece = rest;
-                if (t < 1.0f) {
-                    ssplit(Seg(rest), t, piece, rest);
-                } else {
-                    distance = length;
-                    more = false;
-                }
-                if (idx % 2 == 0) put_seg(piece);
-                left = fs(left, distance);
-                if (left < kFloatEps) {
-                    if (idx % 2 == 0) flush();
-                    idx = idx + 1 == count ? 0 : idx + 1;
-                    left = ahead;
-                    ahead = dashes[idx + 1 == count ? 0 : idx + 1];
-                }
-            }
+        while (it.has_next && !failed) {
+            const Seg s = it.next();
+            if (s.kind == kNone) break;
+            if (steps >= kDashStepLimit) failed = true;
+            else if (s.kind == kLine) walk(s, std::integral_constant<int, kLine>{});
+            else if (s.kind == kQuad) walk(s, std::integral_constant<int, kQuad>{});
+            else walk(s, std::integral_constant<int, kCubic>{});
         }
     }
-    if (idx % 2 == 0) flush();  // OutlineDash::into_outline, dash.cpp:57-63
+    if (failed) {
+        if (lane == 0) atomicOr(&status[kStErr], kErrStroke);
+        return;
+    }
+    if (idx % 2 == 0) end_contour();  // OutlineDash::into_outline, dash.cpp:57-63
+    drain();
+    if (kWrite && lane == 0 && begun > 0) in.dash_end[c0 + begun - 1] = pt0 + pts;
     if (!kWrite && lane == 0) {
         in.dash_pts[p] = pts;
-        in.dash_cnt[p] = cnt;
+        in.dash_cnt[p] = begun;
         // 64-bit total beside the 32-bit scan, so that an overflowing batch is caught
         atomicAdd(reinterpret_cast<unsigned long long *>(status + kStFill64), (unsigned long long)pts);
     }
@@ -1227,26 +1289,36 @@ __global__ void __launch_bounds__(256) k_order(StrokeIn in, uint32_t *ctl, uint3
 }
 
 // Each block's first slot per bucket, largest bucket first; ctl[kOrderBuckets * kOrderBlocks]
-// receives the number of items placed.
-__global__ void k_order_starts(uint32_t *ctl) {
+// receives the number of items placed.  A warp per bucket, all its counts in registers (a thread per
+// bucket, one count after the other, took 21 us).
+__global__ void __launch_bounds__(kOrderBuckets * 32) k_order_starts(uint32_t *ctl) {
+    constexpr int kRounds = kOrderBlocks / 32;
+    static_assert(kOrderBlocks % 32 == 0, "whole warps of blocks");
     __shared__ uint32_t total[kOrderBuckets];
-    const int bk = threadIdx.x;
-    if (bk < kOrderBuckets) {
-        uint32_t t = 0;
-        for (int blk = 0; blk < kOrderBlocks; blk++) t += ctl[kOrderBuckets * blk + bk];
-        total[bk] = t;
-    }
-    __syncthreads();
-    if (bk < kOrderBuckets) {
-        uint32_t run = 0;
-        for (int d = kOrderBuckets - 1; d > bk; d--) run += total[d];
-        for (int blk = 0; blk < kOrderBlocks; blk++) {
-            const uint32_t c = ctl[kOrderBuckets * blk + bk];
-            ctl[kOrderBuckets * blk + bk] = run;
-            run += c;
+    const int bk = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    uint32_t own[kRounds], incl[kRounds], t = 0;
+#pragma unroll
+    for (int r = 0; r < kRounds; r++) own[r] = ctl[kOrderBuckets * (r * 32 + lane) + bk];
+#pragma unroll
+    for (int r = 0; r < kRounds; r++) {
+        incl[r] = own[r];
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const uint32_t v = __shfl_up_sync(0xffffffffu, incl[r], o);
+            if (lane >= o) incl[r] += v;
         }
-        if (bk == 0) ctl[kOrderBuckets * kOrderBlocks] = run;
+        t += __shfl_sync(0xffffffffu, incl[r], 31);
     }
+    if (lane == 0) total[bk] = t;
+    __syncthreads();
+    uint32_t run = 0;
+    for (int d = kOrderBuckets - 1; d > bk; d--) run += total[d];
+#pragma unroll
+    for (int r = 0; r < kRounds; r++) {
+        ctl[kOrderBuckets * (r * 32 + lane) + bk] = run + incl[r] - own[r];
+        run += __shfl_sync(0xffffffffu, incl[r], 31);
+    }
+    if (bk == 0 && lane == 0) ctl[kOrderBuckets * kOrderBlocks] = run;
 }
 
 // The new outline's per-scene offset arrays (the layout the upload uses: scene s's contour
@@ -1308,12 +1380,12 @@ cudaError_t launch_stroke_order(const StrokeIn &in, int what, uint32_t *ctl, uin
     if (what == 0) {
         if (!in.n_units) return cudaSuccess;
         k_order<0, false><<<kOrderBlocks, 256, 0, st>>>(in, ctl, order);
-        k_order_starts<<<1, 32, 0, st>>>(ctl);
+        k_order_starts<<<1, kOrderBuckets * 32, 0, st>>>(ctl);
         k_order<0, true><<<kOrderBlocks, 256, 0, st>>>(in, ctl, order);
     } else {
         if (!in.n_paths) return cudaSuccess;
         k_order<1, false><<<kOrderBlocks, 256, 0, st>>>(in, ctl, order);
-        k_order_starts<<<1, 32, 0, st>>>(ctl);
+        k_order_starts<<<1, kOrderBuckets * 32, 0, st>>>(ctl);
         k_order<1, true><<<kOrderBlocks, 256, 0, st>>>(in, ctl, order);
     }
     count_launches(3);
