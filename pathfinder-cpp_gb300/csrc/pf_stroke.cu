@@ -339,8 +339,10 @@ __device__ bool within_tol(const Seg &s, const Seg &o, float d) {
     float lo = fs(fabsf(d), kStrokeTol), hi = fa(fabsf(d), kStrokeTol);
     lo = lo <= 0.0f ? 0.0f : fm(lo, lo);
     hi = hi <= 0.0f ? 0.0f : fm(hi, hi);
+    // unrolled: the parameters, their divisions and the splits' tests of them are then constants
+#pragma unroll
     for (uint32_t k = 0; k < kSamples + 1; k++) {
-        const float t = fd((float)k, (float)kSamples);
+        const float t = (float)k / (float)kSamples;
         const float sq = vsqlen(vsub(ssample(s, t), ssample(o, t)));
         if (sq < lo || sq > hi) return false;
     }
@@ -778,52 +780,56 @@ __global__ void __launch_bounds__(256) k_dash_gather(StrokeIn in) {
 // --- Jobs --------------------------------------------------------------------------------
 // count: job_first[p] = output contours of path p.  fill: the jobs (x: first point, y: points,
 // z: kind | closed << 2 | from the dash buffer << 3, w: path).
+// A warp per path: a dashed one can have thousands of contours, which kept its thread at it for 150 us.
 template <bool kFill>
-__global__ void k_stroke_jobs(StrokeIn in) {
-    const uint32_t p = blockIdx.x * blockDim.x + threadIdx.x;
+__global__ void __launch_bounds__(128) k_stroke_jobs(StrokeIn in) {
+    const uint32_t p = blockIdx.x * 4 + (threadIdx.x >> 5);
+    const uint32_t lane = threadIdx.x & 31;
     if (p >= in.n_paths) return;
     uint32_t j = kFill ? in.job_first[p] : 0u;
-    if (stroked(in, p) && path_stroke(in, p).dash_count) {
+    const bool st = stroked(in, p);
+    if (st && path_stroke(in, p).dash_count) {
         // the dashed contours, all open (dash_cnt is scanned by now: the path's contours are
         // [dash_cnt[p], dash_cnt[p + 1]))
         const uint32_t c0 = in.dash_cnt[p], n = in.dash_cnt[p + 1] - c0;
         if (kFill) {
-            for (uint32_t k = 0; k < n; k++) {
+            for (uint32_t k = lane; k < n; k += 32) {
                 const uint32_t a = c0 + k == 0 ? 0u : in.dash_end[c0 + k - 1], e = in.dash_end[c0 + k];
-                in.jobs[j++] = make_uint4(a, e - a, kJobOpen | 8u, p);
+                in.jobs[j + k] = make_uint4(a, e - a, kJobOpen | 8u, p);
             }
-        } else {
+        } else if (lane == 0) {
             in.job_first[p] = n;
         }
         return;
     }
     const uint2 kr = path_contours(in, p);
-    const bool st = stroked(in, p);
-    uint32_t n = 0;
-    for (uint32_t k = kr.x; k < kr.y; k++) {
-        const uint32_t s = upper_bound(in.scene_contour_first, in.n_scenes + 1, k) - 1;
-        const SceneDev &S = in.scenes[s];
-        const uint32_t local = k - S.contour_first;
-        const uint32_t a = in.cstart[S.cstart_base + local], e = in.cstart[S.cstart_base + local + 1];
-        const uint32_t first = S.point_first + a, np = e - a;
-        if (!st) {
-            if (kFill) in.jobs[j++] = make_uint4(first, np, kJobCopy, p);
-            n++;
-        } else if (np) {  // an outline has no empty contours (Outline::push_contour)
-            const bool closed = in.closed && in.closed[k];
-            if (closed) {
-                if (kFill) {
-                    in.jobs[j++] = make_uint4(first, np, kJobClosedFwd | 4u, p);
-                    in.jobs[j++] = make_uint4(first, np, kJobClosedBwd | 4u, p);
-                }
-                n += 2;
-            } else {
-                if (kFill) in.jobs[j++] = make_uint4(first, np, kJobOpen, p);
-                n++;
+    const unsigned below = (1u << lane) - 1u;
+    for (uint32_t k0 = kr.x; k0 < kr.y; k0 += 32) {
+        const uint32_t k = k0 + lane;
+        uint32_t first = 0, np = 0, jobs = 0;
+        if (k < kr.y) {
+            const uint32_t s = upper_bound(in.scene_contour_first, in.n_scenes + 1, k) - 1;
+            const SceneDev &S = in.scenes[s];
+            const uint32_t local = k - S.contour_first;
+            const uint32_t a = in.cstart[S.cstart_base + local], e = in.cstart[S.cstart_base + local + 1];
+            first = S.point_first + a;
+            np = e - a;
+            if (!st) jobs = 1;
+            else if (np) jobs = in.closed && in.closed[k] ? 2 : 1;  // an outline has no empty contours
+        }
+        const unsigned one = __ballot_sync(0xffffffffu, jobs >= 1), two = __ballot_sync(0xffffffffu, jobs == 2);
+        if (kFill) {
+            const uint32_t at = j + __popc(one & below) + __popc(two & below);
+            if (jobs == 2) {
+                in.jobs[at] = make_uint4(first, np, kJobClosedFwd | 4u, p);
+                in.jobs[at + 1] = make_uint4(first, np, kJobClosedBwd | 4u, p);
+            } else if (jobs == 1) {
+                in.jobs[at] = make_uint4(first, np, st ? kJobOpen : kJobCopy, p);
             }
         }
+        j += __popc(one) + __popc(two);
     }
-    if (!kFill) in.job_first[p] = n;
+    if (!kFill && lane == 0) in.job_first[p] = j;
 }
 
 // One output contour.  count: job_pts[j]; write: its points at job_pts[j] (scanned).
@@ -985,11 +991,10 @@ __global__ void __launch_bounds__(128) k_unit_leaves(StrokeIn in) {
     const float d = -fm(in.stroke[in.jobs[job].w].line_width, 0.5f);
     uint32_t leaf = kWrite ? in.unit_leaves[u] : 0u;
     const uint32_t l0 = leaf;
-    Seg stack[kStack];
+    // the right halves still to do (the left one is in hand; splits keep the kind)
+    float4 stack[2 * kStack];
     uint8_t depth[kStack];
-    stack[0] = root;
-    depth[0] = 0;
-    int sp = 1;
+    int sp = 0;
     const float tol2 = fm(kStrokeTol, kStrokeTol);
     bool bad = false;
     auto emit = [&](const Seg &s, V2 jp) {
@@ -1003,28 +1008,35 @@ __global__ void __launch_bounds__(128) k_unit_leaves(StrokeIn in) {
         }
         leaf++;
     };
-    while (sp > 0) {
-        sp--;
-        const Seg s = stack[sp];
-        const uint32_t dep = depth[sp];
-        if (!svalid(s)) continue;
-        const V2 jp = s.b.f;
-        if (lsqlen(s.b) < tol2 || dep >= 16) {
-            emit(s, jp);
-            continue;
+    Seg s = root;
+    uint32_t dep = 0;
+    for (;;) {
+        bool split = false;
+        if (svalid(s)) {
+            const V2 jp = s.b.f;
+            if (lsqlen(s.b) < tol2 || dep >= 16) {
+                emit(s, jp);
+            } else {
+                const Seg cand = offset_once(s, d);
+                split = s.kind != kLine && !within_tol(s, cand, d);
+                if (!split) emit(cand, jp);
+            }
         }
-        const Seg cand = offset_once(s, d);
-        if (s.kind == kLine || within_tol(s, cand, d)) {
-            emit(cand, jp);
-            continue;
+        if (split) {
+            Seg a, b;
+            ssplit(s, 0.5f, a, b);
+            stack[2 * sp] = make_float4(b.b.f.x, b.b.f.y, b.b.t.x, b.b.t.y);
+            stack[2 * sp + 1] = make_float4(b.c.f.x, b.c.f.y, b.c.t.x, b.c.t.y);
+            depth[sp++] = (uint8_t)++dep;
+            s = a;
+        } else {
+            if (sp == 0) break;
+            sp--;
+            const float4 q = stack[2 * sp], r = stack[2 * sp + 1];
+            s.b = ls(mk(q.x, q.y), mk(q.z, q.w));
+            s.c = ls(mk(r.x, r.y), mk(r.z, r.w));
+            dep = depth[sp];
         }
-        Seg a, b;
-        ssplit(s, 0.5f, a, b);
-        stack[sp] = b;
-        depth[sp] = (uint8_t)(dep + 1);
-        stack[sp + 1] = a;
-        depth[sp + 1] = (uint8_t)(dep + 1);
-        sp += 2;
     }
     if (!kWrite) in.unit_leaves[u] = leaf - l0;
     // an invalid leaf, or a unit without leaves (a later leaf's predecessor would not be its
@@ -1394,8 +1406,8 @@ cudaError_t launch_stroke_order(const StrokeIn &in, int what, uint32_t *ctl, uin
 
 cudaError_t launch_stroke_jobs(const StrokeIn &in, bool fill, cudaStream_t st) {
     if (!in.n_paths) return cudaSuccess;
-    if (fill) k_stroke_jobs<true><<<blocks(in.n_paths, 128), 128, 0, st>>>(in);
-    else k_stroke_jobs<false><<<blocks(in.n_paths, 128), 128, 0, st>>>(in);
+    if (fill) k_stroke_jobs<true><<<blocks(in.n_paths, 4), 128, 0, st>>>(in);
+    else k_stroke_jobs<false><<<blocks(in.n_paths, 4), 128, 0, st>>>(in);
     count_launches(1);
     return cudaGetLastError();
 }
