@@ -941,8 +941,12 @@ __device__ __forceinline__ void walk_lines(const WalkCtx &w, float4 f, bool have
 // are the same lines bit for bit; only their order within a path's region differs, which no
 // output depends on (fills are counted and placed per tile, coverage sums are integers).  The
 // pool is a stack, so it stays near 32 pieces per level of the warp's deepest segments; a half
-// that finds it full is flattened depth first by its lane alone (about 0.02% of the lines of the
-// 512-scene batch, in a CPU model of this kernel).  Warps take their segments a group at a time from
+// that finds it full is flattened depth first by its lane alone.  The pool and the segment table are
+// what limits the warps per SM, so they are as small as that stays rare: 256 scenes by the learned
+// frame, 2.00 ms with 224 pieces and 128 segments, 1.89 with 192 and 64 (11 blocks per SM instead of
+// 9), 1.95 with 176; taking fewer pieces when the pool is nearly full, so that none is left alone,
+// 1.96.  The exact passes keep 128 segments (stroked batch 0.565 ms with 224 pieces, 0.548 with 192,
+// 0.576 with 64 segments).  Warps take their segments a group at a time from
 // a frame-wide ticket: 32, or fewer (a power of two) when that would leave a resident warp under 8
 // groups, so the last groups end together and small frames use every SM.  A group's slots in the
 // segment table are reused once no pending piece or queued line refers to them.
@@ -953,10 +957,11 @@ __device__ __forceinline__ void walk_lines(const WalkCtx &w, float4 f, bool have
 // against not: 256 scenes by the learned frame 10.06 / 10.00 ms, 20,000 paths 1.26 / 1.28 ms, 24
 // clipped scenes 0.72 / 0.70 ms, 240 paths 0.20 / 0.18 ms).
 constexpr int kPoolWarps = 2;     // warps per block
-constexpr int kPoolCap = 224;     // pending pieces per warp
+constexpr int kPoolCap = 192;     // pending pieces per warp
 constexpr int kPoolLeafCap = 96;  // queued leaf lines per warp: < 32 before a round, + 2 per lane
-constexpr int kPoolEntries = 128; // segments in flight per warp (at most 32 groups)
 enum : int { kPoolLearned = 0, kPoolCount = 1, kPoolWrite = 2 };
+// segments in flight per warp (at most 32 groups)
+__host__ __device__ constexpr int pool_entries(int mode) { return mode == kPoolLearned ? 64 : 128; }
 // piece and line tags: bits 0-6 the segment's table entry (group * 32 + lane), bit 7 the
 // segment's leftmost piece, bit 8 a cubic (else a quadratic), bits 9-13 the depth
 constexpr uint32_t kTagEntry = 127u, kTagLeft = 1u << 7, kTagCubic = 1u << 8;
@@ -971,8 +976,8 @@ struct FlattenPool {
     uint32_t leaf_tag[kMode == kPoolCount ? 1 : kPoolLeafCap];
     // learned frame: path, region, budget, own slot; write pass: the segment's first leaf slot and
     // its lines stored so far; count pass: the segment (kNone: none) and its lines so far
-    uint4 seg[kMode == kPoolLearned ? kPoolEntries : 1];
-    uint2 seg2[kMode == kPoolLearned ? 1 : kPoolEntries];
+    uint4 seg[kMode == kPoolLearned ? pool_entries(kMode) : 1];
+    uint2 seg2[kMode == kPoolLearned ? 1 : pool_entries(kMode)];
 };
 
 // Where a lane stores leaf lines by itself.
@@ -1066,7 +1071,7 @@ __global__ void __launch_bounds__(kPoolWarps * 32) k_flatten_pool(Batch b, uint3
     n_segs = min(n_segs, b.status[kStSegs]);
     constexpr int kTicket = kMode == kPoolWrite ? kStFlatTicket2 : kStFlatTicket;
     const uint32_t group = 1u << group_shift, n_groups = (n_segs + group - 1u) >> group_shift;
-    const uint32_t n_sets = min(32u, (uint32_t)kPoolEntries >> group_shift);
+    const uint32_t n_sets = min(32u, (uint32_t)pool_entries(kMode) >> group_shift);
     const uint32_t all_sets = n_sets == 32u ? ~0u : (1u << n_sets) - 1u;
     // a group of segments: lane 0 takes the ticket, and the lanes read it when they need it, so the
     // atomic's round trip overlaps the work in between
