@@ -26,6 +26,9 @@ namespace {
 // the status words and the binning's control words, which share a buffer with the scans' state
 constexpr size_t kZeroBytes = kStBinCtl * 4 + kBinCtlBytes;
 constexpr size_t kStageBytes = 64 << 10;  // mapped host staging for small device reads
+constexpr size_t kSmallUpload = 256 << 10;  // and for uploads of that much (longer ones allocate)
+constexpr size_t kHostBlock = kStageBytes + 1024 + kSmallUpload;
+static_assert(kStHostWords * 4 <= 1024, "the status words' part of the mapped block");
 
 struct DevBuf {
     void *p = nullptr;
@@ -139,9 +142,14 @@ struct Ctx {
     uint32_t *h_status_dev = nullptr;  // the same memory as the device addresses it
     uint8_t *h_stage = nullptr, *h_stage_dev = nullptr;  // mapped staging for small reads
     // mapped staging for uploads (CopyPlan): its bytes in use by this upload; busy: not yet waited for
-    uint8_t *up_host = nullptr, *up_dev = nullptr;
+    uint8_t *up_host = nullptr, *up_dev = nullptr, *up_block = nullptr;  // up_block: allocated for it
     size_t up_cap = 0, up_used = 0;
     bool up_busy = false;
+    void small_upload() {
+        up_host = h_stage + kStageBytes + 1024;
+        up_dev = h_stage_dev + kStageBytes + 1024;
+        up_cap = kSmallUpload;
+    }
 
     // the scene range of the last frame and its totals
     uint32_t r_first = 0, r_count = 0, r_paths = 0, r_contours = 0, r_fb = 0, r_rows = 0;
@@ -398,18 +406,21 @@ struct CopyPlan {
         c->up_busy = false;
         c->up_used = 0;
         if (bytes <= c->up_cap) return true;
-        if (c->up_host) cudaFreeHost(c->up_host);
-        c->up_host = nullptr;
-        c->up_cap = 0;
-        size_t want = size_t(1) << 18;
+        if (c->up_block) cudaFreeHost(c->up_block);
+        c->up_block = nullptr;
+        c->small_upload();
+        size_t want = 2 * kSmallUpload;
         while (want < bytes) want *= 2;
-        if (cudaHostAlloc(&c->up_host, want, cudaHostAllocMapped) != cudaSuccess ||
-            cudaHostGetDevicePointer(reinterpret_cast<void **>(&c->up_dev), c->up_host, 0) != cudaSuccess) {
+        uint8_t *dev = nullptr;
+        if (cudaHostAlloc(&c->up_block, want, cudaHostAllocMapped) != cudaSuccess ||
+            cudaHostGetDevicePointer(reinterpret_cast<void **>(&dev), c->up_block, 0) != cudaSuccess) {
             cudaGetLastError();
-            if (c->up_host) cudaFreeHost(c->up_host);
-            c->up_host = nullptr;
+            if (c->up_block) cudaFreeHost(c->up_block);
+            c->up_block = nullptr;
             return false;
         }
+        c->up_host = c->up_block;
+        c->up_dev = dev;
         c->up_cap = want;
         return true;
     }
@@ -2015,10 +2026,14 @@ int pf_ctx_create(const pf_config *config, void **out) {
         e = cudaStreamCreateWithFlags(&c->stream, cudaStreamNonBlocking);
         c->own_stream = e == cudaSuccess;
     }
-    if (e == cudaSuccess) e = cudaHostAlloc(&c->h_status, kStHostWords * 4, cudaHostAllocMapped);
-    if (e == cudaSuccess) e = cudaHostGetDevicePointer(reinterpret_cast<void **>(&c->h_status_dev), c->h_status, 0);
-    if (e == cudaSuccess) e = cudaHostAlloc(&c->h_stage, kStageBytes, cudaHostAllocMapped);
+    // one mapped block: small reads, the status words, small uploads
+    if (e == cudaSuccess) e = cudaHostAlloc(&c->h_stage, kHostBlock, cudaHostAllocMapped);
     if (e == cudaSuccess) e = cudaHostGetDevicePointer(reinterpret_cast<void **>(&c->h_stage_dev), c->h_stage, 0);
+    if (e == cudaSuccess) {
+        c->h_status = reinterpret_cast<uint32_t *>(c->h_stage + kStageBytes);
+        c->h_status_dev = reinterpret_cast<uint32_t *>(c->h_stage_dev + kStageBytes);
+        c->small_upload();
+    }
     for (int i = 0; i < 8 && e == cudaSuccess; i++) e = cudaEventCreate(&c->ev[i]);
     if (e == cudaSuccess) e = c->status.ensure(kZeroBytes);
     if (e != cudaSuccess) {
@@ -2076,9 +2091,8 @@ int pf_ctx_destroy(void *ctx) {
     }
     c->canon_state.release();
     c->canon_clip.release();
-    if (c->h_status) cudaFreeHost(c->h_status);
     if (c->h_stage) cudaFreeHost(c->h_stage);
-    if (c->up_host) cudaFreeHost(c->up_host);
+    if (c->up_block) cudaFreeHost(c->up_block);
     if (c->own_stream) cudaStreamDestroy(c->stream);
     delete c;
     return PF_OK;
