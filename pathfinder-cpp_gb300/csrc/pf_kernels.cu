@@ -3441,7 +3441,8 @@ cudaError_t launch_bin_paths(const Batch &b, const Tuning &t, const BinClasses &
         return c;
     };
     if (has.cluster) {
-        PF_LAUNCH(k_bin_cluster<<<std::min(gc, has.cluster * kClusterCtas), kClusterThreads, kClusterSmem, st>>>(slice(sc)));
+        const unsigned ctas = (unsigned)std::min<uint64_t>(gc, uint64_t(has.cluster) * kClusterCtas);
+        PF_LAUNCH(k_bin_cluster<<<ctas, kClusterThreads, kClusterSmem, st>>>(slice(sc)));
         if ((e = cudaGetLastError()) != cudaSuccess) return e;
     }
     cudaStream_t const st2 = bs ? bs->side[0] : st, st0 = bs ? bs->side[1] : st;
@@ -3449,7 +3450,7 @@ cudaError_t launch_bin_paths(const Batch &b, const Tuning &t, const BinClasses &
     if (has.cta[1] && (e = launch_fused<1>(slice(s1), std::min(g[1], has.cta[1]), st)) != cudaSuccess) return e;
     if (has.cta[0] && (e = launch_fused<0>(slice(s0), std::min(g[0], has.cta[0]), st0)) != cudaSuccess) return e;
     if (has.small) {
-        PF_LAUNCH(k_bin_small<<<std::min(gs, (has.small + kSmallWarps - 1u) / kSmallWarps), kSmallThreads, 0, st0>>>(slice(ss)));
+        PF_LAUNCH(k_bin_small<<<std::min(gs, (has.small - 1u) / kSmallWarps + 1u), kSmallThreads, 0, st0>>>(slice(ss)));
         if ((e = cudaGetLastError()) != cudaSuccess) return e;
     }
     for (int k = 0; bs && k < 2; k++) {

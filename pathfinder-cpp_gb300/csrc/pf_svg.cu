@@ -61,6 +61,8 @@
 #include <cstdio>
 #include <cstdlib>
 #include <cstring>
+#include <memory>
+#include <new>
 #include <string>
 #include <vector>
 
@@ -1725,16 +1727,19 @@ extern "C" {
 int pf_svg_parse(const char *text, size_t length, float dpi, pf_svg **out) {
     if (!text || !out) return PF_ERR_INVALID_ARGUMENT;
     *out = nullptr;
+    const size_t n_text = strnlen(text, length);  // the text ends at its first NUL, as C text does
+    std::unique_ptr<char[]> copy(new (std::nothrow) char[n_text + 1]);
     Parser *p = new (std::nothrow) Parser();
     pf_svg *svg = new (std::nothrow) pf_svg();
-    if (!p || !svg) {
+    if (!copy || !p || !svg) {
         delete p;
         delete svg;
         return PF_ERR_OUT_OF_MEMORY;
     }
     p->dpi = dpi;
-    std::string copy(text, strnlen(text, length));  // the text ends at its first NUL, as C text does
-    parse_document(*p, &copy[0], copy.size());
+    std::memcpy(copy.get(), text, n_text);
+    copy[n_text] = '\0';
+    parse_document(*p, copy.get(), n_text);
     scale_to_viewbox(*p);
     SceneOut &o = svg->out;
     o.width = p->width;
