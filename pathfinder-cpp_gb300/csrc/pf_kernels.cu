@@ -1422,10 +1422,11 @@ constexpr int kCtaClasses = 3;
 // a class's words, and up to 3 before the tiles and 3 after them
 __host__ __device__ constexpr size_t class_smem(int c) { return (size_t(class_words(c)) + 8) * 4; }
 __host__ __device__ constexpr int class_threads(int c) { return c == 2 ? 384 : c == 1 ? 128 : 64; }
-// CTAs per SM the register budget is set for (shared memory allows 3 of class 2, 12 of class 1):
-// class 0 at 20 (48 registers) and class 1 at 8 (64 registers, no spills) beat 24 and 12 at 40
-// registers with 148-208 B of spills (binning 20.00 -> 19.30 ms per 512-scene frame)
-__host__ __device__ constexpr int class_min_ctas(int c) { return c == 2 ? 3 : c == 1 ? 8 : 20; }
+// CTAs per SM the register budget is set for (shared memory allows 3 of class 2, 12 of class 1).
+// Binning of 256 scenes / 20,000 paths: class 0 at 16, 18, 20 and 22 CTAs 7.63 / 0.696, 7.61 / 0.706, 7.64
+// / 0.718 and 8.13 / 0.868 ms (more CTAs leave too few registers and spill); class 1 at 7, 8, 9 and 10
+// 7.70, 7.64, 7.64 and 7.75 ms.
+__host__ __device__ constexpr int class_min_ctas(int c) { return c == 2 ? 3 : c == 1 ? 8 : 18; }
 // Tile visits with fills a CTA stages during its count walk (12 bytes each, in its own slice of a
 // global buffer that stays in L2, an equal part for each of its warps): the fills are then placed
 // without walking the lines again.  A path with more than this walks its lines twice.
