@@ -3,20 +3,23 @@
 // Stage map (reference -> here):
 //   SegmentsD3D11::add_path / SegmentsIter   -> k_contour_segments (count + emit)
 //   BuiltPath / round_rect_out_to_tile_bounds -> k_paths
-//   dice.comp (here: the d3d9 recursive bisection, tiler.cpp:284-315)  -> k_flatten<count|write>
+//   dice.comp (here: the d3d9 recursive bisection, tiler.cpp:284-315)
+//                                              -> k_flatten_pool<learned|count|write>; k_flatten
+//                                                 where segments are shallow
 //   bin.comp (here: the d3d9 tile walk + add_fill, tiler.cpp:131-279,
 //             object_builder.cpp:19-114),
 //   bound.comp (tile records), propagate.comp / Tiler::prepare_tiles
 //                                              -> k_bin_fused (one CTA per path: counts, backdrops,
 //                                                 offsets, fills grouped by tile; no linked lists);
-//                                                 k_bin_large* for rects too big for a CTA
+//                                                 k_bin_small (a warp) for small rects, k_bin_cluster
+//                                                 and k_bin_large* for rects too big for a CTA
 //   sort.comp (z-culled per-framebuffer-tile lists)
 //                                              -> k_rows (per framebuffer row: the spanning paths in
 //                                                 path order) + the front-to-back walk of k_composite,
 //                                                 which stops at the first occluder; k_list_dump
 //                                                 writes the lists out for the canonical read-back
 //   fill.comp + tile.comp                      -> k_composite (coverage never leaves the SM)
-//   (learned frame) per-path budgets            -> pf_sizer.cu: k_features, k_mlp_predict, k_budgets;
+//   (learned frame) per-path budgets            -> pf_sizer.cu: k_features, k_mlp, k_budgets;
 //                                                 here k_flatten_pool and the spill-pool lists
 //
 // Integer outputs follow the reference's d3d9 CPU tiler bit for bit, so every float
