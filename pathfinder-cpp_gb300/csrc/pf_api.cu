@@ -559,7 +559,7 @@ int stroke_upload(Ctx *c, const pf_scene_view *scenes, uint32_t n, const std::ve
         if (int e = read_words(c, {in.dash_pts + N, in.dash_cnt + N, status + kStFill64, status + kStFill64 + 1,
                                    status + kStErr, status + kStDashChunks}, w))
             return e;
-        tot[0] = w[0], tot[1] = w[1], tot[2] = w[4];
+        tot[0] = w[0], tot[1] = w[1], tot[2] = w[4] & ~kErrOverflowTotal;  // `wide` catches that
         const uint64_t wide = uint64_t(w[2]) | uint64_t(w[3]) << 32;  // the dash points' 64-bit total
         if (tot[2] & kErrStroke)
             return fail(c, PF_ERR_KERNEL_LIMIT, "a dash pattern needs more than 2^22 steps on one path");
@@ -588,9 +588,12 @@ int stroke_upload(Ctx *c, const pf_scene_view *scenes, uint32_t n, const std::ve
         ms_stroke += t;
         return PF_OK;
     };
-    auto read_u32 = [&](const uint32_t *dev, uint32_t &v) -> int {
+    auto read_u32 = [&](const uint32_t *dev, uint32_t &v) -> int {  // a scan's total
         PF_CUDA(mark(5));
-        if (int e = d2h_wait(c, &v, dev, 1)) return e;
+        uint32_t w[2];
+        if (int e = read_words(c, {dev, status + kStErr}, w)) return e;
+        if (w[1] & kErrOverflowTotal) return fail(c, PF_ERR_OVERFLOW, "stroked outline too large (2^32 pieces)");
+        v = w[0];
         return span();
     };
     PF_CUDA(mark(4));
@@ -665,7 +668,8 @@ int stroke_upload(Ctx *c, const pf_scene_view *scenes, uint32_t n, const std::ve
     tot[0] = w[0], tot[1] = w[3];
     const uint64_t wide = uint64_t(w[1]) | uint64_t(w[2]) << 32;  // the output points' 64-bit total
     if (int e = span()) return e;
-    if (wide >= (1ull << 31)) return fail(c, PF_ERR_OVERFLOW, "stroked outline too large (2^31 points)");
+    if (wide >= (1ull << 31) || (tot[1] & kErrOverflowTotal))
+        return fail(c, PF_ERR_OVERFLOW, "stroked outline too large (2^31 points)");
     if (tot[1] & kErrStroke)
         return fail(c, PF_ERR_KERNEL_LIMIT, "stroking hit a limit (a dash pattern over 2^22 steps on one path, "
                                             "or a cap searching back past 64 points)");
@@ -1072,7 +1076,8 @@ int check_kernel_status(Ctx *c) {
         std::snprintf(m, sizeof m, "a kernel hit an iteration bound (flags 0x%x)", e);
         return fail(c, PF_ERR_KERNEL_LIMIT, m);
     }
-    if (e & (kErrOverflowSeg | kErrOverflowLeaf | kErrOverflowFill | kErrOverflowList))
+    if (e & (kErrOverflowSeg | kErrOverflowLeaf | kErrOverflowFill | kErrOverflowList |
+             kErrOverflowTotal))
         return fail(c, PF_ERR_OVERFLOW, "a buffer capacity was exceeded");
     return PF_OK;
 }
@@ -1085,13 +1090,14 @@ int scan(Ctx *c, uint32_t *arr, uint32_t n, int slot) {
 }
 
 // A frame's scans, several in one launch, in place; the total goes to a status word and, with_end,
-// behind the array.  copy: the status words go to the host with them (read_status then only waits).
+// behind the array; over: the error bit of a total past 2^32.  copy: the status words go to the host with them (read_status then only waits).
 // Their state lies in the buffer of the status words, which begin_frame clears.
 struct FrameScan {
     uint32_t *arr;
     uint32_t n;
     int slot;
     bool with_end;
+    uint32_t over = kErrOverflowTotal;
 };
 
 int scan_frame(Ctx *c, std::initializer_list<FrameScan> scans, bool copy) {
@@ -1100,7 +1106,7 @@ int scan_frame(Ctx *c, std::initializer_list<FrameScan> scans, bool copy) {
     size_t at = c->zero_used;
     for (const FrameScan &f : scans) {
         j.job[j.n++] = ScanJob{f.arr, f.arr, f.n, status + f.slot, f.with_end ? f.arr + f.n : nullptr,
-                               reinterpret_cast<unsigned long long *>(c->status.as<char>() + at), 0, 0};
+                               reinterpret_cast<unsigned long long *>(c->status.as<char>() + at), f.over, 0, 0};
         at += scan_state_words(f.n) * 8;
     }
     j.err = status + kStErr;
@@ -1217,8 +1223,9 @@ int stage_setup(Ctx *c, bool learned) {
                                c->path_fill_budget.as<uint32_t>(), b.path_leaf_cursor, st));
         PF_CUDA(cudaMemcpyAsync(b.path_leaf_budget, b.path_leaf_first, size_t(N) * 4, cudaMemcpyDeviceToDevice, st));
         if (int e = scan_frame(c,
-                               {{b.path_leaf_first, N, kStLeafBudget, true},
-                                {c->path_fill_budget.as<uint32_t>(), N, kStFillBudget, true}},
+                               {{b.path_leaf_first, N, kStLeafBudget, true, kErrOverflowBudget},
+                                // only a first size for the fills, which grow when it was too small
+                                {c->path_fill_budget.as<uint32_t>(), N, kStFillBudget, true, 0}},
                                true))
             return e;
     }
@@ -1396,6 +1403,7 @@ int render_learned_frame(Ctx *c, uint32_t first, uint32_t count, pf_frame_stats 
     cudaStream_t st = c->stream;
     record(c, 0);
     if (int e = stage_setup(c, true)) return e;
+    if (c->h_status[kStErr] & kErrOverflowBudget) return render_exact(c, first, count, stats);
     // per-path regions, then a shared spill pool sized as a fraction of them
     const uint64_t leaf_regions = c->h_status[kStLeafBudget];
     const uint64_t leaf_pool = uint64_t(double(leaf_regions) * c->sz_pool) + 4096;

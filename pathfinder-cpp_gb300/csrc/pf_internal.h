@@ -39,6 +39,8 @@ enum : uint32_t {
     kErrOverflowLeaf = 1u << 9,
     kErrOverflowFill = 1u << 10,
     kErrOverflowList = 1u << 11,
+    kErrOverflowTotal = 1u << 12,   // a scan's total passed 2^32
+    kErrOverflowBudget = 1u << 13,  // the same of a learned frame's leaf budgets (it is then run exactly)
 };
 
 // Per scene of a batch (device).
@@ -234,7 +236,8 @@ void count_launches(uint32_t n);
 // Scans (exclusive, in place allowed); the total lands in *total (device).
 size_t scan_temp_bytes(uint32_t n);
 // Several scans in one launch: in and out (may be equal), the total to *total and behind the output to
-// *end (either may be null), state: scan_state_words(n) zeroed words.  With host set, the last block
+// *end (either may be null), state: scan_state_words(n) zeroed words, over: the error bit of a total that
+// passes 2^32 (0: none).  With host set, the last block
 // copies n_status status words there (done: a zeroed counter).
 struct ScanJob {
     const uint32_t *in;
@@ -242,6 +245,7 @@ struct ScanJob {
     uint32_t n;
     uint32_t *total, *end;
     unsigned long long *state;
+    uint32_t over;
     uint32_t first_block, blocks;  // set by scan_jobs
 };
 constexpr uint32_t kMaxScanJobs = 6;
