@@ -725,20 +725,19 @@ int stroke_upload(Ctx *c, const pf_scene_view *scenes, uint32_t n, const std::ve
     return PF_OK;
 }
 
+// A batch that is rejected leaves the one before as it was; one whose upload fails later leaves none.
 int upload(Ctx *c, const pf_scene_view *scenes, uint32_t n) {
     if (!scenes || n == 0) return fail(c, PF_ERR_INVALID_ARGUMENT, "no scenes");
-    forget_learned(c);
     uint64_t P = 0, C = 0, N = 0, fb = 0, img = 0, cs = 0, ps = 0;
-    c->h_scenes.assign(n, SceneDev{});
-    c->h_scene_fb_first.assign(n + 1, 0);
-    c->h_scene_row_first.assign(n + 1, 0);
+    std::vector<SceneDev> table(n, SceneDev{});
+    std::vector<uint32_t> scene_fb_first(n + 1, 0), scene_row_first(n + 1, 0);
     uint64_t rows = 0;
     std::vector<uint32_t> spf(n + 1, 0), scf(n + 1, 0);
     for (uint32_t i = 0; i < n; i++) {
         int st = validate_scene(c, &scenes[i]);
         if (st) return st;
         const pf_scene_view &s = scenes[i];
-        SceneDev &S = c->h_scenes[i];
+        SceneDev &S = table[i];
         // the view box (Scene::set_view_box rounds its right edge up to a multiple of 16);
         // framebuffer tiles cover the destination image from (0, 0)
         S.vb_left = s.view_box ? s.view_box[0] : 0.0f;
@@ -763,9 +762,9 @@ int upload(Ctx *c, const pf_scene_view *scenes, uint32_t n) {
         S.pstart_base = (uint32_t)ps;
         spf[i] = (uint32_t)N;
         scf[i] = (uint32_t)C;
-        c->h_scene_fb_first[i] = (uint32_t)fb;
+        scene_fb_first[i] = (uint32_t)fb;
         S.row_first = (uint32_t)rows;
-        c->h_scene_row_first[i] = (uint32_t)rows;
+        scene_row_first[i] = (uint32_t)rows;
         rows += S.fbh;
         P += s.n_points;
         C += s.n_contours;
@@ -778,10 +777,15 @@ int upload(Ctx *c, const pf_scene_view *scenes, uint32_t n) {
     }
     spf[n] = (uint32_t)N;
     scf[n] = (uint32_t)C;
-    c->h_scene_fb_first[n] = (uint32_t)fb;
-    c->h_scene_row_first[n] = (uint32_t)rows;
+    scene_fb_first[n] = (uint32_t)fb;
+    scene_row_first[n] = (uint32_t)rows;
     if (P >= (1ull << 31) || C >= (1ull << 31) || N >= (1ull << 31) || fb >= (1ull << 31))
         return fail(c, PF_ERR_OVERFLOW, "batch too large (2^31 points, contours, paths or tiles)");
+    forget_learned(c);
+    c->uploaded = c->rendered = false;
+    c->h_scenes.swap(table);
+    c->h_scene_fb_first.swap(scene_fb_first);
+    c->h_scene_row_first.swap(scene_row_first);
     c->n_scenes = n;
     c->n_points = (uint32_t)P;
     c->n_contours = (uint32_t)C;
@@ -958,7 +962,6 @@ int upload(Ctx *c, const pf_scene_view *scenes, uint32_t n) {
     if (strokes) {
         if (int e = stroke_upload(c, scenes, n, scf)) {
             cudaStreamSynchronize(c->stream);
-            c->uploaded = false;
             return e;
         }
     } else {
@@ -968,7 +971,6 @@ int upload(Ctx *c, const pf_scene_view *scenes, uint32_t n) {
     PF_CUDA(cudaStreamSynchronize(c->stream));
     c->up_busy = false;
     c->uploaded = true;
-    c->rendered = false;
     c->upload_epoch++;
     return PF_OK;
 }
