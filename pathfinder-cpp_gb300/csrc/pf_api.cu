@@ -225,6 +225,7 @@ int fail(Ctx *c, int code, const std::string &msg) {
 }
 
 int cuda_fail(Ctx *c, cudaError_t e, const char *what) {
+    cudaGetLastError();  // reported here: a later launch must not find it and fail
     std::string m = std::string(what) + ": " + cudaGetErrorString(e);
     return fail(c, e == cudaErrorMemoryAllocation ? PF_ERR_OUT_OF_MEMORY : PF_ERR_CUDA, m);
 }

@@ -51,3 +51,18 @@ def test_batch_that_does_not_fit_leaves_none(pf):
             with pytest.raises(pf.PfError) as e:
                 call()
             assert e.value.status == NOT_READY
+
+
+def test_failed_allocation_does_not_fail_the_next_call(pf):
+    good = _batch(4)
+    huge = [dataclasses.replace(S.plain_small(seed=3, n_paths=2, side=64), width=65536.0, height=65536.0)] * 25
+    with pf.Renderer() as r:
+        r.upload(good)
+        r.render()
+        want = r.image(2)
+        with pytest.raises(pf.PfError) as e:
+            r.upload(huge)
+        assert e.value.status == OUT_OF_MEMORY
+        r.upload(good)
+        r.render()
+        assert np.array_equal(r.image(2), want)
