@@ -1458,8 +1458,8 @@ int render_learned_frame(Ctx *c, uint32_t first, uint32_t count, pf_frame_stats 
 // The buffers a learned frame uses, by address (a reallocated one invalidates the graph).
 std::vector<void *> frame_buffers(const Ctx *c) {
     const DevBuf *bufs[] = {&c->status, &c->contour_point_first, &c->contour_path, &c->paths, &c->path_tiles,
-                            &c->path_cols, &c->path_contours, &c->path_bounds, &c->row_first, &c->row_mat, &c->bin_list,
-                            &c->path_leaf_range, &c->path_fill, &c->path_cls, &c->bin_stage,
+                            &c->path_cols, &c->contour_segs, &c->path_contours, &c->path_bounds, &c->row_first,
+                            &c->row_mat, &c->bin_list, &c->path_leaf_range, &c->path_fill, &c->path_cls, &c->bin_stage,
                             &c->path_feat, &c->contour_feat, &c->path_pred, &c->path_leaf_first, &c->path_leaf_budget,
                             &c->path_leaf_cursor, &c->path_fill_budget, &c->path_seg_first, &c->segs, &c->seg_leaves,
                             &c->row_paths, &c->tile_fills, &c->tile_state, &c->col_above,
