@@ -1512,6 +1512,16 @@ __device__ __forceinline__ PathLeaves path_leaves(const Batch &b, uint32_t p) {
     return L;
 }
 
+// Whether a walk of this frame hit its bound (the frame then ends with that error).  The lane form walks
+// such a line through other tiles than walk_line, so its counts are not to be filled by a second walk,
+// nor the fills read.  Past a barrier, a block sees what its own walks have found.  The CTA classes ask
+// while the block of fills is being reserved (20,000 paths 1,432.9 us without, 1,430.3 so; asked at the
+// second walk instead, 1.7% more, as its code then changes the kernel's), a warp only before its second
+// walk (150,000 glyphs 986 and 989 us; asked by every path, 1,130).
+__device__ __forceinline__ bool walk_failed(const uint32_t *status) {
+    return (*(const volatile uint32_t *)status & kErrWalk) != 0;
+}
+
 __device__ __forceinline__ WalkCtx walk_ctx(const Batch &b, const PathDev &P) {
     const SceneDev &S = b.scenes[P.scene];
     WalkCtx w;
@@ -1794,7 +1804,9 @@ __global__ void __launch_bounds__(class_threads(kCls), class_min_ctas(kCls)) k_b
         if (lane == 0) s_wsum[warp] = wsum;
         __syncthreads();
         unsigned long long base = 0, total = 0;
+        bool failed = false;
         if (tid == 0) {
+            failed = walk_failed(err);  // in flight with the atomic
             for (int k = 0; k < kWarps; k++) {
                 const unsigned long long v = s_wsum[k];
                 s_warp[k] = (uint32_t)total;
@@ -1835,7 +1847,7 @@ __global__ void __launch_bounds__(class_threads(kCls), class_min_ctas(kCls)) k_b
             if (!fits) atomicOr(err, kErrOverflowFill);
             b.path_fill[p] = (uint32_t)base;
             s_base = (uint32_t)base;
-            s_write = fits && total > 0;
+            s_write = fits && total > 0 && !failed;
         }
         __syncthreads();
 
@@ -2050,7 +2062,7 @@ __global__ void __launch_bounds__(kSmallThreads, 8) k_bin_small(Batch b) {
                 if (m) b.fills[slot] = q;
                 if (e) b.fills[slot + m] = t & kVisitDown ? make_uint2(0u, q.x) : make_uint2(q.y, 0u);
             }
-        } else if (fits) {
+        } else if (fits && !walk_failed(err)) {
             for (uint32_t k = lane; k < L.n; k += 32) {
                 const float4 f = b.leaves[L.index(b, k)];
                 walk_line(
@@ -2228,13 +2240,14 @@ __global__ void __cluster_dims__(kClusterCtas, 1, 1) __launch_bounds__(kClusterT
             total += v;
         }
         if (rank == 0 && tid == 0) {
+            const bool failed = walk_failed(err);  // in flight with the atomic
             const unsigned long long base = atomicAdd(fill_total(b), total);
             const bool fits = base + total <= (unsigned long long)b.fill_cap;
             if (!fits) atomicOr(err, kErrOverflowFill);
             b.path_fill[p] = (uint32_t)base;
             for (uint32_t r = 0; r < kClusterCtas; r++) {
                 cluster_store(cluster_addr(&s_base, r), (uint32_t)base);
-                cluster_store(cluster_addr(&s_write, r), fits && total > 0 ? 1u : 0u);
+                cluster_store(cluster_addr(&s_write, r), fits && total > 0 && !failed ? 1u : 0u);
             }
         }
 
@@ -2944,8 +2957,9 @@ __global__ void __launch_bounds__(kCompWarps * 32, (kPaint ? 20 : kClip ? 24 : 3
     __shared__ int cells[kCompWarps][kCovCells];
     __shared__ FillPrep prep[kCompWarps][32];
     __shared__ int park[kCompWarps][8][32];  // kMaskBoth: the clip tile's |coverage|
-    // a frame whose leaf lines or fills overran their buffers is redone; nothing to read here
-    if (b.status[kStErr] & (kErrOverflowLeaf | kErrOverflowFill)) return;
+    // a frame whose leaf lines or fills overran their buffers is redone, one with a walk that hit its
+    // bound is an error; nothing to read here
+    if (b.status[kStErr] & (kErrOverflowLeaf | kErrOverflowFill | kErrWalk)) return;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     int *D = cells[warp];
     zero_cells(D);  // once: coverage_raw leaves the cells it reads zero
