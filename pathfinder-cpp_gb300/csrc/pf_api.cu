@@ -123,7 +123,6 @@ struct Ctx {
     uint32_t last_paths_over = 0, last_pool_used = 0;
     DevBuf segs, path_seg_first, seg_leaves, leaves, pool_path, pool_cnt, pool_idx;
     DevBuf tile_fills, tile_state, col_above, col_final, fills, path_fill, path_cls, bin_stage;
-    size_t stage_slots = 0;
     DevBuf row_first, row_mat, row_paths, scene_rblk_first;
     DevBuf z, fb_count, list, image, status, scan_temp;
     DevBuf canon_state, canon_clip;  // clipped frames: tile states after the clip rules (read-back only)
@@ -1043,8 +1042,6 @@ Batch make_batch(Ctx *c) {
     b.col_final = c->col_final.as<int32_t>();
     b.fills = c->fills.as<uint2>();
     b.fill_cap = (uint32_t)std::min<size_t>(c->fills.cap / 8, 0xffffffffu);
-    b.stage = c->bin_stage.as<uint2>();
-    b.stage_tile = c->bin_stage.as<uint32_t>() + 2 * c->stage_slots;
     b.row_first = c->row_first.as<uint32_t>();
     b.row_paths = c->row_paths.as<uint4>();
     b.row_cap = (uint32_t)std::min<size_t>(c->row_paths.cap / 16, 0xffffffffu);
@@ -1185,8 +1182,6 @@ int begin_frame(Ctx *c, uint32_t first, uint32_t count) {
     PF_CUDA(c->bin_list.ensure(size_t(N) * 28 + 16));
     PF_CUDA(c->path_fill.ensure(size_t(N) * 4 + 16));
     PF_CUDA(c->path_seg_first.ensure(size_t(N) * 4 + 16));
-    PF_CUDA(bin_stage_slots(c->tune, c->n_sms, c->r_paths, &c->stage_slots));
-    PF_CUDA(c->bin_stage.ensure(c->stage_slots * 12));
     PF_CUDA(c->path_cls.ensure(size_t(N) + 16));
     PF_CUDA(c->path_leaf_range.ensure(size_t(N) * 8 + 16));
     if (!c->h_path_clip.empty()) PF_CUDA(c->path_clip_rel.ensure(size_t(N) * 4 + 16));
@@ -1278,6 +1273,11 @@ int bin_and_composite(Ctx *c, Batch b, bool learned, uint64_t max_leaves) {
     int classes = (has.small != 0) + (has.cluster != 0) + (has.large != 0);
     for (int k = 0; k < 3; k++) classes += (learned ? rects[k] : has.cta[k]) != 0;
     const bool at_once = c->tune.bin_concurrent || (classes > 1 && N <= 1u << 16);
+    size_t slots = 0;
+    PF_CUDA(bin_stage_slots(c->tune, c->n_sms, has, at_once, &slots));
+    PF_CUDA(c->bin_stage.ensure(slots * 12));
+    b.stage = c->bin_stage.as<uint2>();
+    b.stage_tile = reinterpret_cast<uint32_t *>(b.stage + slots);
     for (int attempt = 0;; attempt++) {
         if (attempt > 0) {  // else begin_frame cleared them
             PF_CUDA(cudaMemsetAsync(b.bin_ctl, 0, kBinCtlBytes, st));

@@ -401,8 +401,9 @@ cudaError_t launch_bin_paths(const Batch &b, const Tuning &t, const BinClasses &
 // The most CTAs of each binning class one SM holds.
 cudaError_t bin_class_max_ctas(int out[3]);
 cudaError_t launch_pool_lists(const Batch &b, bool scatter, cudaStream_t st);
-// Slots of the binning CTAs' stage on the current device for these launch parameters.
-cudaError_t bin_stage_slots(const Tuning &t, uint32_t n_sms, uint32_t n_paths, size_t *slots);
+// Slots of the stage that launch_bin_paths uses with these launch parameters and classes on the current
+// device.
+cudaError_t bin_stage_slots(const Tuning &t, uint32_t n_sms, const BinClasses &has, bool at_once, size_t *slots);
 cudaError_t launch_mlp_predict(const __nv_bfloat16 *w, const float *feat, uint32_t n, float *out, cudaStream_t st);
 cudaError_t launch_mlp_grad(const __nv_bfloat16 *w, const float *feat, const float *target, const uint32_t *index,
                             uint32_t n, float *grad, float *loss, cudaStream_t st);

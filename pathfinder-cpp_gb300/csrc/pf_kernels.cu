@@ -3355,13 +3355,6 @@ static cudaError_t launch_fused(const Batch &b, unsigned grid, cudaStream_t st) 
     return cudaGetLastError();
 }
 
-static cudaError_t fused_grids(const Tuning &t, uint32_t n_sms, uint32_t n_paths, unsigned g[3]) {
-    cudaError_t e = fused_grid<0>(&g[0], n_sms, n_paths, t.bin_ctas_per_sm[0]);
-    if (e == cudaSuccess) e = fused_grid<1>(&g[1], n_sms, n_paths, t.bin_ctas_per_sm[1]);
-    if (e == cudaSuccess) e = fused_grid<2>(&g[2], n_sms, n_paths, t.bin_ctas_per_sm[2]);
-    return e;
-}
-
 // The small class's grid: as many CTAs as fit on every SM, a path per warp at least.
 static cudaError_t small_grid(unsigned *grid, uint32_t n_sms, uint32_t n_paths) {
     static std::atomic<int> per_sm{0};  // the same on every device of the one architecture this is built for
@@ -3408,16 +3401,43 @@ static cudaError_t cluster_grid(unsigned *grid, uint32_t n_paths) {
     return cudaSuccess;
 }
 
-// The classes' slices of the stage follow each other, largest class first: they may run at once.
-cudaError_t bin_stage_slots(const Tuning &t, uint32_t n_sms, uint32_t n_paths, size_t *slots) {
-    unsigned g[3];
-    if (const cudaError_t e = fused_grids(t, n_sms, n_paths, g)) return e;
-    unsigned gs = 0, gc = 0;
-    if (const cudaError_t e = small_grid(&gs, n_sms, n_paths)) return e;
-    if (const cudaError_t e = cluster_grid(&gc, n_paths)) return e;
-    *slots = size_t(g[0]) * class_stage(0) + size_t(g[1]) * class_stage(1) + size_t(g[2]) * class_stage(2) +
-             size_t(gs) * kSmallWarps * kSmallSpill + size_t(gc) * kClusterWarps * kClusterStage;
+// The grids of the classes that can have paths, and their slices of the stage.  Classes of one stream run
+// one after the other and share a slice: on their own streams the cluster class with class 1, and class
+// 0 with the small one; all of them in a frame that runs them in turn.  (A slice for each of the five
+// classes, whether the frame has it or not: a first frame of 240 paths took 178 MB and 614 us, now 68 MB
+// and 550 us, one of 20,000 paths 4.07 ms, now 2.25; later frames are the same.)
+struct BinLaunch {
+    unsigned cta[3] = {}, small = 0, cluster = 0;
+    size_t first[3] = {};                         // class c's slice
+    size_t first_small = 0, first_cluster = 0, slots = 0;
+};
+
+static cudaError_t bin_launch(const Tuning &t, uint32_t n_sms, const BinClasses &has, bool at_once, BinLaunch &l) {
+    cudaError_t e = cudaSuccess;
+    if (has.cta[0]) e = fused_grid<0>(&l.cta[0], n_sms, has.cta[0], t.bin_ctas_per_sm[0]);
+    if (e == cudaSuccess && has.cta[1]) e = fused_grid<1>(&l.cta[1], n_sms, has.cta[1], t.bin_ctas_per_sm[1]);
+    if (e == cudaSuccess && has.cta[2]) e = fused_grid<2>(&l.cta[2], n_sms, has.cta[2], t.bin_ctas_per_sm[2]);
+    if (e == cudaSuccess && has.small) e = small_grid(&l.small, n_sms, has.small);
+    if (e == cudaSuccess && has.cluster) e = cluster_grid(&l.cluster, has.cluster);
+    if (e != cudaSuccess) return e;
+    const size_t own = std::max(size_t(l.cta[1]) * class_stage(1), size_t(l.cluster) * kClusterWarps * kClusterStage);
+    const size_t side0 = size_t(l.cta[2]) * class_stage(2);
+    const size_t side1 = std::max(size_t(l.cta[0]) * class_stage(0), size_t(l.small) * kSmallWarps * kSmallSpill);
+    if (at_once) {
+        l.first[2] = own;
+        l.first[0] = l.first_small = own + side0;
+        l.slots = own + side0 + side1;
+    } else {
+        l.slots = std::max(own, std::max(side0, side1));
+    }
     return cudaSuccess;
+}
+
+cudaError_t bin_stage_slots(const Tuning &t, uint32_t n_sms, const BinClasses &has, bool at_once, size_t *slots) {
+    BinLaunch l;
+    const cudaError_t e = bin_launch(t, n_sms, has, at_once, l);
+    *slots = l.slots;
+    return e;
 }
 
 cudaError_t bin_class_max_ctas(int out[3]) {
@@ -3433,10 +3453,8 @@ cudaError_t bin_class_max_ctas(int out[3]) {
 cudaError_t launch_bin_paths(const Batch &b, const Tuning &t, const BinClasses &has, const BinStreams *bs,
                              cudaStream_t st) {
     if (!b.n_paths) return cudaSuccess;
-    unsigned g[3], gs = 0, gc = 0;
-    cudaError_t e = fused_grids(t, b.n_sms, b.n_paths, g);
-    if (e == cudaSuccess) e = small_grid(&gs, b.n_sms, b.n_paths);
-    if (e == cudaSuccess) e = cluster_grid(&gc, b.n_paths);
+    BinLaunch l;
+    cudaError_t e = bin_launch(t, b.n_sms, has, bs != nullptr, l);
     if (e != cudaSuccess) return e;
     if (bs) {
         if ((e = cudaEventRecord(bs->fork, st)) != cudaSuccess) return e;
@@ -3449,9 +3467,6 @@ cudaError_t launch_bin_paths(const Batch &b, const Tuning &t, const BinClasses &
         PF_LAUNCH(k_bin_large_prep<<<b.n_sms * 2, kPrepThreads, 0, st>>>(b));
         PF_LAUNCH(k_bin_large<true><<<b.n_sms * 8, kThreads, 0, st>>>(b));
     }
-    // the classes' slices of the stage, as bin_stage_slots sizes them
-    const size_t s1 = size_t(g[2]) * class_stage(2), s0 = s1 + size_t(g[1]) * class_stage(1);
-    const size_t ss = s0 + size_t(g[0]) * class_stage(0), sc = ss + size_t(gs) * kSmallWarps * kSmallSpill;
     auto slice = [&](size_t first) {
         Batch c = b;
         c.stage += first;
@@ -3459,16 +3474,15 @@ cudaError_t launch_bin_paths(const Batch &b, const Tuning &t, const BinClasses &
         return c;
     };
     if (has.cluster) {
-        const unsigned ctas = (unsigned)std::min<uint64_t>(gc, uint64_t(has.cluster) * kClusterCtas);
-        PF_LAUNCH(k_bin_cluster<<<ctas, kClusterThreads, kClusterSmem, st>>>(slice(sc)));
+        PF_LAUNCH(k_bin_cluster<<<l.cluster, kClusterThreads, kClusterSmem, st>>>(slice(l.first_cluster)));
         if ((e = cudaGetLastError()) != cudaSuccess) return e;
     }
     cudaStream_t const st2 = bs ? bs->side[0] : st, st0 = bs ? bs->side[1] : st;
-    if (has.cta[2] && (e = launch_fused<2>(slice(0), std::min(g[2], has.cta[2]), st2)) != cudaSuccess) return e;
-    if (has.cta[1] && (e = launch_fused<1>(slice(s1), std::min(g[1], has.cta[1]), st)) != cudaSuccess) return e;
-    if (has.cta[0] && (e = launch_fused<0>(slice(s0), std::min(g[0], has.cta[0]), st0)) != cudaSuccess) return e;
+    if (has.cta[2] && (e = launch_fused<2>(slice(l.first[2]), l.cta[2], st2)) != cudaSuccess) return e;
+    if (has.cta[1] && (e = launch_fused<1>(slice(l.first[1]), l.cta[1], st)) != cudaSuccess) return e;
+    if (has.cta[0] && (e = launch_fused<0>(slice(l.first[0]), l.cta[0], st0)) != cudaSuccess) return e;
     if (has.small) {
-        PF_LAUNCH(k_bin_small<<<std::min(gs, (has.small - 1u) / kSmallWarps + 1u), kSmallThreads, 0, st0>>>(slice(ss)));
+        PF_LAUNCH(k_bin_small<<<l.small, kSmallThreads, 0, st0>>>(slice(l.first_small)));
         if ((e = cudaGetLastError()) != cudaSuccess) return e;
     }
     for (int k = 0; bs && k < 2; k++) {
