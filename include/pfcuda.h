@@ -338,9 +338,10 @@ typedef struct pf_tuning {
     uint32_t bin_concurrent;     /* 1: the binning classes always run at once, on side streams; 0: they do
                                     where several classes have paths and the frame is not too long */
     uint32_t seg_sorted;         /* 0 or 1; changes nothing (segments are no longer ordered by depth) */
-    uint32_t composite_ticket;   /* 0: the composite runs a warp per framebuffer tile; n > 0: its warps
-                                    stay resident and take n consecutive tiles per ticket from a
-                                    frame-wide queue (at most 4096) */
+    uint32_t composite_ticket;   /* n > 0: the composite's warps stay resident and take n consecutive
+                                    framebuffer tiles per ticket from a frame-wide queue (at most
+                                    4096); 0: a warp per tile, or a tile per ticket in frames of many
+                                    tiles with gradients or clip paths, where that is faster */
     uint32_t reserved[8];
 } pf_tuning;
 int pf_tuning_get(void *ctx, pf_tuning *out);

@@ -2672,9 +2672,11 @@ __device__ __forceinline__ void raster_column(const FillPrep &fp, int i, int *D)
 // items counts: an item's fill comes from a mask of the items that begin one (a binary search over
 // the fills' first items was five dependent shared loads), its set-up in two loads.
 // backdrop + the fills' area sums (fixed point) of the warp's 8 pixels per lane, before the fill rule
-// src: the tile's n fills; q: this lane's fill of the first 32 (any value from lane n on).
+// src: the tile's n fills; q: with kLoaded this lane's fill of the first 32 (any value from lane n on),
+// else not read.
 // lane: the caller's, passed down because the composite spills more when each of these functions asks
 // for its own (256 scenes, composite 2.90 -> 2.83 ms).
+template <bool kLoaded>
 __device__ __forceinline__ void coverage_raw(int lane, const uint2 *src, uint32_t n, uint2 q, int8_t bd, int *D,
                                              FillPrep *prep, int raw[8]) {
     const unsigned below = (1u << lane) - 1u;
@@ -2683,7 +2685,7 @@ __device__ __forceinline__ void coverage_raw(int lane, const uint2 *src, uint32_
         int items = 0;
         FillPrep fp;
         if ((uint32_t)lane < left) {
-            if (base > 0) q = src[base + lane];
+            if (!kLoaded || base > 0) q = src[base + lane];
             const float x0 = (float)(q.x & 0xffffu) * (1.0f / 256.0f), y0 = (float)(q.x >> 16) * (1.0f / 256.0f);
             const float x1 = (float)(q.y & 0xffffu) * (1.0f / 256.0f), y1 = (float)(q.y >> 16) * (1.0f / 256.0f);
             fp.s = x0 > x1 ? 1.0f : -1.0f;
@@ -2767,7 +2769,7 @@ __device__ __forceinline__ void alpha_coverage(const Batch &b, uint32_t f0, uint
     int raw[8];
     const uint32_t lane = threadIdx.x & 31;
     const uint2 q = lane < f1 - f0 ? b.fills[f0 + lane] : make_uint2(0u, 0u);
-    coverage_raw((int)lane, b.fills + f0, f1 - f0, q, bd, D, prep, raw);
+    coverage_raw<true>((int)lane, b.fills + f0, f1 - f0, q, bd, D, prep, raw);
     coverage_rule(raw, eo, cov);
 }
 
@@ -2786,7 +2788,8 @@ constexpr int kCompWarps = 1;
 // (the d3d11 z-buffer rule, propagate.comp:190-205) - so the tiles visited are exactly the
 // framebuffer tile's composite list after z-culling (sort.comp:49-83), in reverse order.
 // With kFetch, every visible candidate also loads its colour and (alpha tiles) its fill
-// range in parallel before the visits, so a visit waits on its fills alone.
+// range in parallel before the visits, so a visit waits on its fills alone; with kAhead, the next
+// candidate's first fills are loaded during the visit before it.
 // visit(candidate) returns true to stop the walk.
 struct Cand {
     uint32_t p, gt, st, flags;  // st: the tile state, with a clipped tile's mask source in bits 9-10
@@ -2827,7 +2830,7 @@ __device__ __forceinline__ void apply_clip(const Batch &b, uint32_t p, int32_t t
     }
 }
 
-template <bool kFetch, bool kClip, class Visit>
+template <bool kFetch, bool kClip, bool kAhead, class Visit>
 __device__ __forceinline__ void walk_fb_tile(const Batch &b, int lane, uint32_t row, uint32_t fx, uint32_t fy,
                                              Visit &&visit, uint32_t &chunks) {
     const uint32_t k_lo = b.row_first[row], k_hi = b.row_first[row + 1];
@@ -2857,7 +2860,6 @@ __device__ __forceinline__ void walk_fb_tile(const Batch &b, int lane, uint32_t 
             }
         }
         uint32_t mask = __ballot_sync(0xffffffffu, vis);
-        // kFetch: the next candidate's first fills are loaded while the one before it is visited
         uint32_t nf0 = 0, nf1 = 0;
         uint2 nq = make_uint2(0u, 0u);
         auto next_fills = [&]() {
@@ -2866,7 +2868,7 @@ __device__ __forceinline__ void walk_fb_tile(const Batch &b, int lane, uint32_t 
             nf1 = __shfl_sync(0xffffffffu, c.f1, l);
             if ((uint32_t)lane < nf1 - nf0) nq = b.fills[nf0 + lane];
         };
-        if (kFetch && mask) next_fills();
+        if (kFetch && kAhead && mask) next_fills();
         while (mask) {
             const int l = __ffs(mask) - 1;
             mask &= mask - 1;
@@ -2876,12 +2878,17 @@ __device__ __forceinline__ void walk_fb_tile(const Batch &b, int lane, uint32_t 
             v.st = __shfl_sync(0xffffffffu, c.st, l);
             v.flags = __shfl_sync(0xffffffffu, c.flags, l);
             if (kFetch) {
-                v.f0 = nf0;
-                v.f1 = nf1;
-                v.q = nq;
+                if (!kAhead) {
+                    v.f0 = __shfl_sync(0xffffffffu, c.f0, l);
+                    v.f1 = __shfl_sync(0xffffffffu, c.f1, l);
+                } else {
+                    v.f0 = nf0;
+                    v.f1 = nf1;
+                    v.q = nq;
+                }
                 v.color = __shfl_sync(0xffffffffu, c.color, l);
                 if (kClip) v.gc = __shfl_sync(0xffffffffu, c.gc, l);
-                if (mask) next_fills();
+                if (kAhead && mask) next_fills();
             }
             if (visit(v)) return;
         }
@@ -2949,11 +2956,18 @@ __device__ __forceinline__ float4 gradient_color(const Batch &b, uint32_t g, flo
     return o;
 }
 
+// Warps per SM the registers are capped for.
+__host__ __device__ constexpr int comp_warps(bool clip, bool paint) { return paint ? 20 : clip ? 24 : 32; }
+
 // kClip: the batch has clip paths; kPaint: it has gradient paints; kTicket: resident warps
 // take tiles by ticket (b.comp_ticket > 0).  Variants of their own, so that code one frame does
-// not need costs it no registers.
+// not need costs it no registers.  The loop over tiles costs the ticketed ones registers, so they keep
+// their place in the queue in shared memory, ask for their lane in every tile and don't load the next
+// candidate's fills ahead (with all that in registers 276 and 236 bytes of spills, without and with clips,
+// now 192 and 92; 256 scenes, a ticket per tile: 3.65 -> 3.09 ms, with clips 4.34 -> 3.62, with gradients
+// 6.63 -> 6.10).
 template <bool kClip, bool kPaint, bool kTicket>
-__global__ void __launch_bounds__(kCompWarps * 32, (kPaint ? 20 : kClip ? 24 : 32) / kCompWarps) k_composite(Batch b) {
+__global__ void __launch_bounds__(kCompWarps * 32, comp_warps(kClip, kPaint) / kCompWarps) k_composite(Batch b) {
     __shared__ int cells[kCompWarps][kCovCells];
     __shared__ FillPrep prep[kCompWarps][32];
     __shared__ int park[kCompWarps][8][32];  // kMaskBoth: the clip tile's |coverage|
@@ -2967,24 +2981,31 @@ __global__ void __launch_bounds__(kCompWarps * 32, (kPaint ? 20 : kClip ? 24 : 3
     uint32_t entries = 0, comp_fills = 0, chunks = 0;
     // one framebuffer tile per warp, or (kTicket) warps that stay and take comp_ticket
     // consecutive tiles at a time from a frame-wide ticket counter
-    uint32_t next = 0, left = 0;
+    __shared__ uint32_t s_next[kCompWarps], s_left[kCompWarps];
+    if (kTicket && lane == 0) s_left[warp] = 0;
+    __syncwarp();
     for (uint32_t round = 0;; round++) {
         uint32_t fb;
         if (!kTicket) {
             if (round > 0) break;
             fb = blockIdx.x * kCompWarps + warp;
         } else {
-            if (left == 0) {
-                uint32_t t = 0;
-                if (lane == 0) t = atomicAdd(&b.bin_ctl[kCtlCompTicket], b.comp_ticket);
-                next = __shfl_sync(0xffffffffu, t, 0);
-                left = b.comp_ticket;
+            if (lane == 0) {
+                if (s_left[warp] == 0) {
+                    s_next[warp] = atomicAdd(&b.bin_ctl[kCtlCompTicket], b.comp_ticket);
+                    s_left[warp] = b.comp_ticket;
+                }
+                s_left[warp]--;
             }
-            fb = next++;
-            left--;
+            __syncwarp();
+            fb = s_next[warp];
+            __syncwarp();
+            if (lane == 0) s_next[warp] = fb + 1;
         }
         if (fb >= b.n_fb) break;
-        const int col = lane & 15, h = lane >> 4;
+        int ln = lane;
+        if (kTicket) asm volatile("mov.u32 %0, %%laneid;" : "=r"(ln));
+        const int col = ln & 15, h = ln >> 4;
         const uint32_t fbg = b.fb_base + fb;
         const uint32_t s = b.fb_scene[fbg];
         const SceneDev &S = b.scenes[s];
@@ -2998,7 +3019,7 @@ __global__ void __launch_bounds__(kCompWarps * 32, (kPaint ? 20 : kClip ? 24 : 3
             ar[k] = ag[k] = ab[k] = 0.0f;
             tr[k] = 1.0f;
         }
-        walk_fb_tile<true, kClip>(b, lane, S.row_first - b.row_base + fy, fx, fy, [&](const Cand &v) -> bool {
+        walk_fb_tile<true, kClip, !kTicket>(b, ln, S.row_first - b.row_base + fy, fx, fy, [&](const Cand &v) -> bool {
             const bool eo = (v.flags & 1u) != 0;
             const int8_t bd = (int8_t)(v.st & 0xffu);
             float cov[8];
@@ -3022,13 +3043,13 @@ __global__ void __launch_bounds__(kCompWarps * 32, (kPaint ? 20 : kClip ? 24 : 3
                     const uint32_t cp = b.path_clip_rel[v.p];
                     f0 = fill_begin(b, cp, v.gc);
                     f1 = b.tile_fills[v.gc];
-                    if ((uint32_t)lane < f1 - f0) q = b.fills[f0 + lane];
+                    if (!kTicket && (uint32_t)lane < f1 - f0) q = b.fills[f0 + lane];
                     tbd = (int8_t)(b.tile_state[v.gc] & 0xffu);
                 }
                 int raw[8];
                 for (;;) {
                     comp_fills += f1 - f0;
-                    coverage_raw(lane, b.fills + f0, f1 - f0, q, tbd, D, prep[warp], raw);
+                    coverage_raw<!kTicket>(ln, b.fills + f0, f1 - f0, q, tbd, D, prep[warp], raw);
                     __syncwarp();
                     if (!both) break;
 #pragma unroll
@@ -3170,7 +3191,7 @@ __global__ void __launch_bounds__(kCompWarps * 32) k_list_dump(Batch b) {
         first = b.fb_count[fb];
         count = b.fb_count[fb + 1] - first;
     }
-    walk_fb_tile<false, true>(b, threadIdx.x & 31, S.row_first - b.row_base + fy, fx, fy, [&](const Cand &v) -> bool {
+    walk_fb_tile<false, true, false>(b, threadIdx.x & 31, S.row_first - b.row_base + fy, fx, fy, [&](const Cand &v) -> bool {
         if (kWrite && lane == 0) b.list[first + count - 1 - n] = v.gt;
         n++;
         const int8_t bd = (int8_t)(v.st & 0xffu);
@@ -3563,11 +3584,20 @@ cudaError_t launch_rows(const Batch &b, bool write, cudaStream_t st) {
 }
 
 // Grid of the composite: a warp per framebuffer tile, or (ticketed) as many resident blocks as
-// fit on every SM.
+// fit on every SM.  With no tickets asked for (comp_ticket 0) the frame decides: gradients and clips make
+// some tiles many times as long as others, and in a frame of many tiles resident warps that take the next
+// one are ahead of the block scheduler's order.  The lines, in tiles per resident warp (20 per SM with
+// gradients, 24 with clips): 4 with gradients (4,096 tiles, 1.3 a warp, 0-5% slower with a ticket a tile;
+// from 16,384 on, 5 a warp, 4-14% faster; 512 scenes 14.43 -> 12.16 ms), 64 with clips alone (below, from
+// 15% slower to 7% faster; from 230,000 tiles on 1-9% faster; 512 scenes 7.63 -> 6.93 ms); without either
+// it never pays (64 scenes 0.91 -> 1.03 ms, 512 the same).
 template <bool kClip, bool kPaint>
 static cudaError_t launch_composite_variant(const Batch &b, cudaStream_t st) {
-    if (!b.comp_ticket) {
-        PF_LAUNCH(k_composite<kClip, kPaint, false><<<grid_for(b.n_fb, kCompWarps), kCompWarps * 32, 0, st>>>(b));
+    Batch c = b;
+    const uint64_t resident = uint64_t(comp_warps(kClip, kPaint)) * b.n_sms;
+    if (!c.comp_ticket && (kPaint || kClip) && b.n_fb >= resident * (kPaint ? 4 : 64)) c.comp_ticket = 1;
+    if (!c.comp_ticket) {
+        PF_LAUNCH(k_composite<kClip, kPaint, false><<<grid_for(b.n_fb, kCompWarps), kCompWarps * 32, 0, st>>>(c));
         return cudaGetLastError();
     }
     int dev = 0, sms = 152, per_sm = 1;
@@ -3578,7 +3608,7 @@ static cudaError_t launch_composite_variant(const Batch &b, cudaStream_t st) {
     if (e != cudaSuccess) return e;
     const unsigned grid =
         std::min<unsigned>(grid_for(b.n_fb, kCompWarps), (unsigned)std::max(per_sm, 1) * (unsigned)sms);
-    PF_LAUNCH(k_composite<kClip, kPaint, true><<<grid, kCompWarps * 32, 0, st>>>(b));
+    PF_LAUNCH(k_composite<kClip, kPaint, true><<<grid, kCompWarps * 32, 0, st>>>(c));
     return cudaGetLastError();
 }
 
