@@ -12,10 +12,13 @@
 // started before it.  Every wait is bounded: after kSpinLimit polls the block records an
 // error bit and stops.
 //
-// The offsets are 32 bits wide, the sums behind them 64: a total that 32 bits do not hold sets the
-// job's error bit (`over`), and the caller neither sizes nor writes anything by the wrapped offsets.
-// (The 64-bit sums cost nothing that shows: 240 paths 198.9 us with 32-bit ones, 197.4 so; 150,000
-// glyphs 986.8 and 984.5.)
+// The offsets are 32 bits wide, the tiles' aggregates and prefixes 64: a total that 32 bits do not hold
+// sets the job's error bit (`over`), and the caller neither sizes nor writes anything by the wrapped
+// offsets.  Within a tile the sums have 32 bits, which is exact while its 4,096 elements are below 2^20;
+// a tile with a larger one adds up again in 64.  Eight blocks an SM, so that all tiles of most frames are
+// resident and look back side by side: at five (48 registers, which the second sum asks for) 150,000
+// glyphs, some 4 million segments in 980 tiles, took 220.6 us to flatten, at eight 216.1 (215.8 without the
+// second sum).
 //
 // One launch scans several arrays (their tiles one after the other in the grid): a frame's set-up
 // has four of a few thousand elements, whose launches and clears were most of their time.  The last
@@ -33,21 +36,22 @@ constexpr uint32_t kScanTile = kScanThreads * kScanItems;  // 4096
 constexpr uint64_t kFlagAgg = 1ull << 62, kFlagInc = 2ull << 62, kValMask = (1ull << 62) - 1;
 constexpr uint32_t kSpinLimit = 1u << 20;
 
-__device__ __forceinline__ uint64_t warp_inclusive(uint64_t v) {
+__device__ __forceinline__ uint32_t warp_inclusive(uint32_t v) {
     const int lane = threadIdx.x & 31;
 #pragma unroll
     for (int d = 1; d < 32; d <<= 1) {
-        const uint64_t t = __shfl_up_sync(0xffffffffu, v, d);
+        const uint32_t t = __shfl_up_sync(0xffffffffu, v, d);
         if (lane >= d) v += t;
     }
     return v;
 }
 
 // state[0] = ticket counter, state[1 + t] = status of tile t (all zero at the start)
-__global__ void __launch_bounds__(kScanThreads) k_scan(ScanJobs jobs) {
-    __shared__ uint64_t warp_sums[kScanThreads / 32];
+__global__ void __launch_bounds__(kScanThreads, 8) k_scan(ScanJobs jobs) {
+    __shared__ uint32_t warp_sums[kScanThreads / 32];
+    __shared__ uint64_t wide_sums[kScanThreads / 32];
     __shared__ uint32_t s_tile;
-    __shared__ uint64_t s_prefix;
+    __shared__ uint32_t s_prefix;
     __shared__ bool s_last;
     uint32_t k = 0;
     while (k + 1 < jobs.n && jobs.job[k + 1].first_block <= blockIdx.x) k++;
@@ -75,18 +79,33 @@ __global__ void __launch_bounds__(kScanThreads) k_scan(ScanJobs jobs) {
 #pragma unroll
         for (int k = 0; k < kScanItems; k++) v[k] = base + k < n ? in[base + k] : 0u;
     }
-    uint64_t sum = 0;
+    uint32_t sum = 0, bits = 0;
 #pragma unroll
-    for (int k = 0; k < kScanItems; k++) sum += v[k];
+    for (int k = 0; k < kScanItems; k++) {
+        sum += v[k];
+        bits |= v[k];
+    }
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    const uint64_t inc = warp_inclusive(sum);
+    const uint32_t inc = warp_inclusive(sum);
     if (lane == 31) warp_sums[warp] = inc;
-    __syncthreads();
+    static_assert(kScanTile <= 1u << 12, "elements below 2^20 add up to 32 bits");
+    const bool wide = __syncthreads_or(bits >> 20);
+    if (wide) {
+        uint64_t w = 0;
+        for (int k = 0; k < kScanItems; k++) w += v[k];
+        for (int d = 16; d > 0; d >>= 1) w += __shfl_xor_sync(0xffffffffu, w, d);
+        if (lane == 0) wide_sums[warp] = w;
+        __syncthreads();
+    }
     if (warp == 0) {
-        const uint64_t w = lane < kScanThreads / 32 ? warp_sums[lane] : 0u;
-        const uint64_t wi = warp_inclusive(w);
+        const uint32_t w = lane < kScanThreads / 32 ? warp_sums[lane] : 0u;
+        const uint32_t wi = warp_inclusive(w);
         if (lane < kScanThreads / 32) warp_sums[lane] = wi - w;
-        const uint64_t agg = __shfl_sync(0xffffffffu, wi, kScanThreads / 32 - 1);
+        uint64_t agg = __shfl_sync(0xffffffffu, wi, kScanThreads / 32 - 1), prefix = 0;
+        if (wide) {
+            agg = 0;
+            for (int k = 0; k < kScanThreads / 32; k++) agg += wide_sums[k];
+        }
         // publish the aggregate, then look back over a window of 32 predecessors at a time
         // (lane l reads tile `base - l`); stop at the nearest inclusive prefix
         volatile unsigned long long *st = state + 1;
@@ -97,7 +116,6 @@ __global__ void __launch_bounds__(kScanThreads) k_scan(ScanJobs jobs) {
             }
         } else {
             if (lane == 0) st[tile] = kFlagAgg | agg;
-            uint64_t prefix = 0;
             int64_t base = (int64_t)tile - 1;
             uint32_t spins = 0;
             for (;;) {
@@ -123,17 +141,16 @@ __global__ void __launch_bounds__(kScanThreads) k_scan(ScanJobs jobs) {
             }
             if (lane == 0) {
                 st[tile] = kFlagInc | (prefix + agg);
-                s_prefix = prefix;
+                s_prefix = (uint32_t)prefix;
             }
         }
+        if (lane == 0 && tile == tiles - 1 && job.over && (prefix + agg) >> 32) atomicOr(err, job.over);
     }
     __syncthreads();
-    const uint64_t upto = s_prefix + warp_sums[warp] + inc;  // this thread's elements included
-    uint32_t run = (uint32_t)(upto - sum);
+    uint32_t run = s_prefix + warp_sums[warp] + inc - sum;
     if (tile == tiles - 1 && threadIdx.x == kScanThreads - 1) {
-        if (job.total) *job.total = (uint32_t)upto;
-        if (job.end) *job.end = (uint32_t)upto;
-        if (job.over && upto >> 32) atomicOr(err, job.over);
+        if (job.total) *job.total = run + sum;
+        if (job.end) *job.end = run + sum;
     }
     if (base + kScanItems <= n && ((reinterpret_cast<uintptr_t>(out + base) & 15) == 0)) {
         uint32_t o[kScanItems];
