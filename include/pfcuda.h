@@ -336,7 +336,7 @@ typedef struct pf_tuning {
                                     16896 words); 0: as many as fit */
     float long_line;             /* lines spanning more tiles than this are walked by a whole warp */
     uint32_t bin_concurrent;     /* 1: the binning classes always run at once, on side streams; 0: they do
-                                    where several classes have paths and the frame is not too long */
+                                    where several classes have paths */
     uint32_t seg_sorted;         /* 0 or 1; changes nothing (segments are no longer ordered by depth) */
     uint32_t composite_ticket;   /* n > 0: the composite's warps stay resident and take n consecutive
                                     framebuffer tiles per ticket from a frame-wide queue (at most

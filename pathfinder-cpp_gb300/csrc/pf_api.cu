@@ -1266,13 +1266,15 @@ int bin_and_composite(Ctx *c, Batch b, bool learned, uint64_t max_leaves) {
         has.cluster = counts[4];
         has.large = counts[13] >> 8;  // the paths, above 40 bits of their lines
     }
-    // the binning classes at once where several have paths (20,000 paths 1607 -> 1497 us, mixed 8,192
-    // paths 1456 -> 1247 us, stroked batch 3.10 -> 2.63 ms), but not in frames so long that their
-    // tails no longer count (256 scenes, 178,734 paths, 13.43 -> 13.45 ms); the forks and joins cost
-    // 10 to 15 us (150,000 glyphs, all of one class, 1219 -> 1233 us)
+    // the binning classes at once where several have paths: the last paths of one then overlap the next
+    // (binning of 8,192 and 70,000 mixed paths 0.36 -> 0.29 and 1.83 -> 1.70 ms, of 20,000 and 200,000 large
+    // ones 0.79 -> 0.71 and 6.01 -> 5.97, of 256 scenes with 190,295 paths 8.77 -> 8.72); with one class
+    // only the fork and join are left (150,000 glyphs 0.292 -> 0.295).  A learned frame goes by the
+    // classes that its rects ask for: which paths go up one for their lines is not known yet, and they
+    // are few
     int classes = (has.small != 0) + (has.cluster != 0) + (has.large != 0);
     for (int k = 0; k < 3; k++) classes += (learned ? rects[k] : has.cta[k]) != 0;
-    const bool at_once = c->tune.bin_concurrent || (classes > 1 && N <= 1u << 16);
+    const bool at_once = c->tune.bin_concurrent || classes > 1;
     size_t slots = 0;
     PF_CUDA(bin_stage_slots(c->tune, c->n_sms, has, at_once, &slots));
     PF_CUDA(c->bin_stage.ensure(slots * 12));
