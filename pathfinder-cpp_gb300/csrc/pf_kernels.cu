@@ -1512,6 +1512,16 @@ __device__ __forceinline__ PathLeaves path_leaves(const Batch &b, uint32_t p) {
     return L;
 }
 
+// Lines a warp of a CTA (or cluster) of `warps` takes at a time: 32, one a lane, or fewer where they are
+// long.  A closed outline crosses its rect there and back, so its n lines span at least 2 (rw + rh) / n
+// tiles on average; past long_line the warp walks its lines one after the other, and so many lines fill
+// its part of the stage.  They are then dealt out evenly.  (Binning of 2,000 paths of 40 points, about
+// 375 x 375 tiles each: 8.75 ms by groups of 32, 4.72 so; 300 quadrilaterals on 8,192 px 3.61 and 3.09.)
+__device__ __forceinline__ uint32_t line_group(const Batch &b, uint32_t rw, uint32_t rh, uint32_t n, uint32_t warps) {
+    const bool spread = (float)(2u * (rw + rh)) > b.long_line * (float)n;
+    return spread ? min(32u, max(1u, (n + warps - 1u) / warps)) : 32u;
+}
+
 // Whether a walk of this frame hit its bound (the frame then ends with that error).  The lane form walks
 // such a line through other tiles than walk_line, so its counts are not to be filled by a second walk,
 // nor the fills read.  Past a barrier, a block sees what its own walks have found.  The CTA classes ask
@@ -1737,7 +1747,7 @@ __global__ void __launch_bounds__(class_threads(kCls), class_min_ctas(kCls)) k_b
         __syncthreads();
 
         // 1. fill counts and backdrop deltas, the fills staged with their tiles.  Warps take
-        //    the lines 32 at a time, so a warp that drew short lines takes more.
+        //    the lines a group at a time, so a warp that drew short lines takes more.
         //    A line of many tiles (a contour's closing line spans the canvas) would hold its
         //    warp, and at the barrier its CTA, for tens of steps: such lines are walked by the
         //    whole warp after its short lines.
@@ -1776,13 +1786,14 @@ __global__ void __launch_bounds__(class_threads(kCls), class_min_ctas(kCls)) k_b
             }
             nstage += __popc(keep);
         };
+        const uint32_t group = line_group(b, rw, rh, L.n, kWarps);
         for (;;) {
             uint32_t k0 = 0;
-            if (lane == 0) k0 = atomicAdd(&s_next, 32u);
+            if (lane == 0) k0 = atomicAdd(&s_next, group);
             k0 = __shfl_sync(0xffffffffu, k0, 0);
             if (k0 >= L.n) break;
             const uint32_t k = k0 + (uint32_t)lane;
-            const bool have = k < L.n;
+            const bool have = (uint32_t)lane < group && k < L.n;
             const float4 f = have ? b.leaves[L.index(b, k)] : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
             walk_lines(w, f, have, b.long_line, visit, on_above, on_fill, on_delta, begin_single, end_single, err);
         }
@@ -2155,7 +2166,7 @@ __global__ void __cluster_dims__(kClusterCtas, 1, 1) __launch_bounds__(kClusterT
         cluster_sync();
 
         // 1. fill counts and backdrop deltas into the bands' counters, the visits staged.  CTA r
-        //    takes every fourth group of 32 lines from group r.
+        //    takes every fourth group of lines from group r.
         auto tile_addr = [&](uint32_t local) {
             const uint32_t r = (uint32_t)(local >= band) + (uint32_t)(local >= 2 * band) + (uint32_t)(local >= 3 * band);
             return cluster_addr(cnt + (local - r * band), r);
@@ -2193,13 +2204,14 @@ __global__ void __cluster_dims__(kClusterCtas, 1, 1) __launch_bounds__(kClusterT
             }
             nstage += __popc(keep);
         };
+        const uint32_t group = line_group(b, rw, rh, L.n, kClusterWarps * kClusterCtas);
         for (;;) {
             uint32_t g = 0;
             if (lane == 0) g = atomicAdd(&s_next, 1u);
-            const uint32_t k0 = (__shfl_sync(0xffffffffu, g, 0) * kClusterCtas + rank) * 32u;
+            const uint32_t k0 = (__shfl_sync(0xffffffffu, g, 0) * kClusterCtas + rank) * group;
             if (k0 >= L.n) break;
             const uint32_t k = k0 + (uint32_t)lane;
-            const bool have = k < L.n;
+            const bool have = (uint32_t)lane < group && k < L.n;
             const float4 f = have ? b.leaves[L.index(b, k)] : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
             walk_lines(w, f, have, b.long_line, visit, on_above, on_fill, on_delta, begin_single, end_single, err);
         }
