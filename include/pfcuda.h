@@ -334,7 +334,8 @@ typedef struct pf_tuning {
     uint32_t bin_ctas_per_sm[3]; /* binning CTAs resident per SM for the three CTA classes (paths
                                     whose rect plus a row of column sums takes <= 1088, 4352,
                                     16896 words); 0: as many as fit */
-    float long_line;             /* lines spanning more tiles than this are walked by a whole warp */
+    float long_line;             /* lines spanning more tiles than this are walked by a whole warp,
+                                    where they are few among the warp's 32 */
     uint32_t bin_concurrent;     /* 1: the binning classes always run at once, on side streams; 0: they do
                                     where several classes have paths */
     uint32_t seg_sorted;         /* 0 or 1; changes nothing (segments are no longer ordered by depth) */
