@@ -3447,14 +3447,16 @@ static cudaError_t cluster_grid(unsigned *grid, uint32_t n_paths) {
 }
 
 // The grids of the classes that can have paths, and their slices of the stage.  Classes of one stream run
-// one after the other and share a slice: on their own streams the cluster class with class 1, and class
-// 0 with the small one; all of them in a frame that runs them in turn.  (A slice for each of the five
+// one after the other and share a slice: on their own streams the cluster class with class 1 (in frames
+// with class 3, whose passes come first on that stream, with class 2: three paths of 4,000 long lines on
+// 8,192 px, two of them of class 3, 3.33 -> 1.98 ms), and class 0 with the small one; all of them in a frame that runs them in turn.  (A slice for each of the five
 // classes, whether the frame has it or not: a first frame of 240 paths took 178 MB and 614 us, now 68 MB
 // and 550 us, one of 20,000 paths 4.07 ms, now 2.25; later frames are the same.)
 struct BinLaunch {
     unsigned cta[3] = {}, small = 0, cluster = 0;
     size_t first[3] = {};                         // class c's slice
     size_t first_small = 0, first_cluster = 0, slots = 0;
+    bool cluster_aside = false;                   // the cluster class on class 2's stream
 };
 
 static cudaError_t bin_launch(const Tuning &t, uint32_t n_sms, const BinClasses &has, bool at_once, BinLaunch &l) {
@@ -3465,11 +3467,15 @@ static cudaError_t bin_launch(const Tuning &t, uint32_t n_sms, const BinClasses 
     if (e == cudaSuccess && has.small) e = small_grid(&l.small, n_sms, has.small);
     if (e == cudaSuccess && has.cluster) e = cluster_grid(&l.cluster, has.cluster);
     if (e != cudaSuccess) return e;
-    const size_t own = std::max(size_t(l.cta[1]) * class_stage(1), size_t(l.cluster) * kClusterWarps * kClusterStage);
-    const size_t side0 = size_t(l.cta[2]) * class_stage(2);
+    const size_t cluster = size_t(l.cluster) * kClusterWarps * kClusterStage;
+    size_t own = size_t(l.cta[1]) * class_stage(1), side0 = size_t(l.cta[2]) * class_stage(2);
+    l.cluster_aside = at_once && has.large;
+    size_t &with = l.cluster_aside ? side0 : own;
+    with = std::max(with, cluster);
     const size_t side1 = std::max(size_t(l.cta[0]) * class_stage(0), size_t(l.small) * kSmallWarps * kSmallSpill);
     if (at_once) {
         l.first[2] = own;
+        if (l.cluster_aside) l.first_cluster = own;
         l.first[0] = l.first_small = own + side0;
         l.slots = own + side0 + side1;
     } else {
@@ -3518,11 +3524,12 @@ cudaError_t launch_bin_paths(const Batch &b, const Tuning &t, const BinClasses &
         c.stage_tile += first;
         return c;
     };
+    cudaStream_t const st2 = bs ? bs->side[0] : st, st0 = bs ? bs->side[1] : st;
     if (has.cluster) {
-        PF_LAUNCH(k_bin_cluster<<<l.cluster, kClusterThreads, kClusterSmem, st>>>(slice(l.first_cluster)));
+        PF_LAUNCH(k_bin_cluster<<<l.cluster, kClusterThreads, kClusterSmem, l.cluster_aside ? st2 : st>>>(
+            slice(l.first_cluster)));
         if ((e = cudaGetLastError()) != cudaSuccess) return e;
     }
-    cudaStream_t const st2 = bs ? bs->side[0] : st, st0 = bs ? bs->side[1] : st;
     if (has.cta[2] && (e = launch_fused<2>(slice(l.first[2]), l.cta[2], st2)) != cudaSuccess) return e;
     if (has.cta[1] && (e = launch_fused<1>(slice(l.first[1]), l.cta[1], st)) != cudaSuccess) return e;
     if (has.cta[0] && (e = launch_fused<0>(slice(l.first[0]), l.cta[0], st0)) != cudaSuccess) return e;
