@@ -2316,16 +2316,18 @@ __global__ void __cluster_dims__(kClusterCtas, 1, 1) __launch_bounds__(kClusterT
                 if (e) b.fills[at + m] = t & kVisitDown ? make_uint2(0u, q.x) : make_uint2(q.y, 0u);
             }
         } else if (s_write) {
-            for (uint32_t k0 = ((uint32_t)warp * kClusterCtas + rank) * 32u; k0 < L.n;
-                 k0 += kClusterWarps * kClusterCtas * 32u) {
-                if (k0 + (uint32_t)lane >= L.n) continue;
-                const float4 f = b.leaves[L.index(b, k0 + (uint32_t)lane)];
+            // the lines that this CTA's warps counted: every fourth group, from group `rank`
+            for (uint32_t j = tid;; j += kClusterThreads) {
+                const uint32_t k = (j / group * kClusterCtas + rank) * group + j % group;
+                if (k >= L.n) break;
+                const float4 f = b.leaves[L.index(b, k)];
                 walk_line(
                     w, f.x, f.y, f.z, f.w,
                     [&](int32_t local, uint2 q) { b.fills[cluster_fetch_add(tile_addr((uint32_t)local), 1u)] = q; },
                     [&](int32_t, int) {}, err);
             }
         }
+        __syncwarp();  // whole warps at the barrier
     }
 }
 
