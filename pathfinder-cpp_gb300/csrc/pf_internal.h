@@ -386,10 +386,10 @@ struct StatusCopy {
 // (counts, backdrops, fill offsets, fills).  A learned frame first lists its pooled lines by path:
 // count, scan pool_cnt, scatter.
 cudaError_t launch_bin_lists(const Batch &b, bool learned, const StatusCopy &copy, cudaStream_t st);
-// side[0..1], fork, join[0..1]: streams and events for running the classes at once, or null.
+// Streams and events for running the classes at once, or null.
 struct BinStreams {
-    cudaStream_t side[2];
-    cudaEvent_t fork, join[2];
+    cudaStream_t side[3];
+    cudaEvent_t fork, join[3];
 };
 // The paths each class can have at most (0: none): the CTA classes, a warp's, a cluster's, that of the
 // global passes.

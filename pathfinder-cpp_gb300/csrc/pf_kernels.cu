@@ -841,7 +841,7 @@ __device__ __forceinline__ void lane_steps(const WalkCtx &w, const LaneLine &s, 
 // the whole warp, one after the other - unless they are so many that 32 lanes in step are done sooner: a
 // step in lockstep costs what some four of a warp's do, so where the long lines' steps add up to more than
 // four times the longest's, they stay with their lanes.  (A hatching of 1,000 paths with 400 lines of
-// about 100 tiles: binning 4.70 -> 1.89 ms; of 40 tiles 0.96 -> 0.32; 256 scenes the same.)  The few
+// about 100 tiles: binning 4.80 -> 2.02 ms; of 40 tiles 0.97 -> 0.32; 256 scenes the same.)  The few
 // outside the fast form's range (coordinates beyond 2^20, or tiny) are walked by their lane alone, both
 // with on_fill / on_delta after begin_single() and before end_single().
 template <class Visit, class OnAbove, class OnFill, class OnDelta, class Begin, class End>
@@ -1528,7 +1528,7 @@ __device__ __forceinline__ PathLeaves path_leaves(const Batch &b, uint32_t p) {
 // long.  A closed outline crosses its rect there and back, so its n lines span at least 2 (rw + rh) / n
 // tiles on average; past long_line the warp walks its lines one after the other, and so many lines fill
 // its part of the stage.  They are then dealt out evenly.  (Binning of 2,000 paths of 40 points, about
-// 375 x 375 tiles each: 8.75 ms by groups of 32, 4.72 so; 300 quadrilaterals on 8,192 px 3.61 and 3.09.)
+// 375 x 375 tiles each: 8.75 ms by groups of 32, 4.80 so; 300 quadrilaterals on 8,192 px 3.61 and 3.09.)
 __device__ __forceinline__ uint32_t line_group(const Batch &b, uint32_t rw, uint32_t rh, uint32_t n, uint32_t warps) {
     const bool spread = (float)(2u * (rw + rh)) > b.long_line * (float)n;
     return spread ? min(32u, max(1u, (n + warps - 1u) / warps)) : 32u;
@@ -3449,16 +3449,18 @@ static cudaError_t cluster_grid(unsigned *grid, uint32_t n_paths) {
 }
 
 // The grids of the classes that can have paths, and their slices of the stage.  Classes of one stream run
-// one after the other and share a slice: on their own streams the cluster class with class 1 (in frames
-// with class 3, whose passes come first on that stream, with class 2: three paths of 4,000 long lines on
-// 8,192 px, two of them of class 3, 3.33 -> 1.98 ms), and class 0 with the small one; all of them in a frame that runs them in turn.  (A slice for each of the five
+// one after the other and share a slice: on their own streams the cluster class with class 1, and class
+// 0 with the small one; all of them in a frame that runs them in turn.  Where there is a class 3, whose
+// passes come first on the main stream, the cluster class has a stream of its own: binning of three paths
+// of 4,000 long lines, two of them of class 3, 3.86 -> 2.53 ms, of 100 quadrilaterals on 6,000 px 1.93 ->
+// 1.82; on class 2's stream it held that up (20,000 paths, 0.66 -> 0.72).  (A slice for each of the five
 // classes, whether the frame has it or not: a first frame of 240 paths took 178 MB and 614 us, now 68 MB
 // and 550 us, one of 20,000 paths 4.07 ms, now 2.25; later frames are the same.)
 struct BinLaunch {
     unsigned cta[3] = {}, small = 0, cluster = 0;
     size_t first[3] = {};                         // class c's slice
     size_t first_small = 0, first_cluster = 0, slots = 0;
-    bool cluster_aside = false;                   // the cluster class on class 2's stream
+    bool cluster_aside = false;                   // the cluster class on a stream of its own
 };
 
 static cudaError_t bin_launch(const Tuning &t, uint32_t n_sms, const BinClasses &has, bool at_once, BinLaunch &l) {
@@ -3470,16 +3472,18 @@ static cudaError_t bin_launch(const Tuning &t, uint32_t n_sms, const BinClasses 
     if (e == cudaSuccess && has.cluster) e = cluster_grid(&l.cluster, has.cluster);
     if (e != cudaSuccess) return e;
     const size_t cluster = size_t(l.cluster) * kClusterWarps * kClusterStage;
-    size_t own = size_t(l.cta[1]) * class_stage(1), side0 = size_t(l.cta[2]) * class_stage(2);
     l.cluster_aside = at_once && has.large;
-    size_t &with = l.cluster_aside ? side0 : own;
-    with = std::max(with, cluster);
+    const size_t own = std::max(size_t(l.cta[1]) * class_stage(1), l.cluster_aside ? 0 : cluster);
+    const size_t side0 = size_t(l.cta[2]) * class_stage(2);
     const size_t side1 = std::max(size_t(l.cta[0]) * class_stage(0), size_t(l.small) * kSmallWarps * kSmallSpill);
     if (at_once) {
         l.first[2] = own;
-        if (l.cluster_aside) l.first_cluster = own;
         l.first[0] = l.first_small = own + side0;
         l.slots = own + side0 + side1;
+        if (l.cluster_aside) {
+            l.first_cluster = l.slots;
+            l.slots += cluster;
+        }
     } else {
         l.slots = std::max(own, std::max(side0, side1));
     }
@@ -3509,9 +3513,10 @@ cudaError_t launch_bin_paths(const Batch &b, const Tuning &t, const BinClasses &
     BinLaunch l;
     cudaError_t e = bin_launch(t, b.n_sms, has, bs != nullptr, l);
     if (e != cudaSuccess) return e;
+    const int sides = l.cluster_aside ? 3 : 2;
     if (bs) {
         if ((e = cudaEventRecord(bs->fork, st)) != cudaSuccess) return e;
-        for (int k = 0; k < 2; k++)
+        for (int k = 0; k < sides; k++)
             if ((e = cudaStreamWaitEvent(bs->side[k], bs->fork, 0)) != cudaSuccess) return e;
     }
     if (has.large) {
@@ -3528,7 +3533,7 @@ cudaError_t launch_bin_paths(const Batch &b, const Tuning &t, const BinClasses &
     };
     cudaStream_t const st2 = bs ? bs->side[0] : st, st0 = bs ? bs->side[1] : st;
     if (has.cluster) {
-        PF_LAUNCH(k_bin_cluster<<<l.cluster, kClusterThreads, kClusterSmem, l.cluster_aside ? st2 : st>>>(
+        PF_LAUNCH(k_bin_cluster<<<l.cluster, kClusterThreads, kClusterSmem, l.cluster_aside ? bs->side[2] : st>>>(
             slice(l.first_cluster)));
         if ((e = cudaGetLastError()) != cudaSuccess) return e;
     }
@@ -3539,7 +3544,7 @@ cudaError_t launch_bin_paths(const Batch &b, const Tuning &t, const BinClasses &
         PF_LAUNCH(k_bin_small<<<l.small, kSmallThreads, 0, st0>>>(slice(l.first_small)));
         if ((e = cudaGetLastError()) != cudaSuccess) return e;
     }
-    for (int k = 0; bs && k < 2; k++) {
+    for (int k = 0; bs && k < sides; k++) {
         if ((e = cudaEventRecord(bs->join[k], bs->side[k])) != cudaSuccess) return e;
         if ((e = cudaStreamWaitEvent(st, bs->join[k], 0)) != cudaSuccess) return e;
     }
