@@ -538,10 +538,10 @@ int stroke_upload(Ctx *c, const pf_scene_view *scenes, uint32_t n, const std::ve
         PF_CUDA(launch_stroke_order(in, 1, c->st_order_ctl.as<uint32_t>(), c->dash_order.as<uint32_t>(), st));
         in.dash_order = c->dash_order.as<uint32_t>();
         in.n_dashed = c->ustats.dashed_paths;
-        // the chunk pool: two chunks to begin each path, and 16 points for each input point or what
-        // the largest upload so far took; at most 2^26 points (0.6 GB)
+        // the chunk pool: a chunk to begin each path, and 16 points for each input point or what the
+        // largest upload so far took; at most 2^26 points (0.6 GB)
         const uint64_t chunk_points = std::max<uint64_t>(c->dash_points_hint, uint64_t(c->n_points) * 16);
-        const uint64_t chunk_cap = std::min<uint64_t>(2 * uint64_t(in.n_dashed) + chunk_points / kDashChunk,
+        const uint64_t chunk_cap = std::min<uint64_t>(uint64_t(in.n_dashed) + chunk_points / kDashChunk,
                                                       (1ull << 26) / kDashChunk);
         PF_CUDA(c->dash_chunks.ensure(chunk_cap * (16 + 9 * kDashChunk) + 16));
         char *pool = c->dash_chunks.as<char>();
@@ -554,17 +554,16 @@ int stroke_upload(Ctx *c, const pf_scene_view *scenes, uint32_t n, const std::ve
         PF_CUDA(launch_dash(in, false, status, st));
         PF_CUDA(scan_exclusive_u32(in.dash_pts, in.dash_pts, N, in.dash_pts + N, c->scan_temp.p, st, status));
         PF_CUDA(scan_exclusive_u32(in.dash_cnt, in.dash_cnt, N, in.dash_cnt + N, c->scan_temp.p, st, status));
-        uint32_t tot[3], w[6];
+        uint32_t w[4];
         PF_CUDA(mark(1));
-        if (int e = read_words(c, {in.dash_pts + N, in.dash_cnt + N, status + kStFill64, status + kStFill64 + 1,
-                                   status + kStErr, status + kStDashChunks}, w))
+        if (int e = read_words(c, {in.dash_pts + N, in.dash_cnt + N, status + kStErr, status + kStDashChunks}, w))
             return e;
-        tot[0] = w[0], tot[1] = w[1], tot[2] = w[4] & ~kErrOverflowTotal;  // `wide` catches that
-        const uint64_t wide = uint64_t(w[2]) | uint64_t(w[3]) << 32;  // the dash points' 64-bit total
-        if (tot[2] & kErrStroke)
+        const uint32_t tot[2] = {w[0], w[1]};
+        if (w[2] & kErrStroke)
             return fail(c, PF_ERR_KERNEL_LIMIT, "a dash pattern needs more than 2^22 steps on one path");
-        if (tot[2]) return fail(c, PF_ERR_CUDA, "dash pass failed");
-        if (wide >= (1ull << 31)) return fail(c, PF_ERR_OVERFLOW, "dashed outline too large (2^31 points)");
+        if (w[2] & ~kErrOverflowTotal) return fail(c, PF_ERR_CUDA, "dash pass failed");
+        if ((w[2] & kErrOverflowTotal) || tot[0] >= (1u << 31))
+            return fail(c, PF_ERR_OVERFLOW, "dashed outline too large (2^31 points)");
         c->stroke_dash_points = tot[0];
         PF_CUDA(c->dash_points.ensure(size_t(tot[0]) * 8 + 16));
         PF_CUDA(c->dash_flags.ensure(size_t(tot[0]) + 16));
@@ -573,9 +572,10 @@ int stroke_upload(Ctx *c, const pf_scene_view *scenes, uint32_t n, const std::ve
         in.dash_flags = c->dash_flags.as<uint8_t>();
         in.dash_end = c->dash_end.as<uint32_t>();
         PF_CUDA(mark(2));
-        in.n_dash_chunks = w[5];
-        c->dash_points_hint = std::max(c->dash_points_hint, uint64_t(w[5]) * kDashChunk);
-        if (w[5] <= in.dash_chunk_cap) PF_CUDA(launch_dash_gather(in, st));
+        const uint64_t chunks = uint64_t(in.n_dashed) + w[3];
+        in.n_dash_chunks = (uint32_t)chunks;
+        c->dash_points_hint = std::max(c->dash_points_hint, uint64_t(w[3]) * kDashChunk);
+        if (chunks <= in.dash_chunk_cap) PF_CUDA(launch_dash_gather(in, st));
         else PF_CUDA(launch_dash(in, true, status, st));
         PF_CUDA(mark(3));
     }

@@ -297,7 +297,7 @@ struct StrokeIn {
     uint4 *dash_chunk_head;
     float2 *dash_chunk_points;
     uint8_t *dash_chunk_flags;
-    uint32_t *dash_chunk_count;         // chunks taken (may run past dash_chunk_cap)
+    uint32_t *dash_chunk_count;         // chunks taken beyond each path's first (may run past dash_chunk_cap)
     uint32_t dash_chunk_cap, n_dash_chunks;
     uint32_t *job_first;                // [n_paths + 1] counts -> scanned
     uint4 *jobs;                        // [n_jobs]

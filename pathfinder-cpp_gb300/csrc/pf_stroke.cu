@@ -559,9 +559,11 @@ __device__ __forceinline__ uint2 path_contours(const StrokeIn &in, uint32_t p) {
 // * no state beside the segment in hand: pieces stay in the lanes, a point each, until the next would
 //   not fit, and all then go out together; the loop over a segment knows its kind and selects rather
 //   than branches, since a lone warp waits out each branch (a step is some 130 instructions);
-// * the path is walked once.  Its points go to chunks of kDashChunk points, taken from a pool as
-//   they are needed (the next one a chunk ahead), and k_dash_gather copies them to the path's place
-//   once the counts are scanned.  A pool that runs out costs a second walk, straight to that place.
+// * the path is walked once.  Its points go to chunks of kDashChunk points, and k_dash_gather copies them
+//   to the path's place once the counts are scanned.  Each path has a first chunk; further ones are taken
+//   from a pool when the next points may not fit, as all paths count at one address (a chunk always asked
+//   for ahead, and the points added up there too, took 0.69 ms for 200,000 dashed lines, now 0.34).
+//   A pool that runs out costs a second walk, straight to that place.
 //
 // (5,689 dashed paths, 1.3M points, the longest of 4,000 steps: 5.65 ms for the two passes of one
 // path per lane, 2.30 ms with a warp per path walked by one lane, 1.85 by all with each piece put out
@@ -620,9 +622,9 @@ __global__ void __launch_bounds__(64) k_dash(StrokeIn in, uint32_t *status) {
     const uint32_t pt0 = kWrite ? in.dash_pts[p] : 0u, c0 = kWrite ? in.dash_cnt[p] : 0u;
     uint32_t pts = 0, begun = 0;  // points of the path so far, and the contours they begin
     bool open = false;            // the last of those contours has not ended
-    // count pass: the chunk in hand, and the next one (lane 0)
-    uint32_t chunk = 0, next_chunk = 0;
-    if (!kWrite && lane == 0) next_chunk = atomicAdd(in.dash_chunk_count, 1u);
+    // count pass: the chunk in hand, and the next one (lane 0), which every path has to begin with
+    uint32_t chunk = 0, next_chunk = t0;
+    bool ahead_of_use = true;  // there is a next one
     // the pieces since the last drain: a point per lane, the lanes where pieces begin, and those
     // whose points end a contour
     float2 point = make_float2(0.0f, 0.0f);
@@ -663,13 +665,18 @@ __global__ void __launch_bounds__(64) k_dash(StrokeIn in, uint32_t *status) {
                 if (lane == 0) {
                     if (chunk < in.dash_chunk_cap)
                         in.dash_chunk_head[chunk] = make_uint4(p, border, begun + __popc(before), 0u);
-                    next_chunk = atomicAdd(in.dash_chunk_count, 1u);
                 }
+                ahead_of_use = false;
             }
             if (out && mychunk < in.dash_chunk_cap) {
                 const uint32_t slot = mychunk * kDashChunk + at % kDashChunk;
                 in.dash_chunk_points[slot] = point;
                 in.dash_chunk_flags[slot] = (uint8_t)(flag | (first ? 0x80u : 0u));  // bit 7: of a contour
+            }
+            // the next drain's points (32 at most) may not fit
+            if (!ahead_of_use && (0u - (pts + n)) % kDashChunk < 32) {
+                if (lane == 0) next_chunk = in.n_dashed + atomicAdd(in.dash_chunk_count, 1u);
+                ahead_of_use = true;
             }
         }
         begun += __popc(starts);
@@ -745,8 +752,6 @@ __global__ void __launch_bounds__(64) k_dash(StrokeIn in, uint32_t *status) {
     if (!kWrite && lane == 0) {
         in.dash_pts[p] = pts;
         in.dash_cnt[p] = begun;
-        // 64-bit total beside the 32-bit scan, so that an overflowing batch is caught
-        atomicAdd(reinterpret_cast<unsigned long long *>(status + kStFill64), (unsigned long long)pts);
     }
 }
 
