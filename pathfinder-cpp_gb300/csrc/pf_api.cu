@@ -98,7 +98,7 @@ struct Ctx {
     uint64_t dash_points_hint = 0;  // points of the chunks the largest dashed upload took
     DevBuf dash_pts, dash_cnt, dash_end, dash_points, dash_flags, job_first, jobs, job_pts, st_bounds;
     DevBuf job_units, job_nfwd, job_flags, job_cap1, job_end, units, unit_leaves, st_leaves, leaf_pts;
-    DevBuf st_order_ctl, unit_order, dash_order;
+    DevBuf st_order_ctl, unit_order, dash_order, dash_list;
     uint32_t stroke_jobs = 0, stroke_dash_points = 0;  // of the last upload with strokes
     // gradient paints: per uploaded path its gradient (kNone: solid), per gradient its paint,
     // sorted stops, ramp and shader metadata; empty when the batch has no gradient
@@ -551,6 +551,12 @@ int stroke_upload(Ctx *c, const pf_scene_view *scenes, uint32_t n, const std::ve
         in.dash_chunk_count = status + kStDashChunks;
         in.dash_chunk_cap = (uint32_t)chunk_cap;
         PF_CUDA(cudaMemsetAsync(pool, 0xff, chunk_cap * 16, st));  // no path
+        in.n_sms = c->n_sms;
+        if (in.n_dashed >= kDashLanes) {
+            PF_CUDA(c->dash_list.ensure(size_t(in.n_dashed) * 4));
+            in.dash_list = c->dash_list.as<uint32_t>();
+            PF_CUDA(launch_dash_lanes(in, false, status, st));
+        }
         PF_CUDA(launch_dash(in, false, status, st));
         PF_CUDA(scan_exclusive_u32(in.dash_pts, in.dash_pts, N, in.dash_pts + N, c->scan_temp.p, st, status));
         PF_CUDA(scan_exclusive_u32(in.dash_cnt, in.dash_cnt, N, in.dash_cnt + N, c->scan_temp.p, st, status));
@@ -575,6 +581,7 @@ int stroke_upload(Ctx *c, const pf_scene_view *scenes, uint32_t n, const std::ve
         const uint64_t chunks = uint64_t(in.n_dashed) + w[3];
         in.n_dash_chunks = (uint32_t)chunks;
         c->dash_points_hint = std::max(c->dash_points_hint, uint64_t(w[3]) * kDashChunk);
+        if (in.dash_list) PF_CUDA(launch_dash_lanes(in, true, status, st));
         if (chunks <= in.dash_chunk_cap) PF_CUDA(launch_dash_gather(in, st));
         else PF_CUDA(launch_dash(in, true, status, st));
         PF_CUDA(mark(3));
@@ -2089,7 +2096,7 @@ int pf_ctx_destroy(void *ctx) {
                       &c->job_units, &c->job_nfwd, &c->job_flags, &c->job_cap1, &c->job_end, &c->units,
                       &c->unit_leaves, &c->st_leaves, &c->leaf_pts, &c->path_grad, &c->grad_paint, &c->image_snap,
                       &c->grad_stop_range, &c->grad_stops, &c->grad_meta, &c->grad_ramp, &c->st_order_ctl,
-                      &c->unit_order, &c->dash_order};
+                      &c->unit_order, &c->dash_order, &c->dash_list};
     for (DevBuf *b : bufs) b->release();
     for (auto &e : c->ev)
         if (e) cudaEventDestroy(e);

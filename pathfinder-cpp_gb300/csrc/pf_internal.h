@@ -223,7 +223,8 @@ enum : int {
     kStSampledDeep = 23,
     kStDashChunks = 24,// upload: chunks of dashed points taken
     kStRectClass = 25, // six words: nonzero if a path's rect asks for that binning class
-    kStCount = 31,
+    kStDashLong = 31,  // upload: dashed paths left to the warps
+    kStCount = 32,
     // the binning's control words follow in the same buffer; the host reads the first of them too
     kStBinCtl = 64,
     kStHostWords = kStBinCtl + 16,
@@ -316,13 +317,17 @@ struct StrokeIn {
     float4 *leaves;                     // [n_leaves][3] piece, join point, (job, meta)
     uint32_t *leaf_pts;                 // [n_leaves + 1] counts -> scanned
     const uint32_t *unit_order;         // [n_units] units, the most work first (or null)
-    const uint32_t *dash_order;         // [n_dashed] the dashed paths, the most work first
+    uint32_t *dash_order;               // [n_dashed] the dashed paths, the most work first
     uint32_t n_dashed;
+    uint32_t *dash_list;                // the paths that a lane each left to the warps (null: warps take all)
+    uint32_t n_sms;
 };
 size_t stroke_order_ctl_bytes();
 cudaError_t launch_stroke_order(const StrokeIn &in, int what, uint32_t *ctl, uint32_t *order, cudaStream_t st);
 constexpr uint32_t kDashChunk = 64;  // points
 cudaError_t launch_dash(const StrokeIn &in, bool write, uint32_t *status, cudaStream_t st);
+constexpr uint32_t kDashLanes = 16384;  // dashed paths from which on short ones take a lane each: figures there
+cudaError_t launch_dash_lanes(const StrokeIn &in, bool write, uint32_t *status, cudaStream_t st);
 cudaError_t launch_dash_gather(const StrokeIn &in, cudaStream_t st);
 cudaError_t launch_copy_words(uint32_t *dst, const uint32_t *src, uint32_t n, cudaStream_t st);
 // up to 8 single words gathered into dst[0, n)

@@ -21,6 +21,7 @@
 // bit: Segment::offset and its helpers (core/stroke.cpp:370-540), LineSegmentF
 // (core/data/line_segment.cpp), Segment (core/data/segment.cpp), Mat2 / Transform2 /
 // UnitVector (common/math).
+#include <algorithm>
 #include <type_traits>
 
 #include "pf_internal.h"
@@ -569,8 +570,20 @@ __device__ __forceinline__ uint2 path_contours(const StrokeIn &in, uint32_t p) {
 // path per lane, 2.30 ms with a warp per path walked by one lane, 1.85 by all with each piece put out
 // by itself, 1.42 so; all with the ordering by size before and the gather after.)
 
-// Segment::arc_length (core/data/segment.cpp:141-187) of a segment all lanes hold; lane l % 4 takes
-// leg l of the control polygon (quadratics through to_cubic).
+// Segment::arc_length (core/data/segment.cpp:141-187; quadratics through to_cubic), by a lane.
+__device__ __forceinline__ float arc_length(const Seg &s) {
+    if (s.kind == kLine) return vlen(lvec(s.b));
+    LSeg c = s.c;
+    if (s.kind == kQuad) {
+        const V2 p1_2 = vadd(s.c.f, s.c.f);
+        const V2 c0 = vadd(s.b.f, p1_2), c1 = vadd(p1_2, s.b.t);
+        c = ls(mk(fd(c0.x, 3.0f), fd(c0.y, 3.0f)), mk(fd(c1.x, 3.0f), fd(c1.y, 3.0f)));
+    }
+    const float net = fa(fa(vlen(vsub(s.b.f, c.f)), vlen(lvec(c))), vlen(vsub(s.b.t, c.t)));
+    return fm(fa(net, vlen(lvec(s.b))), 0.5f);
+}
+
+// The same of a segment all lanes hold; lane l % 4 takes leg l of the control polygon.
 __device__ __forceinline__ float warp_arc_length(const Seg &s) {
     if (s.kind == kLine) return vlen(lvec(s.b));
     const int l = threadIdx.x & 3;
@@ -589,14 +602,10 @@ __device__ __forceinline__ float warp_arc_length(const Seg &s) {
     return fm(fa(net, __shfl_sync(0xffffffffu, leg, 3)), 0.5f);
 }
 
+// Path p, the t0-th that warps take.
 template <bool kWrite>
-__global__ void __launch_bounds__(64) k_dash(StrokeIn in, uint32_t *status) {
-    // the dashed paths, largest first (dash_order); every other path's counts are zeroed
-    // before the count pass
-    const uint32_t t0 = blockIdx.x * 2 + (threadIdx.x >> 5);
-    if (t0 >= in.n_dashed) return;
+__device__ __forceinline__ void dash_by_warp(const StrokeIn &in, uint32_t *status, uint32_t t0, uint32_t p) {
     const uint32_t lane = threadIdx.x & 31;
-    const uint32_t p = in.dash_order[t0];
     const pf_stroke &st = path_stroke(in, p);
     if (!stroked(in, p) || st.dash_count == 0) return;
     // DashState::DashState, dash.cpp:9-29
@@ -752,6 +761,109 @@ __global__ void __launch_bounds__(64) k_dash(StrokeIn in, uint32_t *status) {
     if (!kWrite && lane == 0) {
         in.dash_pts[p] = pts;
         in.dash_cnt[p] = begun;
+    }
+}
+
+// The dashed paths, largest first (dash_order); every other path's counts are zeroed before the count
+// pass.  kListed: those that k_dash_lanes has left.
+template <bool kWrite, bool kListed>
+__global__ void __launch_bounds__(64) k_dash(StrokeIn in, uint32_t *status) {
+    uint32_t t = blockIdx.x * 2 + (threadIdx.x >> 5);
+    if (!kListed) {
+        if (t < in.n_dashed) dash_by_warp<kWrite>(in, status, t, in.dash_order[t]);
+        return;
+    }
+    const uint32_t n = status[kStDashLong];
+    for (; t < n; t += gridDim.x * 2) {
+        dash_by_warp<kWrite>(in, status, t, in.dash_list[t]);
+        __syncwarp();
+    }
+}
+
+// Many short paths: a lane each.  With some 20,000 paths the chains fill the GPU whoever walks them, and
+// what counts is how many instructions they take together; a warp's 32 lanes on one chain are then 31
+// too many.  A lane counts its path's points and contours, and walks it again to write them; a path of more
+// than kLaneSteps steps is left to the warps (its place in dash_order marked), as its chain would keep 31
+// other lanes waiting.  (Dashing 200,000 lines of 7 points of dashes each: 0.34 ms by warps, 0.12 so; of 32
+// points 0.82 and 0.30; 60,000 lines 0.14 and 0.09; 20,000, 0.086 and 0.080, of 32 points 0.148 and 0.132.)
+constexpr uint32_t kLaneSteps = 64, kLongPath = 1u << 31;
+
+template <bool kWrite>
+__global__ void __launch_bounds__(128) k_dash_lanes(StrokeIn in, uint32_t *status) {
+    const uint32_t t = blockIdx.x * blockDim.x + threadIdx.x;
+    if (t >= in.n_dashed) return;
+    const uint32_t p = in.dash_order[t];
+    if (kWrite && (p & kLongPath)) return;
+    const pf_stroke &st = path_stroke(in, p);
+    if (!stroked(in, p) || st.dash_count == 0) return;
+    // DashState::DashState, dash.cpp:9-29
+    const float *const dashes = in.dashes + st.dash_first;
+    const uint32_t count = st.dash_count;
+    float total = 0.0f;
+    for (uint32_t i = 0; i < count; i++) total = fa(total, dashes[i]);
+    float left = fmodf(st.dash_offset, total);
+    uint32_t idx = 0;
+    for (; idx < count && !(left < dashes[idx]); idx++) left = fs(left, dashes[idx]);
+    if (idx >= count) {  // the phase ran past the pattern
+        atomicOr(&status[kStErr], kErrStroke);
+        return;
+    }
+    uint32_t at = kWrite ? in.dash_pts[p] : 0u, contours = kWrite ? in.dash_cnt[p] : 0u, first = at, steps = 0;
+    auto push = [&](V2 q, uint8_t f) {
+        if (kWrite) {
+            in.dash_points[at] = make_float2(q.x, q.y);
+            in.dash_flags[at] = f;
+        }
+        at++;
+    };
+    auto end_contour = [&]() {  // Outline::push_contour: empty contours are dropped
+        if (at == first) return;
+        if (kWrite) in.dash_end[contours] = at;
+        contours++;
+        first = at;
+    };
+    const uint2 kr = path_contours(in, p);
+    for (uint32_t k = kr.x; k < kr.y; k++) {
+        const Contour c = raw_contour(in, k);
+        // ContourDash::dash, dash.cpp:68-124
+        SegIter it{&c, 0, true};
+        while (it.has_next) {
+            Seg rest = it.next();
+            if (rest.kind == kNone) break;
+            bool more;
+            do {
+                if (++steps > kLaneSteps && !kWrite) {
+                    in.dash_order[t] = p | kLongPath;
+                    in.dash_list[atomicAdd(&status[kStDashLong], 1u)] = p;
+                    return;
+                }
+                float distance = left;
+                const float length = arc_length(rest), u = fd(left, length);
+                Seg piece = rest;
+                more = u < 1.0f;
+                if (more) split_below(Seg(rest), u, piece, rest);
+                else distance = length;
+                if ((idx & 1u) == 0 && svalid(piece)) {  // core/data/contour.cpp:11-41
+                    push(piece.b.f, kOn);
+                    if (piece.kind != kLine) {
+                        push(piece.c.f, kC0);
+                        if (piece.kind != kQuad) push(piece.c.t, kC1);
+                    }
+                    push(piece.b.t, kOn);
+                }
+                left = fs(left, distance);
+                if (left < kFloatEps) {
+                    if ((idx & 1u) == 0) end_contour();
+                    idx = idx + 1 == count ? 0u : idx + 1;
+                    left = dashes[idx];
+                }
+            } while (more);
+        }
+    }
+    if ((idx & 1u) == 0) end_contour();  // OutlineDash::into_outline, dash.cpp:57-63
+    if (!kWrite) {
+        in.dash_pts[p] = at;
+        in.dash_cnt[p] = contours;
     }
 }
 
@@ -1376,8 +1488,22 @@ static uint32_t blocks(uint32_t n, uint32_t t) { return (n + t - 1) / t; }
 
 cudaError_t launch_dash(const StrokeIn &in, bool write, uint32_t *status, cudaStream_t st) {
     if (!in.n_dashed) return cudaSuccess;
-    if (write) k_dash<true><<<blocks(in.n_dashed, 2), 64, 0, st>>>(in, status);
-    else k_dash<false><<<blocks(in.n_dashed, 2), 64, 0, st>>>(in, status);
+    if (!in.dash_list) {
+        if (write) k_dash<true, false><<<blocks(in.n_dashed, 2), 64, 0, st>>>(in, status);
+        else k_dash<false, false><<<blocks(in.n_dashed, 2), 64, 0, st>>>(in, status);
+    } else {
+        // as many warps as there could be work for, no more than the SMs hold
+        const uint32_t grid = std::min(blocks(in.n_dashed, 2), 16u * in.n_sms);
+        if (write) k_dash<true, true><<<grid, 64, 0, st>>>(in, status);
+        else k_dash<false, true><<<grid, 64, 0, st>>>(in, status);
+    }
+    count_launches(1);
+    return cudaGetLastError();
+}
+
+cudaError_t launch_dash_lanes(const StrokeIn &in, bool write, uint32_t *status, cudaStream_t st) {
+    if (write) k_dash_lanes<true><<<blocks(in.n_dashed, 128), 128, 0, st>>>(in, status);
+    else k_dash_lanes<false><<<blocks(in.n_dashed, 128), 128, 0, st>>>(in, status);
     count_launches(1);
     return cudaGetLastError();
 }
