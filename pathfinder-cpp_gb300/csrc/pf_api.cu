@@ -529,6 +529,7 @@ int stroke_upload(Ctx *c, const pf_scene_view *scenes, uint32_t n, const std::ve
     PF_CUDA(c->scan_temp.ensure(scan_temp_bytes(N + 1)));
 
     PF_CUDA(c->st_order_ctl.ensure(stroke_order_ctl_bytes()));
+    uint64_t contours = C;  // and the dashed ones
     // dashing: counts, offsets, the dashed contours (the dashed paths taken longest first)
     if (dashed) {
         PF_CUDA(mark(0));
@@ -571,6 +572,7 @@ int stroke_upload(Ctx *c, const pf_scene_view *scenes, uint32_t n, const std::ve
         if ((w[2] & kErrOverflowTotal) || tot[0] >= (1u << 31))
             return fail(c, PF_ERR_OVERFLOW, "dashed outline too large (2^31 points)");
         c->stroke_dash_points = tot[0];
+        contours += tot[1];
         PF_CUDA(c->dash_points.ensure(size_t(tot[0]) * 8 + 16));
         PF_CUDA(c->dash_flags.ensure(size_t(tot[0]) + 16));
         PF_CUDA(c->dash_end.ensure(size_t(tot[1]) * 4 + 16));
@@ -604,7 +606,7 @@ int stroke_upload(Ctx *c, const pf_scene_view *scenes, uint32_t n, const std::ve
         return span();
     };
     PF_CUDA(mark(4));
-    PF_CUDA(launch_stroke_jobs(in, false, st));
+    PF_CUDA(launch_stroke_jobs(in, contours, false, st));
     PF_CUDA(scan_exclusive_u32(in.job_first, in.job_first, N, in.job_first + N, c->scan_temp.p, st, status));
     uint32_t J = 0;
     if (int e = read_u32(in.job_first + N, J)) return e;
@@ -628,7 +630,7 @@ int stroke_upload(Ctx *c, const pf_scene_view *scenes, uint32_t n, const std::ve
     c->stroke_jobs = J;
     // units: every stroked contour's segments, forward and backward
     PF_CUDA(mark(4));
-    PF_CUDA(launch_stroke_jobs(in, true, st));
+    PF_CUDA(launch_stroke_jobs(in, contours, true, st));
     PF_CUDA(cudaMemsetAsync(in.job_flags, 0, size_t(J) * 4, st));
     PF_CUDA(launch_units(in, false, st));
     PF_CUDA(scan_exclusive_u32(in.job_units, in.job_units, J, in.job_units + J, c->scan_temp.p, st, status));

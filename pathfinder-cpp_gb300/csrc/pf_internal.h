@@ -337,7 +337,8 @@ struct WordSources {
 };
 cudaError_t launch_gather_words(uint32_t *dst, const WordSources &s, cudaStream_t st);
 cudaError_t launch_copy_bytes(uint8_t *dst, const uint8_t *src, uint32_t n, cudaStream_t st);
-cudaError_t launch_stroke_jobs(const StrokeIn &in, bool fill, cudaStream_t st);
+// n_contours: of the outline and the dash pass together.
+cudaError_t launch_stroke_jobs(const StrokeIn &in, uint64_t n_contours, bool fill, cudaStream_t st);
 cudaError_t launch_stroke(const StrokeIn &in, bool write, uint32_t *status, cudaStream_t st);
 cudaError_t launch_units(const StrokeIn &in, bool write, cudaStream_t st);
 cudaError_t launch_unit_leaves(const StrokeIn &in, bool write, cudaStream_t st);
