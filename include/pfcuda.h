@@ -275,7 +275,10 @@ int pf_scene_upload(void *ctx, const pf_scene_view *scene);
 
 /*
  * Upload a batch of independent scenes (each keeps its own canvas and image).
- * Host ranges that are contiguous across scenes are copied with one transfer.
+ * Short arrays are gathered in mapped host memory and spread over the device by one kernel; longer
+ * ones are copied, those that are contiguous across scenes with one transfer.  A batch that is
+ * rejected (PF_ERR_INVALID_ARGUMENT, PF_ERR_OVERFLOW for too many points, contours, paths or
+ * tiles) leaves the one before it in place; one whose upload fails later leaves none.
  */
 int pf_scene_upload_batch(void *ctx, const pf_scene_view *scenes, uint32_t n_scenes);
 
@@ -333,7 +336,10 @@ int pf_auto_choice(void *ctx, int *last, int *choice, float *exact_ms, float *le
 typedef struct pf_tuning {
     uint32_t bin_ctas_per_sm[3]; /* binning CTAs resident per SM for the three CTA classes (paths
                                     whose rect plus a row of column sums takes <= 1088, 4352,
-                                    16896 words); 0: as many as fit */
+                                    16896 words); 0: as many as fit.  A path of many lines for its
+                                    rect goes up a class, one of <= 128 words and 384 lines to
+                                    single warps, and a rect past the largest class to clusters of
+                                    CTAs or global passes: no parameter sets their grids */
     float long_line;             /* lines spanning more tiles than this are walked by a whole warp,
                                     where they are few among the warp's 32 */
     uint32_t bin_concurrent;     /* 1: the binning classes always run at once, on side streams; 0: they do

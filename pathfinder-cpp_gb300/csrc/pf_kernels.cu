@@ -215,7 +215,6 @@ __global__ void __launch_bounds__(kPathThreads) k_paths(Batch b, uint2 *path_con
 // last, each with a kind read off the three flags after it, and their order is a ballot's.  (A
 // thread walking its contour point by point: 101 + 16 us for 300,000 glyph contours, 270 + 126 us
 // for the 420,000 of a stroked batch, 22 + 11 us where 240 contours are all there is.)
-
 //
 // The count pass also looks at the segments of every sample-th contour (about 2048 of them): how
 // many would bisect into more than kDeepLines lines, by the flatness value at the root, which a
@@ -931,15 +930,14 @@ __device__ __forceinline__ void walk_lines(const WalkCtx &w, float4 f, bool have
 //   the sizer's budget; lines past the budget spill into the shared pool, and an exhausted pool
 //   sets the overflow bit (the frame is then redone by the exact two-pass method);
 // * exact frame's write pass: each segment's lines go to its range of the leaf
-//   buffer, counted by the count pass.
-//
+//   buffer, counted by the count pass;
 // * exact frame's count pass: only the number of each segment's lines is kept.
 //
-// The bisection is shared by the 32 lanes of a warp.  With one segment per lane (as the exact
-// frame's k_flatten does) a warp runs the split branch and the emit branch of every step one after
+// The bisection is shared by the 32 lanes of a warp.  With one segment per lane (as k_flatten does where
+// segments are shallow) a warp runs the split branch and the emit branch of every step one after
 // the other, with only the lanes on one side doing work in each (13 of 32 lanes active on the
-// 512-scene batch, flattening 5.93 ms of the learned frame).  Here the lanes share the work of the
-// warp's segments instead (flattening 4.54 ms):
+// 512-scene batch; flattening took 5.93 ms of the learned frame that way, and 4.54 when this form came
+// in).  Here the lanes share the work of the warp's segments instead:
 //
 // * a split round: each lane takes a pending (not flat) piece from the warp's pool in shared
 //   memory, splits it at t = 0.5, and tests both halves: a flat half (or one at the depth bound)
@@ -1950,8 +1948,9 @@ __global__ void __launch_bounds__(class_threads(kCls), class_min_ctas(kCls)) k_b
 // lines and 10 tiles; a CTA spends most of its time on it in barriers and in waiting for the path's
 // record, while warps on paths of their own have no barriers and wait side by side.  Visits are
 // staged in shared memory (the rest, if any, in the warp's slice of the global stage).  Binning
-// 150,000 glyphs 0.47 -> 0.34 ms, 20,000 paths (half of them small) 0.73 -> 0.69 ms; 10 CTAs per SM
-// (48 registers, spills) instead of 8 take 0.37 ms, the next path's record loaded ahead 0.35 ms.
+// 150,000 glyphs 0.47 -> 0.34 ms, 20,000 paths (half of them small) 0.73 -> 0.69 ms; 8 CTAs
+// per SM leave 64 registers, and 68 bytes of spills; 10 (48 registers, more spills) take 0.37 ms, the next
+// path's record loaded ahead 0.35 ms.
 constexpr int kSmallThreads = 128, kSmallWarps = kSmallThreads / 32;
 constexpr uint32_t kSmallStage = 160, kSmallSpill = 640;  // visits staged per warp: shared, then global
 

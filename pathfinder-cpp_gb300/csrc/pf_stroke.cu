@@ -6,6 +6,7 @@
 //   k_dash<count/write>        one warp per dashed path walks its contours in order (the dash
 //                              state runs on across contours, core/dash.cpp:51-55), writing the
 //                              dashed contours into chunks that k_dash_gather puts in their place;
+//                              of many paths, k_dash_lanes takes the short ones, a lane each;
 //   k_stroke_jobs<count/fill>  one job per output contour: a copied contour (filled paths), an
 //                              open stroked contour (forward offset, cap, backward offset, cap)
 //                              or one of the two contours of a closed stroked contour (forward

@@ -4,8 +4,8 @@
 
 Uploads the batched configuration (scenes.batched: 512 scenes, seeds 1000+i), loads the sizer,
 and runs pf_autotune: coordinate descent over the binning CTAs per SM of each CTA class, the
-long-line threshold of the tile walk, concurrent binning classes, the flatten's segment order
-and the composite's tiles per ticket, each trial the default frame (pf_render_auto's choice)
+long-line threshold of the tile walk, concurrent binning classes and the composite's tiles per
+ticket, each trial the default frame (pf_render_auto's choice)
 timed on the device.  The file records the parameters, the frame time with the starting (built-in)
 parameters and with the tuned ones, the GPU, and the workload.  bench.py and
 pfcuda.Renderer.load_render_config apply it.
