@@ -98,7 +98,7 @@ struct Ctx {
     uint64_t dash_points_hint = 0;  // points of the chunks the largest dashed upload took
     DevBuf dash_pts, dash_cnt, dash_end, dash_points, dash_flags, job_first, jobs, job_pts, st_bounds;
     DevBuf job_units, job_nfwd, job_flags, job_cap1, job_end, units, unit_leaves, st_leaves, leaf_pts;
-    DevBuf st_order_ctl, unit_order, dash_order, dash_list;
+    DevBuf st_order_ctl, unit_order, dash_order, dash_steps;
     uint32_t stroke_jobs = 0, stroke_dash_points = 0;  // of the last upload with strokes
     // gradient paints: per uploaded path its gradient (kNone: solid), per gradient its paint,
     // sorted stops, ramp and shader metadata; empty when the batch has no gradient
@@ -536,9 +536,15 @@ int stroke_upload(Ctx *c, const pf_scene_view *scenes, uint32_t n, const std::ve
         PF_CUDA(c->dash_order.ensure(size_t(N) * 4 + 16));
         PF_CUDA(cudaMemsetAsync(in.dash_pts, 0, size_t(N) * 4, st));
         PF_CUDA(cudaMemsetAsync(in.dash_cnt, 0, size_t(N) * 4, st));
+        in.n_sms = c->n_sms;
+        in.n_dashed = c->ustats.dashed_paths;
+        if (in.n_dashed >= kDashLanes) {
+            PF_CUDA(c->dash_steps.ensure(N));
+            in.dash_steps = c->dash_steps.as<int8_t>();
+            in.dash_split = status + kStDashSplit;
+        }
         PF_CUDA(launch_stroke_order(in, 1, c->st_order_ctl.as<uint32_t>(), c->dash_order.as<uint32_t>(), st));
         in.dash_order = c->dash_order.as<uint32_t>();
-        in.n_dashed = c->ustats.dashed_paths;
         // the chunk pool: a chunk to begin each path, and 16 points for each input point or what the
         // largest upload so far took; at most 2^26 points (0.6 GB)
         const uint64_t chunk_points = std::max<uint64_t>(c->dash_points_hint, uint64_t(c->n_points) * 16);
@@ -552,12 +558,6 @@ int stroke_upload(Ctx *c, const pf_scene_view *scenes, uint32_t n, const std::ve
         in.dash_chunk_count = status + kStDashChunks;
         in.dash_chunk_cap = (uint32_t)chunk_cap;
         PF_CUDA(cudaMemsetAsync(pool, 0xff, chunk_cap * 16, st));  // no path
-        in.n_sms = c->n_sms;
-        if (in.n_dashed >= kDashLanes) {
-            PF_CUDA(c->dash_list.ensure(size_t(in.n_dashed) * 4));
-            in.dash_list = c->dash_list.as<uint32_t>();
-            PF_CUDA(launch_dash_lanes(in, false, status, st));
-        }
         PF_CUDA(launch_dash(in, false, status, st));
         PF_CUDA(scan_exclusive_u32(in.dash_pts, in.dash_pts, N, in.dash_pts + N, c->scan_temp.p, st, status));
         PF_CUDA(scan_exclusive_u32(in.dash_cnt, in.dash_cnt, N, in.dash_cnt + N, c->scan_temp.p, st, status));
@@ -583,9 +583,12 @@ int stroke_upload(Ctx *c, const pf_scene_view *scenes, uint32_t n, const std::ve
         const uint64_t chunks = uint64_t(in.n_dashed) + w[3];
         in.n_dash_chunks = (uint32_t)chunks;
         c->dash_points_hint = std::max(c->dash_points_hint, uint64_t(w[3]) * kDashChunk);
-        if (in.dash_list) PF_CUDA(launch_dash_lanes(in, true, status, st));
-        if (chunks <= in.dash_chunk_cap) PF_CUDA(launch_dash_gather(in, st));
-        else PF_CUDA(launch_dash(in, true, status, st));
+        if (chunks <= in.dash_chunk_cap) {
+            PF_CUDA(launch_dash_lanes_write(in, status, st));
+            PF_CUDA(launch_dash_gather(in, st));
+        } else {
+            PF_CUDA(launch_dash(in, true, status, st));
+        }
         PF_CUDA(mark(3));
     }
     // one job per output contour
@@ -2098,7 +2101,7 @@ int pf_ctx_destroy(void *ctx) {
                       &c->job_units, &c->job_nfwd, &c->job_flags, &c->job_cap1, &c->job_end, &c->units,
                       &c->unit_leaves, &c->st_leaves, &c->leaf_pts, &c->path_grad, &c->grad_paint, &c->image_snap,
                       &c->grad_stop_range, &c->grad_stops, &c->grad_meta, &c->grad_ramp, &c->st_order_ctl,
-                      &c->unit_order, &c->dash_order, &c->dash_list};
+                      &c->unit_order, &c->dash_order, &c->dash_steps};
     for (DevBuf *b : bufs) b->release();
     for (auto &e : c->ev)
         if (e) cudaEventDestroy(e);

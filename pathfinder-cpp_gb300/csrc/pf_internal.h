@@ -223,7 +223,7 @@ enum : int {
     kStSampledDeep = 23,
     kStDashChunks = 24,// upload: chunks of dashed points taken
     kStRectClass = 25, // six words: nonzero if a path's rect asks for that binning class
-    kStDashLong = 31,  // upload: dashed paths left to the warps
+    kStDashSplit = 31, // upload: dashed paths that warps take
     kStCount = 32,
     // the binning's control words follow in the same buffer; the host reads the first of them too
     kStBinCtl = 64,
@@ -317,17 +317,19 @@ struct StrokeIn {
     float4 *leaves;                     // [n_leaves][3] piece, join point, (job, meta)
     uint32_t *leaf_pts;                 // [n_leaves + 1] counts -> scanned
     const uint32_t *unit_order;         // [n_units] units, the most work first (or null)
-    uint32_t *dash_order;               // [n_dashed] the dashed paths, the most work first
-    uint32_t n_dashed;
-    uint32_t *dash_list;                // the paths that a lane each left to the warps (null: warps take all)
-    uint32_t n_sms;
+    const uint32_t *dash_order;         // [n_dashed] the dashed paths, the most work first
+    uint32_t n_dashed, n_sms;
+    // many dashed paths: the first *dash_split are for warps, the rest for lanes (null: warps take all)
+    uint32_t *dash_split;
+    int8_t *dash_steps;                 // [n_paths] log2 of about their steps, -1: not dashed
 };
 size_t stroke_order_ctl_bytes();
 cudaError_t launch_stroke_order(const StrokeIn &in, int what, uint32_t *ctl, uint32_t *order, cudaStream_t st);
 constexpr uint32_t kDashChunk = 64;  // points
 cudaError_t launch_dash(const StrokeIn &in, bool write, uint32_t *status, cudaStream_t st);
-constexpr uint32_t kDashLanes = 16384;  // dashed paths from which on short ones take a lane each: figures there
-cudaError_t launch_dash_lanes(const StrokeIn &in, bool write, uint32_t *status, cudaStream_t st);
+constexpr uint32_t kDashLanes = 16384;  // dashed paths from which on short ones may take a lane each
+// The lanes' paths written, beside launch_dash_gather for the warps'.
+cudaError_t launch_dash_lanes_write(const StrokeIn &in, uint32_t *status, cudaStream_t st);
 cudaError_t launch_dash_gather(const StrokeIn &in, cudaStream_t st);
 cudaError_t launch_copy_words(uint32_t *dst, const uint32_t *src, uint32_t n, cudaStream_t st);
 // up to 8 single words gathered into dst[0, n)

@@ -766,35 +766,16 @@ __device__ __forceinline__ void dash_by_warp(const StrokeIn &in, uint32_t *statu
 }
 
 // The dashed paths, largest first (dash_order); every other path's counts are zeroed before the count
-// pass.  kListed: those that k_dash_lanes has left.
-template <bool kWrite, bool kListed>
+// pass.
+template <bool kWrite>
 __global__ void __launch_bounds__(64) k_dash(StrokeIn in, uint32_t *status) {
-    uint32_t t = blockIdx.x * 2 + (threadIdx.x >> 5);
-    if (!kListed) {
-        if (t < in.n_dashed) dash_by_warp<kWrite>(in, status, t, in.dash_order[t]);
-        return;
-    }
-    const uint32_t n = status[kStDashLong];
-    for (; t < n; t += gridDim.x * 2) {
-        dash_by_warp<kWrite>(in, status, t, in.dash_list[t]);
-        __syncwarp();
-    }
+    const uint32_t t = blockIdx.x * 2 + (threadIdx.x >> 5);
+    if (t < in.n_dashed) dash_by_warp<kWrite>(in, status, t, in.dash_order[t]);
 }
 
-// Many short paths: a lane each.  With some 20,000 paths the chains fill the GPU whoever walks them, and
-// what counts is how many instructions they take together; a warp's 32 lanes on one chain are then 31
-// too many.  A lane counts its path's points and contours, and walks it again to write them; a path of more
-// than kLaneSteps steps is left to the warps (its place in dash_order marked), as its chain would keep 31
-// other lanes waiting.  (Dashing 200,000 lines of 7 points of dashes each: 0.34 ms by warps, 0.12 so; of 32
-// points 0.82 and 0.30; 60,000 lines 0.14 and 0.09; 20,000, 0.086 and 0.080, of 32 points 0.148 and 0.132.)
-constexpr uint32_t kLaneSteps = 64, kLongPath = 1u << 31;
-
+// Path p by a lane, which counts its points and contours, and walks it again to write them.
 template <bool kWrite>
-__global__ void __launch_bounds__(128) k_dash_lanes(StrokeIn in, uint32_t *status) {
-    const uint32_t t = blockIdx.x * blockDim.x + threadIdx.x;
-    if (t >= in.n_dashed) return;
-    const uint32_t p = in.dash_order[t];
-    if (kWrite && (p & kLongPath)) return;
+__device__ __forceinline__ void dash_by_lane(const StrokeIn &in, uint32_t *status, uint32_t p) {
     const pf_stroke &st = path_stroke(in, p);
     if (!stroked(in, p) || st.dash_count == 0) return;
     // DashState::DashState, dash.cpp:9-29
@@ -833,9 +814,8 @@ __global__ void __launch_bounds__(128) k_dash_lanes(StrokeIn in, uint32_t *statu
             if (rest.kind == kNone) break;
             bool more;
             do {
-                if (++steps > kLaneSteps && !kWrite) {
-                    in.dash_order[t] = p | kLongPath;
-                    in.dash_list[atomicAdd(&status[kStDashLong], 1u)] = p;
+                if (++steps > kDashStepLimit) {
+                    atomicOr(&status[kStErr], kErrStroke);
                     return;
                 }
                 float distance = left;
@@ -865,6 +845,23 @@ __global__ void __launch_bounds__(128) k_dash_lanes(StrokeIn in, uint32_t *statu
     if (!kWrite) {
         in.dash_pts[p] = at;
         in.dash_cnt[p] = contours;
+    }
+}
+
+// Many paths: those of more steps (the first *dash_split in dash_order) by a warp each, the rest by lanes,
+// in one launch, so that the short ones fill what the long chains leave idle.  A warp's 32 lanes on one
+// chain take a step in half a lane's time, with some ten times the instructions.  TIMING
+template <bool kWrite>
+__global__ void __launch_bounds__(64) k_dash_split(StrokeIn in, uint32_t warp_blocks, uint32_t *status) {
+    const uint32_t split = *in.dash_split;
+    if (blockIdx.x < warp_blocks) {
+        for (uint32_t t = blockIdx.x * 2 + (threadIdx.x >> 5); t < split; t += warp_blocks * 2) {
+            dash_by_warp<kWrite>(in, status, t, in.dash_order[t]);
+            __syncwarp();
+        }
+    } else {
+        const uint32_t t = split + (blockIdx.x - warp_blocks) * 64 + threadIdx.x;
+        if (t < in.n_dashed) dash_by_lane<kWrite>(in, status, in.dash_order[t]);
     }
 }
 
@@ -1469,7 +1466,59 @@ __device__ __forceinline__ int dash_bucket(const StrokeIn &in, uint32_t p) {
     return d < kOrderBuckets - 1 ? d : kOrderBuckets - 1;
 }
 
-// kWhat 0: units, 1: dashed paths.  ctl[kOrderBuckets * block + bucket].
+// The log2 of about the most steps a dashed path can take: a pattern's entries for every time its length
+// fits into the outline's, and its points.  A path of very many points counts as long unseen.
+__device__ __forceinline__ int dash_steps_bucket(const StrokeIn &in, uint32_t p) {
+    if (!stroked(in, p) || path_stroke(in, p).dash_count == 0) return -1;
+    const pf_stroke &st = path_stroke(in, p);
+    const uint2 kr = path_contours(in, p);
+    if (kr.y - kr.x > 256) return kOrderBuckets - 1;
+    uint32_t pts = 0;
+    float length = 0.0f, total = 0.0f;
+    for (uint32_t k = kr.x; k < kr.y; k++) {
+        const Contour c = raw_contour(in, k);
+        if ((pts += c.n) > 1024) return kOrderBuckets - 1;
+        if (!c.n) continue;
+        V2 a = c.at(c.closed ? c.n - 1 : 0);
+        for (uint32_t i = 0; i < c.n; i++) {
+            const V2 q = c.at(i);
+            length += sqrtf((q.x - a.x) * (q.x - a.x) + (q.y - a.y) * (q.y - a.y));
+            a = q;
+        }
+    }
+    for (uint32_t i = 0; i < st.dash_count; i++) total += in.dashes[st.dash_first + i];
+    const float steps = (floorf(length / total) + 1.0f) * (float)st.dash_count + (float)pts;
+    return steps < 32768.0f ? 31 - __clz(max((uint32_t)steps, 1u)) : kOrderBuckets - 1;
+}
+
+// How many of the paths, longest first, are for warps: all but those of up to 2^b steps, for the b (or
+// none) that takes least time by what each side was measured to take, in ms: a warp 0.35 us a step on its
+// chain and, with many side by side, 0.1 ns a step and 1 ns a path of the whole GPU's time; a lane 0.7 us a
+// step on its chain, in the count pass, which runs beside the warps, and again to write.
+// total: paths by bucket of dash_steps_bucket.
+__device__ __forceinline__ uint32_t dash_border(const uint32_t *total) {
+    uint32_t n = 0, lanes = 0, short_paths = 0;
+    float work = 0.0f, chain = 0.0f;  // of the warps' paths
+    for (int b = 0; b < kOrderBuckets; b++) {
+        n += total[b];
+        work += (1.5f * (float)(1u << b) + 10.0f) * (float)total[b] * 1.0e-7f;
+        if (total[b]) chain = (float)(2u << b) * 0.35e-3f;
+    }
+    float best = fmaxf(work, chain);
+    for (int b = 0; b < kOrderBuckets - 1; b++) {
+        short_paths += total[b];
+        work -= (1.5f * (float)(1u << b) + 10.0f) * (float)total[b] * 1.0e-7f;
+        const float pass = (float)(2u << b) * 0.7e-3f;
+        const float time = fmaxf(pass, short_paths < n ? fmaxf(work, chain) : 0.0f) + pass;
+        if (time < best) {
+            best = time;
+            lanes = short_paths;
+        }
+    }
+    return n - lanes;
+}
+
+// kWhat 0: units, 1: dashed paths by points, 2: dashed paths by steps.  ctl[kOrderBuckets * block + bucket].
 template <int kWhat, bool kScatter>
 __global__ void __launch_bounds__(256) k_order(StrokeIn in, uint32_t *ctl, uint32_t *order) {
     __shared__ uint32_t s_cnt[kOrderBuckets];
@@ -1479,7 +1528,13 @@ __global__ void __launch_bounds__(256) k_order(StrokeIn in, uint32_t *ctl, uint3
     __syncthreads();
     for (uint32_t base = blockIdx.x * blockDim.x; base < n; base += gridDim.x * blockDim.x) {
         const uint32_t i = base + threadIdx.x;
-        const int bk = i < n ? (kWhat == 0 ? unit_bucket(in, i) : dash_bucket(in, i)) : -1;
+        int bk = -1;
+        if (i < n) {
+            if (kWhat == 0) bk = unit_bucket(in, i);
+            else if (kWhat == 1) bk = dash_bucket(in, i);
+            else if (kScatter) bk = in.dash_steps[i];
+            else in.dash_steps[i] = (int8_t)(bk = dash_steps_bucket(in, i));
+        }
         const unsigned group = __match_any_sync(0xffffffffu, bk);
         const int leader = __ffs(group) - 1;
         uint32_t slot = 0;
@@ -1493,8 +1548,8 @@ __global__ void __launch_bounds__(256) k_order(StrokeIn in, uint32_t *ctl, uint3
 
 // Each block's first slot per bucket, largest bucket first; ctl[kOrderBuckets * kOrderBlocks]
 // receives the number of items placed.  A warp per bucket, all its counts in registers (a thread per
-// bucket, one count after the other, took 21 us).
-__global__ void __launch_bounds__(kOrderBuckets * 32) k_order_starts(uint32_t *ctl) {
+// bucket, one count after the other, took 21 us).  split: where dash_border goes, or null.
+__global__ void __launch_bounds__(kOrderBuckets * 32) k_order_starts(uint32_t *ctl, uint32_t *split) {
     constexpr int kRounds = kOrderBlocks / 32;
     static_assert(kOrderBlocks % 32 == 0, "whole warps of blocks");
     __shared__ uint32_t total[kOrderBuckets];
@@ -1522,6 +1577,7 @@ __global__ void __launch_bounds__(kOrderBuckets * 32) k_order_starts(uint32_t *c
         run += __shfl_sync(0xffffffffu, incl[r], 31);
     }
     if (bk == 0 && lane == 0) ctl[kOrderBuckets * kOrderBlocks] = run;
+    if (split && threadIdx.x == 32) *split = dash_border(total);
 }
 
 // The new outline's per-scene offset arrays (the layout the upload uses: scene s's contour
@@ -1562,22 +1618,22 @@ static uint32_t blocks(uint32_t n, uint32_t t) { return (n + t - 1) / t; }
 
 cudaError_t launch_dash(const StrokeIn &in, bool write, uint32_t *status, cudaStream_t st) {
     if (!in.n_dashed) return cudaSuccess;
-    if (!in.dash_list) {
-        if (write) k_dash<true, false><<<blocks(in.n_dashed, 2), 64, 0, st>>>(in, status);
-        else k_dash<false, false><<<blocks(in.n_dashed, 2), 64, 0, st>>>(in, status);
+    if (!in.dash_split) {
+        if (write) k_dash<true><<<blocks(in.n_dashed, 2), 64, 0, st>>>(in, status);
+        else k_dash<false><<<blocks(in.n_dashed, 2), 64, 0, st>>>(in, status);
     } else {
         // as many warps as there could be work for, no more than the SMs hold
-        const uint32_t grid = std::min(blocks(in.n_dashed, 2), 16u * in.n_sms);
-        if (write) k_dash<true, true><<<grid, 64, 0, st>>>(in, status);
-        else k_dash<false, true><<<grid, 64, 0, st>>>(in, status);
+        const uint32_t wb = std::min(blocks(in.n_dashed, 2), 32u * in.n_sms), lb = blocks(in.n_dashed, 64);
+        if (write) k_dash_split<true><<<wb + lb, 64, 0, st>>>(in, wb, status);
+        else k_dash_split<false><<<wb + lb, 64, 0, st>>>(in, wb, status);
     }
     count_launches(1);
     return cudaGetLastError();
 }
 
-cudaError_t launch_dash_lanes(const StrokeIn &in, bool write, uint32_t *status, cudaStream_t st) {
-    if (write) k_dash_lanes<true><<<blocks(in.n_dashed, 128), 128, 0, st>>>(in, status);
-    else k_dash_lanes<false><<<blocks(in.n_dashed, 128), 128, 0, st>>>(in, status);
+cudaError_t launch_dash_lanes_write(const StrokeIn &in, uint32_t *status, cudaStream_t st) {
+    if (!in.n_dashed || !in.dash_split) return cudaSuccess;
+    k_dash_split<true><<<blocks(in.n_dashed, 64), 64, 0, st>>>(in, 0, status);
     count_launches(1);
     return cudaGetLastError();
 }
@@ -1597,13 +1653,17 @@ cudaError_t launch_stroke_order(const StrokeIn &in, int what, uint32_t *ctl, uin
     if (what == 0) {
         if (!in.n_units) return cudaSuccess;
         k_order<0, false><<<kOrderBlocks, 256, 0, st>>>(in, ctl, order);
-        k_order_starts<<<1, kOrderBuckets * 32, 0, st>>>(ctl);
+        k_order_starts<<<1, kOrderBuckets * 32, 0, st>>>(ctl, nullptr);
         k_order<0, true><<<kOrderBlocks, 256, 0, st>>>(in, ctl, order);
-    } else {
+    } else if (!in.dash_split) {
         if (!in.n_paths) return cudaSuccess;
         k_order<1, false><<<kOrderBlocks, 256, 0, st>>>(in, ctl, order);
-        k_order_starts<<<1, kOrderBuckets * 32, 0, st>>>(ctl);
+        k_order_starts<<<1, kOrderBuckets * 32, 0, st>>>(ctl, nullptr);
         k_order<1, true><<<kOrderBlocks, 256, 0, st>>>(in, ctl, order);
+    } else {
+        k_order<2, false><<<kOrderBlocks, 256, 0, st>>>(in, ctl, order);
+        k_order_starts<<<1, kOrderBuckets * 32, 0, st>>>(ctl, in.dash_split);
+        k_order<2, true><<<kOrderBlocks, 256, 0, st>>>(in, ctl, order);
     }
     count_launches(3);
     return cudaGetLastError();
