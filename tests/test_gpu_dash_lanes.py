@@ -1,13 +1,14 @@
 """Many dashed paths, of which the short ones are dashed by a lane each and the rest by warps, against the oracle's
-outline bit for bit: on either side of the number of paths and of the number of steps where that
-changes, with lines and curves, and with a pool of chunks that the long ones overrun at first."""
+outline bit for bit: on either side of the number of paths from which on that is so, with the border
+between them at different numbers of steps, with lines and curves, and with a pool of chunks that the long
+ones overrun at first."""
 import numpy as np
 import pytest
 
 import scenes as S
 from conftest import OUTLINE_KEYS
 
-MANY, STEPS = 16384, 64  # paths from which on lanes dash, steps a lane walks at most
+MANY, STEPS = 16384, 64  # paths from which on lanes dash, and a number of steps
 
 
 def _scene(n, long, lengths, quads):
@@ -40,8 +41,8 @@ def _scene(n, long, lengths, quads):
 @pytest.mark.parametrize("long,lengths", [
     (0, (0.0, 1.0, 12.0, 40.0)),           # every path by a lane
     (40, (3.0, 20.0, 20000.0)),            # chains of thousands of steps among them
-    (5000, (3.0, 1.5 * STEPS, 2.0 * STEPS)),  # about the number of steps itself
-    (MANY - 1, (5.0, 300.0))])             # nearly all by warps, past the first pool
+    (5000, (3.0, 1.5 * STEPS, 2.0 * STEPS)),  # two lengths, near each other
+    (MANY - 1, (5.0, 300.0))])             # nearly all of one length, past the first pool
 @pytest.mark.parametrize("quads", [False, True])
 def test_many_dashed_paths_match_oracle(pf, oracle_mod, n, long, lengths, quads):
     sc = _scene(n, long, lengths, quads)
