@@ -1287,11 +1287,11 @@ int bin_and_composite(Ctx *c, Batch b, bool learned, uint64_t max_leaves) {
     int classes = (has.small != 0) + (has.cluster != 0) + (has.large != 0);
     for (int k = 0; k < 3; k++) classes += (learned ? rects[k] : has.cta[k]) != 0;
     const bool at_once = c->tune.bin_concurrent || classes > 1;
-    size_t slots = 0;
-    PF_CUDA(bin_stage_slots(c->tune, c->n_sms, has, at_once, &slots));
-    PF_CUDA(c->bin_stage.ensure(slots * 12));
+    BinLaunch plan;
+    PF_CUDA(bin_launch(c->tune, c->n_sms, has, at_once, plan));
+    PF_CUDA(c->bin_stage.ensure(plan.slots * 12));
     b.stage = c->bin_stage.as<uint2>();
-    b.stage_tile = reinterpret_cast<uint32_t *>(b.stage + slots);
+    b.stage_tile = reinterpret_cast<uint32_t *>(b.stage + plan.slots);
     for (int attempt = 0;; attempt++) {
         if (attempt > 0) {  // else begin_frame cleared them
             PF_CUDA(cudaMemsetAsync(b.bin_ctl, 0, kBinCtlBytes, st));
@@ -1304,7 +1304,7 @@ int bin_and_composite(Ctx *c, Batch b, bool learned, uint64_t max_leaves) {
             for (auto &e : c->bs.join) PF_CUDA(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
             c->bs_ready = true;
         }
-        PF_CUDA(launch_bin_paths(b, c->tune, has, at_once ? &c->bs : nullptr, st));
+        PF_CUDA(launch_bin_paths(b, plan, has, at_once ? &c->bs : nullptr, st));
         record(c, 3);
         record(c, 4);
         record(c, 5);

@@ -404,14 +404,20 @@ struct BinStreams {
 struct BinClasses {
     uint32_t cta[3], small, cluster, large;
 };
-cudaError_t launch_bin_paths(const Batch &b, const Tuning &t, const BinClasses &has, const BinStreams *bs,
+// The grids of these classes on the current device, and their slices of the stage (12 bytes a slot).
+struct BinLaunch {
+    unsigned cta[3] = {}, small = 0, cluster = 0;
+    size_t first[3] = {};                         // class c's slice
+    size_t first_small = 0, first_cluster = 0, slots = 0;
+    bool cluster_aside = false;                   // the cluster class on a stream of its own
+};
+cudaError_t bin_launch(const Tuning &t, uint32_t n_sms, const BinClasses &has, bool at_once, BinLaunch &l);
+// bs: not null where bin_launch was told at_once.
+cudaError_t launch_bin_paths(const Batch &b, const BinLaunch &l, const BinClasses &has, const BinStreams *bs,
                              cudaStream_t st);
 // The most CTAs of each binning class one SM holds.
 cudaError_t bin_class_max_ctas(int out[3]);
 cudaError_t launch_pool_lists(const Batch &b, bool scatter, cudaStream_t st);
-// Slots of the stage that launch_bin_paths uses with these launch parameters and classes on the current
-// device.
-cudaError_t bin_stage_slots(const Tuning &t, uint32_t n_sms, const BinClasses &has, bool at_once, size_t *slots);
 cudaError_t launch_mlp_predict(const __nv_bfloat16 *w, const float *feat, uint32_t n, float *out, cudaStream_t st);
 cudaError_t launch_mlp_grad(const __nv_bfloat16 *w, const float *feat, const float *target, const uint32_t *index,
                             uint32_t n, float *grad, float *loss, cudaStream_t st);

@@ -3455,14 +3455,7 @@ static cudaError_t cluster_grid(unsigned *grid, uint32_t n_paths) {
 // 1.82; on class 2's stream it held that up (20,000 paths, 0.66 -> 0.72).  (A slice for each of the five
 // classes, whether the frame has it or not: a first frame of 240 paths took 178 MB and 614 us, now 68 MB
 // and 550 us, one of 20,000 paths 4.07 ms, now 2.25; later frames are the same.)
-struct BinLaunch {
-    unsigned cta[3] = {}, small = 0, cluster = 0;
-    size_t first[3] = {};                         // class c's slice
-    size_t first_small = 0, first_cluster = 0, slots = 0;
-    bool cluster_aside = false;                   // the cluster class on a stream of its own
-};
-
-static cudaError_t bin_launch(const Tuning &t, uint32_t n_sms, const BinClasses &has, bool at_once, BinLaunch &l) {
+cudaError_t bin_launch(const Tuning &t, uint32_t n_sms, const BinClasses &has, bool at_once, BinLaunch &l) {
     cudaError_t e = cudaSuccess;
     if (has.cta[0]) e = fused_grid<0>(&l.cta[0], n_sms, has.cta[0], t.bin_ctas_per_sm[0]);
     if (e == cudaSuccess && has.cta[1]) e = fused_grid<1>(&l.cta[1], n_sms, has.cta[1], t.bin_ctas_per_sm[1]);
@@ -3489,13 +3482,6 @@ static cudaError_t bin_launch(const Tuning &t, uint32_t n_sms, const BinClasses 
     return cudaSuccess;
 }
 
-cudaError_t bin_stage_slots(const Tuning &t, uint32_t n_sms, const BinClasses &has, bool at_once, size_t *slots) {
-    BinLaunch l;
-    const cudaError_t e = bin_launch(t, n_sms, has, at_once, l);
-    *slots = l.slots;
-    return e;
-}
-
 cudaError_t bin_class_max_ctas(int out[3]) {
     cudaError_t e = fused_per_sm<0>(&out[0]);
     if (e == cudaSuccess) e = fused_per_sm<1>(&out[1]);
@@ -3506,12 +3492,10 @@ cudaError_t bin_class_max_ctas(int out[3]) {
 // Class 3, the cluster class, the CTA classes, largest rects first, and the small class, those that can
 // have paths; at once (bs not null) on streams of their own, joined before the composite, so that the
 // block scheduler fills the SMs that one class's last paths leave idle with the others'.
-cudaError_t launch_bin_paths(const Batch &b, const Tuning &t, const BinClasses &has, const BinStreams *bs,
+cudaError_t launch_bin_paths(const Batch &b, const BinLaunch &l, const BinClasses &has, const BinStreams *bs,
                              cudaStream_t st) {
     if (!b.n_paths) return cudaSuccess;
-    BinLaunch l;
-    cudaError_t e = bin_launch(t, b.n_sms, has, bs != nullptr, l);
-    if (e != cudaSuccess) return e;
+    cudaError_t e = cudaSuccess;
     const int sides = l.cluster_aside ? 3 : 2;
     if (bs) {
         if ((e = cudaEventRecord(bs->fork, st)) != cudaSuccess) return e;
